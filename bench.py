@@ -300,8 +300,8 @@ def bench_ours(args, rank, world):
     sim.step(args.warmup)
     sim.synchronize()
     active = sim.active_schedule
-    # fused: shell E, sweep, shell H (and the CPML sweep); two-pass: E and H
-    launches_per_step = {2: 3, 3: 4}.get(active, 2)
+    # fused: one sweep per step; two-pass: E and H
+    launches_per_step = {2: 1, 3: 1}.get(active, 2)
     e0 = torch.cuda.Event(enable_timing=True)
     e1 = torch.cuda.Event(enable_timing=True)
     clocks = ClockSampler(torch.cuda.current_device())

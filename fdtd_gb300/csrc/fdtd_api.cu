@@ -11,6 +11,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -102,23 +103,23 @@ struct fdtd_handle {
     PsiSet psi[2] = {};
     int cur = 0;
     bool have_second = false;
-    FusedMaps maps[2];
-    CpmlMaps cmaps[2];  // the CPML sweep's maps per input buffer
+    FusedMaps maps[2];  // the sweep's tensor maps per input buffer
     char* psi_base[2] = {nullptr, nullptr};  // the allocation holding each CPML memory set
-    FusedFork fork{};  // second stream and events of the fused step (created with the fused buffers)
-    struct PlanCache {  // the last fused plan and what it was made for (chunk, schedule, design box)
-        bool valid = false;
-        int key[9] = {};
-        FusedPlan plan;
-    } plan_cache;
-    int kc = 0;  // planes per CTA chunk of the fused sweep
-    FusedWork work{};
-    bool replan = false;  // the design region or the CPML-sweep choice changed since the fused work was planned
+    long long psi_off[6] = {}, psi_stride[6] = {}, psi_total = 0;  // its arrays by face (StepParams::psi_off)
+    float4 *te[3] = {}, *th[3] = {};   // StepParams::te, th
+    BgNode bg_node{};
+    SweepPlan sweep{};  // tiles and chunks of the sweep
     uint8_t* mat = nullptr;
     uint8_t* cls = nullptr;  // node classes, built by ensure_prepared
     uint16_t* rec = nullptr;          // coefficient row per node, built with the classes
     MatCoef* coef_rows = nullptr;     // material rows then interface rows (StepParams::coef)
     int n_iface_rows = 0;
+    int src_row0 = kRecGeneral;       // rows of lumped source edges (StepParams::src_row0)
+    SrcRow* src_rows = nullptr;
+    ProbeAt* d_probes_at = nullptr;   // probes outside the CPML slabs
+    int n_probes_at = 0;
+    int edge_mat = 0;                 // SweepStep::mat (read back by ensure_prepared)
+    int4* d_special = nullptr;        // special_nodes, while and after their rows are built
     // interface-key hash set and its lists (launch_iface_set / launch_iface_rows)
     unsigned long long* iface_table = nullptr;
     unsigned long long* iface_keys = nullptr;
@@ -149,6 +150,7 @@ struct fdtd_handle {
     LumpedEdge* d_lumped = nullptr;
     int* d_lumped_k = nullptr;
     std::vector<PlateDef> plates;
+    std::vector<long long> plate_list;  // nodes with a plate-covered edge, (k * ny + j) * nx + i, sorted
     PlateEdges* d_plates = nullptr;
     int* d_plate_k = nullptr;
     int4* d_plate_nodes = nullptr;
@@ -204,13 +206,6 @@ struct fdtd_handle {
         cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};  // recompute[2], reverse[2], start / end
         long long key[8] = {};         // steps, interval and design box the buffers were sized for
     } adj;
-
-    // work list of fdtd_step_static_scratch (interior items first) in pinned host memory, planned
-    // on first use; each call uploads it into the scratch with one asynchronous copy
-    int4* static_items = nullptr;
-    size_t static_n_items = 0;
-    int static_counts[6] = {};     // items per list (interior, the four shell lists, CPML items)
-    bool static_planned = false;
 
     std::vector<size_t> alloc_sizes;  // bytes of each entry of allocs
 
@@ -286,6 +281,14 @@ StepParams make_params(fdtd_handle* h) {
             p.bg.e[a][s] = h->bg_curl[4 * a + s];
             p.bg.h[a][s] = h->bg_curl[4 * a + 2 + s];
         }
+    p.bgn = h->bg_node;
+    p.src_row0 = h->src_row0;
+    p.src_rows = h->src_rows;
+    std::copy(h->te, h->te + 3, p.te);
+    std::copy(h->th, h->th + 3, p.th);
+    std::copy(h->psi_off, h->psi_off + 6, p.psi_off);
+    std::copy(h->psi_stride, h->psi_stride + 6, p.psi_stride);
+    p.psi_total = h->psi_total;
     return p;
 }
 
@@ -319,13 +322,17 @@ int alloc_psi_set(fdtd_handle* h, int s) {
         bytes[f] = ((size_t)h->psi_elems[f] * sizeof(float) + 255) / 256 * 256;
         off[f] = total;
         total += 4 * bytes[f];
+        h->psi_off[f] = (long long)(off[f] / sizeof(float));
+        h->psi_stride[f] = (long long)(bytes[f] / sizeof(float));
     }
+    h->psi_total = (long long)(total / sizeof(float));
     h->psi[s] = PsiSet{};
     h->psi_base[s] = nullptr;
     if (total == 0) return FDTD_OK;
     char* base = nullptr;
     if (h->alloc((void**)&base, total) != cudaSuccess) return fail(FDTD_ERR_OOM, "CPML memory allocation failed");
     h->psi_base[s] = base;
+    h->psi[s].base = (float*)base;
     if (launch_fill((float*)base, (long long)(total / sizeof(float)), kTiny, nullptr) != cudaSuccess)
         return fail(FDTD_ERR_CUDA, "fill failed");
     for (int f = 0; f < 6; ++f) {
@@ -355,105 +362,65 @@ void* tensor_map_encoder() {
     return fn;
 }
 
-PlanGrid plan_grid(const DeviceGrid& g) {
-    return PlanGrid{g.nx, g.ny, g.nz, g.pxn, g.pxp, g.pyn, g.pyp, g.pzn, g.pzp};
-}
+// AUTO: the fused schedule (one sweep per step) or two passes, by the grid's cells. Measured on GB300,
+// two-pass against sweep per step, vacuum and random boxes: 40^3 13.8 / 8.6 and 15.2 / 10.5 us, 64^3
+// 19.0 / 11.9 and 19.1 / 15.4, 96^3 29.0 / 19.9 and 29.1 / 23.9, 112^3 39.7 / 37.4 and 40.0 / 38.8,
+// 128^3 50.0 / 50.3 and 51.3 / 51.6, 144^3 90.5 / 71.7 and 90.9 / 76.7, 200^3 226 / 139 and 227 / 144.
+// Between about 1 and 2.6 Mi cells, where the fields still sit in L2 and the sweep's CTAs fill the
+// device once, the two are level, and two-pass needs no second buffers; nor do grids below
+// kAutoSweepCells, a few CTAs' work. Grids with a design region take the sweep from kAutoDesignCells
+// on (smaller ones record in their two-pass kernels). Two-pass also serves where the second buffers
+// cannot be allocated.
+constexpr long long kAutoSweepCells = 32LL << 10;
+constexpr long long kAutoLevelLo = 1000LL << 10, kAutoLevelHi = 2600LL << 10;
+constexpr long long kAutoDesignCells = 64LL << 20;
 
-// The lists of a plan one after the other (interior, the shell lists, the CPML items) and their
-// counts.
-constexpr int kWorkLists = 2 + kPlanShellLists;
-static_assert(kWorkLists == 6, "fdtd_handle::static_counts holds one count per work list");
-std::vector<PlanItem> flatten(const FusedPlan& plan, int counts[kWorkLists]) {
-    std::vector<PlanItem> all;
-    const std::vector<PlanItem>* lists[kWorkLists] = {&plan.interior, &plan.shell[0], &plan.shell[1], &plan.shell[2],
-                                                      &plan.shell[3], &plan.cpml};
-    for (int q = 0; q < kWorkLists; ++q) {
-        counts[q] = (int)lists[q]->size();
-        all.insert(all.end(), lists[q]->begin(), lists[q]->end());
+// The background material's coefficients (StepParams::bgn), evaluated on the host with the rounding steps of
+// k_material_tables (coef3, harm2; IEEE float operations and fma on both sides).
+BgNode make_bg_node(const DeviceGrid& g, const fdtd_material_axes& m) {
+    struct C { float a, bp, bm; };
+    auto coef = [&](float rel, float cond, float c0, float dp, float dm) {
+        const float two_r = 2.0f * rel, dts = g.dt * cond;
+        const float num = std::fmaf(two_r, c0, -dts), den = std::fmaf(two_r, c0, dts);
+        return C{num / den, (2.0f * g.dt) / (den * dp), (-2.0f * g.dt) / (den * dm)};
+    };
+    auto harm = [](float a, float b) { return ((2.0f * a) * b) / (a + b); };
+    const float dpe[3] = {g.dy, g.dz, g.dx}, dme[3] = {g.dz, g.dx, g.dy};
+    const float dph[3] = {g.dz, g.dx, g.dy}, dmh[3] = {g.dy, g.dz, g.dx};
+    C e[3], hh[3];
+    BgNode b{};
+    b.low_ok = 1;
+    for (int q = 0; q < 3; ++q) {
+        e[q] = coef(avg4(m.eps_r[q], m.eps_r[q], m.eps_r[q], m.eps_r[q]),
+                    avg4(m.sigma_e[q], m.sigma_e[q], m.sigma_e[q], m.sigma_e[q]), g.eps0, dpe[q], dme[q]);
+        hh[q] = coef(harm(m.mu_r[q], m.mu_r[q]), harm(m.sigma_m[q], m.sigma_m[q]), g.mu0, dph[q], dmh[q]);
+        const C d = coef(1.0f, kTiny, g.mu0, dph[q], dmh[q]);
+        if (std::memcmp(&d, &hh[q], sizeof(C)) != 0) b.low_ok = 0;
+        b.ea[q] = e[q].a;
+        b.ha[q] = hh[q].a;
+        b.ec[2 * q] = e[q].bp; b.ec[2 * q + 1] = e[q].bm;
+        b.hc[2 * q] = hh[q].bp; b.hc[2 * q + 1] = hh[q].bm;
     }
-    return all;
+    const float ce[6] = {e[1].bm * g.dx, e[2].bp * g.dx, e[0].bp * g.dy, e[2].bm * g.dy, e[0].bm * g.dz, e[1].bp * g.dz};
+    const float ch[6] = {hh[1].bp * g.dx, hh[2].bm * g.dx, hh[0].bm * g.dy, hh[2].bp * g.dy, hh[0].bp * g.dz, hh[1].bm * g.dz};
+    std::copy(ce, ce + 6, b.ce);
+    std::copy(ch, ch + 6, b.ch);
+    return b;
 }
 
-// The work lists over a device copy of the flattened plan.
-FusedWork work_of(const int4* d, const int counts[kWorkLists]) {
-    static_assert(kShellLists == kPlanShellLists && kShellZ == kPlanShellZ && kShellYZ == kPlanShellYZ &&
-                      kShellX == kPlanShellX && kShellAny == kPlanShellAny,
-                  "planner and shell kernels agree on the shell lists");
-    FusedWork w{};
-    w.interior = d;
-    w.n_interior = counts[0];
-    const int4* at = d + counts[0];
-    for (int q = 0; q < kShellLists; ++q) {
-        w.shell.items[q] = at;
-        w.shell.n[q] = counts[1 + q];
-        at += counts[1 + q];
-    }
-    w.cpml = at;
-    w.n_cpml = counts[1 + kShellLists];
-    return w;
-}
-
-// The AUTO trial: on grids of at least kAutoTrialCells cells, the first fdtd_step call of at least
-// 2 * kAutoTrialSteps steps times kAutoTrialSteps fused steps and then as many two-pass steps (real
-// steps: both schedules give the same bits) and keeps the faster schedule for the handle. Which one
-// wins depends on the grid: on GB300 random-box cubes with 10-cell CPML, two-pass below about
-// 224^3 and fused above. Smaller grids take two-pass without a trial. Grids of at least
-// kAutoDirectCells cells whose interior tiles hold at least kAutoDirectInterior of the nodes
-// (512^3 with 10-cell CPML: 0.86) take fused without a trial: there fused won by 16-30 % on every
-// grid measured, and the trial's two-pass steps and synchronisation cost more than a step. The
-// fused buffers are freed when two-pass wins or cannot be allocated.
-constexpr int64_t kAutoTrialSteps = 4;
-constexpr long long kAutoTrialCells = 8LL << 20;
-constexpr long long kAutoDirectCells = 64LL << 20;
-constexpr double kAutoDirectInterior = 0.8;
-
-// The fused plan for the handle's current design box and schedule, from the cache when it holds
-// that plan (planning a 512^3 grid takes a few hundred microseconds on the host).
-const FusedPlan& plan_current(fdtd_handle* h) {
-    const PlanGrid pg = plan_grid(h->g);
-    const int kc = h->kc > 0 ? h->kc : plan_chunk(pg);
-    const bool cpml = h->schedule == FDTD_SCHEDULE_FUSED_CPML;
-    int key[9] = {kc, cpml, h->has_design, 0, 0, 0, 0, 0, 0};
-    if (h->has_design) std::copy(h->dbox, h->dbox + 6, key + 3);
-    auto& C = h->plan_cache;
-    if (!(C.valid && std::equal(key, key + 9, C.key))) {
-        C.plan = FusedPlan{};
-        plan_fused(pg, kc, h->has_design ? h->dbox : nullptr, C.plan, cpml);
-        std::copy(key, key + 9, C.key);
-        C.valid = true;
-    }
-    return C.plan;
-}
-
-// Work items of the fused schedule (planner.cpp), with CPML items under FDTD_SCHEDULE_FUSED_CPML.
-// The design region, if any, stays with the shell; planned again when it or the schedule changes.
-int plan_work(fdtd_handle* h) {
-    const FusedPlan& plan = plan_current(h);
-    int counts[kWorkLists];
-    const std::vector<PlanItem> all = flatten(plan, counts);
-    h->release((void*)h->work.interior);
-    h->work = FusedWork{};
-    int4* d = nullptr;
-    CUDA_TRY(h->alloc((void**)&d, sizeof(int4) * (all.size() + 1)));
-    if (!all.empty()) CUDA_TRY(cudaMemcpy(d, all.data(), sizeof(int4) * all.size(), cudaMemcpyHostToDevice));
-    h->work = work_of(d, counts);
-    h->replan = false;
-    return FDTD_OK;
-}
-
-// Second field buffer, second CPML set and the TMA tensor maps of both buffers for the fused sweep.
+// Second field buffer, second CPML set and the TMA tensor maps of both buffers for the sweep.
 int ensure_fused(fdtd_handle* h) {
-    if (h->have_second && h->replan) return plan_work(h);
     if (h->have_second) return FDTD_OK;
-    // no copy of the state and no fill: a fused step writes every node of its target buffer (the
-    // planner's items cover each node once; plate and design nodes by their own kernels); only
-    // the row padding, which no kernel writes, gets buffer 0's initial value so that saved
-    // states agree
+    // no copy of the state and no fill: a fused step writes every node of its target buffer; only
+    // the row padding, which no kernel writes, gets buffer 0's initial value so that saved states
+    // agree
     const long long V = vol(h);
-    for (int c = 0; c < 6; ++c) {
-        CUDA_TRY(h->alloc((void**)&h->field[1][c], (size_t)V * sizeof(float)));
-        CUDA_TRY(launch_fill_padding(h->field[1][c], h->g, kTiny, h->stream));
-    }
+    float* base = nullptr;  // the six fields in one allocation (separate ones cost tens of microseconds each)
+    CUDA_TRY(h->alloc((void**)&base, 6 * (size_t)V * sizeof(float)));
+    for (int c = 0; c < 6; ++c) h->field[1][c] = base + c * V;
+    DeviceGrid all = h->g;
+    all.nz *= 6;
+    CUDA_TRY(launch_fill_padding(base, all, kTiny, h->stream));
     int rc = alloc_psi_set(h, 1);
     if (rc) return rc;
     void* enc = tensor_map_encoder();
@@ -461,27 +428,16 @@ int ensure_fused(fdtd_handle* h) {
     for (int b = 0; b < 2; ++b) {
         float* hh[3] = {h->field[b][3], h->field[b][4], h->field[b][5]};
         float* ee[3] = {h->field[b][0], h->field[b][1], h->field[b][2]};
-        if (encode_fused_maps(&h->maps[b], h->g, hh, ee, h->rec, enc) != 0 ||
-            encode_cpml_maps(&h->cmaps[b], h->g, hh, ee, h->rec, h->psi[b], enc) != 0)
+        if (encode_sweep_maps(&h->maps[b], h->g, hh, ee, h->rec, enc) != 0)
             return fail(FDTD_ERR_CUDA, "tensor map encoding failed");
     }
-    CUDA_TRY(fused_configure());
-    if (!h->fork.aux) {  // the sweep's stream: as high a priority as the handle's
-        int prio = 0;
-        CUDA_TRY(cudaStreamGetPriority(h->stream, &prio));
-        CUDA_TRY(cudaStreamCreateWithPriority(&h->fork.aux, cudaStreamNonBlocking, prio));
-        CUDA_TRY(cudaEventCreateWithFlags(&h->fork.fork, cudaEventDisableTiming));
-        CUDA_TRY(cudaEventCreateWithFlags(&h->fork.join, cudaEventDisableTiming));
-    }
-    h->kc = plan_chunk(plan_grid(h->g));
-    rc = plan_work(h);
-    if (rc) return rc;
+    CUDA_TRY(sweep_configure());
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     h->have_second = true;
     return FDTD_OK;
 }
 
-// AUTO runs two-pass until a trial on the handle's own grid has chosen (auto_trial).
+// AUTO runs two-pass until auto_choose has taken the fused schedule.
 bool use_fused(const fdtd_handle* h) {
     return h->schedule == FDTD_SCHEDULE_FUSED || h->schedule == FDTD_SCHEDULE_FUSED_CPML ||
            (h->schedule == FDTD_SCHEDULE_AUTO && h->auto_choice == FDTD_SCHEDULE_FUSED);
@@ -489,16 +445,37 @@ bool use_fused(const fdtd_handle* h) {
 
 // Frees what ensure_fused allocated; the state must be in buffer 0.
 void release_fused(fdtd_handle* h) {
-    for (int c = 0; c < 6; ++c) {
-        h->release(h->field[1][c]);
-        h->field[1][c] = nullptr;
-    }
+    h->release(h->field[1][0]);  // the allocation holds all six
+    for (int c = 0; c < 6; ++c) h->field[1][c] = nullptr;
     h->release(h->psi_base[1]);
     h->psi_base[1] = nullptr;
     h->psi[1] = PsiSet{};
-    h->release((void*)h->work.interior);
-    h->work = FusedWork{};
     h->have_second = false;
+}
+
+// AUTO's choice, made by the first step or by fdtd_tune_schedule. The second buffers are allocated
+// here, not under stream capture: a handle first stepped there takes two-pass until later.
+void auto_choose(fdtd_handle* h) {
+    if (h->schedule != FDTD_SCHEDULE_AUTO || h->auto_choice != FDTD_SCHEDULE_AUTO) return;
+    const long long cells = (long long)h->g.nx * h->g.ny * h->g.nz;
+    if (cells < (h->has_design ? kAutoDesignCells : kAutoSweepCells) || (cells >= kAutoLevelLo && cells < kAutoLevelHi)) {
+        h->auto_choice = FDTD_SCHEDULE_TWO_PASS;
+        return;
+    }
+    if (!h->have_second) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();
+            return;
+        }
+    }
+    if (ensure_fused(h) == FDTD_OK) {
+        h->auto_choice = FDTD_SCHEDULE_FUSED;
+    } else {  // no room for the second buffers
+        cudaGetLastError();
+        if (h->cur == 0) release_fused(h);
+        h->auto_choice = FDTD_SCHEDULE_TWO_PASS;
+    }
 }
 
 }  // namespace
@@ -551,6 +528,16 @@ int fdtd_create(const fdtd_grid* grid, fdtd_handle** out) {
         for (int q = 0; q < 4; ++q)
             if (h->alloc((void**)&h->bg_curl[4 * a + q], sizeof(float) * ns[a]) != cudaSuccess)
                 return cleanup(fail(FDTD_ERR_OOM, "profile allocation failed"));
+    {   // the packed tables, in one allocation
+        float4* t = nullptr;
+        if (h->alloc((void**)&t, sizeof(float4) * 2 * (size_t)(ns[0] + ns[1] + ns[2])) != cudaSuccess)
+            return cleanup(fail(FDTD_ERR_OOM, "profile allocation failed"));
+        for (int a = 0; a < 3; ++a) {
+            h->te[a] = t;
+            h->th[a] = t + ns[a];
+            t += 2 * ns[a];
+        }
+    }
     if (h->alloc((void**)&h->d_kappa_ptrs, sizeof(float*) * 6) != cudaSuccess ||
         h->alloc((void**)&h->d_bg_ptrs, sizeof(float*) * 12) != cudaSuccess)
         return cleanup(fail(FDTD_ERR_OOM, "table allocation failed"));
@@ -587,9 +574,7 @@ int fdtd_create(const fdtd_grid* grid, fdtd_handle** out) {
     if (cudaMemset(h->mat, 0, (size_t)V) != cudaSuccess || cudaMemset(h->status, 0, sizeof(int)) != cudaSuccess)
         return cleanup(fail(FDTD_ERR_CUDA, "memset failed"));
     h->materials.push_back(axes_of(fdtd_material{1.0f, kTiny, 1.0f, kTiny}));
-    // grids large enough for AUTO to weigh the fused schedule: plan its work on the host while the
-    // fills run (the plan is cached for the first step)
-    if ((long long)g.nx * g.ny * g.nz >= kAutoTrialCells) plan_current(h);
+    h->sweep = plan_sweep(PlanGrid{g.nx, g.ny, g.nz, g.pxn, g.pxp, g.pyn, g.pyp, g.pzn, g.pzp});
     cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return cleanup(fail(FDTD_ERR_CUDA, std::string("init: ") + cudaGetErrorString(e)));
     *out = h;
@@ -603,7 +588,6 @@ int fdtd_destroy(fdtd_handle* h) {
     for (void* p : h->allocs) cudaFree(p);
     h->allocs.clear();
     h->alloc_sizes.clear();
-    if (h->static_items) cudaFreeHost(h->static_items);
     if (h->adj.pinned_samples) cudaFreeHost(h->adj.pinned_samples);
     if (h->adj.pinned_grad) cudaFreeHost(h->adj.pinned_grad);
     if (h->adj.rev) {
@@ -611,12 +595,6 @@ int fdtd_destroy(fdtd_handle* h) {
         for (cudaEvent_t e : h->adj.ev)
             if (e) cudaEventDestroy(e);
         cudaStreamDestroy(h->adj.rev);
-    }
-    if (h->fork.aux) {
-        cudaStreamSynchronize(h->fork.aux);
-        cudaEventDestroy(h->fork.fork);
-        cudaEventDestroy(h->fork.join);
-        cudaStreamDestroy(h->fork.aux);
     }
     delete h;
     return FDTD_OK;
@@ -632,7 +610,6 @@ int fdtd_set_schedule(fdtd_handle* h, int32_t schedule) {
     if (!h) return fail(FDTD_ERR_INVALID, "handle is NULL");
     if (schedule < FDTD_SCHEDULE_AUTO || schedule > FDTD_SCHEDULE_FUSED_CPML)
         return fail(FDTD_ERR_INVALID, "unknown schedule");
-    if ((schedule == FDTD_SCHEDULE_FUSED_CPML) != (h->schedule == FDTD_SCHEDULE_FUSED_CPML)) h->replan = true;
     h->schedule = schedule;
     h->auto_choice = FDTD_SCHEDULE_AUTO;  // AUTO runs its trial again
     return FDTD_OK;
@@ -882,18 +859,29 @@ int fdtd_prepare(fdtd_handle* h) {
 
 namespace {
 
+// What the sweep of the handle's next step takes besides its fields; late: the step before it is
+// one of the same call, whose probes are still to be sampled.
+SweepStep sweep_step(const fdtd_handle* h, bool late) {
+    SweepStep s{h->d_probes_at, h->n_probes_at, late, h->edge_mat || !h->plates.empty(), {}};
+    for (size_t w = 0; w < h->waves.size() && w < (size_t)kSweepSources; ++w)
+        s.sig[w] = h->step < (long long)h->waves[w].size() ? h->waves[w][(size_t)h->step] : 0.f;
+    return s;
+}
+
 int steps_fused(fdtd_handle* h, const StepParams& p, int64_t n) {
     int rc = ensure_fused(h);
     if (rc) return rc;
+    auto fields = [&](int b) {
+        return FieldPtrs{h->field[b][0], h->field[b][1], h->field[b][2], h->field[b][3], h->field[b][4], h->field[b][5]};
+    };
     for (int64_t s = 0; s < n; ++s) {
         const int a = h->cur, b = 1 - h->cur;
-        FieldPtrs fi{h->field[a][0], h->field[a][1], h->field[a][2], h->field[a][3], h->field[a][4], h->field[a][5]};
-        FieldPtrs fo{h->field[b][0], h->field[b][1], h->field[b][2], h->field[b][3], h->field[b][4], h->field[b][5]};
-        CUDA_TRY(launch_fused(h->maps[a], p, fi, fo, h->psi[a], h->psi[b], h->step, h->work, h->stream,
-                              h->fork.aux ? &h->fork : nullptr, &h->cmaps[a]));
+        CUDA_TRY(launch_sweep(h->maps[a], p, fields(a), fields(b), h->psi[a], h->psi[b], h->sweep, sweep_step(h, s > 0), h->step,
+                              h->stream));
         h->cur = b;
         ++h->step;
     }
+    if (n > 0) CUDA_TRY(launch_sample_probes(p, fields(h->cur), h->d_probes_at, h->n_probes_at, h->step - 1, h->stream));
     return FDTD_OK;
 }
 
@@ -907,60 +895,6 @@ int steps_two_pass(fdtd_handle* h, const StepParams& p, int64_t n) {
     return FDTD_OK;
 }
 
-// Share of the grid's nodes that the interior sweep's tiles hold (overlapping tiles counted once
-// per tile, a slight overestimate).
-double interior_share(fdtd_handle* h) {
-    const FusedPlan& plan = plan_current(h);
-    long long n = 0;
-    for (const PlanItem& it : plan.interior) n += (long long)(it.w - it.z) * kTileX * kTileY;
-    return (double)n / ((double)h->g.nx * h->g.ny * h->g.nz);
-}
-
-// AUTO's choice without a trial where it is clear (see above); false: run the trial.
-bool auto_direct(fdtd_handle* h) {
-    if ((long long)h->g.nx * h->g.ny * h->g.nz < kAutoDirectCells || interior_share(h) < kAutoDirectInterior) return false;
-    if (ensure_fused(h) != FDTD_OK) {  // no room for the second buffers
-        cudaGetLastError();
-        if (h->cur == 0) release_fused(h);
-        h->auto_choice = FDTD_SCHEDULE_TWO_PASS;
-        return true;
-    }
-    h->auto_choice = FDTD_SCHEDULE_FUSED;
-    return true;
-}
-
-int auto_trial(fdtd_handle* h, const StepParams& p) {
-    if (ensure_fused(h) != FDTD_OK) {  // no room for the second buffers
-        cudaGetLastError();
-        if (h->cur == 0) release_fused(h);
-        h->auto_choice = FDTD_SCHEDULE_TWO_PASS;
-        return FDTD_OK;
-    }
-    cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
-    struct Guard {
-        cudaEvent_t* e;
-        ~Guard() {
-            for (int q = 0; q < 3; ++q)
-                if (e[q]) cudaEventDestroy(e[q]);
-        }
-    } guard{ev};
-    for (cudaEvent_t& e : ev) CUDA_TRY(cudaEventCreate(&e));
-    CUDA_TRY(cudaEventRecord(ev[0], h->stream));
-    int rc = steps_fused(h, p, kAutoTrialSteps);  // an even count
-    if (rc) return rc;
-    CUDA_TRY(cudaEventRecord(ev[1], h->stream));
-    if ((rc = steps_two_pass(h, p, kAutoTrialSteps))) return rc;
-    CUDA_TRY(cudaEventRecord(ev[2], h->stream));
-    CUDA_TRY(cudaEventSynchronize(ev[2]));
-    float t_fused = 0.f, t_two = 0.f;
-    CUDA_TRY(cudaEventElapsedTime(&t_fused, ev[0], ev[1]));
-    CUDA_TRY(cudaEventElapsedTime(&t_two, ev[1], ev[2]));
-    h->auto_choice = t_fused < t_two ? FDTD_SCHEDULE_FUSED : FDTD_SCHEDULE_TWO_PASS;
-    // the fused steps came in pairs, so the state is back in the buffer it started in
-    if (h->auto_choice == FDTD_SCHEDULE_TWO_PASS && h->cur == 0) release_fused(h);
-    return FDTD_OK;
-}
-
 }  // namespace
 
 int fdtd_step(fdtd_handle* h, int64_t n) {
@@ -969,11 +903,7 @@ int fdtd_step(fdtd_handle* h, int64_t n) {
     int rc = ensure_prepared(h);
     if (rc) return rc;
     StepParams p = make_params(h);
-    if (h->schedule == FDTD_SCHEDULE_AUTO && h->auto_choice == FDTD_SCHEDULE_AUTO && n >= 2 * kAutoTrialSteps &&
-        (long long)h->g.nx * h->g.ny * h->g.nz >= kAutoTrialCells && !auto_direct(h)) {
-        if ((rc = auto_trial(h, p))) return rc;
-        n -= 2 * kAutoTrialSteps;
-    }
+    auto_choose(h);
     return use_fused(h) ? steps_fused(h, p, n) : steps_two_pass(h, p, n);
 }
 
@@ -1141,32 +1071,7 @@ int fdtd_tune_schedule(fdtd_handle* h) {
     if (!h) return fail(FDTD_ERR_INVALID, "handle is NULL");
     int rc = ensure_prepared(h);
     if (rc) return rc;
-    if (h->schedule != FDTD_SCHEDULE_AUTO || h->auto_choice != FDTD_SCHEDULE_AUTO) return FDTD_OK;
-    if ((long long)h->g.nx * h->g.ny * h->g.nz < kAutoTrialCells) {
-        h->auto_choice = FDTD_SCHEDULE_TWO_PASS;
-        return FDTD_OK;
-    }
-    if (auto_direct(h)) return FDTD_OK;
-    // the trial's steps are undone: state and probe ring saved before, restored after
-    const size_t ring = sizeof(float) * (size_t)h->ring_cap * std::max<size_t>(h->probes.size(), 1);
-    void* saved = nullptr;
-    if (cudaMalloc(&saved, (size_t)fdtd_state_bytes(h) + ring) != cudaSuccess) {
-        cudaGetLastError();
-        return FDTD_OK;  // no room: the first long fdtd_step call runs the trial instead
-    }
-    struct Free {
-        void* p;
-        ~Free() { cudaFree(p); }
-    } guard{saved};
-    char* ring_copy = (char*)saved + fdtd_state_bytes(h);
-    if ((rc = state_copy(h, saved, true))) return rc;
-    CUDA_TRY(cudaMemcpyAsync(ring_copy, h->ring, ring, cudaMemcpyDeviceToDevice, h->stream));
-    const long long step = h->step;
-    if ((rc = auto_trial(h, make_params(h)))) return rc;
-    if ((rc = state_copy(h, saved, false))) return rc;
-    CUDA_TRY(cudaMemcpyAsync(h->ring, ring_copy, ring, cudaMemcpyDeviceToDevice, h->stream));
-    h->step = step;
-    CUDA_TRY(cudaStreamSynchronize(h->stream));
+    auto_choose(h);
     return FDTD_OK;
 }
 
@@ -1301,6 +1206,7 @@ int build_plates(fdtd_handle* h) {
     h->release(h->d_plates); h->release(h->d_plate_k); h->release(h->d_plate_nodes);
     h->d_plates = nullptr; h->d_plate_k = nullptr; h->d_plate_nodes = nullptr;
     h->n_plate_nodes = 0;
+    h->plate_list.clear();
     if (h->plates.empty()) return FDTD_OK;
     const DeviceGrid& g = h->g;
     std::vector<std::vector<PlateEdges>> per_k(g.nz);
@@ -1347,7 +1253,34 @@ int build_plates(fdtd_handle* h) {
     CUDA_TRY(cudaMemcpy(h->d_plate_k, koff.data(), sizeof(int) * (g.nz + 1), cudaMemcpyHostToDevice));
     if (!list.empty()) CUDA_TRY(cudaMemcpy(h->d_plate_nodes, list.data(), sizeof(int4) * list.size(), cudaMemcpyHostToDevice));
     h->n_plate_nodes = (int)list.size();
+    h->plate_list = std::move(nodes);
     return FDTD_OK;
+}
+
+// The nodes whose coefficients no seven-cell key describes but a row can: those with a plate-covered
+// edge (none of them a lumped edge), and those with a lumped edge outside the CPML slabs, with the
+// source that drives their Ez edge (-1: none; sources past kSweepSources stay on the general path).
+// {i, j, k, source}.
+constexpr size_t kSpecialEach = 256;
+size_t special_nodes(const fdtd_handle* h, std::vector<int4>& out) {
+    const DeviceGrid& g = h->g;
+    constexpr int kInSlab = kSweepSources;  // never a row
+    std::map<long long, int> lumped;        // node -> source
+    for (const LumpedDef& L : h->lumped)
+        lumped_edges(L, [&](int i, int j, int k) {
+            const bool slab = in_slab_host(i, g.nx, g.pxn, g.pxp) || in_slab_host(j, g.ny, g.pyn, g.pyp) ||
+                              in_slab_host(k, g.nz, g.pzn, g.pzp);
+            int& s = lumped.emplace(((long long)k * g.ny + j) * g.nx + i, -1).first->second;
+            s = std::max(s, slab ? kInSlab : L.source);
+        });
+    auto node = [&](long long v, int s) {
+        return make_int4((int)(v % g.nx), (int)((v / g.nx) % g.ny), (int)(v / ((long long)g.nx * g.ny)), s);
+    };
+    for (const auto& e : lumped)
+        if (e.second < kSweepSources) out.push_back(node(e.first, e.second));
+    for (long long v : h->plate_list)
+        if (!lumped.count(v)) out.push_back(node(v, -1));
+    return out.size();
 }
 
 // Interface rows (kInterfaceNode and kGeneral nodes): gather the seven-cell keys, sort and unique
@@ -1381,29 +1314,92 @@ int build_interface_rows(fdtd_handle* h) {
                                  h->stream));
     }
     const int n_rows = (int)hk.size();
+    CUDA_TRY(launch_iface_rows(g, h->cls, h->mat, h->iface_table, h->iface_keys, n_rows, h->iface_slot_row, h->rec,
+                               h->small, h->stream));
+    CUDA_TRY(launch_rec_general(g, h->d_lumped, h->n_lumped_edges, h->rec, h->stream));
+    StepParams p = make_params(h);  // the rows come from the material rows and properties, plates and lumped edges
+    p.coef = h->coef;
+    // nodes with plate-covered edges, and lumped edges outside the CPML slabs: rows of their own
+    std::vector<int4> special;
+    std::vector<unsigned long long> sk;
+    h->release(h->d_special);
+    h->d_special = nullptr;
+    const int room = kMaxInterfaceRows - n_rows;
+    // a few such nodes (lumped edges): a row each; more (plates): their distinct rows
+    const bool each = special_nodes(h, special) <= kSpecialEach && (int)special.size() <= room;
+    std::stable_sort(special.begin(), special.end(), [](const int4& a, const int4& b) { return (a.w >= 0) < (b.w >= 0); });
+    if (!special.empty()) {
+        CUDA_TRY(h->alloc((void**)&h->d_special, sizeof(int4) * special.size()));
+        CUDA_TRY(cudaMemcpyAsync(h->d_special, special.data(), sizeof(int4) * special.size(), cudaMemcpyHostToDevice, h->stream));
+    }
+    if (each) {
+        for (size_t q = 0; q < special.size(); ++q) sk.push_back(special[q].w >= 0 ? 1ull << 63 : 0ull);
+    } else if (room > 0) {
+        CUDA_TRY(launch_special_set(p, h->d_special, (int)special.size(), h->iface_table, h->iface_counters, h->iface_keys, h->stream));
+        CUDA_TRY(cudaMemcpyAsync(counters, h->iface_counters, sizeof(counters), cudaMemcpyDeviceToHost, h->stream));
+        CUDA_TRY(cudaStreamSynchronize(h->stream));
+        sk.resize((size_t)std::min(counters[1], kIfaceTableSize));
+        CUDA_TRY(cudaMemcpyAsync(sk.data(), h->iface_keys, sk.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, h->stream));
+        CUDA_TRY(cudaStreamSynchronize(h->stream));
+        std::sort(sk.begin(), sk.end());  // source rows (bit 63) last
+        if (sk.size() > (size_t)room) sk.resize((size_t)room);
+    }
+    const int n_special = (int)sk.size();
+    int n_plain = 0;
+    while (n_plain < n_special && !(sk[(size_t)n_plain] >> 63)) ++n_plain;
     h->release(h->coef_rows);
     h->coef_rows = nullptr;
+    h->release(h->src_rows);
+    h->src_rows = nullptr;
+    h->src_row0 = kRecGeneral;
     h->n_iface_rows = 0;
-    CUDA_TRY(h->alloc((void**)&h->coef_rows, sizeof(MatCoef) * (size_t)(kFirstInterfaceRow + n_rows)));
+    CUDA_TRY(h->alloc((void**)&h->coef_rows, sizeof(MatCoef) * (size_t)(kFirstInterfaceRow + n_rows + n_special)));
     CUDA_TRY(cudaMemcpyAsync(h->coef_rows, h->coef, sizeof(MatCoef) * (size_t)kFirstInterfaceRow, cudaMemcpyDeviceToDevice,
                              h->stream));
-    CUDA_TRY(launch_iface_rows(g, h->cls, h->mat, h->iface_table, h->iface_keys, n_rows, h->iface_slot_row, h->rec,
-                               h->stream));
-    CUDA_TRY(launch_rec_general(g, h->d_lumped, h->n_lumped_edges, h->rec, h->stream));
-    StepParams p{};  // the rows come from the material rows and properties only
-    p.g = g;
-    p.props = h->props;
-    p.coef = h->coef;
-    CUDA_TRY(launch_iface_coefs(p, h->iface_keys, n_rows, h->coef_rows, h->stream));
+    if (n_special > 0) {
+        const int first = kFirstInterfaceRow + n_rows;
+        if (n_special > n_plain) {
+            CUDA_TRY(h->alloc((void**)&h->src_rows, sizeof(SrcRow) * (size_t)(n_special - n_plain)));
+            h->src_row0 = first + n_plain;
+        }
+        if (each) {
+            CUDA_TRY(launch_special_each(p, h->d_special, n_special, n_plain, first, h->coef_rows, h->src_rows, h->rec, h->stream));
+        } else {
+            CUDA_TRY(cudaMemcpyAsync(h->iface_keys, sk.data(), sk.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice, h->stream));
+            CUDA_TRY(launch_special_rows(p, h->d_special, (int)special.size(), h->iface_table, h->iface_keys, n_special, n_plain,
+                                         first, h->iface_slot_row, h->coef_rows, h->src_rows, h->rec, h->stream));
+            CUDA_TRY(cudaMemcpyAsync(h->iface_keys, hk.data(), hk.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice, h->stream));
+        }
+    }
+    StepParams pi{};
+    pi.g = g;
+    pi.props = h->props;
+    pi.coef = h->coef;
+    CUDA_TRY(launch_iface_coefs(pi, h->iface_keys, n_rows, h->coef_rows, h->stream));
     h->n_iface_rows = n_rows;
+    CUDA_TRY(cudaMemcpyAsync(&h->edge_mat, h->small, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     return FDTD_OK;
 }
 
 int build_probes(fdtd_handle* h) {
     h->release(h->d_probes); h->release(h->d_probe_k); h->release(h->d_probe_ids); h->release(h->ring);
     h->d_probes = nullptr; h->d_probe_k = nullptr; h->d_probe_ids = nullptr; h->ring = nullptr;
+    h->release(h->d_probes_at);
+    h->d_probes_at = nullptr;
     const DeviceGrid& g = h->g;
     const size_t np = h->probes.size();
+    std::vector<ProbeAt> at;
+    for (size_t q = 0; q < np; ++q) {
+        const Probe& r = h->probes[q];
+        if (in_slab_host(r.i, g.nx, g.pxn, g.pxp) || in_slab_host(r.j, g.ny, g.pyn, g.pyp) || in_slab_host(r.k, g.nz, g.pzn, g.pzp))
+            continue;
+        at.push_back(ProbeAt{r.comp, (int)q, (long long)r.k * g.plane + (long long)r.j * g.pitch + r.i});
+    }
+    h->n_probes_at = (int)at.size();
+    if (!at.empty()) {
+        CUDA_TRY(h->alloc((void**)&h->d_probes_at, sizeof(ProbeAt) * at.size()));
+        CUDA_TRY(cudaMemcpy(h->d_probes_at, at.data(), sizeof(ProbeAt) * at.size(), cudaMemcpyHostToDevice));
+    }
     std::vector<int> order(np);
     for (size_t q = 0; q < np; ++q) order[q] = (int)q;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return h->probes[a].k < h->probes[b].k; });
@@ -1441,6 +1437,8 @@ int ensure_prepared(fdtd_handle* h) {
         if (!h->prepared || h->dirty_cpml) CUDA_TRY(launch_cpml_profiles(h->g, h->grid.pi, h->cpml_r0, h->prof, h->stream));
         h->dirty_cpml = false;
         CUDA_TRY(launch_bg_curl(h->g, h->coef, 0, h->d_kappa_ptrs, h->d_bg_ptrs, h->stream));
+        CUDA_TRY(launch_axis_tables(h->g, h->prof, h->bg_curl, h->te, h->th, h->stream));
+        h->bg_node = make_bg_node(h->g, h->materials[0]);
         h->dirty_materials = false;
         h->dirty_lumped = true;
     }
@@ -1464,6 +1462,7 @@ int ensure_prepared(fdtd_handle* h) {
         int rc = build_probes(h);
         if (rc) return rc;
     }
+    CUDA_TRY(launch_rec_probes(h->g, h->d_probes, (int)h->probes.size(), h->rec, h->stream));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     h->prepared = true;
     return FDTD_OK;
@@ -1495,26 +1494,21 @@ bool g_scratch_configured[kMaxScratchDevices] = {};
 
 size_t align_up(size_t v) { return (v + kScratchAlign - 1) / kScratchAlign * kScratchAlign; }
 
-// Offsets of the pieces of the scratch for handle h: 6 fields, 24 CPML arrays, work list.
+// Offsets of the pieces of the scratch for handle h: 6 fields, then the 24 CPML arrays, laid out
+// like a CPML memory set (alloc_psi_set).
 struct ScratchLayout {
     size_t field[6];
-    size_t psi[6][4];
-    size_t items;
+    size_t psi;
     size_t total;
 };
 
-ScratchLayout scratch_layout(const fdtd_handle* h, size_t n_items) {
+ScratchLayout scratch_layout(const fdtd_handle* h) {
     ScratchLayout L{};
     size_t off = 0;
     const size_t fb = align_up((size_t)vol(h) * sizeof(float));
     for (int c = 0; c < 6; ++c, off += fb) L.field[c] = off;
-    for (int f = 0; f < 6; ++f) {
-        const size_t pb = align_up((size_t)h->psi_elems[f] * sizeof(float));
-        for (int q = 0; q < 4; ++q, off += pb) L.psi[f][q] = off;
-    }
-    L.items = off;
-    off += align_up(n_items * sizeof(int4));
-    L.total = off;
+    L.psi = off;
+    L.total = off + (size_t)h->psi_total * sizeof(float);
     return L;
 }
 
@@ -1529,7 +1523,7 @@ int scratch_setup(int dev, unsigned char** base) {
         g_scratch_addr[dev] = (unsigned char*)a;
     }
     if (!g_scratch_configured[dev]) {
-        CUDA_TRY(fused_configure());
+        CUDA_TRY(sweep_configure());
         g_scratch_configured[dev] = true;
     }
     *base = g_scratch_addr[dev];
@@ -1548,22 +1542,7 @@ extern "C" int fdtd_step_static_scratch(fdtd_handle* h, int64_t n) {
     int dev = -1;
     CUDA_TRY(cudaGetDevice(&dev));
     if (dev != h->device) return fail(FDTD_ERR_STATE, "the current device is not the handle's device");
-    if (!h->static_planned) {  // planning, as for the fused schedule; host memory only
-        FusedPlan plan;
-        const PlanGrid pg = plan_grid(h->g);
-        plan_fused(pg, plan_chunk(pg), h->has_design ? h->dbox : nullptr, plan);  // no CPML items: shell only
-        const std::vector<PlanItem> all = flatten(plan, h->static_counts);
-        if (h->static_items) CUDA_TRY(cudaFreeHost(h->static_items));
-        h->static_items = nullptr;
-        h->static_n_items = 0;
-        if (!all.empty()) {
-            CUDA_TRY(cudaHostAlloc((void**)&h->static_items, all.size() * sizeof(int4), cudaHostAllocDefault));
-            std::memcpy(h->static_items, all.data(), all.size() * sizeof(int4));
-        }
-        h->static_n_items = all.size();
-        h->static_planned = true;
-    }
-    const ScratchLayout L = scratch_layout(h, h->static_n_items);
+    const ScratchLayout L = scratch_layout(h);
     if (L.total > kStaticScratchBytes)
         return fail(FDTD_ERR_RANGE, "grid needs " + std::to_string(L.total) + " bytes of step scratch; the static scratch holds " +
                                         std::to_string(kStaticScratchBytes) + " (about a 64^3 grid with 10-cell CPML)");
@@ -1578,11 +1557,14 @@ extern "C" int fdtd_step_static_scratch(fdtd_handle* h, int64_t n) {
     float* sf[6];
     for (int c = 0; c < 6; ++c) sf[c] = (float*)(base + L.field[c]);
     PsiSet sp{};
+    sp.base = (float*)(base + L.psi);
     for (int f = 0; f < 6; ++f) {
-        sp.f[f].e[0] = h->psi_elems[f] ? (float*)(base + L.psi[f][0]) : nullptr;
-        sp.f[f].e[1] = h->psi_elems[f] ? (float*)(base + L.psi[f][1]) : nullptr;
-        sp.f[f].h[0] = h->psi_elems[f] ? (float*)(base + L.psi[f][2]) : nullptr;
-        sp.f[f].h[1] = h->psi_elems[f] ? (float*)(base + L.psi[f][3]) : nullptr;
+        if (!h->psi_elems[f]) continue;
+        float* at = (float*)(base + L.psi) + h->psi_off[f];
+        sp.f[f].e[0] = at;
+        sp.f[f].e[1] = at + h->psi_stride[f];
+        sp.f[f].h[0] = at + 2 * h->psi_stride[f];
+        sp.f[f].h[1] = at + 3 * h->psi_stride[f];
     }
     FusedMaps maps_h, maps_s;  // tensor maps (host structs) of the handle's buffer and the scratch
     {
@@ -1590,14 +1572,10 @@ extern "C" int fdtd_step_static_scratch(fdtd_handle* h, int64_t n) {
         float* ee[3] = {h->field[a][0], h->field[a][1], h->field[a][2]};
         float* sh[3] = {sf[3], sf[4], sf[5]};
         float* se[3] = {sf[0], sf[1], sf[2]};
-        if (encode_fused_maps(&maps_h, h->g, hh, ee, h->rec, enc) != 0 ||
-            encode_fused_maps(&maps_s, h->g, sh, se, h->rec, enc) != 0)
+        if (encode_sweep_maps(&maps_h, h->g, hh, ee, h->rec, enc) != 0 ||
+            encode_sweep_maps(&maps_s, h->g, sh, se, h->rec, enc) != 0)
             return fail(FDTD_ERR_CUDA, "tensor map encoding failed");
     }
-    int4* d_items = (int4*)(base + L.items);
-    const size_t n_items = h->static_n_items;
-    if (n_items) CUDA_TRY(cudaMemcpyAsync(d_items, h->static_items, n_items * sizeof(int4), cudaMemcpyHostToDevice, h->stream));
-    const FusedWork w = work_of(d_items, h->static_counts);
     // With an odd count the result ends in the scratch and is copied back whole, so the scratch's
     // CPML arrays start as copies of the handle's: the elements no step writes then agree. With an
     // even count the last step writes the handle's own buffers and the scratch needs no copy.
@@ -1613,10 +1591,13 @@ extern "C" int fdtd_step_static_scratch(fdtd_handle* h, int64_t n) {
     const FieldPtrs fh{h->field[a][0], h->field[a][1], h->field[a][2], h->field[a][3], h->field[a][4], h->field[a][5]};
     const FieldPtrs fs{sf[0], sf[1], sf[2], sf[3], sf[4], sf[5]};
     for (int64_t s = 0; s < n; ++s) {
-        if ((s & 1) == 0) CUDA_TRY(launch_fused(maps_h, p, fh, fs, h->psi[a], sp, h->step, w, h->stream));
-        else CUDA_TRY(launch_fused(maps_s, p, fs, fh, sp, h->psi[a], h->step, w, h->stream));
+        if ((s & 1) == 0)
+            CUDA_TRY(launch_sweep(maps_h, p, fh, fs, h->psi[a], sp, h->sweep, sweep_step(h, s > 0), h->step, h->stream));
+        else
+            CUDA_TRY(launch_sweep(maps_s, p, fs, fh, sp, h->psi[a], h->sweep, sweep_step(h, s > 0), h->step, h->stream));
         ++h->step;
     }
+    CUDA_TRY(launch_sample_probes(p, n & 1 ? fs : fh, h->d_probes_at, h->n_probes_at, h->step - 1, h->stream));
     if (n & 1) {  // the last step wrote the scratch: copy the state back into the handle's buffers
         // only the nx columns of each row: the sweep never writes the row padding
         const DeviceGrid& g = h->g;
@@ -1677,9 +1658,8 @@ extern "C" int fdtd_set_design_region(fdtd_handle* h, const int32_t box[6], cons
     CUDA_TRY(cudaMemcpyAsync(h->d_deps, eps_r, nd * sizeof(float), cudaMemcpyHostToDevice, h->stream));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     h->design_base = *base;
+    if (!h->has_design) h->auto_choice = FDTD_SCHEDULE_AUTO;  // AUTO weighs the grid anew
     h->has_design = true;
-    h->replan = true;            // fused work items
-    h->static_planned = false;   // and those of fdtd_step_static_scratch
     h->dirty_materials = true;  // table entry 255, node classes
     h->adj.ready = false;
     return FDTD_OK;
@@ -1866,11 +1846,7 @@ int adj_forward_enqueue(fdtd_handle* h, int64_t n, int32_t checkpoint_every, int
         CUDA_TRY(launch_after_step(h->field[c][0], h->field[c][1], h->field[c][2], g, A.probe, nullptr, h->dbox, adj_slot(h, 0),
                                    h->stream));
     }
-    // one step per fdtd_step call never runs AUTO's trial: apply its direct choice (large grids
-    // with mostly interior tiles take fused) before stepping
-    if (h->schedule == FDTD_SCHEDULE_AUTO && h->auto_choice == FDTD_SCHEDULE_AUTO &&
-        (long long)g.nx * g.ny * g.nz >= kAutoTrialCells)
-        auto_direct(h);
+    auto_choose(h);
     // two-pass steps take their records in k_design_e (no launch of their own): the E of the
     // design edge box is final there, and so is every other E
     const bool two_pass = !use_fused(h);

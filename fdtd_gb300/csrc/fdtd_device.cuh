@@ -109,6 +109,30 @@ struct BgCurl {
     const float* h[3][2];
 };
 
+// The background material's own update coefficients and the factors of its CPML memory (curl
+// coefficient times cell size), for kernels that keep them in constant memory. Own: ea = {Ca of Ex,
+// Ey, Ez}; curl: ec = {Ex plus, Ex minus, Ey plus, Ey minus, Ez plus, Ez minus}; psi: ce = {x: Ey,
+// Ez; y: Ex, Ez; z: Ex, Ey}; ha, hc, ch the same for H. low_ok: the H coefficients equal the
+// default entry's, which faces on the low boundary planes take.
+struct BgNode {
+    float ea[3], ha[3];
+    float ec[6], hc[6];
+    float ce[6], ch[6];
+    int low_ok;
+};
+
+// A coefficient row of a lumped source's Ez edges (rows from StepParams::src_row0 on): its injection
+// coefficient and its waveform.
+struct SrcRow {
+    float cezj;
+    int source;
+};
+// A probe outside the CPML slabs: component, node offset, id.
+struct ProbeAt {
+    int comp, id;
+    long long node;
+};
+
 // Everything an update kernel reads besides the fields.
 struct StepParams {
     DeviceGrid g;
@@ -142,6 +166,17 @@ struct StepParams {
     long long ring_cap;
     int* status;                 // device error word
     BgCurl bg;                   // kappa-divided curl coefficients of the CPML background material
+    BgNode bgn;
+    // coefficient rows from src_row0 on belong to lumped source edges (kRecGeneral: none do)
+    int src_row0;
+    const SrcRow* src_rows;
+    // the same curl coefficients packed with the CPML profiles, per axis and node: {slot 0, slot 1,
+    // b, a} of E and of H (BgCurl's slots)
+    const float4 *te[3], *th[3];
+    // CPML memory by offset from PsiSet::base: array a of face f (E 0, E 1, H 0, H 1) at
+    // psi_off[f] + a * psi_stride[f] floats
+    long long psi_off[6], psi_stride[6];
+    long long psi_total;
     // design region: cells of material kDesign inside dbox = [d0,d3) x [d1,d4) x [d2,d5) take eps_r
     // from deps ((d5-d2), (d4-d1), (d3-d0), x fastest); NULL when the handle has none
     const float* deps;

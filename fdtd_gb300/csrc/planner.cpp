@@ -49,6 +49,41 @@ std::vector<int> starts(int lo, int hi, int size, int align, bool overlap) {
 
 }  // namespace
 
+// Chunks per tile column. A chunk of n planes costs about n + 2 plane steps (the plane below is
+// streamed, the E of the plane above recomputed), and about kSweepSlots CTAs run at once, so short
+// grids want enough chunks to fill the device and tall ones few. The cheapest count wins. Where the
+// chunks come out long, cuts at the z slabs keep the slabs' rules out of the middle chunks.
+SweepPlan plan_sweep(const PlanGrid& g) {
+#ifndef FDTD_SWEEP_SLOTS
+#define FDTD_SWEEP_SLOTS 3
+#endif
+    constexpr int kSweepSlots = FDTD_SWEEP_SLOTS * 152;
+    SweepPlan p{(g.nx + kTileX - 1) / kTileX, (g.ny + kSweepRows - 1) / kSweepRows, g.nz, 0, g.nz, 0, 1, 0};
+    const long long tiles = (long long)p.nbx * p.nby;
+    double best = -1.0;
+    for (int nch = (g.nz + kMaxSweepChunk - 1) / kMaxSweepChunk; nch <= g.nz; ++nch) {
+        const int kc = (g.nz + nch - 1) / nch;
+        const double ctas = (double)tiles * nch;
+        const double waves = ctas <= kSweepSlots ? 1.0 : ctas / kSweepSlots + 0.5;
+        const double cost = waves * (kc + 2);
+        if (best < 0 || cost < best) {
+            best = cost;
+            p.n_mid = nch;
+        }
+    }
+    const int kc = (g.nz + p.n_mid - 1) / p.n_mid;
+    const int lo = g.pzn > 1 ? g.pzn : 1, hi = (g.pzp > 1 ? g.nz - g.pzp : g.nz - 1) - 1;
+    if (kc >= 24 && hi - lo >= kc) {
+        auto chunks = [&](int n) { return (n + kc - 1) / kc; };
+        p.zlo = lo;
+        p.zhi = hi;
+        p.n_lo = chunks(lo);
+        p.n_mid = chunks(hi - lo);
+        p.n_hi = chunks(g.nz - hi);
+    }
+    return p;
+}
+
 // Planes per interior item: chunks are halved until the grid has at least kMinItems of them, and
 // no chunk is longer than kMaxChunk planes (an item also streams the plane below and recomputes
 // the one above). 8192 items measured best at 512^3 against 2048, 4096 and 16384 (32 planes

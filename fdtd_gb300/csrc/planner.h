@@ -32,10 +32,6 @@ struct PlanItem {
     int x, y, z, w;  // same layout as int4
 };
 
-struct PlanGrid {
-    int nx, ny, nz;
-    int pxn, pxp, pyn, pyp, pzn, pzp;
-};
 
 struct FusedPlan {
     std::vector<PlanItem> interior;
@@ -45,6 +41,38 @@ struct FusedPlan {
 
 // Thickest CPML slab (cells) the CPML sweep takes: a slab then fits in one tile row band.
 constexpr int kCpmlMaxSlab = kTileY - 1;
+
+struct PlanGrid {
+    int nx, ny, nz;
+    int pxn, pxp, pyn, pyp, pzn, pzp;
+};
+
+// The sweep of the whole grid (yee_sweep.cu): tiles of kTileX x kSweepRows nodes from the origin, each
+// cut into chunks of planes of nearly equal length: n_lo chunks of the planes below zlo, n_mid of
+// [zlo, zhi) and n_hi of the rest. The middle chunks, and the E above their top plane, meet neither a
+// z slab nor a z wall; grids where cutting there does not pay have n_mid chunks only (zlo 0, zhi nz).
+#ifndef FDTD_SWEEP_ROWS
+#define FDTD_SWEEP_ROWS 16
+#endif
+constexpr int kSweepRows = FDTD_SWEEP_ROWS;
+constexpr int kMaxSweepChunk = 32;                   // planes of a chunk
+constexpr int kMaxSweepPlanes = kMaxSweepChunk + 2;  // planes a chunk streams
+#ifdef __CUDACC__
+#define FDTD_HD __host__ __device__
+#else
+#define FDTD_HD
+#endif
+struct SweepPlan {
+    int nbx, nby, nz;
+    int zlo, zhi, n_lo, n_mid, n_hi;
+    FDTD_HD int chunks() const { return n_lo + n_mid + n_hi; }
+    FDTD_HD int chunk(int c) const {  // first plane of chunk c; nz for c = chunks()
+        if (c < n_lo) return (int)((long long)c * zlo / n_lo);
+        if (c < n_lo + n_mid) return zlo + (int)((long long)(c - n_lo) * (zhi - zlo) / n_mid);
+        return c == chunks() ? nz : zhi + (int)((long long)(c - n_lo - n_mid) * (nz - zhi) / n_hi);
+    }
+};
+SweepPlan plan_sweep(const PlanGrid& g);
 
 // Planes per interior item (see plan_chunk in planner.cpp).
 int plan_chunk(const PlanGrid& g);

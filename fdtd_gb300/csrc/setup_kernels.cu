@@ -195,6 +195,26 @@ cudaError_t launch_bg_curl(const DeviceGrid& g, const MatCoef* coef, int bg, con
     return cudaGetLastError();
 }
 
+// One axis of StepParams::te / th.
+__global__ void k_axis_table(float4* te, float4* th, int n, const float* be, const float* ae, const float* bm,
+                             const float* am, const float* e0, const float* e1, const float* h0, const float* h1) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    te[q] = make_float4(e0[q], e1[q], be[q], ae[q]);
+    th[q] = make_float4(h0[q], h1[q], bm[q], am[q]);
+}
+
+cudaError_t launch_axis_tables(const DeviceGrid& g, float* const prof[18], float* const bg_curl[12], float4* const te[3],
+                               float4* const th[3], cudaStream_t st) {
+    const int ns[3] = {g.nx, g.ny, g.nz};
+    for (int a = 0; a < 3; ++a) {
+        float* const* P = prof + 6 * a;
+        float* const* C = bg_curl + 4 * a;
+        k_axis_table<<<(ns[a] + 127) / 128, 128, 0, st>>>(te[a], th[a], ns[a], P[0], P[1], P[2], P[3], C[0], C[1], C[2], C[3]);
+    }
+    return cudaGetLastError();
+}
+
 __global__ void k_fill(float* p, long long n, float v) {
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
         p[q] = v;
@@ -431,12 +451,19 @@ __device__ __forceinline__ void iface_row(uint8_t* __restrict__ cls, const uint8
                                           uint16_t* __restrict__ rec, int i, int j, int k);
 __global__ void k_iface_rows(uint8_t* __restrict__ cls, const uint8_t* __restrict__ mat, DeviceGrid g,
                              const unsigned long long* __restrict__ table, const int* __restrict__ slot_row,
-                             uint16_t* __restrict__ rec) {
+                             uint16_t* __restrict__ rec, int* __restrict__ edge_mat) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= g.nx || j >= g.ny) return;
-    for (int k = blockIdx.z * kSetupPlanes, k1 = min(g.nz, k + kSetupPlanes); k < k1; ++k)
-        iface_row(cls, mat, g, table, slot_row, rec, i, j, k);
+    if (j >= g.ny) return;  // i < g.pitch: the blocks cover whole rows
+    for (int k = blockIdx.z * kSetupPlanes, k1 = min(g.nz, k + kSetupPlanes); k < k1; ++k) {
+        if (i < g.nx) {
+            iface_row(cls, mat, g, table, slot_row, rec, i, j, k);
+            const int r = rec[(long long)k * g.plane + (long long)j * g.pitch + i];
+            if (r != 0 && r < kRecGeneral && (i == 0 || j == 0 || k == 0 || in_slab(i, g.nx, g.pxn, g.pxp) ||
+                                              in_slab(j, g.ny, g.pyn, g.pyp) || in_slab(k, g.nz, g.pzn, g.pzp)))
+                *edge_mat = 1;
+        } else rec[(long long)k * g.plane + (long long)j * g.pitch + i] = 0;  // row padding: the sweep's tiles read it
+    }
 }
 __device__ __forceinline__ void iface_row(uint8_t* __restrict__ cls, const uint8_t* __restrict__ mat, const DeviceGrid& g,
                                           const unsigned long long* __restrict__ table, const int* __restrict__ slot_row,
@@ -466,6 +493,23 @@ __global__ void k_rec_general(uint16_t* rec, DeviceGrid g, const LumpedEdge* edg
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q < n_edges)
         rec[(long long)edges[q].k * g.plane + (long long)edges[q].j * g.pitch + edges[q].i] = (uint16_t)(kRecGeneral | kGeneral);
+}
+
+// The nodes of probes inside a CPML slab too: the general path samples them before the CPML
+// correction. The classes, which the per-node kernels go by, stay: those kernels sample themselves.
+__global__ void k_rec_probes(uint16_t* rec, DeviceGrid g, const Probe* probes, int n) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    const Probe& r = probes[q];
+    if (!in_slab(r.i, g.nx, g.pxn, g.pxp) && !in_slab(r.j, g.ny, g.pyn, g.pyp) && !in_slab(r.k, g.nz, g.pzn, g.pzp)) return;
+    const long long v = (long long)r.k * g.plane + (long long)r.j * g.pitch + r.i;
+    if (rec[v] < kRecGeneral) rec[v] = (uint16_t)(kRecGeneral | kGeneral);
+}
+
+cudaError_t launch_rec_probes(const DeviceGrid& g, const Probe* probes, int n, uint16_t* rec, cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    k_rec_probes<<<(n + 127) / 128, 128, 0, st>>>(rec, g, probes, n);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_rec_general(const DeviceGrid& g, const LumpedEdge* edges, int n_edges, uint16_t* rec, cudaStream_t st) {
@@ -513,12 +557,14 @@ cudaError_t launch_iface_set(const DeviceGrid& g, const uint8_t* cls, const uint
 }
 
 cudaError_t launch_iface_rows(const DeviceGrid& g, uint8_t* cls, const uint8_t* mat, const unsigned long long* table,
-                              const unsigned long long* keys, int n_keys, int* slot_row, uint16_t* rec, cudaStream_t st) {
+                              const unsigned long long* keys, int n_keys, int* slot_row, uint16_t* rec, int* edge_mat,
+                              cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(slot_row, 0xff, sizeof(int) * kIfaceTableSize, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(edge_mat, 0, sizeof(int), st);
     if (e != cudaSuccess) return e;
     if (n_keys > 0) k_iface_slot_rows<<<(n_keys + 127) / 128, 128, 0, st>>>(table, keys, n_keys, slot_row);
     const dim3 block(32, 8, 1), grid((g.nx + 31) / 32, (g.ny + 7) / 8, (g.nz + kSetupPlanes - 1) / kSetupPlanes);
-    k_iface_rows<<<grid, block, 0, st>>>(cls, mat, g, table, slot_row, rec);
+    k_iface_rows<<<grid, block, 0, st>>>(cls, mat, g, table, slot_row, rec, edge_mat);
     return cudaGetLastError();
 }
 
@@ -526,6 +572,126 @@ cudaError_t launch_iface_coefs(const StepParams& p, const unsigned long long* ke
                                cudaStream_t st) {
     if (n_keys <= 0) return cudaSuccess;
     k_iface_coefs<<<(n_keys + 127) / 128, 128, 0, st>>>(p, keys, n_keys, coef);
+    return cudaGetLastError();
+}
+
+// The coefficient row of a node with plate-covered or lumped edges: as e_update builds its
+// coefficients (cell averages, plate conductivity, lumped override), and its H faces'. Interior
+// position rules (CPML kappa, default entries of the low walls) are the sweep's. cezj: the source's.
+namespace {
+__device__ __forceinline__ MatCoef special_row(const StepParams& p, int i, int j, int k, float& cezj) {
+    const DeviceGrid& g = p.g;
+    const unsigned long long key = cell_key(p.mat, g, i, j, k);
+    const int m0 = (int)(key & 0xff), mi = (int)((key >> 8) & 0xff), mj = (int)((key >> 16) & 0xff);
+    const int mk = (int)((key >> 24) & 0xff), mij = (int)((key >> 32) & 0xff), mik = (int)((key >> 40) & 0xff);
+    const int mjk = (int)((key >> 48) & 0xff);
+    Coef3 e[3] = {e_coef(p, 0, m0 == mj && m0 == mk && m0 == mjk, m0, mj, mk, mjk, i, j, k),
+                  e_coef(p, 1, m0 == mi && m0 == mk && m0 == mik, m0, mi, mk, mik, i, j, k),
+                  e_coef(p, 2, m0 == mi && m0 == mj && m0 == mij, m0, mi, mj, mij, i, j, k)};
+    if (plane_has_plate(p, k)) {
+        Coef3 pc[3];
+        const int hit = e_plate(&p, i, j, k, m0, mi, mj, mk, mij, mik, mjk, pc);
+        for (int c = 0; c < 3; ++c)
+            if (hit >> c & 1) e[c] = pc[c];
+    }
+    const LumpedEdge* Lx = find_lumped(p, i, j, k, 0);
+    const LumpedEdge* Lz = find_lumped(p, i, j, k, 2);
+    if (Lx) e[0] = Coef3{Lx->ceze, Lx->cezhy, Lx->cezhx};
+    if (Lz) e[2] = Coef3{Lz->ceze, Lz->cezhy, Lz->cezhx};
+    cezj = Lz && Lz->source >= 0 ? Lz->cezj : 0.f;
+    const Coef3 h[3] = {h_coef(p, 0, false, m0 == mi, m0, mi), h_coef(p, 1, false, m0 == mj, m0, mj),
+                        h_coef(p, 2, false, m0 == mk, m0, mk)};
+    MatCoef r;
+    for (int c = 0; c < 3; ++c) {
+        r.e[c] = make_float4(e[c].a, e[c].bp, e[c].bm, 0.f);
+        r.h[c] = make_float4(h[c].a, h[c].bp, h[c].bm, 0.f);
+    }
+    return r;
+}
+__device__ __forceinline__ unsigned long long special_key(const MatCoef& r, float cezj, int source) {
+    unsigned long long h = 0x9E3779B97F4A7C15ull * (unsigned)(source + 2);
+    const unsigned* w = reinterpret_cast<const unsigned*>(&r);
+    for (int q = 0; q < (int)(sizeof(MatCoef) / 4); ++q) {  // splitmix-style mixing of each word
+        h = (h ^ w[q]) * 0xBF58476D1CE4E5B9ull;
+        h ^= h >> 29;
+    }
+    h = (h ^ __float_as_uint(cezj)) * 0x94D049BB133111EBull;
+    h ^= h >> 32;
+    h &= ~(3ull << 62);  // bit 62 stays clear, so that no key equals kEmptyKey
+    return source >= 0 ? h | 1ull << 63 : h;
+}
+}  // namespace
+
+__global__ void k_special_set(const __grid_constant__ StepParams p, const int4* __restrict__ nodes, int n,
+                              unsigned long long* table, int* filled) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    const int4 v = nodes[q];
+    float cezj;
+    const MatCoef r = special_row(p, v.x, v.y, v.z, cezj);
+    iface_insert(table, filled, special_key(r, cezj, v.w));
+}
+// write: the rows; otherwise every node's entry of rec, checked against the row that was written
+// (several nodes of a key write equal rows unless their hashes collide).
+__global__ void k_special_rows(const __grid_constant__ StepParams p, const int4* __restrict__ nodes, int n,
+                               const unsigned long long* __restrict__ table, const int* __restrict__ slot_row, int first,
+                               int n_plain, MatCoef* coef, SrcRow* src, uint16_t* rec, bool write) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    const int4 v = nodes[q];
+    float cezj;
+    const MatCoef r = special_row(p, v.x, v.y, v.z, cezj);
+    const int s = find_slot(table, special_key(r, cezj, v.w));
+    const int row = s >= 0 ? slot_row[s] : -1;
+    if (row < 0) return;  // no room: the node stays general
+    if (write) {
+        coef[first + row] = r;
+        if (v.w >= 0) src[row - n_plain] = SrcRow{cezj, v.w};
+        return;
+    }
+    const unsigned* a = reinterpret_cast<const unsigned*>(&r);
+    const unsigned* b = reinterpret_cast<const unsigned*>(coef + first + row);
+    bool same = v.w < 0 || (src[row - n_plain].source == v.w && __float_as_uint(src[row - n_plain].cezj) == __float_as_uint(cezj));
+    for (int w = 0; w < (int)(sizeof(MatCoef) / 4); ++w) same = same && a[w] == b[w];
+    if (same) rec[(long long)v.z * p.g.plane + (long long)v.y * p.g.pitch + v.x] = (uint16_t)(first + row);
+}
+
+// Row first + q for node q (nodes with a source from n_plain on).
+__global__ void k_special_each(const __grid_constant__ StepParams p, const int4* __restrict__ nodes, int n, int n_plain,
+                               int first, MatCoef* coef, SrcRow* src, uint16_t* rec) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    const int4 v = nodes[q];
+    float cezj;
+    coef[first + q] = special_row(p, v.x, v.y, v.z, cezj);
+    if (q >= n_plain) src[q - n_plain] = SrcRow{cezj, v.w};
+    rec[(long long)v.z * p.g.plane + (long long)v.y * p.g.pitch + v.x] = (uint16_t)(first + q);
+}
+
+cudaError_t launch_special_each(const StepParams& p, const int4* nodes, int n, int n_plain, int first, MatCoef* coef,
+                                SrcRow* src, uint16_t* rec, cudaStream_t st) {
+    k_special_each<<<(n + 127) / 128, 128, 0, st>>>(p, nodes, n, n_plain, first, coef, src, rec);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_special_set(const StepParams& p, const int4* nodes, int n, unsigned long long* table, int* counters,
+                               unsigned long long* keys, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(table, 0xff, sizeof(unsigned long long) * kIfaceTableSize, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(counters, 0, 2 * sizeof(int), st);
+    if (e != cudaSuccess) return e;
+    k_special_set<<<(n + 127) / 128, 128, 0, st>>>(p, nodes, n, table, counters);
+    k_iface_compact<<<kIfaceTableSize / 256, 256, 0, st>>>(table, keys, counters + 1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_special_rows(const StepParams& p, const int4* nodes, int n, const unsigned long long* table,
+                                const unsigned long long* keys, int n_keys, int n_plain, int first, int* slot_row,
+                                MatCoef* coef, SrcRow* src, uint16_t* rec, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(slot_row, 0xff, sizeof(int) * kIfaceTableSize, st);
+    if (e != cudaSuccess || n_keys <= 0) return e;
+    k_iface_slot_rows<<<(n_keys + 127) / 128, 128, 0, st>>>(table, keys, n_keys, slot_row);
+    for (bool write : {true, false})
+        k_special_rows<<<(n + 127) / 128, 128, 0, st>>>(p, nodes, n, table, slot_row, first, n_plain, coef, src, rec, write);
     return cudaGetLastError();
 }
 

@@ -14,6 +14,12 @@
 
 #include "fdtd_device.cuh"
 
+// The rare paths' helpers are calls, which keeps their registers out of the kernels that use them; a
+// file that runs them with much state live inlines them instead (a call would spill that state).
+#ifndef FDTD_RARE
+#define FDTD_RARE __noinline__
+#endif
+
 namespace fdtd {
 
 // True when node coordinate q lies in the CPML slabs of an axis with n nodes (setABCPML regions,
@@ -42,19 +48,19 @@ __device__ __forceinline__ int psi_off_z(const DeviceGrid& g, int i, int j, int 
 // line with scalar arguments: it runs only at material interfaces and keeps its divisions out of
 // the hot loop's instruction footprint.
 // axis: the component's axis, whose cell values are averaged.
-static __device__ __noinline__ Coef3 e_coef_mixed(const MatProps* props, int axis, int m0, int m1, int m2, int m3,
+static __device__ FDTD_RARE Coef3 e_coef_mixed(const MatProps* props, int axis, int m0, int m1, int m2, int m3,
                                                   float dt, float eps0, float dp, float dm) {
     const MatAxis a = props[m0].a[axis], b = props[m1].a[axis], c = props[m2].a[axis], d = props[m3].a[axis];
     return coef3(avg4(a.eps, b.eps, c.eps, d.eps), avg4(a.sig, b.sig, c.sig, d.sig), dt, eps0, dp, dm);
 }
 // Harmonic means of two cells for an H face (fdtdrav.h:1183-1213).
-static __device__ __noinline__ Coef3 h_coef_mixed(const MatProps* props, int axis, int m0, int m1, float dt, float mu0,
+static __device__ FDTD_RARE Coef3 h_coef_mixed(const MatProps* props, int axis, int m0, int m1, float dt, float mu0,
                                                   float dp, float dm) {
     const MatAxis a = props[m0].a[axis], b = props[m1].a[axis];
     return coef3(harm2(a.mu, b.mu), harm2(a.sigm, b.sigm), dt, mu0, dp, dm);
 }
 // A curl coefficient divided by the CPML kappa (setABCPML, fdtdrav.h:1903-1906 and mirrors).
-static __device__ __noinline__ float kappa_div(float c, float kappa) { return __fdiv_rn(c, kappa); }
+static __device__ FDTD_RARE float kappa_div(float c, float kappa) { return __fdiv_rn(c, kappa); }
 
 // eps_r of axis `axis` of cell (ci, cj, ck) holding material m: the design array for design
 // cells (isotropic).
@@ -80,7 +86,7 @@ __device__ __forceinline__ void edge_material(const StepParams& p, int comp, int
 }
 // Coefficients of an E edge with a design cell among its four cells (setCoefficients on the
 // averages, fdtdrav.h:1280-1303). Out of line: design edges are a small region.
-static __device__ __noinline__ Coef3 e_coef_design(const StepParams* pp, int comp, int i, int j, int k, int m0, int m1,
+static __device__ FDTD_RARE Coef3 e_coef_design(const StepParams* pp, int comp, int i, int j, int k, int m0, int m1,
                                                    int m2, int m3) {
     const StepParams& p = *pp;
     float eps, sig;
@@ -99,7 +105,7 @@ __device__ __forceinline__ bool has_design(const StepParams& p, int m0, int m1, 
 // coefficients from the edge's averaged eps_r and the plate's sigma_e (the last plate listed
 // wins, as the reference writes them in order). Returns a bit per overridden component and
 // writes its coefficients to c[comp]. Out of line: it runs only in planes holding a plate.
-static __device__ __noinline__ int e_plate(const StepParams* pp, int i, int j, int k, int m0, int mi, int mj, int mk,
+static __device__ FDTD_RARE int e_plate(const StepParams* pp, int i, int j, int k, int m0, int mi, int mj, int mk,
                                            int mij, int mik, int mjk, Coef3* c) {
     const StepParams& p = *pp;
     const int b = p.plate_k[k], e = p.plate_k[k + 1];
@@ -335,10 +341,17 @@ __device__ __forceinline__ void h_masks(const DeviceGrid& g, int i, int j, int k
 // material and that carries no lumped edge (node class kUniformGeneral + background): the same
 // arithmetic with the uniformity, background and lumped tests decided at compile time.
 // kSlabs: the CPML slabs (bit 0 x, 1 y, 2 z) the node may lie in; the other slab tests compile out.
-template <bool kDesignAware = false, bool kCoherent = false, bool kPlate = false, bool kBg = false, int kSlabs = 7>
-__device__ __forceinline__ void e_update(const StepParams& p, const ENbr& n, int i, int j, int k, long long m,
-                                         bool plane_lumped, const PsiIO& ps, float out[3], float pre[3],
-                                         const PsiOld* old = nullptr) {
+// kRow: the node's coefficients are row `row` of the coefficient table (StepParams::rec) instead of
+// the averages over its cell materials.
+struct EDiff {
+    float dHz_j, dHy_k, dHx_k, dHz_i, dHy_i, dHx_j;
+};
+// diff(): the node's H differences, formed where they are first used (earlier, they would sit in
+// registers across the coefficients' calls: 5 % on the two-pass step at 128^3).
+template <bool kDesignAware, bool kCoherent, bool kPlate, bool kBg, int kSlabs, bool kRow, class Diff>
+__device__ __forceinline__ void e_update_at(const StepParams& p, const ENbr& n, Diff diff, int i, int j, int k,
+                                              long long m, bool plane_lumped, const PsiIO& ps, float out[3],
+                                              float pre[3], const PsiOld* old, int row) {
     const DeviceGrid& g = p.g;
     bool ex_m, ey_m, ez_m;  // fdtdrav.h:665, 696, 720
     e_masks(g, i, j, k, ex_m, ey_m, ez_m);
@@ -350,10 +363,16 @@ __device__ __forceinline__ void e_update(const StepParams& p, const ENbr& n, int
     const bool ux = kBg || (n.m0 == n.mj && n.m0 == n.mk && n.m0 == n.mjk);
     const bool uy = kBg || (n.m0 == n.mi && n.m0 == n.mk && n.m0 == n.mik);
     const bool uz = kBg || (n.m0 == n.mi && n.m0 == n.mj && n.m0 == n.mij);
-    const bool on_bg = kBg || n.m0 == bg;
-    Coef3 cx = e_coef<kDesignAware>(p, 0, ux, m0, n.mj, n.mk, n.mjk, i, j, k);
-    Coef3 cy = e_coef<kDesignAware>(p, 1, uy, m0, n.mi, n.mk, n.mik, i, j, k);
-    Coef3 cz = e_coef<kDesignAware>(p, 2, uz, m0, n.mi, n.mj, n.mij, i, j, k);
+    const bool on_bg = kBg || (!kRow && n.m0 == bg);
+    Coef3 cx, cy, cz;
+    if constexpr (kRow) {
+        const float4 x = __ldg(&p.coef[row].e[0]), y = __ldg(&p.coef[row].e[1]), z = __ldg(&p.coef[row].e[2]);
+        cx = Coef3{x.x, x.y, x.z}; cy = Coef3{y.x, y.y, y.z}; cz = Coef3{z.x, z.y, z.z};
+    } else {
+        cx = e_coef<kDesignAware>(p, 0, ux, m0, n.mj, n.mk, n.mjk, i, j, k);
+        cy = e_coef<kDesignAware>(p, 1, uy, m0, n.mi, n.mk, n.mik, i, j, k);
+        cz = e_coef<kDesignAware>(p, 2, uz, m0, n.mi, n.mj, n.mij, i, j, k);
+    }
     // plate-covered components (kPlate only): plate coefficients, and the background's tabulated
     // kappa-divided values (which belong to its table coefficients) no longer apply
     int pm = 0;
@@ -366,9 +385,8 @@ __device__ __forceinline__ void e_update(const StepParams& p, const ENbr& n, int
             if (pm & 4) cz = pc[2];
         }
     }
-    const float dHz_j = __fsub_rn(n.hz, n.hz_jm), dHy_k = __fsub_rn(n.hy, n.hy_km);
-    const float dHx_k = __fsub_rn(n.hx, n.hx_km), dHz_i = __fsub_rn(n.hz, n.hz_im);
-    const float dHy_i = __fsub_rn(n.hy, n.hy_im), dHx_j = __fsub_rn(n.hx, n.hx_jm);
+    const EDiff d = diff();
+    const float dHz_j = d.dHz_j, dHy_k = d.dHy_k, dHx_k = d.dHx_k, dHz_i = d.dHz_i, dHy_i = d.dHy_i, dHx_j = d.dHx_j;
     const BgCurl& B = p.bg;
     // Ex (fdtdrav.h:665-676), with defineSourceX's coefficients on its edges (fdtdrav.h:1311-1365)
     const LumpedEdge* Lx = (!kBg && plane_lumped) ? find_lumped(p, i, j, k, 0) : nullptr;
@@ -422,11 +440,38 @@ __device__ __forceinline__ void e_update(const StepParams& p, const ENbr& n, int
     out[2] = ez_m ? vz : n.ez;
 }
 
+template <bool kDesignAware = false, bool kCoherent = false, bool kPlate = false, bool kBg = false, int kSlabs = 7>
+__device__ __forceinline__ void e_update(const StepParams& p, const ENbr& n, int i, int j, int k, long long m,
+                                         bool plane_lumped, const PsiIO& ps, float out[3], float pre[3],
+                                         const PsiOld* old = nullptr) {
+    e_update_at<kDesignAware, kCoherent, kPlate, kBg, kSlabs, false>(
+        p, n,
+        [&] {
+            return EDiff{__fsub_rn(n.hz, n.hz_jm), __fsub_rn(n.hy, n.hy_km), __fsub_rn(n.hx, n.hx_km),
+                         __fsub_rn(n.hz, n.hz_im), __fsub_rn(n.hy, n.hy_im), __fsub_rn(n.hx, n.hx_jm)};
+        },
+        i, j, k, m, plane_lumped, ps, out, pre, old, 0);
+}
+// The same from the differences themselves (n: old E and, unless kRow, the cell materials).
+template <bool kDesignAware = false, bool kCoherent = false, bool kPlate = false, bool kBg = false, int kSlabs = 7,
+          bool kRow = false>
+__device__ __forceinline__ void e_update_diff(const StepParams& p, const ENbr& n, const EDiff& d, int i, int j, int k,
+                                              long long m, bool plane_lumped, const PsiIO& ps, float out[3],
+                                              float pre[3], const PsiOld* old = nullptr, int row = 0) {
+    e_update_at<kDesignAware, kCoherent, kPlate, kBg, kSlabs, kRow>(p, n, [&] { return d; }, i, j, k, m, plane_lumped, ps, out,
+                                                                    pre, old, row);
+}
+
 // One H node (calc_h fdtdrav.h:249-573).
-// kSlabs as for e_update.
-template <bool kCoherent = false, bool kBg = false, int kSlabs = 7>
-__device__ __forceinline__ void h_update(const StepParams& p, const HNbr& n, int i, int j, int k,
-                                         const PsiIO& ps, float out[3], float pre[3], const PsiOld* old = nullptr) {
+// kSlabs and kRow as for e_update_diff (a row's faces on the low boundary planes take the default
+// entry).
+struct HDiff {
+    float dEy_k, dEz_j, dEz_i, dEx_k, dEx_j, dEy_i;
+};
+template <bool kCoherent, bool kBg, int kSlabs, bool kRow, class Diff>
+__device__ __forceinline__ void h_update_at(const StepParams& p, const HNbr& n, Diff diff, int i, int j, int k,
+                                              const PsiIO& ps, float out[3], float pre[3],
+                                              const PsiOld* old, int row) {
     const DeviceGrid& g = p.g;
     bool hx_m, hy_m, hz_m;  // fdtdrav.h:328, 357, 382
     h_masks(g, i, j, k, hx_m, hy_m, hz_m);
@@ -436,15 +481,14 @@ __device__ __forceinline__ void h_update(const StepParams& p, const HNbr& n, int
     const int bg = p.bg.mat;
     const int m0 = kBg ? bg : n.m0;
     const bool ux = kBg || n.m0 == n.mi, uy = kBg || n.m0 == n.mj, uz = kBg || n.m0 == n.mk;
-    const bool on_bg = kBg || n.m0 == bg;
-    const Coef3 cx = h_coef(p, 0, i == 0, ux, m0, n.mi);
-    const Coef3 cy = h_coef(p, 1, j == 0, uy, m0, n.mj);
-    const Coef3 cz = h_coef(p, 2, k == 0, uz, m0, n.mk);
+    const bool on_bg = kBg || (!kRow && n.m0 == bg);
+    const Coef3 cx = h_coef(p, 0, i == 0, kRow || ux, kRow ? row : m0, n.mi);
+    const Coef3 cy = h_coef(p, 1, j == 0, kRow || uy, kRow ? row : m0, n.mj);
+    const Coef3 cz = h_coef(p, 2, k == 0, kRow || uz, kRow ? row : m0, n.mk);
     // the tabulated kappa-divided values belong to the background material's table entry
     const bool bx = i != 0 && ux && on_bg, by = j != 0 && uy && on_bg, bz = k != 0 && uz && on_bg;
-    const float dEy_k = __fsub_rn(n.ey_kp, n.ey), dEz_j = __fsub_rn(n.ez_jp, n.ez);
-    const float dEz_i = __fsub_rn(n.ez_ip, n.ez), dEx_k = __fsub_rn(n.ex_kp, n.ex);
-    const float dEx_j = __fsub_rn(n.ex_jp, n.ex), dEy_i = __fsub_rn(n.ey_ip, n.ey);
+    const HDiff d = diff();
+    const float dEy_k = d.dEy_k, dEz_j = d.dEz_j, dEz_i = d.dEz_i, dEx_k = d.dEx_k, dEx_j = d.dEx_j, dEy_i = d.dEy_i;
     const BgCurl& B = p.bg;
     // Hx (fdtdrav.h:331-338)
     float vx = upd3_hx(cx.a, n.hx, zs ? kdiv(cx.bp, bx, B.h[2][0], p.kmz, k) : cx.bp, dEy_k,
@@ -481,6 +525,24 @@ __device__ __forceinline__ void h_update(const StepParams& p, const HNbr& n, int
     out[0] = hx_m ? vx : n.hx;
     out[1] = hy_m ? vy : n.hy;
     out[2] = hz_m ? vz : n.hz;
+}
+
+template <bool kCoherent = false, bool kBg = false, int kSlabs = 7>
+__device__ __forceinline__ void h_update(const StepParams& p, const HNbr& n, int i, int j, int k,
+                                         const PsiIO& ps, float out[3], float pre[3], const PsiOld* old = nullptr) {
+    h_update_at<kCoherent, kBg, kSlabs, false>(
+        p, n,
+        [&] {
+            return HDiff{__fsub_rn(n.ey_kp, n.ey), __fsub_rn(n.ez_jp, n.ez), __fsub_rn(n.ez_ip, n.ez),
+                         __fsub_rn(n.ex_kp, n.ex), __fsub_rn(n.ex_jp, n.ex), __fsub_rn(n.ey_ip, n.ey)};
+        },
+        i, j, k, ps, out, pre, old, 0);
+}
+template <bool kCoherent = false, bool kBg = false, int kSlabs = 7, bool kRow = false>
+__device__ __forceinline__ void h_update_diff(const StepParams& p, const HNbr& n, const HDiff& d, int i, int j, int k,
+                                              const PsiIO& ps, float out[3], float pre[3],
+                                              const PsiOld* old = nullptr, int row = 0) {
+    h_update_at<kCoherent, kBg, kSlabs, kRow>(p, n, [&] { return d; }, i, j, k, ps, out, pre, old, row);
 }
 
 }  // namespace fdtd

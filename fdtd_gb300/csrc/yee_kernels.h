@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "fdtd_device.cuh"
+#include "planner.h"
 
 namespace fdtd {
 
@@ -16,6 +17,8 @@ struct FieldPtrs {
 // Six CPML faces in the order x_n, x_p, y_n, y_p, z_n, z_p.
 struct PsiSet {
     PsiFace f[6];
+    float* base;  // the allocation that holds them all (StepParams::psi_off), 16-byte aligned size
+    long long pad;
 };
 
 // One time step m with the two-pass schedule (E pass then H pass, in place).
@@ -46,70 +49,31 @@ cudaError_t launch_design_e(const StepParams& p, const FieldPtrs& fi, const Fiel
 cudaError_t launch_plate_e(const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fo, const PsiSet& pin,
                            const PsiSet& pout, long long m, cudaStream_t st);
 
-// Shell items of the fused schedule (planner.h), one list per set of CPML slabs their nodes may
-// lie in: kShellZ (z slabs only: planes outside the interior z range within the interior's x / y
-// range, and tiles around a design region), kShellYZ (the y bands beside the interior), kShellX
-// (the x bands beside the swept rows, inside the interior z range), kShellAny (the rest of the x
-// bands, corners included, and whole grids without interior tiles).
-enum { kShellZ = 0, kShellYZ = 1, kShellX = 2, kShellAny = 3, kShellLists = 4 };
-struct ShellWork {
-    const int4* items[kShellLists];
-    int n[kShellLists];
-};
-
-// Shell passes of the fused schedule (yee_two_pass.cu): E (e_pass) or H of the nodes of the shell
-// items, reading fi / pin (buffer A) and writing fo / pout (buffer B). The lists must lie one after
-// the other in device memory (one launch covers them).
-cudaError_t launch_shell(bool e_pass, const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fo, const PsiSet& pin,
-                         const PsiSet& pout, const ShellWork& w, long long m, cudaStream_t st);
-
-// Fused schedule (yee_fused.cu): per step the shell E pass, the z-marching interior sweep (TMA
-// tiles of buffer A: H with halo, old E, coefficient rows) and the shell H pass; fields A -> B, CPML
-// memory psi_in -> psi_out. The items come from plan_fused (planner.h).
-struct FusedMaps {
+// Fused schedule (yee_sweep.cu): one kernel per time step sweeps the whole grid, fields A -> B,
+// CPML memory pin -> pout.
+struct FusedMaps {  // tensor maps of buffer A
     CUtensorMap h[3];
     CUtensorMap e[3];
     CUtensorMap rec;  // coefficient rows (StepParams::rec)
 };
-// Tensor maps of the CPML sweep: the sweep's own, plus the CPML memory of buffer A's y and z faces
-// per side (0: n face, 1: p face) and array (the two E, the two H arrays of the face): E arrays in
-// E-tile boxes (the halo nodes' E needs its old psi too), H arrays in boxes of the tile's own nodes.
-// Faces without CPML cells have no maps: bit s of `faces` is set for y side s, bit 2 + s for z
-// side s, and the sweep loads through no other map.
-struct CpmlMaps {
-    FusedMaps base;
-    CUtensorMap ye[2][2], yh[2][2];
-    CUtensorMap ze[2][2], zh[2][2];
-    int faces;
+constexpr int kSweepSources = 8;  // lumped sources whose signal comes with the launch
+struct SweepStep {
+    const ProbeAt* probes;  // probes outside the CPML slabs
+    int n_probes;
+    int late;               // sample them for step m - 1 from fi
+    int mat;                // coefficient rows other than the background's in a CPML slab or on a low wall
+    float sig[kSweepSources];
 };
-// Work items of one step (device arrays of int4 in the formats of planner.h).
-struct FusedWork {
-    const int4* interior;
-    int n_interior;
-    ShellWork shell;
-    const int4* cpml;  // CPML items (CPML sweep), run after the interior sweep on its stream
-    int n_cpml;
-};
-cudaError_t fused_configure();
-int fused_smem_bytes();
-int cpml_smem_bytes();
-// fork (optional): a second stream and two events; the interior sweep then runs on `aux`,
-// concurrently with the shell E pass on `st` (they read buffer A and write disjoint nodes of B),
-// and `st` waits for it before the shell H pass.
-struct FusedFork {
-    cudaStream_t aux;
-    cudaEvent_t fork, join;
-};
-// cmaps: the CPML sweep's maps (buffer A), needed when w.n_cpml > 0.
-cudaError_t launch_fused(const FusedMaps& maps, const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fo,
-                         const PsiSet& psi_in, const PsiSet& psi_out, long long m, const FusedWork& w, cudaStream_t st,
-                         const FusedFork* fork = nullptr, const CpmlMaps* cmaps = nullptr);
+cudaError_t sweep_configure();
+cudaError_t launch_sweep(const FusedMaps& maps, const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fo,
+                         const PsiSet& pin, const PsiSet& pout, const SweepPlan& sg, const SweepStep& ss, long long m,
+                         cudaStream_t st);
+// The same probes for step m from its finished fields f.
+cudaError_t launch_sample_probes(const StepParams& p, const FieldPtrs& f, const ProbeAt* probes, int n, long long m,
+                                 cudaStream_t st);
 // encode_fn: the driver's cuTensorMapEncodeTiled. Returns 0 on success.
-int encode_fused_maps(FusedMaps* out, const DeviceGrid& g, float* const h[3], float* const e[3], const uint16_t* rec,
+int encode_sweep_maps(FusedMaps* out, const DeviceGrid& g, float* const h[3], float* const e[3], const uint16_t* rec,
                       void* encode_fn);
-// The CPML sweep's maps of a buffer (fields h, e, CPML memory psi) into out.
-int encode_cpml_maps(CpmlMaps* out, const DeviceGrid& g, float* const h[3], float* const e[3], const uint16_t* rec,
-                     const PsiSet& psi, void* encode_fn);
 
 // Setup kernels (setup_kernels.cu).
 // r0 = 0: the reference's grading (sigma_opt); r0 > 0: sigma_max from that reflection coefficient.
@@ -123,6 +87,9 @@ cudaError_t launch_lumped_coefs(const DeviceGrid& g, const uint8_t* mat, const M
 // kappa_m z}; out_dev: device array of 12 pointers, per axis {E slot 0, E slot 1, H slot 0, H slot 1}.
 cudaError_t launch_bg_curl(const DeviceGrid& g, const MatCoef* coef, int bg, const float* const* kappa_dev,
                            float* const* out_dev, cudaStream_t st);
+// tab: per axis the packed E and H tables (StepParams::te, th) from the profiles and out_dev's arrays.
+cudaError_t launch_axis_tables(const DeviceGrid& g, float* const prof[18], float* const bg_curl[12], float4* const te[3],
+                               float4* const th[3], cudaStream_t st);
 cudaError_t launch_fill(float* p, long long n, float v, cudaStream_t st);
 // Columns nx .. pitch-1 of every row of a field array set to v.
 cudaError_t launch_fill_padding(float* p, const DeviceGrid& g, float v, cudaStream_t st);
@@ -146,10 +113,29 @@ constexpr int kIfaceTableBits = 17;
 constexpr int kIfaceTableSize = 1 << kIfaceTableBits;
 cudaError_t launch_iface_set(const DeviceGrid& g, const uint8_t* cls, const uint8_t* mat, unsigned long long* table,
                              int* counters, unsigned long long* keys, cudaStream_t st);
+// *edge_mat (device int) becomes 1 if such a row lies in a CPML slab or on a low wall.
 cudaError_t launch_iface_rows(const DeviceGrid& g, uint8_t* cls, const uint8_t* mat, const unsigned long long* table,
-                              const unsigned long long* keys, int n_keys, int* slot_row, uint16_t* rec, cudaStream_t st);
+                              const unsigned long long* keys, int n_keys, int* slot_row, uint16_t* rec, int* edge_mat,
+                              cudaStream_t st);
 cudaError_t launch_iface_coefs(const StepParams& p, const unsigned long long* keys, int n_keys, MatCoef* coef,
                                cudaStream_t st);
+// The nodes of the probes inside a CPML slab to the general path (after launch_iface_rows), which
+// samples them before the CPML correction.
+cudaError_t launch_rec_probes(const DeviceGrid& g, const Probe* probes, int n, uint16_t* rec, cudaStream_t st);
+// Coefficient rows of listed nodes ({i, j, k, source or -1}: nodes with plate-covered or lumped
+// edges, which no seven-cell key describes). launch_special_set collects their distinct rows by a
+// 64-bit hash of the row and the source in the set of launch_iface_set (bit 63: a source), the list
+// unsorted in keys, counters[1] their number. launch_special_rows, given the sorted keys, writes rows
+// first + q of the coefficient table, the nodes' entries of rec, and the source rows' table (rows from
+// first + n_plain on). A node whose row differs from its key's (equal hashes) stays general.
+// launch_special_each gives node q row first + q instead (nodes with a source from n_plain on).
+cudaError_t launch_special_each(const StepParams& p, const int4* nodes, int n, int n_plain, int first, MatCoef* coef,
+                                SrcRow* src, uint16_t* rec, cudaStream_t st);
+cudaError_t launch_special_set(const StepParams& p, const int4* nodes, int n, unsigned long long* table, int* counters,
+                               unsigned long long* keys, cudaStream_t st);
+cudaError_t launch_special_rows(const StepParams& p, const int4* nodes, int n, const unsigned long long* table,
+                                const unsigned long long* keys, int n_keys, int n_plain, int first, int* slot_row,
+                                MatCoef* coef, SrcRow* src, uint16_t* rec, cudaStream_t st);
 // The lumped edges' nodes back to kRecGeneral | kGeneral in rec (after launch_iface_rows).
 cudaError_t launch_rec_general(const DeviceGrid& g, const LumpedEdge* edges, int n_edges, uint16_t* rec, cudaStream_t st);
 

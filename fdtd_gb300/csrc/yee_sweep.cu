@@ -1,0 +1,876 @@
+// Fused schedule: one kernel per time step sweeps the whole grid, fields A -> B and CPML memory
+// psi_in -> psi_out.
+//
+// A CTA owns a column of 32 x kSweepRows nodes and a chunk of planes [k0, k1) and marches along z, a
+// quad of four x-neighbours per thread: the addresses, tests and parameter loads, which outnumber
+// the arithmetic several times in a kernel of one node per thread, are shared by the quad, and its
+// values move as 16-byte words. Planes stream through a shared-memory ring filled by TMA
+// (cp.async.bulk.tensor, 3-D tiles, the next plane in flight while one is computed): H with a
+// one-node halo, old E, and the 16-bit coefficient row of each node (StepParams::rec). At plane k a
+// thread computes E(k) of its quad and then H(k-1), whose neighbours' E(k-1) lie in shared memory
+// since the step before: one barrier per plane. What it needs of its own nodes at plane k-1 stays
+// in registers. One more warp computes E on the row above the tile and the column beside it, which
+// the H update needs (recomputed from the old fields, not exchanged).
+//
+// Coefficients. A quad whose four nodes share a coefficient row loads it once (the background's comes
+// with the kernel parameters); in a CPML slab the curl coefficients along the slab's axis come from
+// the axis' table for background nodes (StepParams::te, th: divided by kappa) and by division for
+// other rows. Quads of several rows take them node by node. What is left (lumped edges in a slab,
+// design nodes, probes in a slab, keys beyond the table, quads of several rows in a slab) runs
+// e_update_diff / h_update_diff (slow_node). Old CPML memory of the y and z faces is fetched a plane
+// ahead with cp.async into slots of the thread's own.
+//
+// What bounds it: on grids beyond L2, HBM and the latency of a plane step; on smaller ones the latency
+// of a plane step alone (15 warps an SM, about 650 instructions per quad and step, a third of the
+// issue slots). Measured per step, against the schedule it replaced (a sweep of the interior
+// tiles, then one-node-per-thread passes over the CPML shell): 512^3 random boxes 1.650 -> 1.385 ms,
+// 256^3 0.302 -> 0.244 ms, 1024 x 1024 x 896 10.4 -> 8.8 ms; against two-pass, 64^3 18.4 -> 11.8 us. One
+// node per thread in the same march ran 2.0 ms at 512^3 (352 instructions per node against about 165).
+// 3 CTAs an SM (128 registers) against 2 (160): 512^3 1.39 / 1.55 ms, 128^3 52 / 61 us, 64^3 11.8 / 10.4 us.
+// All arithmetic is that of yee_common.cuh, so the results equal the two-pass schedule's bits.
+// Every wait on a TMA barrier is bounded: on timeout the kernel records an error in the status
+// word, drains its own copies (again bounded) and exits.
+#define FDTD_RARE __forceinline__  // calls in the slow path would spill the march's state (512^3: 31.0 -> 28.6 ms for 20 steps)
+#include <cuda.h>
+
+#include <algorithm>
+
+#include "planner.h"
+#include "tma.cuh"
+#include "yee_common.cuh"
+#include "yee_kernels.h"
+
+namespace fdtd {
+
+namespace {
+
+// Stages of the ring: a third one left less of the SM's memory to L1 and was 12-20 % slower.
+#ifndef FDTD_SWEEP_STAGES
+#define FDTD_SWEEP_STAGES 2
+#endif
+#ifndef FDTD_SWEEP_MIN_BLOCKS
+#define FDTD_SWEEP_MIN_BLOCKS 3
+#endif
+constexpr int TX = kTileX, TY = kSweepRows;
+constexpr int QX = TX / 4;                // quads per row
+constexpr int NOWN = QX * TY;             // threads with a quad of the tile; then the halo row and column
+constexpr int NTH = NOWN + (QX + TY + 31) / 32 * 32;
+static_assert(NOWN % 32 == 0, "own quads fill whole warps");
+constexpr int NST = FDTD_SWEEP_STAGES;    // planes in the ring
+constexpr int round128(int b) { return (b + 127) / 128 * 128; }
+// Tiles in shared memory. H and coefficient rows, with rows of W: x in [x0-4, x0+36), y in
+// [y0-1, y0+TY] and x in [x0, x0+40), y in [y0, y0+TY]; old and new E, with rows of WE: x in
+// [x0, x0+36), y in [y0, y0+TY].
+constexpr int W = TX + 8, WE = TX + 4, HR = TY + 2, ER = TY + 1;
+constexpr int H_BYTES = round128(W * HR * 4), E_BYTES = round128(WE * ER * 4), M_BYTES = round128(W * ER * 2);
+constexpr int STAGE_BYTES = 3 * H_BYTES + 3 * E_BYTES + M_BYTES;
+constexpr unsigned H_TX = W * HR * 4, E_TX = WE * ER * 4, M_TX = W * ER * 2;  // bytes the boxes carry
+constexpr int HF = H_BYTES / 4, EF = E_BYTES / 4;
+constexpr int H_OFF = W + 4, E_OFF = 3 * HF;  // float offsets in a stage of a tile node 0's Hx and Ex
+constexpr int NF = WE * ER;               // floats of one new-E component plane
+// CPML memory of a thread's quad on its y face, or its z face where it lies in no y slab, fetched one
+// plane ahead (cp.async): E arrays 0 and 1, H arrays 0 and 1
+enum { kPsiE = 0, kPsiH = 2, kPsiSlots = 4 };
+
+// Where the CPML memory of a plane of a z face begins: E array 0 of node (0, 0) at base, the face's
+// other arrays `stride` apart (E1, H0, H1). on = 0: the plane lies in no z slab.
+template <typename Idx>
+struct __align__(16) PsiAt {
+    Idx base, stride, on, pad;
+};
+
+template <typename Idx>
+struct SweepSmem {
+    unsigned char stage[NST][STAGE_BYTES];  // H (3), old E (3), rows of a plane
+    float enew[2][3][NF];                   // new E of planes k - 1, k
+    float4 psi[kPsiSlots][NTH];
+    float xe[4][W], xh[4][W];               // curl 0, curl 1, b, a of each column, E and H
+    float4 ye[ER], yh[ER];                  // {curl 0, curl 1, b, a} of each row / plane
+    float4 ze[kMaxSweepPlanes], zh[kMaxSweepPlanes];
+    PsiAt<Idx> zo[kMaxSweepPlanes];
+    uint64_t bar[NST];
+};
+
+__device__ __forceinline__ const float* f32(const unsigned char* b) { return reinterpret_cast<const float*>(b); }
+
+// The kernel's parameters, in constant memory.
+struct SweepArgs {
+    FusedMaps maps;
+    StepParams p;
+    FieldPtrs fo;
+    PsiSet pin, pout;
+    SweepPlan sg;
+    long long m;
+    FieldPtrs fi;
+    const ProbeAt* probes;  // probes outside the CPML slabs (n of them), sampled one step late: see k_sweep
+    int n_probes_at;
+    int late;               // the step before this one belongs to the same call
+    float sig[kSweepSources];  // this step's signal of each source
+};
+
+// Slow path, out of line: nodes on the general path (lumped edges, plates, design nodes, probes,
+// keys beyond the table), nodes of another material than the background in a CPML slab, and H faces
+// of such nodes on the low walls. bits: 1 E(k), 2 H(k-1), 4 a node of the tile (stored, probes
+// sampled), 8 E(k) is this chunk's. Old H of plane k - 1 and the node's row there come with the
+// call, the rest from the shared-memory tiles.
+template <typename Idx>
+__device__ __forceinline__ void slow_node(const SweepArgs* pa, SweepSmem<Idx>* ps, int bits, int k, int stage, int i, int j,
+                                       int t, int te, float hxp, float hyp, float hzp, int cp) {
+    const StepParams& p = pa->p;
+    const FieldPtrs& fo = pa->fo;
+    SweepSmem<Idx>& S = *ps;
+    const float* T = f32(S.stage[stage]) + t;
+    const float* TE = f32(S.stage[stage]) + E_OFF + te;
+    float* en = &S.enew[k & 1][0][te];
+    const float* ep = &S.enew[(k - 1) & 1][0][te];
+    const long long R = p.g.pitch, PL = p.g.plane, m = pa->m, rr = m % p.ring_cap;
+    const bool own = bits & 4, store_e = bits & 8;
+    float out[3], pre[3];
+    if (bits & 1) {
+        const float *H0 = T + H_OFF, *H1 = H0 + HF, *H2 = H1 + HF;
+        EDiff d;
+        d.dHz_j = __fsub_rn(H2[0], H2[-W]);
+        d.dHx_j = __fsub_rn(H0[0], H0[-W]);
+        d.dHy_k = __fsub_rn(H1[0], hyp);
+        d.dHx_k = __fsub_rn(H0[0], hxp);
+        d.dHz_i = __fsub_rn(H2[0], H2[-1]);
+        d.dHy_i = __fsub_rn(H1[0], H1[-1]);
+        const int c = reinterpret_cast<const uint16_t*>(S.stage[stage] + 3 * H_BYTES + 3 * E_BYTES)[t];
+        const long long n = (long long)k * PL + (long long)j * R + i;
+        ENbr nb{};
+        nb.ex = TE[0]; nb.ey = TE[EF]; nb.ez = TE[2 * EF];
+        const PsiIO io{pa->pin.f, pa->pout.f, own && store_e};
+        if (c < kRecGeneral) {
+            e_update_diff<false, false, false, false, 7, true>(p, nb, d, i, j, k, m, false, io, out, pre, nullptr, c);
+        } else {
+            const uint8_t* mat = p.mat;
+            nb.m0 = mat[n];
+            nb.mi = i > 0 ? mat[n - 1] : 0;
+            nb.mj = j > 0 ? mat[n - R] : 0;
+            nb.mk = k > 0 ? mat[n - PL] : 0;
+            nb.mij = (i > 0 && j > 0) ? mat[n - 1 - R] : 0;
+            nb.mik = (i > 0 && k > 0) ? mat[n - 1 - PL] : 0;
+            nb.mjk = (j > 0 && k > 0) ? mat[n - R - PL] : 0;
+            const bool lumped = p.lumped_k[k] < p.lumped_k[k + 1];
+            e_update_diff<true, false, true, false, 7>(p, nb, d, i, j, k, m, lumped, io, out, pre);
+            if (own && store_e && p.probe_k[k] < p.probe_k[k + 1])
+                for (int a = 0; a < 3; ++a) sample(p, rr, a, i, j, k, pre[a]);
+        }
+        en[0] = out[0]; en[NF] = out[1]; en[2 * NF] = out[2];
+        if (own && store_e) { fo.ex[n] = out[0]; fo.ey[n] = out[1]; fo.ez[n] = out[2]; }
+    }
+    if (!(bits & 2)) return;
+    const int kh = k - 1;
+    HNbr nb{};
+    nb.hx = hxp; nb.hy = hyp; nb.hz = hzp;
+    HDiff f;
+    f.dEy_k = __fsub_rn(en[NF], ep[NF]);
+    f.dEx_k = __fsub_rn(en[0], ep[0]);
+    f.dEz_j = __fsub_rn(ep[2 * NF + WE], ep[2 * NF]);
+    f.dEx_j = __fsub_rn(ep[WE], ep[0]);
+    f.dEz_i = __fsub_rn(ep[2 * NF + 1], ep[2 * NF]);
+    f.dEy_i = __fsub_rn(ep[NF + 1], ep[NF]);
+    const long long n = (long long)kh * PL + (long long)j * R + i;
+    const PsiIO io{pa->pin.f, pa->pout.f, true};
+    if (cp < kRecGeneral) {
+        h_update_diff<false, false, 7, true>(p, nb, f, i, j, kh, io, out, pre, nullptr, cp);
+    } else {
+        const uint8_t* mat = p.mat;
+        nb.m0 = mat[n];
+        nb.mi = i > 0 ? mat[n - 1] : 0;
+        nb.mj = j > 0 ? mat[n - R] : 0;
+        nb.mk = kh > 0 ? mat[n - PL] : 0;
+        h_update_diff<false, false, 7>(p, nb, f, i, j, kh, io, out, pre);
+        if (p.probe_k[kh] < p.probe_k[kh + 1])
+            for (int a = 0; a < 3; ++a) sample(p, rr, 3 + a, i, j, kh, pre[a]);
+    }
+    fo.hx[n] = out[0]; fo.hy[n] = out[1]; fo.hz[n] = out[2];
+}
+
+__device__ __forceinline__ void sample_at(const ProbeAt& r, const FieldPtrs& f, const StepParams& p, long long m) {
+    const float* c[6] = {f.ex, f.ey, f.ez, f.hx, f.hy, f.hz};
+    const float* a = c[0];
+#pragma unroll
+    for (int q = 1; q < 6; ++q)
+        if (r.comp == q) a = c[q];
+    p.probe_ring[m % p.ring_cap * p.n_probes + r.id] = a[r.node];
+}
+
+struct Quad {
+    float v[4];
+};
+__device__ __forceinline__ Quad lds4(const float* a) {
+    const float4 f = *reinterpret_cast<const float4*>(a);
+    return Quad{f.x, f.y, f.z, f.w};
+}
+__device__ __forceinline__ Quad ldg4(const float* a) {
+    const float4 f = __ldg(reinterpret_cast<const float4*>(a));
+    return Quad{f.x, f.y, f.z, f.w};
+}
+__device__ __forceinline__ void st4(float* a, const Quad& q) {
+    *reinterpret_cast<float4*>(a) = make_float4(q.v[0], q.v[1], q.v[2], q.v[3]);
+}
+// The nodes of a mask (bit r: node r) to a[0 .. 3] (and b, c).
+__device__ __forceinline__ void st_mask3(float* a, float* b, float* c, const Quad& x, const Quad& y, const Quad& z, int mask) {
+    if (mask == 15) {
+        st4(a, x); st4(b, y); st4(c, z);
+    } else {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            if (mask >> r & 1) { a[r] = x.v[r]; b[r] = y.v[r]; c[r] = z.v[r]; }
+    }
+}
+__device__ __forceinline__ void st_mask2(float* a, float* b, const Quad& x, const Quad& y, int ma, int mb) {
+    if ((ma & mb) == 15) {
+        st4(a, x); st4(b, y);
+    } else {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            if (ma >> r & 1) a[r] = x.v[r];
+            if (mb >> r & 1) b[r] = y.v[r];
+        }
+    }
+}
+__device__ __forceinline__ float pick(const Quad& q, int r) { return r == 0 ? q.v[0] : r == 1 ? q.v[1] : r == 2 ? q.v[2] : q.v[3]; }
+
+__device__ __forceinline__ void cp_async16(float4* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(saddr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ Quad quad_of(const float4& f) { return Quad{f.x, f.y, f.z, f.w}; }
+
+// The march of one thread's quad at tile row `row`, first column `col`. kEdge: the tile (halo
+// included) meets a CPML slab or a wall in x (wx) or y (wy), or the chunk one in z; without it no
+// node does. kMat: rows other than the background's lie in a slab or on a low wall (without it the
+// few that may, beside general nodes, take the slow path).
+template <typename Idx, bool kEdge, bool kMat>
+__device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int x0, int y0, int k0, int k1, int row,
+                                      int col, bool own, bool wx, bool wy) {
+    const StepParams& p = A.p;
+    const DeviceGrid& g = p.g;
+    const FieldPtrs& fo = A.fo;
+    const BgNode& B = p.bgn;
+    const float* const pin = A.pin.base;
+    float* const pout = A.pout.base;
+    const int i = x0 + col, j = y0 + row, t = row * W + col, te = row * WE + col, kfirst = k0 - 1;
+    // nodes of the quad (bit r) in the grid, below the high x wall, off both x walls, in an x slab
+    int in4 = 15, lt4 = 15, in_x = 15, xs = 0, xslow = 0;
+    bool ylt = true, yin = true, ys = false;
+    Idx qx = 0, sx = 0, dx = 0, qy = 0, sy = 0, dy = 0;  // CPML memory of the x and y faces at plane k (advanced with it):
+                                                       // E array 0 of the first node, the arrays' stride, the planes'
+    if (kEdge) {
+        if (wx) {
+            in4 = i + 4 <= g.nx ? 15 : i < g.nx ? (1 << (g.nx - i)) - 1 : 0;
+            lt4 = i + 4 <= g.nx - 1 ? 15 : i < g.nx - 1 ? (1 << (g.nx - 1 - i)) - 1 : 0;
+            in_x = i > 0 ? lt4 : lt4 & 14;
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                if (in_slab(i + r, g.nx, g.pxn, g.pxp)) xs |= 1 << r;
+        }
+        if (j >= g.ny) in4 = 0;
+        xs &= in4;
+        // a quad that meets both x slabs: the high side's nodes take the slow path
+        if (xs && i < g.pxn && i + 3 >= g.nx - g.pxp) {
+            xslow = xs & ~((1 << max(0, min(4, g.pxn - i))) - 1);
+            xs &= ~xslow;
+        }
+        ylt = j < g.ny - 1;
+        yin = j > 0 && ylt;
+        ys = wy && in4 && in_slab(j, g.ny, g.pyn, g.pyp);
+        if (xs) {
+            const bool lo = i < g.pxn;
+            const int w = lo ? g.pxn : g.pxp;
+            sx = (Idx)p.psi_stride[lo ? 0 : 1];
+            dx = (Idx)g.ny * (Idx)w;
+            qx = (Idx)p.psi_off[lo ? 0 : 1] + (Idx)k0 * dx + (Idx)j * (Idx)w + (Idx)(lo ? i : i - (g.nx - g.pxp));
+        }
+        if (ys) {
+            const bool lo = j < g.pyn;
+            const int w = lo ? g.pyn : g.pyp;
+            sy = (Idx)p.psi_stride[lo ? 2 : 3];
+            dy = (Idx)w * (Idx)g.pitch;
+            qy = (Idx)p.psi_off[lo ? 2 : 3] + (Idx)k0 * dy + (Idx)(lo ? j : j - (g.ny - g.pyp)) * (Idx)g.pitch + (Idx)i;
+        }
+    }
+    own = own && in4;
+    const Idx nij = (Idx)j * (Idx)g.pitch + (Idx)i;
+    Idx n = (Idx)k0 * (Idx)g.plane + nij;
+    const int bgm = p.bg.mat;
+    float4* const ps = &S.psi[0][threadIdx.x];
+
+    auto issue = [&](int k, int s) {
+        unsigned char* d = S.stage[s];
+        mbar_expect_tx(&S.bar[s], 3 * H_TX + 3 * E_TX + M_TX);
+        for (int c = 0; c < 3; ++c) tma_load_3d(d + c * H_BYTES, &A.maps.h[c], &S.bar[s], x0 - 4, y0 - 1, k);
+        for (int c = 0; c < 3; ++c) tma_load_3d(d + 3 * H_BYTES + c * E_BYTES, &A.maps.e[c], &S.bar[s], x0, y0, k);
+        tma_load_3d(d + 3 * H_BYTES + 3 * E_BYTES, &A.maps.rec, &S.bar[s], x0, y0, k);
+    };
+    // Fetch the old CPML memory of E(k) and H(k-1) into the thread's slots (qk: its y face's offset at plane k).
+    auto fetch_psi = [&](int k, Idx qk) {
+        if (ys) {
+            cp_async16(ps + kPsiE * NTH, pin + qk);
+            cp_async16(ps + (kPsiE + 1) * NTH, pin + qk + sy);
+            if (own && k > k0) {
+                cp_async16(ps + kPsiH * NTH, pin + qk - dy + 2 * sy);
+                cp_async16(ps + (kPsiH + 1) * NTH, pin + qk - dy + 3 * sy);
+            }
+        } else {
+            const PsiAt<Idx> z = S.zo[k - kfirst], zh = S.zo[k - 1 - kfirst];
+            if (z.on && in4) {
+                cp_async16(ps + kPsiE * NTH, pin + z.base + nij);
+                cp_async16(ps + (kPsiE + 1) * NTH, pin + z.base + nij + z.stride);
+            }
+            if (zh.on && own && k > k0) {
+                cp_async16(ps + kPsiH * NTH, pin + zh.base + nij + 2 * zh.stride);
+                cp_async16(ps + (kPsiH + 1) * NTH, pin + zh.base + nij + 3 * zh.stride);
+            }
+        }
+        cp_async_commit();
+    };
+    if (kEdge) fetch_psi(k0, qy);
+    // plane k0 - 1: only its Hx and Hy are needed (loaded by the kernel into stage 0)
+    bool ok = mbar_wait(&S.bar[0], 0);
+    Quad hxp = lds4(f32(S.stage[0]) + t + H_OFF), hyp = lds4(f32(S.stage[0]) + t + H_OFF + HF);  // old H of plane k - 1
+    Quad hzp{};
+    uint2 cp = make_uint2(0, 0);  // the nodes' rows there
+    int s = 1;
+    uint32_t parity = 0;  // of stage s
+#pragma unroll 1
+    for (int k = k0;; ++k) {
+        if (__syncthreads_or(!ok)) {
+            // a plane never arrived: record it, wait (bounded) for the copies still in flight, exit
+            if (kEdge) cp_async_wait_all();
+            if (threadIdx.x == 0) {
+                atomic_flag(p.status, 1);
+                int r = s;
+                uint32_t par = parity;
+                for (int q = k; q <= min(k1, k + NST - 2); ++q) {
+                    mbar_wait(&S.bar[r], par);
+                    if (++r == NST) { r = 0; par ^= 1u; }
+                }
+            }
+            __syncthreads();
+            return;
+        }
+        if (k > k1) return;
+        if (threadIdx.x == 0 && k + NST - 1 <= k1) {
+            fence_proxy_async();  // generic reads of the recycled stage precede the async writes
+            issue(k + NST - 1, s == 0 ? NST - 1 : s - 1);
+        }
+        const int q = k - kfirst;
+        const bool store_e = own && k < k1;
+        bool zs = false, zsh = false, kin = true, klt = true, klh = true;
+        if (kEdge) {
+            zs = S.zo[q].on && in4;
+            zsh = S.zo[q - 1].on;
+            klt = k < g.nz - 1;
+            klh = k - 1 < g.nz - 1;
+            kin = k > 0 && klt;
+        }
+        const float* T = f32(S.stage[s]) + t;
+        const float* TE = f32(S.stage[s]) + E_OFF + te;
+        float* en = &S.enew[k & 1][0][te];
+        const float* ep = &S.enew[(k - 1) & 1][0][te];
+        float xq0[4], xq1[4];
+        if (kEdge && xs) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                if (xs >> r & 1) {
+                    xq0[r] = __ldg(pin + (qx + r));
+                    xq1[r] = __ldg(pin + (qx + sx + r));
+                }
+        }
+        ok = mbar_wait(&S.bar[s], parity);
+        const Quad hx = lds4(T + H_OFF), hy = lds4(T + H_OFF + HF), hz = lds4(T + H_OFF + 2 * HF);
+        const uint2 cw = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(S.stage[s] + 3 * H_BYTES + 3 * E_BYTES) + t);
+        Quad vx, vy, vz;
+        int slow = 0;  // nodes on the slow path: bits 0-3 E(k), bits 4-7 H(k-1)
+        // ---- E(k) ----
+        {
+            const Quad hzj = lds4(T + H_OFF + 2 * HF - W), hxj = lds4(T + H_OFF - W);
+            const float hzi = T[H_OFF + 2 * HF - 1], hyi = T[H_OFF + HF - 1];
+            vx = lds4(TE); vy = lds4(TE + EF); vz = lds4(TE + 2 * EF);
+            float ce[6];  // the nodes' factors of the CPML memory
+            if (kEdge) {
+#pragma unroll
+                for (int r = 0; r < 6; ++r) ce[r] = B.ce[r];
+            }
+            const int c0 = (int)(cw.x & 0xffffu);
+            if (cw.x == cw.y && cw.x == (uint32_t)c0 * 0x10001u && c0 < p.src_row0 &&
+                !(kEdge && (xslow || (!kMat && c0 != bgm && (xs || ys || zs))))) {
+                // one row for the quad
+                float4 a = make_float4(B.ea[0], B.ec[0], B.ec[1], 0.f), b = make_float4(B.ea[1], B.ec[2], B.ec[3], 0.f);
+                float4 d = make_float4(B.ea[2], B.ec[4], B.ec[5], 0.f);
+                if (c0 != bgm) {
+                    const MatCoef* mc = p.coef + c0;
+                    a = __ldg(&mc->e[0]); b = __ldg(&mc->e[1]); d = __ldg(&mc->e[2]);
+                    if (kEdge && kMat) {  // its factors of the CPML memory
+                        ce[0] = __fmul_rn(b.z, g.dx); ce[1] = __fmul_rn(d.y, g.dx);
+                        ce[2] = __fmul_rn(a.y, g.dy); ce[3] = __fmul_rn(d.z, g.dy);
+                        ce[4] = __fmul_rn(a.z, g.dz); ce[5] = __fmul_rn(b.y, g.dz);
+                    }
+                }
+                Quad x0c = {b.z, b.z, b.z, b.z}, x1c = {d.y, d.y, d.y, d.y};
+                if (kEdge && (xs || ys || zs)) {  // curl coefficients along a slab's axis, over kappa
+                    if (!kMat || c0 == bgm) {
+                        if (ys) { a.y = S.ye[row].x; d.z = S.ye[row].y; }
+                        if (zs) { a.z = S.ze[q].x; b.y = S.ze[q].y; }
+                        if (xs) { x0c = lds4(&S.xe[0][col]); x1c = lds4(&S.xe[1][col]); }
+                    } else {
+                        if (ys) { const float kap = __ldg(p.key + j); a.y = __fdiv_rn(a.y, kap); d.z = __fdiv_rn(d.z, kap); }
+                        if (zs) { const float kap = __ldg(p.kez + k); a.z = __fdiv_rn(a.z, kap); b.y = __fdiv_rn(b.y, kap); }
+#pragma unroll
+                        for (int r = 0; r < 4; ++r)
+                            if (xs >> r & 1) {
+                                const float kap = __ldg(p.kex + i + r);
+                                x0c.v[r] = __fdiv_rn(x0c.v[r], kap);
+                                x1c.v[r] = __fdiv_rn(x1c.v[r], kap);
+                            }
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    vx.v[r] = upd3(a.x, vx.v[r], a.y, __fsub_rn(hz.v[r], hzj.v[r]), a.z, __fsub_rn(hy.v[r], hyp.v[r]));
+                    vy.v[r] = upd3(b.x, vy.v[r], b.y, __fsub_rn(hx.v[r], hxp.v[r]), x0c.v[r], __fsub_rn(hz.v[r], r ? hz.v[r - 1] : hzi));
+                    vz.v[r] = upd3(d.x, vz.v[r], x1c.v[r], __fsub_rn(hy.v[r], r ? hy.v[r - 1] : hyi), d.z, __fsub_rn(hx.v[r], hxj.v[r]));
+                }
+            } else {
+                // rows per node; in a slab only background nodes, which take the slab's curl coefficients
+                int cur = -1;
+                float4 a{}, b{}, d{};
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const int c = (int)((r < 2 ? cw.x : cw.y) >> (16 * (r & 1)) & 0xffffu);
+                    const bool x = kEdge && (xs >> r & 1);
+                    if (c >= kRecGeneral || (kEdge && ((c != bgm && (ys || zs || x)) || (xslow >> r & 1)))) {
+                        slow |= 1 << r;
+                        continue;
+                    }
+                    if (c != cur) {
+                        const MatCoef* mc = p.coef + c;
+                        a = __ldg(&mc->e[0]); b = __ldg(&mc->e[1]); d = __ldg(&mc->e[2]);
+                        cur = c;
+                        if (kEdge && ys) { a.y = S.ye[row].x; d.z = S.ye[row].y; }
+                        if (kEdge && zs) { a.z = S.ze[q].x; b.y = S.ze[q].y; }
+                    }
+                    vx.v[r] = upd3(a.x, vx.v[r], a.y, __fsub_rn(hz.v[r], hzj.v[r]), a.z, __fsub_rn(hy.v[r], hyp.v[r]));
+                    vy.v[r] = upd3(b.x, vy.v[r], b.y, __fsub_rn(hx.v[r], hxp.v[r]), x ? S.xe[0][col + r] : b.z,
+                                   __fsub_rn(hz.v[r], r ? hz.v[r - 1] : hzi));
+                    vz.v[r] = upd3(d.x, vz.v[r], x ? S.xe[1][col + r] : d.y, __fsub_rn(hy.v[r], r ? hy.v[r - 1] : hyi), d.z,
+                                   __fsub_rn(hx.v[r], hxj.v[r]));
+                    if (c >= p.src_row0) {  // lumped source edge (fdtdrav.h:728)
+                        const SrcRow sr = p.src_rows[c - p.src_row0];
+                        vz.v[r] = __fmaf_rn(sr.cezj, A.sig[sr.source], vz.v[r]);
+                    }
+                }
+                slow &= in4;
+                if (kEdge && k >= g.nz) slow = 0;
+            }
+            if (kEdge) {
+                cp_async_wait_all();
+                const bool wall = in_x != 15 || !yin || !kin;
+                int mx = 15, my = 15, mz = 15;
+                if (wall) {
+                    mx = yin && kin ? lt4 : 0;
+                    my = ylt && kin ? in_x : 0;
+                    mz = yin && klt ? in_x : 0;
+                }
+                const int st = store_e ? in4 & ~slow : 0;
+                if (xs) {  // fdtdrav.h:752-785
+                    const Quad b = lds4(&S.xe[2][col]), c = lds4(&S.xe[3][col]);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        if (xs >> r & 1) {
+                            xq0[r] = psi_upd(b.v[r], xq0[r], c.v[r], __fsub_rn(hz.v[r], r ? hz.v[r - 1] : hzi));
+                            xq1[r] = psi_upd(b.v[r], xq1[r], c.v[r], __fsub_rn(hy.v[r], r ? hy.v[r - 1] : hyi));
+                            if (st & my & (1 << r)) pout[qx + r] = xq0[r];
+                            if (st & mz & (1 << r)) pout[qx + sx + r] = xq1[r];
+                            vy.v[r] = psi_add(vy.v[r], ce[0], xq0[r]);
+                            vz.v[r] = psi_add(vz.v[r], ce[1], xq1[r]);
+                        }
+                }
+                if (ys) {  // fdtdrav.h:790-827
+                    const float b = S.ye[row].z, c = S.ye[row].w;
+                    Quad u = quad_of(ps[kPsiE * NTH]), w = quad_of(ps[(kPsiE + 1) * NTH]);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        u.v[r] = psi_upd(b, u.v[r], c, __fsub_rn(hz.v[r], hzj.v[r]));
+                        w.v[r] = psi_upd(b, w.v[r], c, __fsub_rn(hx.v[r], hxj.v[r]));
+                        vx.v[r] = psi_add(vx.v[r], ce[2], u.v[r]);
+                        vz.v[r] = psi_add(vz.v[r], ce[3], w.v[r]);
+                    }
+                    st_mask2(pout + qy, pout + qy + sy, u, w, st & mx, st & mz);
+                }
+                if (zs) {  // fdtdrav.h:829-911
+                    const float b = S.ze[q].z, c = S.ze[q].w;
+                    const Idx at = S.zo[q].base + nij;
+                    Quad u, w;
+                    if (ys) { u = ldg4(pin + at); w = ldg4(pin + at + S.zo[q].stride); }
+                    else { u = quad_of(ps[kPsiE * NTH]); w = quad_of(ps[(kPsiE + 1) * NTH]); }
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        u.v[r] = psi_upd(b, u.v[r], c, __fsub_rn(hy.v[r], hyp.v[r]));
+                        w.v[r] = psi_upd(b, w.v[r], c, __fsub_rn(hx.v[r], hxp.v[r]));
+                        vx.v[r] = psi_add(vx.v[r], ce[4], u.v[r]);
+                        vy.v[r] = psi_add(vy.v[r], ce[5], w.v[r]);
+                    }
+                    st_mask2(pout + at, pout + at + S.zo[q].stride, u, w, st & mx, st & my);
+                }
+                if (wall) {  // components the walls keep
+                    const Quad ex = lds4(TE), ey = lds4(TE + EF), ez = lds4(TE + 2 * EF);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        if (!(mx >> r & 1)) vx.v[r] = ex.v[r];
+                        if (!(my >> r & 1)) vy.v[r] = ey.v[r];
+                        if (!(mz >> r & 1)) vz.v[r] = ez.v[r];
+                    }
+                }
+            }
+        }
+        st4(en, vx);
+        st4(en + NF, vy);
+        st4(en + 2 * NF, vz);
+        if (store_e) {
+            const int st = in4 & ~slow;
+            st_mask3(fo.ex + n, fo.ey + n, fo.ez + n, vx, vy, vz, st);
+        }
+        // ---- H(k-1) ----
+        if (k > k0 && own) {
+            const int kh = k - 1;
+            const Idx gx = qx - dx + 2 * sx;
+            if (kEdge && xs) {
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+                    if (xs >> r & 1) {
+                        xq0[r] = __ldg(pin + (gx + r));
+                        xq1[r] = __ldg(pin + (gx + sx + r));
+                    }
+            }
+            // differences of E: along z, y and x
+            const Quad ex = lds4(ep), ey = lds4(ep + NF), ez = lds4(ep + 2 * NF);
+            const Quad ezj = lds4(ep + 2 * NF + WE), exj = lds4(ep + WE);
+            const float ezi = ep[2 * NF + 4], eyi = ep[NF + 4];
+            const bool low_jk = kEdge && (j == 0 || kh == 0);  // faces on a low wall take the default entry
+            float ch[6];  // the nodes' factors of the CPML memory
+            if (kEdge) {
+#pragma unroll
+                for (int r = 0; r < 6; ++r) ch[r] = B.ch[r];
+            }
+            Quad ux = hxp, uy = hyp, uz = hzp;
+            const int c0 = (int)(cp.x & 0xffffu);
+            const bool table = c0 == bgm && (!low_jk || B.low_ok);  // the tabulated coefficients apply
+            if (cp.x == cp.y && cp.x == (uint32_t)c0 * 0x10001u && c0 < kRecGeneral &&
+                !(kEdge && (xslow || (i == 0 && (c0 != bgm || !B.low_ok)) || (!kMat && !table && (xs || ys || zsh || low_jk))))) {
+                float4 a = make_float4(B.ha[0], B.hc[0], B.hc[1], 0.f), b = make_float4(B.ha[1], B.hc[2], B.hc[3], 0.f);
+                float4 d = make_float4(B.ha[2], B.hc[4], B.hc[5], 0.f);
+                if (!table) {
+                    const MatCoef *mc = p.coef + c0, *md = p.coef + kDefaultEntry;
+                    a = __ldg(&mc->h[0]); b = __ldg(kEdge && kMat && j == 0 ? &md->h[1] : &mc->h[1]);
+                    d = __ldg(kEdge && kMat && kh == 0 ? &md->h[2] : &mc->h[2]);
+                    if (kEdge && kMat) {
+                        ch[0] = __fmul_rn(b.y, g.dx); ch[1] = __fmul_rn(d.z, g.dx);
+                        ch[2] = __fmul_rn(a.z, g.dy); ch[3] = __fmul_rn(d.y, g.dy);
+                        ch[4] = __fmul_rn(a.y, g.dz); ch[5] = __fmul_rn(b.z, g.dz);
+                    }
+                }
+                Quad x0c = {b.y, b.y, b.y, b.y}, x1c = {d.z, d.z, d.z, d.z};
+                if (kEdge && (xs || ys || zsh)) {
+                    if (!kMat || table) {
+                        if (ys) { a.z = S.yh[row].x; d.y = S.yh[row].y; }
+                        if (zsh) { a.y = S.zh[q - 1].x; b.z = S.zh[q - 1].y; }
+                        if (xs) { x0c = lds4(&S.xh[0][col]); x1c = lds4(&S.xh[1][col]); }
+                    } else {
+                        if (ys) { const float kap = __ldg(p.kmy + j); a.z = __fdiv_rn(a.z, kap); d.y = __fdiv_rn(d.y, kap); }
+                        if (zsh) { const float kap = __ldg(p.kmz + kh); a.y = __fdiv_rn(a.y, kap); b.z = __fdiv_rn(b.z, kap); }
+#pragma unroll
+                        for (int r = 0; r < 4; ++r)
+                            if (xs >> r & 1) {
+                                const float kap = __ldg(p.kmx + i + r);
+                                x0c.v[r] = __fdiv_rn(x0c.v[r], kap);
+                                x1c.v[r] = __fdiv_rn(x1c.v[r], kap);
+                            }
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    ux.v[r] = upd3_hx(a.x, ux.v[r], a.y, __fsub_rn(vy.v[r], ey.v[r]), a.z, __fsub_rn(ezj.v[r], ez.v[r]));
+                    uy.v[r] = upd3(b.x, uy.v[r], x0c.v[r], __fsub_rn(r < 3 ? ez.v[r + 1] : ezi, ez.v[r]), b.z, __fsub_rn(vx.v[r], ex.v[r]));
+                    uz.v[r] = upd3(d.x, uz.v[r], d.y, __fsub_rn(exj.v[r], ex.v[r]), x1c.v[r], __fsub_rn(r < 3 ? ey.v[r + 1] : eyi, ey.v[r]));
+                }
+            } else {
+                int cur = -1;
+                float4 a{}, b{}, d{};
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const int c = (int)((r < 2 ? cp.x : cp.y) >> (16 * (r & 1)) & 0xffffu);
+                    const bool x = kEdge && (xs >> r & 1), lw = kEdge && (low_jk || (r == 0 && i == 0));
+                    if (c >= kRecGeneral ||
+                        (kEdge && ((c != bgm && (ys || zsh || x || lw)) || (lw && !B.low_ok) || (xslow >> r & 1)))) {
+                        slow |= 16 << r;
+                        continue;
+                    }
+                    if (c != cur) {
+                        const MatCoef* mc = p.coef + c;
+                        a = __ldg(&mc->h[0]); b = __ldg(&mc->h[1]); d = __ldg(&mc->h[2]);
+                        cur = c;
+                        if (kEdge && ys) { a.z = S.yh[row].x; d.y = S.yh[row].y; }
+                        if (kEdge && zsh) { a.y = S.zh[q - 1].x; b.z = S.zh[q - 1].y; }
+                    }
+                    ux.v[r] = upd3_hx(a.x, ux.v[r], a.y, __fsub_rn(vy.v[r], ey.v[r]), a.z, __fsub_rn(ezj.v[r], ez.v[r]));
+                    uy.v[r] = upd3(b.x, uy.v[r], x ? S.xh[0][col + r] : b.y, __fsub_rn(r < 3 ? ez.v[r + 1] : ezi, ez.v[r]), b.z,
+                                   __fsub_rn(vx.v[r], ex.v[r]));
+                    uz.v[r] = upd3(d.x, uz.v[r], d.y, __fsub_rn(exj.v[r], ex.v[r]), x ? S.xh[1][col + r] : d.z,
+                                   __fsub_rn(r < 3 ? ey.v[r + 1] : eyi, ey.v[r]));
+                }
+                slow &= in4 | in4 << 4;
+            }
+            slow |= (slow & 15) << 4;  // H(k-1) of a node whose E(k) is still to come
+            const int st = in4 & ~(slow >> 4);
+            if (kEdge) {
+                int mx = 15, my = 15, mz = 15;
+                const bool wall = lt4 != 15 || !ylt || !klh;
+                if (wall) {
+                    mx = ylt && klh ? 15 : 0;
+                    my = klh ? lt4 : 0;
+                    mz = ylt ? lt4 : 0;
+                }
+                if (xs) {  // fdtdrav.h:401-442
+                    const Quad b = lds4(&S.xh[2][col]), c = lds4(&S.xh[3][col]);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        if (xs >> r & 1) {
+                            xq0[r] = psi_upd(b.v[r], xq0[r], c.v[r], __fsub_rn(r < 3 ? ez.v[r + 1] : ezi, ez.v[r]));
+                            xq1[r] = psi_upd(b.v[r], xq1[r], c.v[r], __fsub_rn(r < 3 ? ey.v[r + 1] : eyi, ey.v[r]));
+                            if (st & my & (1 << r)) pout[gx + r] = xq0[r];
+                            if (st & mz & (1 << r)) pout[gx + sx + r] = xq1[r];
+                            uy.v[r] = psi_add(uy.v[r], ch[0], xq0[r]);
+                            uz.v[r] = psi_add(uz.v[r], ch[1], xq1[r]);
+                        }
+                }
+                if (ys) {  // fdtdrav.h:445-486
+                    const float b = S.yh[row].z, c = S.yh[row].w;
+                    Quad u = quad_of(ps[kPsiH * NTH]), w = quad_of(ps[(kPsiH + 1) * NTH]);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        u.v[r] = psi_upd(b, u.v[r], c, __fsub_rn(ezj.v[r], ez.v[r]));
+                        w.v[r] = psi_upd(b, w.v[r], c, __fsub_rn(exj.v[r], ex.v[r]));
+                        ux.v[r] = psi_add(ux.v[r], ch[2], u.v[r]);
+                        uz.v[r] = psi_add(uz.v[r], ch[3], w.v[r]);
+                    }
+                    const Idx at = qy - dy + 2 * sy;
+                    st_mask2(pout + at, pout + at + sy, u, w, st & mx, st & mz);
+                }
+                if (zsh) {  // fdtdrav.h:489-562
+                    const float b = S.zh[q - 1].z, c = S.zh[q - 1].w;
+                    const Idx sz = S.zo[q - 1].stride, at = S.zo[q - 1].base + nij + 2 * sz;
+                    Quad u, w;
+                    if (ys) { u = ldg4(pin + at); w = ldg4(pin + at + sz); }
+                    else { u = quad_of(ps[kPsiH * NTH]); w = quad_of(ps[(kPsiH + 1) * NTH]); }
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        u.v[r] = psi_upd(b, u.v[r], c, __fsub_rn(vy.v[r], ey.v[r]));
+                        w.v[r] = psi_upd_hyz(b, w.v[r], c, __fsub_rn(vx.v[r], ex.v[r]));
+                        ux.v[r] = psi_add(ux.v[r], ch[4], u.v[r]);
+                        uy.v[r] = psi_add(uy.v[r], ch[5], w.v[r]);
+                    }
+                    st_mask2(pout + at, pout + at + sz, u, w, st & mx, st & my);
+                }
+                if (wall) {
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        if (!(mx >> r & 1)) ux.v[r] = hxp.v[r];
+                        if (!(my >> r & 1)) uy.v[r] = hyp.v[r];
+                        if (!(mz >> r & 1)) uz.v[r] = hzp.v[r];
+                    }
+                }
+            }
+            const Idx nh = n - (Idx)g.plane;
+            st_mask3(fo.hx + nh, fo.hy + nh, fo.hz + nh, ux, uy, uz, st);
+        }
+        if (slow) {
+#pragma unroll 1
+            for (int r = 0; r < 4; ++r) {
+                const int bits = (slow >> r & 1) | (slow >> (3 + r) & 2);
+                if (!bits) continue;
+                const uint32_t c = (r < 2 ? cp.x : cp.y) >> (16 * (r & 1)) & 0xffffu;
+                slow_node<Idx>(&A, &S, bits | (own ? 4 : 0) | (store_e ? 8 : 0), k, s, i + r, j, t + r, te + r, pick(hxp, r), pick(hyp, r),
+                               pick(hzp, r), (int)c);
+            }
+        }
+        hxp = hx; hyp = hy; hzp = hz;
+        cp = cw;
+        n += (Idx)g.plane;
+        if (kEdge) {
+            qx += dx;
+            qy += dy;
+            if (k < k1) fetch_psi(k + 1, qy);
+        }
+        if (++s == NST) { s = 0; parity ^= 1u; }
+    }
+}
+
+}  // namespace
+
+template <typename Idx, bool kMat>
+__global__ void __launch_bounds__(NTH, FDTD_SWEEP_MIN_BLOCKS) k_sweep(const __grid_constant__ SweepArgs A) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    SweepSmem<Idx>& S = *reinterpret_cast<SweepSmem<Idx>*>(smem_raw);
+    const StepParams& p = A.p;
+    const DeviceGrid& g = p.g;
+    const int tid = threadIdx.x;
+    // item: chunk outer, tiles inner (x fastest), so the CTAs in flight work on neighbouring planes
+    int b = blockIdx.x;
+    const int bx = b % A.sg.nbx;
+    b /= A.sg.nbx;
+    const int by = b % A.sg.nby, ch = b / A.sg.nby;
+    const int x0 = bx * TX, y0 = by * TY;
+    const int k0 = A.sg.chunk(ch), k1 = A.sg.chunk(ch + 1);
+    const int kfirst = k0 - 1;  // the planes k0 - 1 .. k1, at most kMaxSweepPlanes (plan_sweep)
+
+    // ---- per-column, per-row and per-plane tables ----
+    if (tid == 0) {
+        for (int q = 0; q < NST; ++q) mbar_init(&S.bar[q], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q = tid; q < W; q += NTH) {
+        const bool in = x0 + q < g.nx;
+        const float4 e = in ? __ldg(p.te[0] + x0 + q) : none, h = in ? __ldg(p.th[0] + x0 + q) : none;
+        S.xe[0][q] = e.x; S.xe[1][q] = e.y; S.xe[2][q] = e.z; S.xe[3][q] = e.w;
+        S.xh[0][q] = h.x; S.xh[1][q] = h.y; S.xh[2][q] = h.z; S.xh[3][q] = h.w;
+    }
+    // (other threads than the ones above where there are enough)
+    for (int r = NTH - 1 - tid; r < ER; r += NTH) {
+        const bool in = y0 + r < g.ny;
+        S.ye[r] = in ? __ldg(p.te[1] + y0 + r) : none;
+        S.yh[r] = in ? __ldg(p.th[1] + y0 + r) : none;
+    }
+    for (int r = (tid + NTH - W) % NTH; r <= k1 - kfirst; r += NTH) {
+        const int q = kfirst + r;
+        const bool in = q >= 0 && q < g.nz;
+        S.ze[r] = in ? __ldg(p.te[2] + q) : none;
+        S.zh[r] = in ? __ldg(p.th[2] + q) : none;
+        PsiAt<Idx> o{0, 0, 0, 0};
+        if (in && in_slab(q, g.nz, g.pzn, g.pzp)) {
+            const bool lo = q < g.pzn;
+            o.base = (Idx)p.psi_off[lo ? 4 : 5] + (Idx)(lo ? q : q - (g.nz - g.pzp)) * (Idx)g.plane;
+            o.stride = (Idx)p.psi_stride[lo ? 4 : 5];
+            o.on = 1;
+        }
+        S.zo[r] = o;
+    }
+    __syncthreads();
+    grid_dependency_wait();  // the previous step wrote what this one reads
+    grid_launch_dependents();
+    if (tid == 0) {
+        mbar_expect_tx(&S.bar[0], 2 * H_TX);
+        for (int c = 0; c < 2; ++c) tma_load_3d(S.stage[0] + c * H_BYTES, &A.maps.h[c], &S.bar[0], x0 - 4, y0 - 1, kfirst);
+        for (int k = k0; k <= min(k1, k0 + NST - 2); ++k) {
+            const int s = 1 + k - k0;
+            unsigned char* d = S.stage[s];
+            mbar_expect_tx(&S.bar[s], 3 * H_TX + 3 * E_TX + M_TX);
+            for (int c = 0; c < 3; ++c) tma_load_3d(d + c * H_BYTES, &A.maps.h[c], &S.bar[s], x0 - 4, y0 - 1, k);
+            for (int c = 0; c < 3; ++c) tma_load_3d(d + 3 * H_BYTES + c * E_BYTES, &A.maps.e[c], &S.bar[s], x0, y0, k);
+            tma_load_3d(d + 3 * H_BYTES + 3 * E_BYTES, &A.maps.rec, &S.bar[s], x0, y0, k);
+        }
+    }
+    // Probes outside the CPML slabs hold the step's final values, so they are read from the finished
+    // fields: here the step before (its fields are this step's input), and after a call's last step by
+    // k_sample_probes. Probes inside a slab are sampled by the slow path, before the CPML correction.
+    if (A.late && blockIdx.x * NTH < (unsigned)A.n_probes_at) {
+        const int q = blockIdx.x * NTH + tid;
+        if (q < A.n_probes_at) sample_at(A.probes[q], A.fi, p, A.m - 1);
+    }
+    // own quads, then those of the halo row and the halo column (spare threads repeat the last one)
+    const bool own = tid < NOWN;
+    const int h = min(tid - NOWN, QX + TY - 1);
+    const int row = own ? tid / QX : h < QX ? TY : h - QX, col = own ? tid % QX * 4 : h < QX ? h * 4 : TX;
+    const bool wx = x0 < max(g.pxn, 1) || x0 + TX >= min(g.nx - g.pxp, g.nx - 1);
+    const bool wy = y0 < max(g.pyn, 1) || y0 + TY >= min(g.ny - g.pyp, g.ny - 1);
+    const bool wz = k0 < max(g.pzn, 1) || k1 >= min(g.nz - g.pzp, g.nz - 1);  // E(k0) .. E(k1), H(k0) .. H(k1 - 1)
+    if (wx || wy || wz) march<Idx, true, kMat>(A, S, x0, y0, k0, k1, row, col, own, wx, wy);
+    else march<Idx, false, kMat>(A, S, x0, y0, k0, k1, row, col, own, false, false);
+}
+
+template <typename Idx>
+constexpr int sweep_smem() { return (int)sizeof(SweepSmem<Idx>); }
+
+template <typename Idx, bool kMat>
+cudaError_t configure() {
+    return cudaFuncSetAttribute(k_sweep<Idx, kMat>, cudaFuncAttributeMaxDynamicSharedMemorySize, sweep_smem<Idx>());
+}
+cudaError_t sweep_configure() {
+    cudaError_t e = configure<uint32_t, false>();
+    if (e == cudaSuccess) e = configure<uint32_t, true>();
+    if (e == cudaSuccess) e = configure<unsigned long long, true>();
+    return e;
+}
+
+__global__ void k_sample_probes(const __grid_constant__ StepParams p, const __grid_constant__ FieldPtrs f,
+                                const ProbeAt* __restrict__ probes, int n, long long m) {
+    grid_dependency_wait();
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < n) sample_at(probes[q], f, p, m);
+}
+
+cudaError_t launch_sample_probes(const StepParams& p, const FieldPtrs& f, const ProbeAt* probes, int n, long long m,
+                                 cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(n + 127) / 128, 1, 1);
+    cfg.blockDim = dim3(128, 1, 1);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_sample_probes, p, f, probes, n, m);
+}
+
+cudaError_t launch_sweep(const FusedMaps& maps, const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fo,
+                         const PsiSet& pin, const PsiSet& pout, const SweepPlan& sg, const SweepStep& ss, long long m,
+                         cudaStream_t st) {
+    SweepArgs args{maps, p, fo, pin, pout, sg, m, fi, ss.probes, ss.n_probes, ss.late, {}};
+    std::copy(ss.sig, ss.sig + kSweepSources, args.sig);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(sg.nbx * sg.nby * sg.chunks()), 1, 1);
+    cfg.blockDim = dim3(NTH, 1, 1);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const bool idx32 = p.g.plane * (long long)(p.g.nz + 1) < (1LL << 31) && p.psi_total < (1LL << 31);
+    cfg.dynamicSmemBytes = idx32 ? sweep_smem<uint32_t>() : sweep_smem<unsigned long long>();
+    if (!idx32) return cudaLaunchKernelEx(&cfg, k_sweep<unsigned long long, true>, args);
+    return ss.mat ? cudaLaunchKernelEx(&cfg, k_sweep<uint32_t, true>, args) : cudaLaunchKernelEx(&cfg, k_sweep<uint32_t, false>, args);
+}
+
+// Tensor maps of the sweep: H tiles with a one-node halo (x from 4 nodes before the tile: a TMA box
+// starts on a 16-byte boundary), old-E and coefficient-row tiles. Coordinates outside the arrays
+// load as zeros.
+int encode_sweep_maps(FusedMaps* out, const DeviceGrid& g, float* const h[3], float* const e[3], const uint16_t* rec,
+                      void* encode_fn) {
+    using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    const EncodeFn encode = reinterpret_cast<EncodeFn>(encode_fn);
+    const cuuint64_t dims[3] = {(cuuint64_t)g.pitch, (cuuint64_t)g.ny, (cuuint64_t)g.nz};
+    const cuuint64_t fstr[2] = {(cuuint64_t)g.pitch * 4, (cuuint64_t)g.plane * 4};
+    const cuuint64_t mstr[2] = {(cuuint64_t)g.pitch * 2, (cuuint64_t)g.plane * 2};
+    const cuuint32_t hbox[3] = {W, HR, 1}, ebox[3] = {WE, ER, 1}, mbox[3] = {W, ER, 1}, es[3] = {1, 1, 1};
+    auto map = [&](CUtensorMap* mp, CUtensorMapDataType t, void* base, const cuuint64_t* str, const cuuint32_t* box) {
+        return encode(mp, t, 3, base, dims, str, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    for (int c = 0; c < 3; ++c)
+        if (!map(&out->h[c], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, h[c], fstr, hbox) ||
+            !map(&out->e[c], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, e[c], fstr, ebox))
+            return -1;
+    return map(&out->rec, CU_TENSOR_MAP_DATA_TYPE_UINT16, const_cast<uint16_t*>(rec), mstr, mbox) ? 0 : -1;
+}
+
+}  // namespace fdtd

@@ -13,18 +13,6 @@ namespace fdtd {
 #ifndef FDTD_TWO_PASS_MIN_BLOCKS
 #define FDTD_TWO_PASS_MIN_BLOCKS 6
 #endif
-#ifndef FDTD_SHELL_MIN_BLOCKS
-#define FDTD_SHELL_MIN_BLOCKS 6
-#endif
-// The shell E pass loads a CPML node's old psi together with its fields (e_node_global's kEarly):
-// measured at 512^3, the fused step 2.2 % faster (256^3: 3.3 %). The shell H pass gains nothing
-// from it, and the two-pass kernels, whose spills it raises, lose 7-9 % at 64^3 and 128^3.
-#ifndef FDTD_SHELL_EARLY_E
-#define FDTD_SHELL_EARLY_E 1
-#endif
-#ifndef FDTD_SHELL_EARLY_H
-#define FDTD_SHELL_EARLY_H 0
-#endif
 template <typename Idx>
 __global__ void __launch_bounds__(256, FDTD_TWO_PASS_MIN_BLOCKS) k_update_e(const __grid_constant__ StepParams p, FieldPtrs f,
                                                   const __grid_constant__ PsiSet ps, long long m) {
@@ -41,90 +29,6 @@ __global__ void __launch_bounds__(256, FDTD_TWO_PASS_MIN_BLOCKS) k_update_h(cons
     const int j = blockIdx.y * 8 + threadIdx.y;
     if (i >= p.g.nx || j >= p.g.ny) return;
     h_node_global<false, Idx>(p, f, f, f, ps, ps, i, j, blockIdx.z, m);
-}
-
-// Shell passes of the fused schedule: the nodes of the shell items (int4 {x0, y0, k, code}: a
-// block of shape s = code & 15 (widths 32, 16, 64, 128, 256, 8, 4, 2, 1; 256 nodes) of which the
-// first (code >> 4) & 511 columns and (code >> 13) & 511 rows are the item's, in planes k ..
-// k + ((code >> 22) & 15)) read buffer A (`fi`,
-// `pin`) and write buffer B (`fo`, `pout`), one node per thread as in the two-pass kernels. The E
-// pass runs before the interior sweep, the H pass after it, since H reads new E at interior nodes
-// next to the shell.
-__device__ __forceinline__ bool shell_node(const int4& it, const DeviceGrid& g, int& i, int& j) {
-    const int s = it.w & 15;
-    const int lw = s == 0 ? 5 : s == 1 ? 4 : s <= 4 ? s + 4 : 8 - s;  // log2 of the block width
-    const int t = (int)(threadIdx.y * 32 + threadIdx.x);
-    const int tx = t & ((1 << lw) - 1), ty = t >> lw;
-    i = it.x + tx;
-    j = it.y + ty;
-    return tx < ((it.w >> 4) & 511) && ty < ((it.w >> 13) & 511) && i < g.nx && j < g.ny;
-}
-
-// One launch per pass covers the four shell lists (yee_kernels.h), which lie one after the other
-// in device memory: a block takes the instantiation of its list, kSlabs = the CPML slabs (bit 0 x,
-// 1 y, 2 z) its nodes may lie in, so the other slab tests compile out of that list's code. One
-// launch, not one per list, since small grids are bound by the chain of launches.
-template <typename Idx, int kSlabs>
-__device__ __forceinline__ void shell_e_item(const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fo,
-                                             const PsiSet& pin, const PsiSet& pout, const int4& it, long long m) {
-    int i, j;
-    if (!shell_node(it, p.g, i, j)) return;
-    for (int k = it.z, k1 = it.z + ((it.w >> 22) & 15); k <= k1; ++k)
-        e_node_global<false, false, false, Idx, kSlabs, FDTD_SHELL_EARLY_E != 0>(p, fi, fo, pin, pout, i, j, k, m);
-}
-template <typename Idx, int kSlabs>
-__device__ __forceinline__ void shell_h_item(const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fo,
-                                             const PsiSet& pin, const PsiSet& pout, const int4& it, long long m) {
-    int i, j;
-    if (!shell_node(it, p.g, i, j)) return;
-    for (int k = it.z, k1 = it.z + ((it.w >> 22) & 15); k <= k1; ++k)
-        h_node_global<false, Idx, kSlabs, FDTD_SHELL_EARLY_H != 0>(p, fi, fo, fo, pin, pout, i, j, k, m);
-}
-
-// e1, e2, e3: the ends of the first three lists in the launch (blocks from e3 on take the fourth).
-template <typename Idx>
-__global__ void __launch_bounds__(256, FDTD_SHELL_MIN_BLOCKS) k_shell_e(const __grid_constant__ StepParams p, FieldPtrs fi, FieldPtrs fo,
-                                                 const __grid_constant__ PsiSet pin, const __grid_constant__ PsiSet pout,
-                                                 const int4* __restrict__ items, int e1, int e2, int e3, long long m) {
-    const int b = blockIdx.x;
-    const int4 it = items[b];
-    if (b < e1) shell_e_item<Idx, 4>(p, fi, fo, pin, pout, it, m);
-    else if (b < e2) shell_e_item<Idx, 6>(p, fi, fo, pin, pout, it, m);
-    else if (b < e3) shell_e_item<Idx, 1>(p, fi, fo, pin, pout, it, m);
-    else shell_e_item<Idx, 7>(p, fi, fo, pin, pout, it, m);
-}
-
-template <typename Idx>
-__global__ void __launch_bounds__(256, FDTD_SHELL_MIN_BLOCKS) k_shell_h(const __grid_constant__ StepParams p, FieldPtrs fi, FieldPtrs fo,
-                                                 const __grid_constant__ PsiSet pin, const __grid_constant__ PsiSet pout,
-                                                 const int4* __restrict__ items, int e1, int e2, int e3, long long m) {
-    const int b = blockIdx.x;
-    const int4 it = items[b];
-    if (b < e1) shell_h_item<Idx, 4>(p, fi, fo, pin, pout, it, m);
-    else if (b < e2) shell_h_item<Idx, 6>(p, fi, fo, pin, pout, it, m);
-    else if (b < e3) shell_h_item<Idx, 1>(p, fi, fo, pin, pout, it, m);
-    else shell_h_item<Idx, 7>(p, fi, fo, pin, pout, it, m);
-}
-
-cudaError_t launch_shell(bool e_pass, const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fo, const PsiSet& pin,
-                         const PsiSet& pout, const ShellWork& w, long long m, cudaStream_t st) {
-    int n = 0;
-    for (int q = 0; q < kShellLists; ++q) {
-        if (q > 0 && w.items[q] != w.items[q - 1] + w.n[q - 1]) return cudaErrorInvalidValue;  // the lists must be contiguous
-        n += w.n[q];
-    }
-    if (n <= 0) return cudaSuccess;
-    const dim3 b(32, 8, 1);
-    const int e1 = w.n[kShellZ], e2 = e1 + w.n[kShellYZ], e3 = e2 + w.n[kShellX];
-    const int4* items = w.items[kShellZ];
-    if (p.g.plane * (long long)(p.g.nz + 1) < (1LL << 31)) {
-        if (e_pass) k_shell_e<uint32_t><<<n, b, 0, st>>>(p, fi, fo, pin, pout, items, e1, e2, e3, m);
-        else k_shell_h<uint32_t><<<n, b, 0, st>>>(p, fi, fo, pin, pout, items, e1, e2, e3, m);
-    } else {
-        if (e_pass) k_shell_e<long long><<<n, b, 0, st>>>(p, fi, fo, pin, pout, items, e1, e2, e3, m);
-        else k_shell_h<long long><<<n, b, 0, st>>>(p, fi, fo, pin, pout, items, e1, e2, e3, m);
-    }
-    return cudaGetLastError();
 }
 
 // E of the nodes of the design region's edge box [d0, d3] x [d1, d4] x [d2, d5] (node class

@@ -36,15 +36,13 @@ enum { FDTD_EX = 0, FDTD_EY = 1, FDTD_EZ = 2, FDTD_HX = 3, FDTD_HY = 4, FDTD_HZ 
 
 /* Update-kernel schedules (fdtd_set_schedule). */
 enum {
-    FDTD_SCHEDULE_AUTO = 0,   /* two passes; on grids of >= 8 Mi cells the first fdtd_step call
-                                 of >= 8 steps times 4 steps of each schedule and keeps the faster
-                                 (that call synchronises the handle's stream) */
+    FDTD_SCHEDULE_AUTO = 0,   /* FUSED or TWO_PASS by the grid's size (the measured faster one),
+                                 chosen by the first step or fdtd_tune_schedule; TWO_PASS where the
+                                 second buffers do not fit or the first step is captured */
     FDTD_SCHEDULE_TWO_PASS = 1, /* E pass then H pass per step, in place (the reference's order) */
-    FDTD_SCHEDULE_FUSED = 2,  /* one z-marching sweep per step over ping-pong field buffers   */
-    FDTD_SCHEDULE_FUSED_CPML = 3 /* FUSED with the z-march also over the z and y CPML slabs and
-                                    the boundary planes beside the interior tiles (slabs of at most
-                                    15 cells, no design region); same bits, slower on the measured
-                                    grids, so AUTO does not choose it */
+    FDTD_SCHEDULE_FUSED = 2,  /* one z-marching sweep of the whole grid per step over ping-pong
+                                 field buffers (second buffers are allocated by the first step)  */
+    FDTD_SCHEDULE_FUSED_CPML = 3 /* the same sweep as FUSED, which covers the CPML */
 };
 
 typedef struct fdtd_handle fdtd_handle;
@@ -88,9 +86,8 @@ int fdtd_set_stream(fdtd_handle* h, void* cuda_stream);
 int fdtd_set_schedule(fdtd_handle* h, int32_t schedule);
 /* The schedule the next step runs: TWO_PASS or FUSED (AUTO resolved; -1 for a NULL handle). */
 int32_t fdtd_active_schedule(const fdtd_handle* h);
-/* Under AUTO, run the schedule trial now without advancing the handle: fields, CPML memory, probe
- * ring and step count are restored afterwards. Nothing to do for other schedules or a trial already
- * taken. Synchronises the handle's stream. */
+/* Under AUTO, make the choice now, before the first step: the second buffers of the fused schedule,
+ * if it takes it, are allocated here. Nothing to do for other schedules or a choice already made. */
 int fdtd_tune_schedule(fdtd_handle* h);
 
 /* Material table (at most 256 entries). Replaces the per-brick material scalars that setBrick
@@ -342,14 +339,14 @@ int fdtd_batch_step(fdtd_batch* b, int64_t steps);
 /* Wait for the batch stream; FDTD_ERR_DEVICE if an instance's kernel reported an error. */
 int fdtd_batch_synchronize(fdtd_batch* b);
 
-/* Maximum bytes of FDTD_STEP_STATIC_SCRATCH: one second field set, one second CPML memory set and
- * the sweep's work list. Enough for a 64^3 grid with 10-cell CPML on all faces (about 9.8 MiB). */
+/* Maximum bytes of FDTD_STEP_STATIC_SCRATCH: one second field set and one second CPML memory set.
+ * Enough for a 64^3 grid with 10-cell CPML on all faces (about 9.8 MiB). */
 #define FDTD_STEP_STATIC_SCRATCH_BYTES (16u << 20)
 
 /* No reference counterpart. Advances n steps with the fused sweep like fdtd_step under
  * FDTD_SCHEDULE_FUSED, with bit-identical fields, CPML memory and probe samples. This call
- * allocates no device memory. fdtd_step allocates a second field set and CPML set (plus the
- * sweep's work list) the first time it runs the fused sweep. The ping-pong target here is instead
+ * allocates no device memory. fdtd_step allocates a second field set and CPML set the first time it
+ * runs the fused sweep. The ping-pong target here is instead
  * a fixed static device array of FDTD_STEP_STATIC_SCRATCH_BYTES inside the library.
  * It is for callers that cannot allocate while stepping: callers whose device memory is reserved
  * in full up front (by their own pool) so that a lazy allocation would fail, and callers that must
@@ -364,8 +361,6 @@ int fdtd_batch_synchronize(fdtd_batch* b);
  *    does only this set-up; make it once per device before a section that must issue nothing
  *    but stream work. The address is kept for the life of the process: after a cudaDeviceReset
  *    it is stale, so do not use this call across a device reset.
- *  - Each call uploads the sweep's work list (planned once per handle into pinned host memory)
- *    into the scratch with one asynchronous host-to-device copy on the handle's stream.
  *  - Nothing in the scratch needs to start at zero or to survive between calls: with an odd n the
  *    call first copies the handle's CPML memory into it, every scratch element a step reads was
  *    written earlier in the same call, and the result is back in the handle's own buffers when

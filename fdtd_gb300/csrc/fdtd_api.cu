@@ -118,7 +118,9 @@ struct fdtd_handle {
     SrcRow* src_rows = nullptr;
     ProbeAt* d_probes_at = nullptr;   // probes outside the CPML slabs
     int n_probes_at = 0;
-    int edge_mat = 0;                 // SweepStep::mat (read back by ensure_prepared)
+    int edge_mat = 0;                 // rows other than the background's in a slab or on a low wall (read back by ensure_prepared)
+    float4* slab_rows = nullptr;      // SlabRows, with edge_mat (NULL: too many rows, their nodes take the general path)
+    int n_coef_rows = 0;
     int4* d_special = nullptr;        // special_nodes, while and after their rows are built
     // interface-key hash set and its lists (launch_iface_set / launch_iface_rows)
     unsigned long long* iface_table = nullptr;
@@ -368,11 +370,15 @@ void* tensor_map_encoder() {
 // 128^3 50.0 / 50.3 and 51.3 / 51.6, 144^3 90.5 / 71.7 and 90.9 / 76.7, 200^3 226 / 139 and 227 / 144.
 // Between about 1 and 2.6 Mi cells, where the fields still sit in L2 and the sweep's CTAs fill the
 // device once, the two are level, and two-pass needs no second buffers; nor do grids below
-// kAutoSweepCells, a few CTAs' work. Grids with a design region take the sweep from kAutoDesignCells
+// kAutoSweepCells, a few CTAs' work. With materials in the CPML slabs (boxes that touch one face) the
+// tiles there take longer than the others and the range is wider: 64^3 18 / 12.5 us, 72^3 22 / 21,
+// 96^3 29 / 29, 112^3 39 / 46, 128^3 47 / 62, 160^3 97 / 113, 176^3 130 / 149, 200^3 178 / 157,
+// 225^3 253 / 217. Grids with a design region take the sweep from kAutoDesignCells
 // on (smaller ones record in their two-pass kernels). Two-pass also serves where the second buffers
 // cannot be allocated.
 constexpr long long kAutoSweepCells = 32LL << 10;
 constexpr long long kAutoLevelLo = 1000LL << 10, kAutoLevelHi = 2600LL << 10;
+constexpr long long kAutoEdgeLo = 900LL << 10, kAutoEdgeHi = 6400LL << 10;  // with slab_rows
 constexpr long long kAutoDesignCells = 64LL << 20;
 
 // The background material's coefficients (StepParams::bgn), evaluated on the host with the rounding steps of
@@ -458,7 +464,8 @@ void release_fused(fdtd_handle* h) {
 void auto_choose(fdtd_handle* h) {
     if (h->schedule != FDTD_SCHEDULE_AUTO || h->auto_choice != FDTD_SCHEDULE_AUTO) return;
     const long long cells = (long long)h->g.nx * h->g.ny * h->g.nz;
-    if (cells < (h->has_design ? kAutoDesignCells : kAutoSweepCells) || (cells >= kAutoLevelLo && cells < kAutoLevelHi)) {
+    const long long lo = h->slab_rows ? kAutoEdgeLo : kAutoLevelLo, hi = h->slab_rows ? kAutoEdgeHi : kAutoLevelHi;
+    if (cells < (h->has_design ? kAutoDesignCells : kAutoSweepCells) || (cells >= lo && cells < hi)) {
         h->auto_choice = FDTD_SCHEDULE_TWO_PASS;
         return;
     }
@@ -862,7 +869,18 @@ namespace {
 // What the sweep of the handle's next step takes besides its fields; late: the step before it is
 // one of the same call, whose probes are still to be sampled.
 SweepStep sweep_step(const fdtd_handle* h, bool late) {
-    SweepStep s{h->d_probes_at, h->n_probes_at, late, h->edge_mat || !h->plates.empty(), {}};
+    SweepStep s{h->d_probes_at, h->n_probes_at, late, h->slab_rows != nullptr, {}, {}};
+    if (s.mat) {
+        const DeviceGrid& g = h->g;
+        const int L[3] = {g.pxn + g.pxp, g.pyn + g.pyp, g.pzn + g.pzp};
+        const float4* r = h->slab_rows;
+        for (int a = 0; a < 3; ++a) {
+            const long long n = (long long)h->n_coef_rows * L[a];
+            s.rows.e[a] = r;
+            s.rows.h[a] = r + n;
+            r += 2 * n;
+        }
+    }
     for (size_t w = 0; w < h->waves.size() && w < (size_t)kSweepSources; ++w)
         s.sig[w] = h->step < (long long)h->waves[w].size() ? h->waves[w][(size_t)h->step] : 0.f;
     return s;
@@ -1377,7 +1395,28 @@ int build_interface_rows(fdtd_handle* h) {
     pi.coef = h->coef;
     CUDA_TRY(launch_iface_coefs(pi, h->iface_keys, n_rows, h->coef_rows, h->stream));
     h->n_iface_rows = n_rows;
+    h->n_coef_rows = kFirstInterfaceRow + n_rows + n_special;
     CUDA_TRY(cudaMemcpyAsync(&h->edge_mat, h->small, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    return FDTD_OK;
+}
+
+// The slab coefficients by row, where rows other than the background's lie in a slab or on a low wall
+// (4 MB for 1000 rows and 60 slab planes; up to kSlabRowsLimit).
+constexpr size_t kSlabRowsLimit = 256u << 20;
+int build_slab_rows(fdtd_handle* h) {
+    const DeviceGrid& g = h->g;
+    h->release(h->slab_rows);
+    h->slab_rows = nullptr;
+    if (!h->edge_mat && h->plates.empty() && h->bg_node.low_ok) return FDTD_OK;
+    const long long L = (long long)g.pxn + g.pxp + g.pyn + g.pyp + g.pzn + g.pzp;
+    const size_t bytes = std::max<size_t>(1, (size_t)(2 * h->n_coef_rows * L) * sizeof(float4));
+    if (bytes > kSlabRowsLimit || h->alloc((void**)&h->slab_rows, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        h->slab_rows = nullptr;
+        return FDTD_OK;
+    }
+    float* const kappa[6] = {h->prof[4], h->prof[10], h->prof[16], h->prof[5], h->prof[11], h->prof[17]};
+    CUDA_TRY(launch_slab_rows(g, h->coef_rows, h->n_coef_rows, kappa, h->slab_rows, h->stream));
     return FDTD_OK;
 }
 
@@ -1442,6 +1481,7 @@ int ensure_prepared(fdtd_handle* h) {
         h->dirty_materials = false;
         h->dirty_lumped = true;
     }
+    const bool rows = h->dirty_lumped;
     if (h->dirty_lumped) {
         int rc = build_lumped(h);
         if (rc) return rc;
@@ -1464,6 +1504,10 @@ int ensure_prepared(fdtd_handle* h) {
     }
     CUDA_TRY(launch_rec_probes(h->g, h->d_probes, (int)h->probes.size(), h->rec, h->stream));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
+    if (rows) {
+        int rc = build_slab_rows(h);
+        if (rc) return rc;
+    }
     h->prepared = true;
     return FDTD_OK;
 }

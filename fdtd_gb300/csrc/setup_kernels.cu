@@ -204,6 +204,34 @@ __global__ void k_axis_table(float4* te, float4* th, int n, const float* be, con
     th[q] = make_float4(h0[q], h1[q], bm[q], am[q]);
 }
 
+// SlabRows: per axis the E entries of every row, then the H entries (rows of H on the low walls are
+// the default entry's, so they need none of their own).
+__global__ void k_slab_rows(const MatCoef* __restrict__ coef, DeviceGrid g, int n_rows, const float* kex, const float* key,
+                            const float* kez, const float* kmx, const float* kmy, const float* kmz, float4* out) {
+    const int lo[3] = {g.pxn, g.pyn, g.pzn}, hi[3] = {g.pxp, g.pyp, g.pzp}, n[3] = {g.nx, g.ny, g.nz};
+    const float *ke[3] = {kex, key, kez}, *km[3] = {kmx, kmy, kmz};
+    const int a = blockIdx.y, L = lo[a] + hi[a];
+    for (int b = 0; b < a; ++b) out += 2LL * n_rows * (lo[b] + hi[b]);
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n_rows * L) return;
+    const int l = q % L, at = l < lo[a] ? l : n[a] - hi[a] + l - lo[a];
+    const MatCoef& c = coef[q / L];
+    const float size = a == 0 ? g.dx : a == 1 ? g.dy : g.dz;
+    const float e0 = a == 0 ? c.e[1].z : a == 1 ? c.e[0].y : c.e[0].z, e1 = a == 0 ? c.e[2].y : a == 1 ? c.e[2].z : c.e[1].y;
+    const float h0 = a == 0 ? c.h[1].y : a == 1 ? c.h[0].z : c.h[0].y, h1 = a == 0 ? c.h[2].z : a == 1 ? c.h[2].y : c.h[1].z;
+    out[q] = make_float4(__fdiv_rn(e0, ke[a][at]), __fdiv_rn(e1, ke[a][at]), __fmul_rn(e0, size), __fmul_rn(e1, size));
+    out[n_rows * L + q] = make_float4(__fdiv_rn(h0, km[a][at]), __fdiv_rn(h1, km[a][at]), __fmul_rn(h0, size), __fmul_rn(h1, size));
+}
+
+cudaError_t launch_slab_rows(const DeviceGrid& g, const MatCoef* coef, int n_rows, float* const kappa[6], float4* out,
+                             cudaStream_t st) {
+    const int L = max(g.pxn + g.pxp, max(g.pyn + g.pyp, g.pzn + g.pzp));
+    if (n_rows <= 0 || L <= 0) return cudaSuccess;
+    k_slab_rows<<<dim3((unsigned)((n_rows * L + 255) / 256), 3), 256, 0, st>>>(coef, g, n_rows, kappa[0], kappa[1], kappa[2], kappa[3],
+                                                                              kappa[4], kappa[5], out);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_axis_tables(const DeviceGrid& g, float* const prof[18], float* const bg_curl[12], float4* const te[3],
                                float4* const th[3], cudaStream_t st) {
     const int ns[3] = {g.nx, g.ny, g.nz};

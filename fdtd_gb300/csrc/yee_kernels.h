@@ -56,12 +56,24 @@ struct FusedMaps {  // tensor maps of buffer A
     CUtensorMap e[3];
     CUtensorMap rec;  // coefficient rows (StepParams::rec)
 };
+// Coefficients of the CPML slabs by coefficient row, for the sweep's nodes whose row is not the
+// background's: entry (row, l) of axis a at e[a][row * (the axis's slab planes) + l], l counting the
+// low slab's planes and then the high slab's: the two E curl coefficients along the axis over kappa,
+// then the factors of the CPML memory; likewise h.
+struct SlabRows {
+    const float4* e[3];
+    const float4* h[3];
+};
+cudaError_t launch_slab_rows(const DeviceGrid& g, const MatCoef* coef, int n_rows, float* const prof_kappa[6], float4* out,
+                             cudaStream_t st);
+
 constexpr int kSweepSources = 8;  // lumped sources whose signal comes with the launch
 struct SweepStep {
     const ProbeAt* probes;  // probes outside the CPML slabs
     int n_probes;
     int late;               // sample them for step m - 1 from fi
     int mat;                // coefficient rows other than the background's in a CPML slab or on a low wall
+    SlabRows rows;          // with mat
     float sig[kSweepSources];
 };
 cudaError_t sweep_configure();

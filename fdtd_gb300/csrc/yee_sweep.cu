@@ -14,19 +14,24 @@
 //
 // Coefficients. A quad whose four nodes share a coefficient row loads it once (the background's comes
 // with the kernel parameters); in a CPML slab the curl coefficients along the slab's axis come from
-// the axis' table for background nodes (StepParams::te, th: divided by kappa) and by division for
+// the axis' table for background nodes (StepParams::te, th: divided by kappa) and from SlabRows for
 // other rows. Quads of several rows take them node by node. What is left (lumped edges in a slab,
-// design nodes, probes in a slab, keys beyond the table, quads of several rows in a slab) runs
-// e_update_diff / h_update_diff (slow_node). Old CPML memory of the y and z faces is fetched a plane
-// ahead with cp.async into slots of the thread's own.
+// design nodes, probes in a slab, keys beyond the table) runs e_update_diff / h_update_diff (slow_node).
+// Old CPML memory of the y and z faces is fetched a plane ahead with cp.async into slots of the
+// thread's own.
 //
 // What bounds it: on grids beyond L2, HBM and the latency of a plane step; on smaller ones the latency
 // of a plane step alone (15 warps an SM, about 650 instructions per quad and step, a third of the
-// issue slots). Measured per step, against the schedule it replaced (a sweep of the interior
-// tiles, then one-node-per-thread passes over the CPML shell): 512^3 random boxes 1.650 -> 1.385 ms,
-// 256^3 0.302 -> 0.244 ms, 1024 x 1024 x 896 10.4 -> 8.8 ms; against two-pass, 64^3 18.4 -> 11.8 us. One
-// node per thread in the same march ran 2.0 ms at 512^3 (352 instructions per node against about 165).
-// 3 CTAs an SM (128 registers) against 2 (160): 512^3 1.39 / 1.55 ms, 128^3 52 / 61 us, 64^3 11.8 / 10.4 us.
+// issue slots) and, with materials in the slabs, the tiles that hold them. Measured per step, against
+// the schedule it replaced (a sweep of the interior tiles, then one-node-per-thread passes over the
+// CPML shell): 512^3 random boxes 1.650 -> 1.38 ms, 256^3 0.302 -> 0.240 ms, 1024 x 1024 x 896 10.4 ->
+// 8.8 ms; against two-pass, 64^3 18.4 -> 10.5 us. One node per thread in the same march ran 2.0 ms at 512^3
+// (352 instructions per node against about 165). 3 CTAs an SM (128 registers) against 2: 512^3 1.39 /
+// 1.55 ms, 128^3 52 / 61 us. Registers decide much: spills of 100 bytes in the march cost 5 % at 512^3 and
+// 20 % at 64^3, so old H of a plane is read again from its stage at the end of the step rather than
+// kept through it; and code, as the march should fit the instruction cache: rows other than the
+// background's have their slab coefficients in a table (SlabRows), since divisions in line made grids
+// with materials in the slabs 10-20 % slower (128^3 73 -> 60 us).
 // All arithmetic is that of yee_common.cuh, so the results equal the two-pass schedule's bits.
 // Every wait on a TMA barrier is bounded: on timeout the kernel records an error in the status
 // word, drains its own copies (again bounded) and exits.
@@ -48,15 +53,16 @@ namespace {
 #ifndef FDTD_SWEEP_STAGES
 #define FDTD_SWEEP_STAGES 2
 #endif
-#ifndef FDTD_SWEEP_MIN_BLOCKS
-#define FDTD_SWEEP_MIN_BLOCKS 3
-#endif
 constexpr int TX = kTileX, TY = kSweepRows;
 constexpr int QX = TX / 4;                // quads per row
 constexpr int NOWN = QX * TY;             // threads with a quad of the tile; then the halo row and column
 constexpr int NTH = NOWN + (QX + TY + 31) / 32 * 32;
 static_assert(NOWN % 32 == 0, "own quads fill whole warps");
 constexpr int NST = FDTD_SWEEP_STAGES;    // planes in the ring
+// Up to this many CTAs, two of 168 registers an SM run the grid at once (kWide) instead of three of 128:
+// a plane step is shorter with the registers to have the loads of a quad of several rows in flight
+// together (64^3: vacuum 11.0 -> 10.4 us a step, boxes 12.5 -> 10.5, boxes that touch a CPML slab 16.7 -> 12.6).
+constexpr unsigned kSweepWideCtas = 2 * 152;
 constexpr int round128(int b) { return (b + 127) / 128 * 128; }
 // Tiles in shared memory. H and coefficient rows, with rows of W: x in [x0-4, x0+36), y in
 // [y0-1, y0+TY] and x in [x0, x0+40), y in [y0, y0+TY]; old and new E, with rows of WE: x in
@@ -105,6 +111,7 @@ struct SweepArgs {
     const ProbeAt* probes;  // probes outside the CPML slabs (n of them), sampled one step late: see k_sweep
     int n_probes_at;
     int late;               // the step before this one belongs to the same call
+    SlabRows rows;          // kMat
     float sig[kSweepSources];  // this step's signal of each source
 };
 
@@ -231,6 +238,8 @@ __device__ __forceinline__ void st_mask2(float* a, float* b, const Quad& x, cons
         }
     }
 }
+// The row of node r of a quad.
+__device__ __forceinline__ int row_at(const uint2& c, int r) { return (int)((r < 2 ? c.x : c.y) >> (16 * (r & 1)) & 0xffffu); }
 __device__ __forceinline__ float pick(const Quad& q, int r) { return r == 0 ? q.v[0] : r == 1 ? q.v[1] : r == 2 ? q.v[2] : q.v[3]; }
 
 __device__ __forceinline__ void cp_async16(float4* dst, const float* src) {
@@ -244,7 +253,7 @@ __device__ __forceinline__ Quad quad_of(const float4& f) { return Quad{f.x, f.y,
 // included) meets a CPML slab or a wall in x (wx) or y (wy), or the chunk one in z; without it no
 // node does. kMat: rows other than the background's lie in a slab or on a low wall (without it the
 // few that may, beside general nodes, take the slow path).
-template <typename Idx, bool kEdge, bool kMat>
+template <typename Idx, bool kEdge, bool kMat, bool kWide>
 __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int x0, int y0, int k0, int k1, int row,
                                       int col, bool own, bool wx, bool wy) {
     const StepParams& p = A.p;
@@ -294,6 +303,12 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
         }
     }
     own = own && in4;
+    // kMat: the slab coefficients of row c (SlabRows); lx, ly, lz(k): the slab planes of the quad's first
+    // node, its row and plane k
+    const int Lx = g.pxn + g.pxp, Ly = g.pyn + g.pyp, Lz = g.pzn + g.pzp;
+    const int lx = i < g.pxn ? i : i - (g.nx - Lx), ly = j < g.pyn ? j : j - (g.ny - Ly);
+    auto lz = [&](int k) { return k < g.pzn ? k : k - (g.nz - Lz); };
+    const SlabRows& SR = A.rows;
     const Idx nij = (Idx)j * (Idx)g.pitch + (Idx)i;
     Idx n = (Idx)k0 * (Idx)g.plane + nij;
     const int bgm = p.bg.mat;
@@ -372,13 +387,13 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
         const float* TE = f32(S.stage[s]) + E_OFF + te;
         float* en = &S.enew[k & 1][0][te];
         const float* ep = &S.enew[(k - 1) & 1][0][te];
-        float xq0[4], xq1[4];
+        Quad xq0, xq1;
         if (kEdge && xs) {
 #pragma unroll
             for (int r = 0; r < 4; ++r)
                 if (xs >> r & 1) {
-                    xq0[r] = __ldg(pin + (qx + r));
-                    xq1[r] = __ldg(pin + (qx + sx + r));
+                    xq0.v[r] = __ldg(pin + (qx + r));
+                    xq1.v[r] = __ldg(pin + (qx + sx + r));
                 }
         }
         ok = mbar_wait(&S.bar[s], parity);
@@ -391,43 +406,21 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
             const Quad hzj = lds4(T + H_OFF + 2 * HF - W), hxj = lds4(T + H_OFF - W);
             const float hzi = T[H_OFF + 2 * HF - 1], hyi = T[H_OFF + HF - 1];
             vx = lds4(TE); vy = lds4(TE + EF); vz = lds4(TE + 2 * EF);
-            float ce[6];  // the nodes' factors of the CPML memory
-            if (kEdge) {
-#pragma unroll
-                for (int r = 0; r < 6; ++r) ce[r] = B.ce[r];
-            }
             const int c0 = (int)(cw.x & 0xffffu);
-            if (cw.x == cw.y && cw.x == (uint32_t)c0 * 0x10001u && c0 < p.src_row0 &&
-                !(kEdge && (xslow || (!kMat && c0 != bgm && (xs || ys || zs))))) {
-                // one row for the quad
+            bool mixed = false;
+            if (cw.x == cw.y && cw.x == (uint32_t)c0 * 0x10001u && (kEdge ? c0 == bgm && !xslow : c0 < p.src_row0)) {
+                // one row for the quad (in tiles at the edge, the background's)
                 float4 a = make_float4(B.ea[0], B.ec[0], B.ec[1], 0.f), b = make_float4(B.ea[1], B.ec[2], B.ec[3], 0.f);
                 float4 d = make_float4(B.ea[2], B.ec[4], B.ec[5], 0.f);
-                if (c0 != bgm) {
+                if (!kEdge && c0 != bgm) {
                     const MatCoef* mc = p.coef + c0;
                     a = __ldg(&mc->e[0]); b = __ldg(&mc->e[1]); d = __ldg(&mc->e[2]);
-                    if (kEdge && kMat) {  // its factors of the CPML memory
-                        ce[0] = __fmul_rn(b.z, g.dx); ce[1] = __fmul_rn(d.y, g.dx);
-                        ce[2] = __fmul_rn(a.y, g.dy); ce[3] = __fmul_rn(d.z, g.dy);
-                        ce[4] = __fmul_rn(a.z, g.dz); ce[5] = __fmul_rn(b.y, g.dz);
-                    }
                 }
                 Quad x0c = {b.z, b.z, b.z, b.z}, x1c = {d.y, d.y, d.y, d.y};
-                if (kEdge && (xs || ys || zs)) {  // curl coefficients along a slab's axis, over kappa
-                    if (!kMat || c0 == bgm) {
-                        if (ys) { a.y = S.ye[row].x; d.z = S.ye[row].y; }
-                        if (zs) { a.z = S.ze[q].x; b.y = S.ze[q].y; }
-                        if (xs) { x0c = lds4(&S.xe[0][col]); x1c = lds4(&S.xe[1][col]); }
-                    } else {
-                        if (ys) { const float kap = __ldg(p.key + j); a.y = __fdiv_rn(a.y, kap); d.z = __fdiv_rn(d.z, kap); }
-                        if (zs) { const float kap = __ldg(p.kez + k); a.z = __fdiv_rn(a.z, kap); b.y = __fdiv_rn(b.y, kap); }
-#pragma unroll
-                        for (int r = 0; r < 4; ++r)
-                            if (xs >> r & 1) {
-                                const float kap = __ldg(p.kex + i + r);
-                                x0c.v[r] = __fdiv_rn(x0c.v[r], kap);
-                                x1c.v[r] = __fdiv_rn(x1c.v[r], kap);
-                            }
-                    }
+                if (kEdge) {  // curl coefficients along a slab's axis, over kappa
+                    if (ys) { a.y = S.ye[row].x; d.z = S.ye[row].y; }
+                    if (zs) { a.z = S.ze[q].x; b.y = S.ze[q].y; }
+                    if (xs) { x0c = lds4(&S.xe[0][col]); x1c = lds4(&S.xe[1][col]); }
                 }
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
@@ -436,32 +429,105 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                     vz.v[r] = upd3(d.x, vz.v[r], x1c.v[r], __fsub_rn(hy.v[r], r ? hy.v[r - 1] : hyi), d.z, __fsub_rn(hx.v[r], hxj.v[r]));
                 }
             } else {
-                // rows per node; in a slab only background nodes, which take the slab's curl coefficients
-                int cur = -1;
-                float4 a{}, b{}, d{};
+                // rows per node; in a slab background nodes take the tabulated curl coefficients, and
+                // without kMat the others the slow path
+                mixed = true;
+                if constexpr (kWide) {
+                    // (component by component, so that the four nodes' loads are in flight together: the quads
+                    // of a material's surface decide how long the plane takes)
+                    int c[4];
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const int c = (int)((r < 2 ? cw.x : cw.y) >> (16 * (r & 1)) & 0xffffu);
-                    const bool x = kEdge && (xs >> r & 1);
-                    if (c >= kRecGeneral || (kEdge && ((c != bgm && (ys || zs || x)) || (xslow >> r & 1)))) {
-                        slow |= 1 << r;
-                        continue;
+                    for (int r = 0; r < 4; ++r) {
+                        c[r] = row_at(cw, r);
+                        if (c[r] >= kRecGeneral || (kEdge && ((!kMat && c[r] != bgm && (ys || zs || (xs >> r & 1))) || (xslow >> r & 1)))) {
+                            slow |= 1 << r;
+                            c[r] = bgm;
+                        }
                     }
-                    if (c != cur) {
-                        const MatCoef* mc = p.coef + c;
-                        a = __ldg(&mc->e[0]); b = __ldg(&mc->e[1]); d = __ldg(&mc->e[2]);
-                        cur = c;
-                        if (kEdge && ys) { a.y = S.ye[row].x; d.z = S.ye[row].y; }
-                        if (kEdge && zs) { a.z = S.ze[q].x; b.y = S.ze[q].y; }
+                    // the curl coefficients along the axes whose slab the nodes lie in, over kappa
+                    auto slab_e = [&](Quad& f, bool in, const float4* T, int L, int l, int w, float bg) {
+                        if (kEdge && in)
+#pragma unroll
+                            for (int r = 0; r < 4; ++r) f.v[r] = kMat ? __ldg(&T[c[r] * L + l].x + w) : bg;
+                    };
+                    auto slab_ex = [&](Quad& f, int w) {
+                        if (kEdge && xs)
+#pragma unroll
+                            for (int r = 0; r < 4; ++r)
+                                if (xs >> r & 1) f.v[r] = kMat ? __ldg(&SR.e[0][c[r] * Lx + lx + r].x + w) : S.xe[w][col + r];
+                    };
+                    Quad f0, f1, f2;
+                    auto rows = [&](int comp) {
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            const float4 f = __ldg(&p.coef[c[r]].e[comp]);
+                            f0.v[r] = f.x; f1.v[r] = f.y; f2.v[r] = f.z;
+                        }
+                    };
+                    rows(0);
+                    slab_e(f1, ys, SR.e[1], Ly, ly, 0, S.ye[row].x);
+                    slab_e(f2, zs, SR.e[2], Lz, lz(k), 0, S.ze[q].x);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        vx.v[r] = upd3(f0.v[r], vx.v[r], f1.v[r], __fsub_rn(hz.v[r], hzj.v[r]), f2.v[r], __fsub_rn(hy.v[r], hyp.v[r]));
+                    rows(1);
+                    slab_e(f1, zs, SR.e[2], Lz, lz(k), 1, S.ze[q].y);
+                    slab_ex(f2, 0);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        vy.v[r] = upd3(f0.v[r], vy.v[r], f1.v[r], __fsub_rn(hx.v[r], hxp.v[r]), f2.v[r],
+                                       __fsub_rn(hz.v[r], r ? hz.v[r - 1] : hzi));
+                    rows(2);
+                    slab_ex(f1, 1);
+                    slab_e(f2, ys, SR.e[1], Ly, ly, 1, S.ye[row].y);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        vz.v[r] = upd3(f0.v[r], vz.v[r], f1.v[r], __fsub_rn(hy.v[r], r ? hy.v[r - 1] : hyi), f2.v[r],
+                                       __fsub_rn(hx.v[r], hxj.v[r]));
+                        if (c[r] >= p.src_row0) {  // lumped source edge (fdtdrav.h:728)
+                            const SrcRow sr = p.src_rows[c[r] - p.src_row0];
+                            vz.v[r] = __fmaf_rn(sr.cezj, A.sig[sr.source], vz.v[r]);
+                        }
                     }
-                    vx.v[r] = upd3(a.x, vx.v[r], a.y, __fsub_rn(hz.v[r], hzj.v[r]), a.z, __fsub_rn(hy.v[r], hyp.v[r]));
-                    vy.v[r] = upd3(b.x, vy.v[r], b.y, __fsub_rn(hx.v[r], hxp.v[r]), x ? S.xe[0][col + r] : b.z,
-                                   __fsub_rn(hz.v[r], r ? hz.v[r - 1] : hzi));
-                    vz.v[r] = upd3(d.x, vz.v[r], x ? S.xe[1][col + r] : d.y, __fsub_rn(hy.v[r], r ? hy.v[r - 1] : hyi), d.z,
-                                   __fsub_rn(hx.v[r], hxj.v[r]));
-                    if (c >= p.src_row0) {  // lumped source edge (fdtdrav.h:728)
-                        const SrcRow sr = p.src_rows[c - p.src_row0];
-                        vz.v[r] = __fmaf_rn(sr.cezj, A.sig[sr.source], vz.v[r]);
+                } else {
+                    int cur = -1;
+                    float4 a{}, b{}, d{};
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const int c = row_at(cw, r);
+                        const bool x = kEdge && (xs >> r & 1);
+                        if (c >= kRecGeneral || (kEdge && ((!kMat && c != bgm && (ys || zs || x)) || (xslow >> r & 1)))) {
+                            slow |= 1 << r;
+                            continue;
+                        }
+                        if (c != cur) {
+                            const MatCoef* mc = p.coef + c;
+                            a = __ldg(&mc->e[0]); b = __ldg(&mc->e[1]); d = __ldg(&mc->e[2]);
+                            cur = c;
+                            if (!kMat || c == bgm) {
+                                if (kEdge && ys) { a.y = S.ye[row].x; d.z = S.ye[row].y; }
+                                if (kEdge && zs) { a.z = S.ze[q].x; b.y = S.ze[q].y; }
+                            } else if (kEdge) {
+                                if (ys) { const float4 f = __ldg(SR.e[1] + c * Ly + ly); a.y = f.x; d.z = f.y; }
+                                if (zs) { const float4 f = __ldg(SR.e[2] + c * Lz + lz(k)); a.z = f.x; b.y = f.y; }
+                            }
+                        }
+                        float xb = b.z, xd = d.y;
+                        if (x) {
+                            if (!kMat || c == bgm) {
+                                xb = S.xe[0][col + r]; xd = S.xe[1][col + r];
+                            } else {
+                                const float4 f = __ldg(SR.e[0] + c * Lx + lx + r);
+                                xb = f.x; xd = f.y;
+                            }
+                        }
+                        vx.v[r] = upd3(a.x, vx.v[r], a.y, __fsub_rn(hz.v[r], hzj.v[r]), a.z, __fsub_rn(hy.v[r], hyp.v[r]));
+                        vy.v[r] = upd3(b.x, vy.v[r], b.y, __fsub_rn(hx.v[r], hxp.v[r]), xb, __fsub_rn(hz.v[r], r ? hz.v[r - 1] : hzi));
+                        vz.v[r] = upd3(d.x, vz.v[r], xd, __fsub_rn(hy.v[r], r ? hy.v[r - 1] : hyi), d.z, __fsub_rn(hx.v[r], hxj.v[r]));
+                        if (c >= p.src_row0) {  // lumped source edge (fdtdrav.h:728)
+                            const SrcRow sr = p.src_rows[c - p.src_row0];
+                            vz.v[r] = __fmaf_rn(sr.cezj, A.sig[sr.source], vz.v[r]);
+                        }
                     }
                 }
                 slow &= in4;
@@ -477,18 +543,40 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                     mz = yin && klt ? in_x : 0;
                 }
                 const int st = store_e ? in4 & ~slow : 0;
+                // v0 and v1 plus the quad's CPML memory u0, u1 along an axis (factors b0, b1, or its rows')
+                const bool own_rows = kMat && (mixed || c0 != bgm);
+                auto add = [&](Quad& v0, Quad& v1, const Quad& u0, const Quad& u1, float b0, float b1, const float4* T, int L, int l,
+                               int dl, int nodes) {
+                    if (own_rows) {
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            const int c = row_at(cw, r);
+                            if (c < kRecGeneral && (nodes >> r & 1)) {
+                                const float4 f = __ldg(T + c * L + l + r * dl);
+                                v0.v[r] = psi_add(v0.v[r], f.z, u0.v[r]);
+                                v1.v[r] = psi_add(v1.v[r], f.w, u1.v[r]);
+                            }
+                        }
+                        return;
+                    }
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        if (nodes >> r & 1) {
+                            v0.v[r] = psi_add(v0.v[r], b0, u0.v[r]);
+                            v1.v[r] = psi_add(v1.v[r], b1, u1.v[r]);
+                        }
+                };
                 if (xs) {  // fdtdrav.h:752-785
                     const Quad b = lds4(&S.xe[2][col]), c = lds4(&S.xe[3][col]);
 #pragma unroll
                     for (int r = 0; r < 4; ++r)
                         if (xs >> r & 1) {
-                            xq0[r] = psi_upd(b.v[r], xq0[r], c.v[r], __fsub_rn(hz.v[r], r ? hz.v[r - 1] : hzi));
-                            xq1[r] = psi_upd(b.v[r], xq1[r], c.v[r], __fsub_rn(hy.v[r], r ? hy.v[r - 1] : hyi));
-                            if (st & my & (1 << r)) pout[qx + r] = xq0[r];
-                            if (st & mz & (1 << r)) pout[qx + sx + r] = xq1[r];
-                            vy.v[r] = psi_add(vy.v[r], ce[0], xq0[r]);
-                            vz.v[r] = psi_add(vz.v[r], ce[1], xq1[r]);
+                            xq0.v[r] = psi_upd(b.v[r], xq0.v[r], c.v[r], __fsub_rn(hz.v[r], r ? hz.v[r - 1] : hzi));
+                            xq1.v[r] = psi_upd(b.v[r], xq1.v[r], c.v[r], __fsub_rn(hy.v[r], r ? hy.v[r - 1] : hyi));
+                            if (st & my & (1 << r)) pout[qx + r] = xq0.v[r];
+                            if (st & mz & (1 << r)) pout[qx + sx + r] = xq1.v[r];
                         }
+                    add(vy, vz, xq0, xq1, B.ce[0], B.ce[1], SR.e[0], Lx, lx, 1, xs);
                 }
                 if (ys) {  // fdtdrav.h:790-827
                     const float b = S.ye[row].z, c = S.ye[row].w;
@@ -497,10 +585,9 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                     for (int r = 0; r < 4; ++r) {
                         u.v[r] = psi_upd(b, u.v[r], c, __fsub_rn(hz.v[r], hzj.v[r]));
                         w.v[r] = psi_upd(b, w.v[r], c, __fsub_rn(hx.v[r], hxj.v[r]));
-                        vx.v[r] = psi_add(vx.v[r], ce[2], u.v[r]);
-                        vz.v[r] = psi_add(vz.v[r], ce[3], w.v[r]);
                     }
                     st_mask2(pout + qy, pout + qy + sy, u, w, st & mx, st & mz);
+                    add(vx, vz, u, w, B.ce[2], B.ce[3], SR.e[1], Ly, ly, 0, 15);
                 }
                 if (zs) {  // fdtdrav.h:829-911
                     const float b = S.ze[q].z, c = S.ze[q].w;
@@ -512,10 +599,9 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                     for (int r = 0; r < 4; ++r) {
                         u.v[r] = psi_upd(b, u.v[r], c, __fsub_rn(hy.v[r], hyp.v[r]));
                         w.v[r] = psi_upd(b, w.v[r], c, __fsub_rn(hx.v[r], hxp.v[r]));
-                        vx.v[r] = psi_add(vx.v[r], ce[4], u.v[r]);
-                        vy.v[r] = psi_add(vy.v[r], ce[5], w.v[r]);
                     }
                     st_mask2(pout + at, pout + at + S.zo[q].stride, u, w, st & mx, st & my);
+                    add(vx, vy, u, w, B.ce[4], B.ce[5], SR.e[2], Lz, lz(k), 0, 15);
                 }
                 if (wall) {  // components the walls keep
                     const Quad ex = lds4(TE), ey = lds4(TE + EF), ez = lds4(TE + 2 * EF);
@@ -543,8 +629,8 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
 #pragma unroll
                 for (int r = 0; r < 4; ++r)
                     if (xs >> r & 1) {
-                        xq0[r] = __ldg(pin + (gx + r));
-                        xq1[r] = __ldg(pin + (gx + sx + r));
+                        xq0.v[r] = __ldg(pin + (gx + r));
+                        xq1.v[r] = __ldg(pin + (gx + sx + r));
                     }
             }
             // differences of E: along z, y and x
@@ -552,45 +638,33 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
             const Quad ezj = lds4(ep + 2 * NF + WE), exj = lds4(ep + WE);
             const float ezi = ep[2 * NF + 4], eyi = ep[NF + 4];
             const bool low_jk = kEdge && (j == 0 || kh == 0);  // faces on a low wall take the default entry
-            float ch[6];  // the nodes' factors of the CPML memory
-            if (kEdge) {
-#pragma unroll
-                for (int r = 0; r < 6; ++r) ch[r] = B.ch[r];
-            }
             Quad ux = hxp, uy = hyp, uz = hzp;
             const int c0 = (int)(cp.x & 0xffffu);
+            bool mixed = false;
+            // the row that component `comp` of node r (row c) takes: the default entry's on a low wall
+            auto hrow = [&](int c, int r, int comp) {
+                if (!kEdge || !kMat) return c;
+                return (comp == 0 ? i + r == 0 : comp == 1 ? j == 0 : kh == 0) ? kDefaultEntry : c;
+            };
+            // entry (row of component p, row of component q) of an axis's slab coefficients
+            auto slab_h = [&](const float4* T, int L, int l, int rp, int rq) {
+                float4 f = __ldg(T + rp * L + l);
+                if (rq != rp) { const float4 o = __ldg(T + rq * L + l); f.y = o.y; f.w = o.w; }
+                return f;
+            };
             const bool table = c0 == bgm && (!low_jk || B.low_ok);  // the tabulated coefficients apply
-            if (cp.x == cp.y && cp.x == (uint32_t)c0 * 0x10001u && c0 < kRecGeneral &&
-                !(kEdge && (xslow || (i == 0 && (c0 != bgm || !B.low_ok)) || (!kMat && !table && (xs || ys || zsh || low_jk))))) {
+            if (cp.x == cp.y && cp.x == (uint32_t)c0 * 0x10001u &&
+                (kEdge ? table && !xslow && (i > 0 || B.low_ok) : c0 < kRecGeneral)) {
                 float4 a = make_float4(B.ha[0], B.hc[0], B.hc[1], 0.f), b = make_float4(B.ha[1], B.hc[2], B.hc[3], 0.f);
                 float4 d = make_float4(B.ha[2], B.hc[4], B.hc[5], 0.f);
-                if (!table) {
-                    const MatCoef *mc = p.coef + c0, *md = p.coef + kDefaultEntry;
-                    a = __ldg(&mc->h[0]); b = __ldg(kEdge && kMat && j == 0 ? &md->h[1] : &mc->h[1]);
-                    d = __ldg(kEdge && kMat && kh == 0 ? &md->h[2] : &mc->h[2]);
-                    if (kEdge && kMat) {
-                        ch[0] = __fmul_rn(b.y, g.dx); ch[1] = __fmul_rn(d.z, g.dx);
-                        ch[2] = __fmul_rn(a.z, g.dy); ch[3] = __fmul_rn(d.y, g.dy);
-                        ch[4] = __fmul_rn(a.y, g.dz); ch[5] = __fmul_rn(b.z, g.dz);
-                    }
+                if (!kEdge && c0 != bgm) {
+                    a = __ldg(&p.coef[c0].h[0]); b = __ldg(&p.coef[c0].h[1]); d = __ldg(&p.coef[c0].h[2]);
                 }
                 Quad x0c = {b.y, b.y, b.y, b.y}, x1c = {d.z, d.z, d.z, d.z};
-                if (kEdge && (xs || ys || zsh)) {
-                    if (!kMat || table) {
-                        if (ys) { a.z = S.yh[row].x; d.y = S.yh[row].y; }
-                        if (zsh) { a.y = S.zh[q - 1].x; b.z = S.zh[q - 1].y; }
-                        if (xs) { x0c = lds4(&S.xh[0][col]); x1c = lds4(&S.xh[1][col]); }
-                    } else {
-                        if (ys) { const float kap = __ldg(p.kmy + j); a.z = __fdiv_rn(a.z, kap); d.y = __fdiv_rn(d.y, kap); }
-                        if (zsh) { const float kap = __ldg(p.kmz + kh); a.y = __fdiv_rn(a.y, kap); b.z = __fdiv_rn(b.z, kap); }
-#pragma unroll
-                        for (int r = 0; r < 4; ++r)
-                            if (xs >> r & 1) {
-                                const float kap = __ldg(p.kmx + i + r);
-                                x0c.v[r] = __fdiv_rn(x0c.v[r], kap);
-                                x1c.v[r] = __fdiv_rn(x1c.v[r], kap);
-                            }
-                    }
+                if (kEdge) {
+                    if (ys) { a.z = S.yh[row].x; d.y = S.yh[row].y; }
+                    if (zsh) { a.y = S.zh[q - 1].x; b.z = S.zh[q - 1].y; }
+                    if (xs) { x0c = lds4(&S.xh[0][col]); x1c = lds4(&S.xh[1][col]); }
                 }
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
@@ -599,29 +673,96 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                     uz.v[r] = upd3(d.x, uz.v[r], d.y, __fsub_rn(exj.v[r], ex.v[r]), x1c.v[r], __fsub_rn(r < 3 ? ey.v[r + 1] : eyi, ey.v[r]));
                 }
             } else {
-                int cur = -1;
-                float4 a{}, b{}, d{};
+                mixed = true;
+                if constexpr (kWide) {
+                    int c[4];
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const int c = (int)((r < 2 ? cp.x : cp.y) >> (16 * (r & 1)) & 0xffffu);
-                    const bool x = kEdge && (xs >> r & 1), lw = kEdge && (low_jk || (r == 0 && i == 0));
-                    if (c >= kRecGeneral ||
-                        (kEdge && ((c != bgm && (ys || zsh || x || lw)) || (lw && !B.low_ok) || (xslow >> r & 1)))) {
-                        slow |= 16 << r;
-                        continue;
+                    for (int r = 0; r < 4; ++r) {
+                        c[r] = row_at(cp, r);
+                        const bool lw = kEdge && (low_jk || i + r == 0);
+                        if (c[r] >= kRecGeneral || (kEdge && ((!kMat && ((c[r] != bgm && (ys || zsh || (xs >> r & 1) || lw)) || (lw && !B.low_ok))) ||
+                                                              (xslow >> r & 1)))) {
+                            slow |= 16 << r;
+                            c[r] = bgm;
+                        }
                     }
-                    if (c != cur) {
-                        const MatCoef* mc = p.coef + c;
-                        a = __ldg(&mc->h[0]); b = __ldg(&mc->h[1]); d = __ldg(&mc->h[2]);
-                        cur = c;
-                        if (kEdge && ys) { a.z = S.yh[row].x; d.y = S.yh[row].y; }
-                        if (kEdge && zsh) { a.y = S.zh[q - 1].x; b.z = S.zh[q - 1].y; }
+                    auto slab_q = [&](Quad& f, bool in, const float4* T, int L, int l, int w, int comp, float bg) {
+                        if (kEdge && in)
+#pragma unroll
+                            for (int r = 0; r < 4; ++r) f.v[r] = kMat ? __ldg(&T[hrow(c[r], r, comp) * L + l].x + w) : bg;
+                    };
+                    auto slab_qx = [&](Quad& f, int w, int comp) {
+                        if (kEdge && xs)
+#pragma unroll
+                            for (int r = 0; r < 4; ++r)
+                                if (xs >> r & 1) f.v[r] = kMat ? __ldg(&SR.h[0][hrow(c[r], r, comp) * Lx + lx + r].x + w) : S.xh[w][col + r];
+                    };
+                    Quad f0, f1, f2;
+                    auto rows = [&](int comp) {
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            const float4 f = __ldg(&p.coef[hrow(c[r], r, comp)].h[comp]);
+                            f0.v[r] = f.x; f1.v[r] = f.y; f2.v[r] = f.z;
+                        }
+                    };
+                    rows(0);
+                    slab_q(f1, zsh, SR.h[2], Lz, lz(kh), 0, 0, S.zh[q - 1].x);
+                    slab_q(f2, ys, SR.h[1], Ly, ly, 0, 0, S.yh[row].x);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        ux.v[r] = upd3_hx(f0.v[r], ux.v[r], f1.v[r], __fsub_rn(vy.v[r], ey.v[r]), f2.v[r], __fsub_rn(ezj.v[r], ez.v[r]));
+                    rows(1);
+                    slab_qx(f1, 0, 1);
+                    slab_q(f2, zsh, SR.h[2], Lz, lz(kh), 1, 1, S.zh[q - 1].y);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        uy.v[r] = upd3(f0.v[r], uy.v[r], f1.v[r], __fsub_rn(r < 3 ? ez.v[r + 1] : ezi, ez.v[r]), f2.v[r],
+                                       __fsub_rn(vx.v[r], ex.v[r]));
+                    rows(2);
+                    slab_q(f1, ys, SR.h[1], Ly, ly, 1, 2, S.yh[row].y);
+                    slab_qx(f2, 1, 2);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        uz.v[r] = upd3(f0.v[r], uz.v[r], f1.v[r], __fsub_rn(exj.v[r], ex.v[r]), f2.v[r],
+                                       __fsub_rn(r < 3 ? ey.v[r + 1] : eyi, ey.v[r]));
+                } else {
+                    int cur = -1;
+                    float4 a{}, b{}, d{};
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const int c = row_at(cp, r);
+                        const bool x = kEdge && (xs >> r & 1), lw = kEdge && (low_jk || (r == 0 && i == 0));
+                        if (c >= kRecGeneral || (kEdge && ((!kMat && ((c != bgm && (ys || zsh || x || lw)) || (lw && !B.low_ok))) ||
+                                                           (xslow >> r & 1)))) {
+                            slow |= 16 << r;
+                            continue;
+                        }
+                        const bool tab = !kMat || (c == bgm && (!lw || B.low_ok));
+                        if (c != cur) {
+                            a = __ldg(&p.coef[hrow(c, r, 0)].h[0]); b = __ldg(&p.coef[hrow(c, r, 1)].h[1]);
+                            d = __ldg(&p.coef[hrow(c, r, 2)].h[2]);
+                            cur = kEdge && kMat && r == 0 && i == 0 ? -1 : c;
+                            if (tab) {
+                                if (kEdge && ys) { a.z = S.yh[row].x; d.y = S.yh[row].y; }
+                                if (kEdge && zsh) { a.y = S.zh[q - 1].x; b.z = S.zh[q - 1].y; }
+                            } else if (kEdge) {
+                                if (ys) { const float4 f = slab_h(SR.h[1], Ly, ly, hrow(c, r, 0), hrow(c, r, 2)); a.z = f.x; d.y = f.y; }
+                                if (zsh) { const float4 f = slab_h(SR.h[2], Lz, lz(kh), hrow(c, r, 0), hrow(c, r, 1)); a.y = f.x; b.z = f.y; }
+                            }
+                        }
+                        float xb = b.y, xd = d.z;
+                        if (x) {
+                            if (tab) {
+                                xb = S.xh[0][col + r]; xd = S.xh[1][col + r];
+                            } else {
+                                const float4 f = slab_h(SR.h[0], Lx, lx + r, hrow(c, r, 1), hrow(c, r, 2));
+                                xb = f.x; xd = f.y;
+                            }
+                        }
+                        ux.v[r] = upd3_hx(a.x, ux.v[r], a.y, __fsub_rn(vy.v[r], ey.v[r]), a.z, __fsub_rn(ezj.v[r], ez.v[r]));
+                        uy.v[r] = upd3(b.x, uy.v[r], xb, __fsub_rn(r < 3 ? ez.v[r + 1] : ezi, ez.v[r]), b.z, __fsub_rn(vx.v[r], ex.v[r]));
+                        uz.v[r] = upd3(d.x, uz.v[r], d.y, __fsub_rn(exj.v[r], ex.v[r]), xd, __fsub_rn(r < 3 ? ey.v[r + 1] : eyi, ey.v[r]));
                     }
-                    ux.v[r] = upd3_hx(a.x, ux.v[r], a.y, __fsub_rn(vy.v[r], ey.v[r]), a.z, __fsub_rn(ezj.v[r], ez.v[r]));
-                    uy.v[r] = upd3(b.x, uy.v[r], x ? S.xh[0][col + r] : b.y, __fsub_rn(r < 3 ? ez.v[r + 1] : ezi, ez.v[r]), b.z,
-                                   __fsub_rn(vx.v[r], ex.v[r]));
-                    uz.v[r] = upd3(d.x, uz.v[r], d.y, __fsub_rn(exj.v[r], ex.v[r]), x ? S.xh[1][col + r] : d.z,
-                                   __fsub_rn(r < 3 ? ey.v[r + 1] : eyi, ey.v[r]));
                 }
                 slow &= in4 | in4 << 4;
             }
@@ -635,18 +776,39 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                     my = klh ? lt4 : 0;
                     mz = ylt ? lt4 : 0;
                 }
+                const bool own_rows = kMat && (mixed || !table);
+                auto add = [&](Quad& v0, Quad& v1, const Quad& u0, const Quad& u1, float b0, float b1, const float4* T, int L, int l,
+                               int dl, int nodes, int p0, int p1) {
+                    if (own_rows) {
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            const int c = row_at(cp, r);
+                            if (c < kRecGeneral && (nodes >> r & 1)) {
+                                const float4 f = slab_h(T, L, l + r * dl, hrow(c, r, p0), hrow(c, r, p1));
+                                v0.v[r] = psi_add(v0.v[r], f.z, u0.v[r]);
+                                v1.v[r] = psi_add(v1.v[r], f.w, u1.v[r]);
+                            }
+                        }
+                        return;
+                    }
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        if (nodes >> r & 1) {
+                            v0.v[r] = psi_add(v0.v[r], b0, u0.v[r]);
+                            v1.v[r] = psi_add(v1.v[r], b1, u1.v[r]);
+                        }
+                };
                 if (xs) {  // fdtdrav.h:401-442
                     const Quad b = lds4(&S.xh[2][col]), c = lds4(&S.xh[3][col]);
 #pragma unroll
                     for (int r = 0; r < 4; ++r)
                         if (xs >> r & 1) {
-                            xq0[r] = psi_upd(b.v[r], xq0[r], c.v[r], __fsub_rn(r < 3 ? ez.v[r + 1] : ezi, ez.v[r]));
-                            xq1[r] = psi_upd(b.v[r], xq1[r], c.v[r], __fsub_rn(r < 3 ? ey.v[r + 1] : eyi, ey.v[r]));
-                            if (st & my & (1 << r)) pout[gx + r] = xq0[r];
-                            if (st & mz & (1 << r)) pout[gx + sx + r] = xq1[r];
-                            uy.v[r] = psi_add(uy.v[r], ch[0], xq0[r]);
-                            uz.v[r] = psi_add(uz.v[r], ch[1], xq1[r]);
+                            xq0.v[r] = psi_upd(b.v[r], xq0.v[r], c.v[r], __fsub_rn(r < 3 ? ez.v[r + 1] : ezi, ez.v[r]));
+                            xq1.v[r] = psi_upd(b.v[r], xq1.v[r], c.v[r], __fsub_rn(r < 3 ? ey.v[r + 1] : eyi, ey.v[r]));
+                            if (st & my & (1 << r)) pout[gx + r] = xq0.v[r];
+                            if (st & mz & (1 << r)) pout[gx + sx + r] = xq1.v[r];
                         }
+                    add(uy, uz, xq0, xq1, B.ch[0], B.ch[1], SR.h[0], Lx, lx, 1, xs, 1, 2);
                 }
                 if (ys) {  // fdtdrav.h:445-486
                     const float b = S.yh[row].z, c = S.yh[row].w;
@@ -655,11 +817,10 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                     for (int r = 0; r < 4; ++r) {
                         u.v[r] = psi_upd(b, u.v[r], c, __fsub_rn(ezj.v[r], ez.v[r]));
                         w.v[r] = psi_upd(b, w.v[r], c, __fsub_rn(exj.v[r], ex.v[r]));
-                        ux.v[r] = psi_add(ux.v[r], ch[2], u.v[r]);
-                        uz.v[r] = psi_add(uz.v[r], ch[3], w.v[r]);
                     }
                     const Idx at = qy - dy + 2 * sy;
                     st_mask2(pout + at, pout + at + sy, u, w, st & mx, st & mz);
+                    add(ux, uz, u, w, B.ch[2], B.ch[3], SR.h[1], Ly, ly, 0, 15, 0, 2);
                 }
                 if (zsh) {  // fdtdrav.h:489-562
                     const float b = S.zh[q - 1].z, c = S.zh[q - 1].w;
@@ -671,10 +832,9 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                     for (int r = 0; r < 4; ++r) {
                         u.v[r] = psi_upd(b, u.v[r], c, __fsub_rn(vy.v[r], ey.v[r]));
                         w.v[r] = psi_upd_hyz(b, w.v[r], c, __fsub_rn(vx.v[r], ex.v[r]));
-                        ux.v[r] = psi_add(ux.v[r], ch[4], u.v[r]);
-                        uy.v[r] = psi_add(uy.v[r], ch[5], w.v[r]);
                     }
                     st_mask2(pout + at, pout + at + sz, u, w, st & mx, st & my);
+                    add(ux, uy, u, w, B.ch[4], B.ch[5], SR.h[2], Lz, lz(kh), 0, 15, 0, 1);
                 }
                 if (wall) {
 #pragma unroll
@@ -698,8 +858,8 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                                pick(hzp, r), (int)c);
             }
         }
-        hxp = hx; hyp = hy; hzp = hz;
-        cp = cw;
+        hxp = lds4(T + H_OFF); hyp = lds4(T + H_OFF + HF); hzp = lds4(T + H_OFF + 2 * HF);  // (again: not kept in registers)
+        cp = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(S.stage[s] + 3 * H_BYTES + 3 * E_BYTES) + t);
         n += (Idx)g.plane;
         if (kEdge) {
             qx += dx;
@@ -712,8 +872,8 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
 
 }  // namespace
 
-template <typename Idx, bool kMat>
-__global__ void __launch_bounds__(NTH, FDTD_SWEEP_MIN_BLOCKS) k_sweep(const __grid_constant__ SweepArgs A) {
+template <typename Idx, bool kMat, bool kWide>
+__global__ void __launch_bounds__(NTH, kWide ? 2 : 3) k_sweep(const __grid_constant__ SweepArgs A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     SweepSmem<Idx>& S = *reinterpret_cast<SweepSmem<Idx>*>(smem_raw);
     const StepParams& p = A.p;
@@ -789,21 +949,23 @@ __global__ void __launch_bounds__(NTH, FDTD_SWEEP_MIN_BLOCKS) k_sweep(const __gr
     const bool wx = x0 < max(g.pxn, 1) || x0 + TX >= min(g.nx - g.pxp, g.nx - 1);
     const bool wy = y0 < max(g.pyn, 1) || y0 + TY >= min(g.ny - g.pyp, g.ny - 1);
     const bool wz = k0 < max(g.pzn, 1) || k1 >= min(g.nz - g.pzp, g.nz - 1);  // E(k0) .. E(k1), H(k0) .. H(k1 - 1)
-    if (wx || wy || wz) march<Idx, true, kMat>(A, S, x0, y0, k0, k1, row, col, own, wx, wy);
-    else march<Idx, false, kMat>(A, S, x0, y0, k0, k1, row, col, own, false, false);
+    if (wx || wy || wz) march<Idx, true, kMat, kWide>(A, S, x0, y0, k0, k1, row, col, own, wx, wy);
+    else march<Idx, false, kMat, kWide>(A, S, x0, y0, k0, k1, row, col, own, false, false);
 }
 
 template <typename Idx>
 constexpr int sweep_smem() { return (int)sizeof(SweepSmem<Idx>); }
 
-template <typename Idx, bool kMat>
+template <typename Idx, bool kMat, bool kWide>
 cudaError_t configure() {
-    return cudaFuncSetAttribute(k_sweep<Idx, kMat>, cudaFuncAttributeMaxDynamicSharedMemorySize, sweep_smem<Idx>());
+    return cudaFuncSetAttribute(k_sweep<Idx, kMat, kWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, sweep_smem<Idx>());
 }
 cudaError_t sweep_configure() {
-    cudaError_t e = configure<uint32_t, false>();
-    if (e == cudaSuccess) e = configure<uint32_t, true>();
-    if (e == cudaSuccess) e = configure<unsigned long long, true>();
+    cudaError_t e = cudaSuccess;
+    for (cudaError_t (*f)() : {configure<uint32_t, false, false>, configure<uint32_t, false, true>, configure<uint32_t, true, false>,
+                               configure<uint32_t, true, true>, configure<unsigned long long, false, false>,
+                               configure<unsigned long long, true, false>})
+        if (e == cudaSuccess) e = f();
     return e;
 }
 
@@ -832,7 +994,7 @@ cudaError_t launch_sample_probes(const StepParams& p, const FieldPtrs& f, const 
 cudaError_t launch_sweep(const FusedMaps& maps, const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fo,
                          const PsiSet& pin, const PsiSet& pout, const SweepPlan& sg, const SweepStep& ss, long long m,
                          cudaStream_t st) {
-    SweepArgs args{maps, p, fo, pin, pout, sg, m, fi, ss.probes, ss.n_probes, ss.late, {}};
+    SweepArgs args{maps, p, fo, pin, pout, sg, m, fi, ss.probes, ss.n_probes, ss.late, ss.rows, {}};
     std::copy(ss.sig, ss.sig + kSweepSources, args.sig);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(sg.nbx * sg.nby * sg.chunks()), 1, 1);
@@ -845,8 +1007,12 @@ cudaError_t launch_sweep(const FusedMaps& maps, const StepParams& p, const Field
     cfg.numAttrs = 1;
     const bool idx32 = p.g.plane * (long long)(p.g.nz + 1) < (1LL << 31) && p.psi_total < (1LL << 31);
     cfg.dynamicSmemBytes = idx32 ? sweep_smem<uint32_t>() : sweep_smem<unsigned long long>();
-    if (!idx32) return cudaLaunchKernelEx(&cfg, k_sweep<unsigned long long, true>, args);
-    return ss.mat ? cudaLaunchKernelEx(&cfg, k_sweep<uint32_t, true>, args) : cudaLaunchKernelEx(&cfg, k_sweep<uint32_t, false>, args);
+    const bool wide = cfg.gridDim.x <= kSweepWideCtas;
+    using K = void (*)(const SweepArgs);
+    const K k = idx32 ? ss.mat ? wide ? K(k_sweep<uint32_t, true, true>) : K(k_sweep<uint32_t, true, false>)
+                               : wide ? K(k_sweep<uint32_t, false, true>) : K(k_sweep<uint32_t, false, false>)
+                      : ss.mat ? K(k_sweep<unsigned long long, true, false>) : K(k_sweep<unsigned long long, false, false>);
+    return cudaLaunchKernelEx(&cfg, k, args);
 }
 
 // Tensor maps of the sweep: H tiles with a one-node halo (x from 4 nodes before the tile: a TMA box

@@ -99,6 +99,7 @@ def check(sc, schedule=2, calls=(5, 4)):
     ((6, 5, 4), (1, 3, 2, 2, 0, 3)),
     ((3, 3, 3), (0,) * 6),
     ((130, 20, 100), (2, 11, 7, 8, 30, 33)),
+    ((130, 210, 45), (5, 4, 8, 7, 6, 6)),  # more CTAs than the two-per-SM kernel takes
 ])
 @pytest.mark.parametrize("materials", [False, True])
 def test_sweep_equals_two_pass(gpu_lib, dims, pml, materials):

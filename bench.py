@@ -523,9 +523,9 @@ def bench_batched(steps=2000):
             "sequential": {"value": round(seq, 3), "unit": "Gcell-updates/s", "seconds": round(t_seq, 3),
                            "gpu_launches": 2 * steps * len(scs)},
             "batched": {"value": round(bat, 3), "unit": "Gcell-updates/s", "seconds": round(t_bat, 3),
-                        "gpu_launches": {-1: 2 * steps * len(scs) + -(-steps // 32), 0: 3 * steps}.get(cfg["cluster"], 1),
+                        "gpu_launches": {-1: (steps + -(-steps // 32)) * len(scs) + -(-steps // 32), 0: 3 * steps}.get(cfg["cluster"], 1),
                         "config": cfg,
-                        "form": {-1: "chains (each instance's two-pass kernels, concurrent graph branches)",
+                        "form": {-1: "chains (each instance's own kernels, concurrent graph branches)",
                                  0: "flat (E, H, step-counter kernels per step)"}.get(cfg["cluster"], "persistent clusters"),
                         "tune_ms_5_steps": round(tune_ms, 2)},
             "speedup": round(bat / seq, 2)}

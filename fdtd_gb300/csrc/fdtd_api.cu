@@ -869,7 +869,7 @@ namespace {
 // What the sweep of the handle's next step takes besides its fields; late: the step before it is
 // one of the same call, whose probes are still to be sampled.
 SweepStep sweep_step(const fdtd_handle* h, bool late) {
-    SweepStep s{h->d_probes_at, h->n_probes_at, late, h->slab_rows != nullptr, {}, {}};
+    SweepStep s{h->d_probes_at, h->n_probes_at, late, nullptr, h->slab_rows != nullptr, {}, {}};
     if (s.mat) {
         const DeviceGrid& g = h->g;
         const int L[3] = {g.pxn + g.pxp, g.pyn + g.pyp, g.pzn + g.pzp};
@@ -899,7 +899,7 @@ int steps_fused(fdtd_handle* h, const StepParams& p, int64_t n) {
         h->cur = b;
         ++h->step;
     }
-    if (n > 0) CUDA_TRY(launch_sample_probes(p, fields(h->cur), h->d_probes_at, h->n_probes_at, h->step - 1, h->stream));
+    if (n > 0) CUDA_TRY(launch_sample_probes(p, fields(h->cur), h->d_probes_at, h->n_probes_at, nullptr, h->step - 1, h->stream));
     return FDTD_OK;
 }
 
@@ -1641,7 +1641,7 @@ extern "C" int fdtd_step_static_scratch(fdtd_handle* h, int64_t n) {
             CUDA_TRY(launch_sweep(maps_s, p, fs, fh, sp, h->psi[a], h->sweep, sweep_step(h, s > 0), h->step, h->stream));
         ++h->step;
     }
-    CUDA_TRY(launch_sample_probes(p, n & 1 ? fs : fh, h->d_probes_at, h->n_probes_at, h->step - 1, h->stream));
+    CUDA_TRY(launch_sample_probes(p, n & 1 ? fs : fh, h->d_probes_at, h->n_probes_at, nullptr, h->step - 1, h->stream));
     if (n & 1) {  // the last step wrote the scratch: copy the state back into the handle's buffers
         // only the nx columns of each row: the sweep never writes the row padding
         const DeviceGrid& g = h->g;
@@ -2095,6 +2095,7 @@ struct fdtd_batch {
     struct Graph {
         long long steps;
         int cfg[3];
+        unsigned long long sig;     // of the descriptors it bakes in (chain form; 0 otherwise)
         cudaGraph_t graph;
         cudaGraphExec_t exec;
     };
@@ -2103,10 +2104,16 @@ struct fdtd_batch {
     // and a signature of the descriptors the captured graphs bake in
     std::vector<cudaStream_t> chain_streams;
     std::vector<cudaEvent_t> chain_events;  // [0]: fork, [1 + q]: join of instance q
-    unsigned long long chain_sig = 0;
+    unsigned long long chain_sig = 0;       // of the current descriptors
+    std::vector<char> sweep;                // instances whose chain runs the sweep (two-pass otherwise)
 };
 
 namespace {
+
+// A batch of n plans each instance's chunks for kBatchShare / n of the device: long chunks repeat
+// fewer halo planes, short ones give the device more CTAs. 64 instances of 32^3 to 96^3, 32 steps:
+// 14.5 ms with a share of 1, 14.6 with 2, 14.8 with 4; 16 of them 5.1, 3.9 and 3.5; 8 of 64^3 2.3, 1.8 and 2.0.
+constexpr double kBatchShare = 2.0;
 
 void batch_drop_graph(fdtd_batch* b) {
     for (auto& G : b->graphs) {
@@ -2136,7 +2143,7 @@ int batch_refresh(fdtd_batch* b) {
 }
 
 int batch_set_config(fdtd_batch* b, int cluster, int threads) {
-    if (cluster == -1) {  // chains: each instance's own two-pass kernels, instances concurrent
+    if (cluster == -1) {  // chains: each instance's own kernels, instances concurrent
         if (threads != 256) return fail(FDTD_ERR_INVALID, "the chain form (cluster -1) runs 256 threads per CTA");
         b->cluster = -1;
         b->threads = 256;
@@ -2161,15 +2168,61 @@ int batch_set_config(fdtd_batch* b, int cluster, int threads) {
     return FDTD_OK;
 }
 
+// Which instances' chains run the sweep: in a batch of at least kBatchSweepCells altogether, those from
+// kAutoSweepCells on whose schedule allows it and that have room for second buffers. Smaller batches
+// leave the device partly idle, and two passes have the shorter chain of dependent loads. Measured,
+// two-pass against sweep, ms for 32 steps of n cubes: 4 x 64^3 0.90 / 1.05, 2 x 96^3 1.17 / 1.39,
+// 16 x 40^3 1.78 / 1.81, 8 x 64^3 2.04 / 1.76, 8 x (32 to 96) 1.56 / 1.99, 16 x 48^3 2.73 / 2.17, 4 x 96^3
+// 3.08 / 2.37, 16 x (32 to 96) 4.74 / 3.93, 64 x 40^3 9.3 / 6.2, 64 x 64^3 21.3 / 12.0, 16 x 128^3 25.4 / 15.7.
+constexpr long long kBatchSweepCells = 2560LL << 10;
+void batch_choose(fdtd_batch* b) {
+    auto cells = [](const fdtd_handle* h) { return (long long)h->g.nx * h->g.ny * h->g.nz; };
+    long long total = 0;
+    for (const fdtd_handle* h : b->hs) total += cells(h);
+    for (size_t q = 0; q < b->hs.size(); ++q) {
+        fdtd_handle* h = b->hs[q];
+        bool s = total >= kBatchSweepCells && cells(h) >= kAutoSweepCells && h->schedule != FDTD_SCHEDULE_TWO_PASS;
+        if (s && ensure_fused(h) != FDTD_OK) {
+            cudaGetLastError();
+            if (h->cur == 0) release_fused(h);
+            s = false;
+        }
+        b->sweep[q] = s;
+    }
+}
+
+// `steps` sweep steps of instance q on stream cs, counted from its device step counter.
+cudaError_t chain_sweep(fdtd_batch* b, int q, long long steps, cudaStream_t cs) {
+    fdtd_handle* h = b->hs[q];
+    const StepParams& p = b->inst[q].p;
+    const DeviceGrid& g = h->g;
+    const SweepPlan plan = plan_sweep(PlanGrid{g.nx, g.ny, g.nz, g.pxn, g.pxp, g.pyn, g.pyp, g.pzn, g.pzp},
+                                      kBatchShare / (double)b->hs.size());
+    auto fields = [&](int c) {
+        return FieldPtrs{h->field[c][0], h->field[c][1], h->field[c][2], h->field[c][3], h->field[c][4], h->field[c][5]};
+    };
+    int a = h->cur;
+    cudaError_t e = cudaSuccess;
+    for (long long t = 0; t < steps && e == cudaSuccess; ++t, a = 1 - a) {
+        SweepStep s = sweep_step(h, t > 0);
+        s.base = &b->d_inst[q].step;
+        e = launch_sweep(h->maps[a], p, fields(a), fields(1 - a), h->psi[a], h->psi[1 - a], plan, s, t, cs);
+    }
+    if (e == cudaSuccess)
+        e = launch_sample_probes(p, fields(a), h->d_probes_at, h->n_probes_at, &b->d_inst[q].step, steps - 1, cs);
+    return e;
+}
+
 // The captured launch of `steps` steps under the current configuration (captured on first use).
 int batch_graph(fdtd_batch* b, long long steps, cudaGraphExec_t* out) {
     const int cfg[3] = {b->cluster, b->threads, b->n_clusters};
+    const unsigned long long sig = b->cluster == -1 ? b->chain_sig : 0;
     for (auto& G : b->graphs)
-        if (G.steps == steps && std::equal(cfg, cfg + 3, G.cfg)) {
+        if (G.steps == steps && std::equal(cfg, cfg + 3, G.cfg) && G.sig == sig) {
             *out = G.exec;
             return FDTD_OK;
         }
-    if (b->graphs.size() >= 4) batch_drop_graph(b);
+    if (b->graphs.size() >= 8) batch_drop_graph(b);
     const int n = (int)b->hs.size();
     if (b->cluster == -1 && b->chain_streams.empty()) {
         b->chain_streams.assign(n, nullptr);
@@ -2180,13 +2233,14 @@ int batch_graph(fdtd_batch* b, long long steps, cudaGraphExec_t* out) {
     CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t e = cudaSuccess;
     if (b->cluster == -1) {
-        // fork one chain per instance, `steps` two-pass steps each, join, advance the counters
+        // fork one chain per instance, `steps` steps each, join, advance the counters
         e = cudaEventRecord(b->chain_events[0], b->stream);
         for (int q = 0; q < n && e == cudaSuccess; ++q) {
             const BatchInstance& I = b->inst[q];
             cudaStream_t cs = b->chain_streams[q];
             e = cudaStreamWaitEvent(cs, b->chain_events[0], 0);
-            for (long long t = 0; t < steps && e == cudaSuccess; ++t)
+            if (e == cudaSuccess && b->sweep[q]) e = chain_sweep(b, q, steps, cs);
+            for (long long t = 0; t < steps && e == cudaSuccess && !b->sweep[q]; ++t)
                 e = launch_two_pass_rel(I.p, I.f, I.ps, &b->d_inst[q].step, (int)t, cs);
             if (e == cudaSuccess) e = cudaEventRecord(b->chain_events[1 + q], cs);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream, b->chain_events[1 + q], 0);
@@ -2203,7 +2257,7 @@ int batch_graph(fdtd_batch* b, long long steps, cudaGraphExec_t* out) {
         if (g) cudaGraphDestroy(g);
         return fail(FDTD_ERR_CUDA, std::string("batch graph capture: ") + cudaGetErrorString(e != cudaSuccess ? e : e2));
     }
-    fdtd_batch::Graph G{steps, {cfg[0], cfg[1], cfg[2]}, g, nullptr};
+    fdtd_batch::Graph G{steps, {cfg[0], cfg[1], cfg[2]}, sig, g, nullptr};
     if (cudaGraphInstantiate(&G.exec, g, 0) != cudaSuccess) {
         cudaGraphDestroy(g);
         return fail(FDTD_ERR_CUDA, "batch graph instantiation");
@@ -2215,9 +2269,9 @@ int batch_graph(fdtd_batch* b, long long steps, cudaGraphExec_t* out) {
 
 // Run `steps` steps on every instance (refresh, graph launches), then advance the step counters.
 // The persistent form is one launch of `steps` steps; the flat and chain forms replay a graph of
-// kFlatChunk steps and one of the remainder. The chain form's graphs bake the descriptors in, so
-// they are captured again when a descriptor changes (a handle stepped alone under the fused
-// schedule, tables rebuilt).
+// kFlatChunk steps and one of the remainder. The chain form's graphs bake the descriptors in, so a
+// graph is captured for each set of descriptors (a handle stepped alone or swept an odd number of
+// steps has its state in the other buffer; tables may be rebuilt); the last few are kept.
 constexpr long long kFlatChunk = 32;
 unsigned long long descriptor_signature(const fdtd_batch* b) {
     unsigned long long h = 1469598103934665603ULL;  // FNV-1a over the descriptors without their steps
@@ -2225,20 +2279,29 @@ unsigned long long descriptor_signature(const fdtd_batch* b) {
         const unsigned char* c = reinterpret_cast<const unsigned char*>(&I);
         for (size_t q = 0; q < offsetof(BatchInstance, step); ++q) h = (h ^ c[q]) * 1099511628211ULL;
     }
+    auto word = [&](unsigned long long w) { h = (h ^ w) * 1099511628211ULL; };
+    for (size_t q = 0; q < b->hs.size(); ++q) {  // what the sweep's launches take besides
+        const fdtd_handle* x = b->hs[q];
+        word(b->sweep[q]);
+        word((unsigned long long)x->cur);
+        word((unsigned long long)(uintptr_t)x->field[1][0]);
+        word((unsigned long long)(uintptr_t)x->psi_base[1]);
+        word((unsigned long long)(uintptr_t)x->d_probes_at);
+        word((unsigned long long)x->n_probes_at);
+        word((unsigned long long)(uintptr_t)x->slab_rows);
+        word((unsigned long long)x->n_coef_rows);
+    }
     return h;
 }
 int batch_run(fdtd_batch* b, long long steps) {
     int rc = batch_refresh(b);
     if (rc) return rc;
     if (b->cluster == -1) {
-        const unsigned long long sig = descriptor_signature(b);
-        if (sig != b->chain_sig) {
-            batch_drop_graph(b);
-            b->chain_sig = sig;
-        }
+        batch_choose(b);
+        b->chain_sig = descriptor_signature(b);
     }
     cudaGraphExec_t ex = nullptr;
-    if (b->cluster <= 0) {
+    if (b->cluster <= 0) {  // (an odd chunk is replayed once only: the state then lies in the other buffer)
         const long long chunk = std::min(steps, kFlatChunk), full = steps / chunk, rem = steps % chunk;
         if ((rc = batch_graph(b, chunk, &ex))) return rc;
         for (long long q = 0; q < full; ++q) CUDA_TRY(cudaGraphLaunch(ex, b->stream));
@@ -2250,7 +2313,10 @@ int batch_run(fdtd_batch* b, long long steps) {
         if ((rc = batch_graph(b, steps, &ex))) return rc;
         CUDA_TRY(cudaGraphLaunch(ex, b->stream));
     }
-    for (fdtd_handle* h : b->hs) h->step += steps;
+    for (size_t q = 0; q < b->hs.size(); ++q) {
+        b->hs[q]->step += steps;
+        if (b->cluster == -1 && b->sweep[q] && (steps & 1)) b->hs[q]->cur = 1 - b->hs[q]->cur;
+    }
     return FDTD_OK;
 }
 
@@ -2273,6 +2339,7 @@ extern "C" int fdtd_batch_create(fdtd_handle* const* handles, int32_t n, fdtd_ba
     b->hs.assign(handles, handles + n);
     b->device = dev;
     b->inst.resize(n);
+    b->sweep.assign(n, 0);
     auto cleanup = [&](int rc) { fdtd_batch_destroy(b); return rc; };
     if (cudaStreamCreateWithFlags(&b->own_stream, cudaStreamNonBlocking) != cudaSuccess)
         return cleanup(fail(FDTD_ERR_CUDA, "batch stream"));

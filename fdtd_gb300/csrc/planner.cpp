@@ -50,21 +50,21 @@ std::vector<int> starts(int lo, int hi, int size, int align, bool overlap) {
 }  // namespace
 
 // Chunks per tile column. A chunk of n planes costs about n + 2 plane steps (the plane below is
-// streamed, the E of the plane above recomputed), and about kSweepSlots CTAs run at once, so short
+// streamed, the E of the plane above recomputed), and FDTD_SWEEP_SLOTS CTAs run at once on each of the 152 SMs, so short
 // grids want enough chunks to fill the device and tall ones few. The cheapest count wins. Where the
 // chunks come out long, cuts at the z slabs keep the slabs' rules out of the middle chunks.
-SweepPlan plan_sweep(const PlanGrid& g) {
+SweepPlan plan_sweep(const PlanGrid& g, double share) {
 #ifndef FDTD_SWEEP_SLOTS
 #define FDTD_SWEEP_SLOTS 3
 #endif
-    constexpr int kSweepSlots = FDTD_SWEEP_SLOTS * 152;
+    const double slots = std::max(1.0, FDTD_SWEEP_SLOTS * 152 * share);
     SweepPlan p{(g.nx + kTileX - 1) / kTileX, (g.ny + kSweepRows - 1) / kSweepRows, g.nz, 0, g.nz, 0, 1, 0};
     const long long tiles = (long long)p.nbx * p.nby;
     double best = -1.0;
     for (int nch = (g.nz + kMaxSweepChunk - 1) / kMaxSweepChunk; nch <= g.nz; ++nch) {
         const int kc = (g.nz + nch - 1) / nch;
         const double ctas = (double)tiles * nch;
-        const double waves = ctas <= kSweepSlots ? 1.0 : ctas / kSweepSlots + 0.5;
+        const double waves = ctas <= slots ? 1.0 : ctas / slots + 0.5;
         const double cost = waves * (kc + 2);
         if (best < 0 || cost < best) {
             best = cost;

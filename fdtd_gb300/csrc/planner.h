@@ -72,7 +72,8 @@ struct SweepPlan {
         return c == chunks() ? nz : zhi + (int)((long long)(c - n_lo - n_mid) * (nz - zhi) / n_hi);
     }
 };
-SweepPlan plan_sweep(const PlanGrid& g);
+// share: the part of the device the grid has to itself (1 / n for one of n grids swept at once).
+SweepPlan plan_sweep(const PlanGrid& g, double share = 1.0);
 
 // Planes per interior item (see plan_chunk in planner.cpp).
 int plan_chunk(const PlanGrid& g);

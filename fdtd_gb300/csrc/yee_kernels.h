@@ -72,6 +72,8 @@ struct SweepStep {
     const ProbeAt* probes;  // probes outside the CPML slabs
     int n_probes;
     int late;               // sample them for step m - 1 from fi
+    const long long* base;  // device step counter that m counts from (captured launches), or NULL: the
+                            // sources' signals are then read on the device
     int mat;                // coefficient rows other than the background's in a CPML slab or on a low wall
     SlabRows rows;          // with mat
     float sig[kSweepSources];
@@ -80,9 +82,9 @@ cudaError_t sweep_configure();
 cudaError_t launch_sweep(const FusedMaps& maps, const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fo,
                          const PsiSet& pin, const PsiSet& pout, const SweepPlan& sg, const SweepStep& ss, long long m,
                          cudaStream_t st);
-// The same probes for step m from its finished fields f.
-cudaError_t launch_sample_probes(const StepParams& p, const FieldPtrs& f, const ProbeAt* probes, int n, long long m,
-                                 cudaStream_t st);
+// The same probes for step m (from *base, if not NULL) from its finished fields f.
+cudaError_t launch_sample_probes(const StepParams& p, const FieldPtrs& f, const ProbeAt* probes, int n, const long long* base,
+                                 long long m, cudaStream_t st);
 // encode_fn: the driver's cuTensorMapEncodeTiled. Returns 0 on success.
 int encode_sweep_maps(FusedMaps* out, const DeviceGrid& g, float* const h[3], float* const e[3], const uint16_t* rec,
                       void* encode_fn);

@@ -59,7 +59,7 @@ constexpr int NOWN = QX * TY;             // threads with a quad of the tile; th
 constexpr int NTH = NOWN + (QX + TY + 31) / 32 * 32;
 static_assert(NOWN % 32 == 0, "own quads fill whole warps");
 constexpr int NST = FDTD_SWEEP_STAGES;    // planes in the ring
-// Up to this many CTAs, two of 168 registers an SM run the grid at once (kWide) instead of three of 128:
+// A grid swept alone of up to this many CTAs: two of 168 registers an SM run the grid at once (kWide) instead of three of 128:
 // a plane step is shorter with the registers to have the loads of a quad of several rows in flight
 // together (64^3: vacuum 11.0 -> 10.4 us a step, boxes 12.5 -> 10.5, boxes that touch a CPML slab 16.7 -> 12.6).
 constexpr unsigned kSweepWideCtas = 2 * 152;
@@ -95,6 +95,7 @@ struct SweepSmem {
     float4 ze[kMaxSweepPlanes], zh[kMaxSweepPlanes];
     PsiAt<Idx> zo[kMaxSweepPlanes];
     uint64_t bar[NST];
+    long long m;                            // the step
 };
 
 __device__ __forceinline__ const float* f32(const unsigned char* b) { return reinterpret_cast<const float*>(b); }
@@ -106,7 +107,8 @@ struct SweepArgs {
     FieldPtrs fo;
     PsiSet pin, pout;
     SweepPlan sg;
-    long long m;
+    long long m;            // the step, or its offset from *base
+    const long long* base;  // device step counter (launches captured in a graph), or NULL
     FieldPtrs fi;
     const ProbeAt* probes;  // probes outside the CPML slabs (n of them), sampled one step late: see k_sweep
     int n_probes_at;
@@ -114,6 +116,13 @@ struct SweepArgs {
     SlabRows rows;          // kMat
     float sig[kSweepSources];  // this step's signal of each source
 };
+
+__device__ __forceinline__ long long sweep_m(const SweepArgs& A) { return A.base ? *A.base + A.m : A.m; }
+__device__ __forceinline__ float sweep_sig(const SweepArgs& A, int source) {
+    if (!A.base) return A.sig[source];
+    const long long m = sweep_m(A);
+    return m < A.p.wave_len[source] ? A.p.waves[source][m] : 0.f;
+}
 
 // Slow path, out of line: nodes on the general path (lumped edges, plates, design nodes, probes,
 // keys beyond the table), nodes of another material than the background in a CPML slab, and H faces
@@ -130,7 +139,7 @@ __device__ __forceinline__ void slow_node(const SweepArgs* pa, SweepSmem<Idx>* p
     const float* TE = f32(S.stage[stage]) + E_OFF + te;
     float* en = &S.enew[k & 1][0][te];
     const float* ep = &S.enew[(k - 1) & 1][0][te];
-    const long long R = p.g.pitch, PL = p.g.plane, m = pa->m, rr = m % p.ring_cap;
+    const long long R = p.g.pitch, PL = p.g.plane, m = S.m, rr = m % p.ring_cap;
     const bool own = bits & 4, store_e = bits & 8;
     float out[3], pre[3];
     if (bits & 1) {
@@ -486,7 +495,7 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                                        __fsub_rn(hx.v[r], hxj.v[r]));
                         if (c[r] >= p.src_row0) {  // lumped source edge (fdtdrav.h:728)
                             const SrcRow sr = p.src_rows[c[r] - p.src_row0];
-                            vz.v[r] = __fmaf_rn(sr.cezj, A.sig[sr.source], vz.v[r]);
+                            vz.v[r] = __fmaf_rn(sr.cezj, sweep_sig(A, sr.source), vz.v[r]);
                         }
                     }
                 } else {
@@ -526,7 +535,7 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                         vz.v[r] = upd3(d.x, vz.v[r], xd, __fsub_rn(hy.v[r], r ? hy.v[r - 1] : hyi), d.z, __fsub_rn(hx.v[r], hxj.v[r]));
                         if (c >= p.src_row0) {  // lumped source edge (fdtdrav.h:728)
                             const SrcRow sr = p.src_rows[c - p.src_row0];
-                            vz.v[r] = __fmaf_rn(sr.cezj, A.sig[sr.source], vz.v[r]);
+                            vz.v[r] = __fmaf_rn(sr.cezj, sweep_sig(A, sr.source), vz.v[r]);
                         }
                     }
                 }
@@ -890,6 +899,7 @@ __global__ void __launch_bounds__(NTH, kWide ? 2 : 3) k_sweep(const __grid_const
 
     // ---- per-column, per-row and per-plane tables ----
     if (tid == 0) {
+        S.m = sweep_m(A);
         for (int q = 0; q < NST; ++q) mbar_init(&S.bar[q], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -940,7 +950,7 @@ __global__ void __launch_bounds__(NTH, kWide ? 2 : 3) k_sweep(const __grid_const
     // k_sample_probes. Probes inside a slab are sampled by the slow path, before the CPML correction.
     if (A.late && blockIdx.x * NTH < (unsigned)A.n_probes_at) {
         const int q = blockIdx.x * NTH + tid;
-        if (q < A.n_probes_at) sample_at(A.probes[q], A.fi, p, A.m - 1);
+        if (q < A.n_probes_at) sample_at(A.probes[q], A.fi, p, S.m - 1);
     }
     // own quads, then those of the halo row and the halo column (spare threads repeat the last one)
     const bool own = tid < NOWN;
@@ -970,14 +980,14 @@ cudaError_t sweep_configure() {
 }
 
 __global__ void k_sample_probes(const __grid_constant__ StepParams p, const __grid_constant__ FieldPtrs f,
-                                const ProbeAt* __restrict__ probes, int n, long long m) {
+                                const ProbeAt* __restrict__ probes, int n, const long long* base, long long m) {
     grid_dependency_wait();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < n) sample_at(probes[q], f, p, m);
+    if (q < n) sample_at(probes[q], f, p, base ? *base + m : m);
 }
 
-cudaError_t launch_sample_probes(const StepParams& p, const FieldPtrs& f, const ProbeAt* probes, int n, long long m,
-                                 cudaStream_t st) {
+cudaError_t launch_sample_probes(const StepParams& p, const FieldPtrs& f, const ProbeAt* probes, int n, const long long* base,
+                                 long long m, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(n + 127) / 128, 1, 1);
@@ -988,13 +998,13 @@ cudaError_t launch_sample_probes(const StepParams& p, const FieldPtrs& f, const 
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_sample_probes, p, f, probes, n, m);
+    return cudaLaunchKernelEx(&cfg, k_sample_probes, p, f, probes, n, base, m);
 }
 
 cudaError_t launch_sweep(const FusedMaps& maps, const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fo,
                          const PsiSet& pin, const PsiSet& pout, const SweepPlan& sg, const SweepStep& ss, long long m,
                          cudaStream_t st) {
-    SweepArgs args{maps, p, fo, pin, pout, sg, m, fi, ss.probes, ss.n_probes, ss.late, ss.rows, {}};
+    SweepArgs args{maps, p, fo, pin, pout, sg, m, ss.base, fi, ss.probes, ss.n_probes, ss.late, ss.rows, {}};
     std::copy(ss.sig, ss.sig + kSweepSources, args.sig);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(sg.nbx * sg.nby * sg.chunks()), 1, 1);
@@ -1007,7 +1017,7 @@ cudaError_t launch_sweep(const FusedMaps& maps, const StepParams& p, const Field
     cfg.numAttrs = 1;
     const bool idx32 = p.g.plane * (long long)(p.g.nz + 1) < (1LL << 31) && p.psi_total < (1LL << 31);
     cfg.dynamicSmemBytes = idx32 ? sweep_smem<uint32_t>() : sweep_smem<unsigned long long>();
-    const bool wide = cfg.gridDim.x <= kSweepWideCtas;
+    const bool wide = !ss.base && cfg.gridDim.x <= kSweepWideCtas;
     using K = void (*)(const SweepArgs);
     const K k = idx32 ? ss.mat ? wide ? K(k_sweep<uint32_t, true, true>) : K(k_sweep<uint32_t, true, false>)
                                : wide ? K(k_sweep<uint32_t, false, true>) : K(k_sweep<uint32_t, false, false>)

@@ -308,7 +308,9 @@ int fdtd_batch_adjoint(fdtd_handle* const* handles, int32_t n, int64_t steps, in
 /* ---- Batched launch (no reference counterpart: the reference runs one domain per process). A
  * batch advances many independent handles of any sizes together, its launches captured in CUDA
  * graphs, in one of three forms. Chains (cluster -1, the default): each instance runs its own
- * two-pass kernels on its own branch of the graph, every branch concurrent with the others. Flat
+ * kernels on its own branch of the graph, every branch concurrent with the others: in batches of
+ * 2.5 Mi cells and more the sweep for instances from 32 Ki cells on (unless the schedule is
+ * FDTD_SCHEDULE_TWO_PASS or second buffers do not fit), the two-pass kernels otherwise. Flat
  * (cluster 0): per step one E kernel and one H kernel over the 32 x 8 blocks of every plane of
  * every instance, one node per thread. Persistent (cluster 1, 2, 4 or 8): one kernel for all
  * steps, each instance owned by a thread-block cluster for all of its steps (E update, cluster

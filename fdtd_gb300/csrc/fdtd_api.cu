@@ -93,7 +93,8 @@ struct fdtd_handle {
     DeviceGrid g{};
     cudaStream_t stream = nullptr;
     int schedule = FDTD_SCHEDULE_AUTO;
-    int auto_choice = FDTD_SCHEDULE_AUTO;  // AUTO: the schedule its trial chose (AUTO = none yet)
+    int auto_choice = FDTD_SCHEDULE_AUTO;  // AUTO: the schedule chosen (AUTO = none yet)
+    long long auto_steps = 0;              // steps asked for under AUTO while none was
     int device = 0;
 
     // device state: two field buffers and two CPML memory sets; `cur` holds the current step.
@@ -156,7 +157,7 @@ struct fdtd_handle {
     PlateEdges* d_plates = nullptr;
     int* d_plate_k = nullptr;
     int4* d_plate_nodes = nullptr;
-    int n_plate_nodes = 0;
+    int n_plate_nodes = 0, n_plate_general = 0;
     Probe* d_probes = nullptr;
     int* d_probe_k = nullptr;
     int* d_probe_ids = nullptr;
@@ -277,6 +278,7 @@ StepParams make_params(fdtd_handle* h) {
     p.plate_k = h->plates.empty() ? nullptr : h->d_plate_k;
     p.plate_nodes = h->d_plate_nodes;
     p.n_plate_nodes = h->plates.empty() ? 0 : h->n_plate_nodes;
+    p.n_plate_general = h->n_plate_general;
     p.bg.mat = 0;  // the background material fills the CPML slabs in the usual layouts
     for (int a = 0; a < 3; ++a)
         for (int s = 0; s < 2; ++s) {
@@ -291,6 +293,17 @@ StepParams make_params(fdtd_handle* h) {
     std::copy(h->psi_off, h->psi_off + 6, p.psi_off);
     std::copy(h->psi_stride, h->psi_stride + 6, p.psi_stride);
     p.psi_total = h->psi_total;
+    if (h->slab_rows) {
+        const DeviceGrid& g = h->g;
+        const int L[3] = {g.pxn + g.pxp, g.pyn + g.pyp, g.pzn + g.pzp};
+        const float4* r = h->slab_rows;
+        for (int a = 0; a < 3; ++a) {
+            const long long n = (long long)h->n_coef_rows * L[a];
+            p.rows.e[a] = r;
+            p.rows.h[a] = r + n;
+            r += 2 * n;
+        }
+    }
     return p;
 }
 
@@ -365,20 +378,17 @@ void* tensor_map_encoder() {
 }
 
 // AUTO: the fused schedule (one sweep per step) or two passes, by the grid's cells. Measured on GB300,
-// two-pass against sweep per step, vacuum and random boxes: 40^3 13.8 / 8.6 and 15.2 / 10.5 us, 64^3
-// 19.0 / 11.9 and 19.1 / 15.4, 96^3 29.0 / 19.9 and 29.1 / 23.9, 112^3 39.7 / 37.4 and 40.0 / 38.8,
-// 128^3 50.0 / 50.3 and 51.3 / 51.6, 144^3 90.5 / 71.7 and 90.9 / 76.7, 200^3 226 / 139 and 227 / 144.
-// Between about 1 and 2.6 Mi cells, where the fields still sit in L2 and the sweep's CTAs fill the
-// device once, the two are level, and two-pass needs no second buffers; nor do grids below
-// kAutoSweepCells, a few CTAs' work. With materials in the CPML slabs (boxes that touch one face) the
-// tiles there take longer than the others and the range is wider: 64^3 18 / 12.5 us, 72^3 22 / 21,
-// 96^3 29 / 29, 112^3 39 / 46, 128^3 47 / 62, 160^3 97 / 113, 176^3 130 / 149, 200^3 178 / 157,
-// 225^3 253 / 217. Grids with a design region take the sweep from kAutoDesignCells
-// on (smaller ones record in their two-pass kernels). Two-pass also serves where the second buffers
-// cannot be allocated.
+// two-pass against sweep per step, boxes outside the CPML: 40^3 8.5 / 7.4 us, 64^3 11.3 / 10.4, 72^3 14.5 /
+// 15.9, 96^3 20.9 / 20.7, 112^3 31.7 / 34.3, 128^3 39.8 / 45.3, 136^3 60.0 / 59.0, 144^3 70 / 65, 160^3 89 / 78,
+// 200^3 175 / 129, 225^3 247 / 182. In between, where the fields sit in L2 and the sweep's CTAs do not
+// fill the device evenly, two-pass is ahead. Boxes that touch the CPML make the sweep's tiles there
+// slower than the others: 40^3 8.5 / 8.7 us, 64^3 11.3 / 12.5, 128^3 40 / 62, 160^3 90 / 113, 192^3 145 / 188,
+// 200^3 176 / 157, 225^3 253 / 217. Grids below kAutoSweepCells, a few CTAs' work, gain little. Grids with
+// a design region take the sweep from kAutoDesignCells on (smaller ones record in their two-pass
+// kernels). Two-pass also serves where the second buffers cannot be allocated.
 constexpr long long kAutoSweepCells = 32LL << 10;
-constexpr long long kAutoLevelLo = 1000LL << 10, kAutoLevelHi = 2600LL << 10;
-constexpr long long kAutoEdgeLo = 900LL << 10, kAutoEdgeHi = 6400LL << 10;  // with slab_rows
+constexpr long long kAutoTwoPassLo = 300LL << 10, kAutoTwoPassHi = 2450LL << 10;
+constexpr long long kAutoEdgeHi = 7400LL << 10;  // with slab_rows, two-pass below this
 constexpr long long kAutoDesignCells = 64LL << 20;
 
 // The background material's coefficients (StepParams::bgn), evaluated on the host with the rounding steps of
@@ -459,17 +469,25 @@ void release_fused(fdtd_handle* h) {
     h->have_second = false;
 }
 
-// AUTO's choice, made by the first step or by fdtd_tune_schedule. The second buffers are allocated
-// here, not under stream capture: a handle first stepped there takes two-pass until later.
-void auto_choose(fdtd_handle* h) {
+// AUTO's choice, made by fdtd_tune_schedule (n < 0) or by the call whose n steps bring the handle to
+// where the second buffers repay what it costs to allocate and free them: measured 0.2 ms at 64^3,
+// 0.55 at 256^3, 0.84 at 28 M cells, against the 1, 92 and 190 us that the sweep saves a step; some
+// 200 steps at 64^3, 20 at 160^3, 5 from 256^3 on. The buffers are allocated here, not under stream
+// capture: a handle stepped there takes two-pass until later.
+void auto_choose(fdtd_handle* h, int64_t n) {
     if (h->schedule != FDTD_SCHEDULE_AUTO || h->auto_choice != FDTD_SCHEDULE_AUTO) return;
     const long long cells = (long long)h->g.nx * h->g.ny * h->g.nz;
-    const long long lo = h->slab_rows ? kAutoEdgeLo : kAutoLevelLo, hi = h->slab_rows ? kAutoEdgeHi : kAutoLevelHi;
-    if (cells < (h->has_design ? kAutoDesignCells : kAutoSweepCells) || (cells >= lo && cells < hi)) {
+    const bool small = cells < kAutoTwoPassLo;
+    if (h->has_design ? cells < kAutoDesignCells
+        : h->slab_rows ? cells < kAutoEdgeHi
+                       : cells < kAutoSweepCells || (!small && cells < kAutoTwoPassHi)) {
         h->auto_choice = FDTD_SCHEDULE_TWO_PASS;
         return;
     }
     if (!h->have_second) {
+        if (n > 0) h->auto_steps += n;
+        const double saved = small ? 1.0 : std::max(1.0, 7e-6 * (cells - 2.2e6)), cost = 200.0 + 23e-6 * cells;
+        if (n >= 0 && h->auto_steps * saved < cost) return;
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
             cudaGetLastError();
@@ -618,7 +636,7 @@ int fdtd_set_schedule(fdtd_handle* h, int32_t schedule) {
     if (schedule < FDTD_SCHEDULE_AUTO || schedule > FDTD_SCHEDULE_FUSED_CPML)
         return fail(FDTD_ERR_INVALID, "unknown schedule");
     h->schedule = schedule;
-    h->auto_choice = FDTD_SCHEDULE_AUTO;  // AUTO runs its trial again
+    h->auto_choice = FDTD_SCHEDULE_AUTO;  // AUTO chooses again
     return FDTD_OK;
 }
 
@@ -869,18 +887,7 @@ namespace {
 // What the sweep of the handle's next step takes besides its fields; late: the step before it is
 // one of the same call, whose probes are still to be sampled.
 SweepStep sweep_step(const fdtd_handle* h, bool late) {
-    SweepStep s{h->d_probes_at, h->n_probes_at, late, nullptr, h->slab_rows != nullptr, {}, {}};
-    if (s.mat) {
-        const DeviceGrid& g = h->g;
-        const int L[3] = {g.pxn + g.pxp, g.pyn + g.pyp, g.pzn + g.pzp};
-        const float4* r = h->slab_rows;
-        for (int a = 0; a < 3; ++a) {
-            const long long n = (long long)h->n_coef_rows * L[a];
-            s.rows.e[a] = r;
-            s.rows.h[a] = r + n;
-            r += 2 * n;
-        }
-    }
+    SweepStep s{h->d_probes_at, h->n_probes_at, late, nullptr, h->slab_rows != nullptr, {}};
     for (size_t w = 0; w < h->waves.size() && w < (size_t)kSweepSources; ++w)
         s.sig[w] = h->step < (long long)h->waves[w].size() ? h->waves[w][(size_t)h->step] : 0.f;
     return s;
@@ -907,9 +914,10 @@ int steps_two_pass(fdtd_handle* h, const StepParams& p, int64_t n) {
     const int a = h->cur;
     FieldPtrs f{h->field[a][0], h->field[a][1], h->field[a][2], h->field[a][3], h->field[a][4], h->field[a][5]};
     for (int64_t s = 0; s < n; ++s) {
-        CUDA_TRY(launch_two_pass(p, f, h->psi[a], h->step, h->stream));
+        CUDA_TRY(launch_two_pass(p, f, h->psi[a], h->d_probes_at, h->n_probes_at, s > 0, h->step, h->stream));
         ++h->step;
     }
+    if (n > 0) CUDA_TRY(launch_sample_probes(p, f, h->d_probes_at, h->n_probes_at, nullptr, h->step - 1, h->stream));
     return FDTD_OK;
 }
 
@@ -921,7 +929,7 @@ int fdtd_step(fdtd_handle* h, int64_t n) {
     int rc = ensure_prepared(h);
     if (rc) return rc;
     StepParams p = make_params(h);
-    auto_choose(h);
+    auto_choose(h, n);
     return use_fused(h) ? steps_fused(h, p, n) : steps_two_pass(h, p, n);
 }
 
@@ -1089,7 +1097,7 @@ int fdtd_tune_schedule(fdtd_handle* h) {
     if (!h) return fail(FDTD_ERR_INVALID, "handle is NULL");
     int rc = ensure_prepared(h);
     if (rc) return rc;
-    auto_choose(h);
+    auto_choose(h, -1);
     return FDTD_OK;
 }
 
@@ -1503,6 +1511,11 @@ int ensure_prepared(fdtd_handle* h) {
         if (rc) return rc;
     }
     CUDA_TRY(launch_rec_probes(h->g, h->d_probes, (int)h->probes.size(), h->rec, h->stream));
+    h->n_plate_general = 0;
+    if (!h->plates.empty() && h->n_plate_nodes > 0) {
+        CUDA_TRY(launch_count_general(h->g, h->rec, h->d_plate_nodes, h->n_plate_nodes, h->small + 1, h->stream));
+        CUDA_TRY(cudaMemcpyAsync(&h->n_plate_general, h->small + 1, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    }
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     if (rows) {
         int rc = build_slab_rows(h);
@@ -1890,7 +1903,7 @@ int adj_forward_enqueue(fdtd_handle* h, int64_t n, int32_t checkpoint_every, int
         CUDA_TRY(launch_after_step(h->field[c][0], h->field[c][1], h->field[c][2], g, A.probe, nullptr, h->dbox, adj_slot(h, 0),
                                    h->stream));
     }
-    auto_choose(h);
+    auto_choose(h, n);
     // two-pass steps take their records in k_design_e (no launch of their own): the E of the
     // design edge box is final there, and so is every other E
     const bool two_pass = !use_fused(h);
@@ -1910,12 +1923,14 @@ int adj_forward_enqueue(fdtd_handle* h, int64_t n, int32_t checkpoint_every, int
         if (two_pass) {
             pa.fom_sample = A.samples + s;
             pa.design_snap = K == 0 ? adj_slot(h, s + 1) : nullptr;
-            CUDA_TRY(launch_two_pass(pa, cur_fields(h), h->psi[h->cur], h->step, h->stream));
+            CUDA_TRY(launch_two_pass(pa, cur_fields(h), h->psi[h->cur], h->d_probes_at, h->n_probes_at, s > 0, h->step, h->stream));
             ++h->step;
         } else if ((rc = adj_forward_step(h, A.samples + s, K == 0 ? adj_slot(h, s + 1) : nullptr))) {
             return rc;
         }
     }
+    if (two_pass && n > 0)
+        CUDA_TRY(launch_sample_probes(pa, cur_fields(h), h->d_probes_at, h->n_probes_at, nullptr, h->step - 1, h->stream));
     if ((rc = state_copy(h, adj_ckpt(h, A.ckpt_slots - 1), true))) return rc;  // final state
     CUDA_TRY(cudaMemcpyAsync(A.pinned_samples, A.samples, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost, h->stream));
     return FDTD_OK;
@@ -2171,9 +2186,9 @@ int batch_set_config(fdtd_batch* b, int cluster, int threads) {
 // Which instances' chains run the sweep: in a batch of at least kBatchSweepCells altogether, those from
 // kAutoSweepCells on whose schedule allows it and that have room for second buffers. Smaller batches
 // leave the device partly idle, and two passes have the shorter chain of dependent loads. Measured,
-// two-pass against sweep, ms for 32 steps of n cubes: 4 x 64^3 0.90 / 1.05, 2 x 96^3 1.17 / 1.39,
-// 16 x 40^3 1.78 / 1.81, 8 x 64^3 2.04 / 1.76, 8 x (32 to 96) 1.56 / 1.99, 16 x 48^3 2.73 / 2.17, 4 x 96^3
-// 3.08 / 2.37, 16 x (32 to 96) 4.74 / 3.93, 64 x 40^3 9.3 / 6.2, 64 x 64^3 21.3 / 12.0, 16 x 128^3 25.4 / 15.7.
+// two-pass against sweep, ms for 32 steps of n cubes: 4 x 64^3 0.77 / 1.05, 2 x 96^3 1.02 / 1.38,
+// 16 x 40^3 1.40 / 1.83, 8 x 64^3 1.61 / 1.78, 16 x 48^3 2.11 / 2.18, 16 x 56^3 3.6 / 2.8, 4 x 96^3 2.67 / 2.36,
+// 16 x (32 to 96) 4.24 / 3.96, 64 x 40^3 8.5 / 6.2, 64 x 64^3 18.7 / 12.0, 16 x 128^3 23.2 / 15.7.
 constexpr long long kBatchSweepCells = 2560LL << 10;
 void batch_choose(fdtd_batch* b) {
     auto cells = [](const fdtd_handle* h) { return (long long)h->g.nx * h->g.ny * h->g.nz; };
@@ -2241,7 +2256,9 @@ int batch_graph(fdtd_batch* b, long long steps, cudaGraphExec_t* out) {
             e = cudaStreamWaitEvent(cs, b->chain_events[0], 0);
             if (e == cudaSuccess && b->sweep[q]) e = chain_sweep(b, q, steps, cs);
             for (long long t = 0; t < steps && e == cudaSuccess && !b->sweep[q]; ++t)
-                e = launch_two_pass_rel(I.p, I.f, I.ps, &b->d_inst[q].step, (int)t, cs);
+                e = launch_two_pass_rel(I.p, I.f, I.ps, b->hs[q]->d_probes_at, b->hs[q]->n_probes_at, &b->d_inst[q].step, (int)t, cs);
+            if (e == cudaSuccess && !b->sweep[q])
+                e = launch_sample_probes(I.p, I.f, b->hs[q]->d_probes_at, b->hs[q]->n_probes_at, &b->d_inst[q].step, steps - 1, cs);
             if (e == cudaSuccess) e = cudaEventRecord(b->chain_events[1 + q], cs);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream, b->chain_events[1 + q], 0);
         }
@@ -2288,8 +2305,6 @@ unsigned long long descriptor_signature(const fdtd_batch* b) {
         word((unsigned long long)(uintptr_t)x->psi_base[1]);
         word((unsigned long long)(uintptr_t)x->d_probes_at);
         word((unsigned long long)x->n_probes_at);
-        word((unsigned long long)(uintptr_t)x->slab_rows);
-        word((unsigned long long)x->n_coef_rows);
     }
     return h;
 }

@@ -133,6 +133,15 @@ struct ProbeAt {
     long long node;
 };
 
+// Coefficients of the CPML slabs by coefficient row, for nodes whose row is not the background's: entry
+// (row, l) of axis a at e[a][row * (the axis's slab planes) + l], l counting the low slab's planes and
+// then the high slab's: the two E curl coefficients along the axis over kappa, then the factors of the
+// CPML memory; likewise h.
+struct SlabRows {
+    const float4* e[3];
+    const float4* h[3];
+};
+
 // Everything an update kernel reads besides the fields.
 struct StepParams {
     DeviceGrid g;
@@ -177,6 +186,7 @@ struct StepParams {
     // psi_off[f] + a * psi_stride[f] floats
     long long psi_off[6], psi_stride[6];
     long long psi_total;
+    SlabRows rows;  // e[0] NULL: not built (no such nodes, or too many rows)
     // design region: cells of material kDesign inside dbox = [d0,d3) x [d1,d4) x [d2,d5) take eps_r
     // from deps ((d5-d2), (d4-d1), (d3-d0), x fastest); NULL when the handle has none
     const float* deps;
@@ -187,6 +197,7 @@ struct StepParams {
     const int* plate_k;
     const int4* plate_nodes;     // nodes of class kPlateNode {i, j, k, 0} (updated by k_plate_e)
     int n_plate_nodes;
+    int n_plate_general;         // those of them without a coefficient row
     // records of an adjoint run that k_design_e takes in two-pass steps (NULL otherwise): the new
     // E of the design edge box into design_snap (three arrays of the box volume, x fastest), and
     // the FoM sample Ez into *fom_sample, from the design node fom_node when the probe is one

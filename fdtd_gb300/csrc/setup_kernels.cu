@@ -540,6 +540,19 @@ cudaError_t launch_rec_probes(const DeviceGrid& g, const Probe* probes, int n, u
     return cudaGetLastError();
 }
 
+// How many of the listed nodes take the general path.
+__global__ void k_count_general(const uint16_t* rec, DeviceGrid g, const int4* nodes, int n, int* count) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < n && rec[(long long)nodes[q].z * g.plane + (long long)nodes[q].y * g.pitch + nodes[q].x] >= kRecGeneral) atomicAdd(count, 1);
+}
+
+cudaError_t launch_count_general(const DeviceGrid& g, const uint16_t* rec, const int4* nodes, int n, int* count, cudaStream_t st) {
+    const cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int), st);
+    if (e != cudaSuccess || n <= 0) return e;
+    k_count_general<<<(n + 127) / 128, 128, 0, st>>>(rec, g, nodes, n, count);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_rec_general(const DeviceGrid& g, const LumpedEdge* edges, int n_edges, uint16_t* rec, cudaStream_t st) {
     if (n_edges <= 0) return cudaSuccess;
     k_rec_general<<<(n_edges + 127) / 128, 128, 0, st>>>(rec, g, edges, n_edges);

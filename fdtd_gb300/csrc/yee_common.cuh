@@ -222,6 +222,17 @@ __device__ __forceinline__ void sample(const StepParams& p, long long row, int c
     }
 }
 
+// The value of probe r at step m from the step's finished fields.
+template <class Fields>
+__device__ __forceinline__ void sample_at(const ProbeAt& r, const Fields& f, const StepParams& p, long long m) {
+    const float* c[6] = {f.ex, f.ey, f.ez, f.hx, f.hy, f.hz};
+    const float* a = c[0];
+#pragma unroll
+    for (int q = 1; q < 6; ++q)
+        if (r.comp == q) a = c[q];
+    p.probe_ring[m % p.ring_cap * p.n_probes + r.id] = a[r.node];
+}
+
 // Neighbourhood of E(i,j,k): old E, H at the node and its lower neighbours, and the materials of the
 // seven cells the three edge averages touch. Entries whose neighbour lies outside the grid are never
 // used (the masks exclude those edges).

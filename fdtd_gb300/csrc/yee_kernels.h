@@ -21,9 +21,11 @@ struct PsiSet {
     long long pad;
 };
 
-// One time step m with the two-pass schedule (E pass then H pass, in place).
-cudaError_t launch_two_pass(const StepParams& p, const FieldPtrs& f, const PsiSet& ps, long long m,
-                            cudaStream_t st);
+// One time step m with the two-pass schedule (E pass then H pass, in place). probes: those outside the
+// CPML slabs; late: step m - 1 belongs to the same call, and its H probes are sampled here. After a call's
+// last step launch_sample_probes does that.
+cudaError_t launch_two_pass(const StepParams& p, const FieldPtrs& f, const PsiSet& ps, const ProbeAt* probes, int n_probes, bool late,
+                            long long m, cudaStream_t st);
 
 // A box of nodes [x0, x1) x [y0, y1) x [z0, z1).
 struct NodeBox {
@@ -35,19 +37,20 @@ struct NodeBox {
 cudaError_t launch_two_pass_box(const StepParams& p, const FieldPtrs& f, const PsiSet& ps, const NodeBox& b, long long m,
                                 cudaStream_t st);
 
-// One two-pass step whose step index is *base + s (device counter), for graph replay; handles
-// without a design region or plates only.
-cudaError_t launch_two_pass_rel(const StepParams& p, const FieldPtrs& f, const PsiSet& ps, const long long* base, int s,
-                                cudaStream_t st);
+// One two-pass step whose step index is *base + s (device counter; s counts a call's steps), for graph
+// replay; handles without a design region or plates only.
+cudaError_t launch_two_pass_rel(const StepParams& p, const FieldPtrs& f, const PsiSet& ps, const ProbeAt* probes, int n_probes,
+                                const long long* base, int s, cudaStream_t st);
 
 // E of the design region's nodes, fi/pin -> fo/pout, after a schedule's E kernels; nothing
 // without a design region.
 cudaError_t launch_design_e(const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fo, const PsiSet& pin,
                             const PsiSet& pout, long long m, cudaStream_t st);
 
-// E of the plate nodes (StepParams::plate_nodes), fi/pin -> fo/pout, after a schedule's E kernels.
+// E of the plate nodes (StepParams::plate_nodes), fi/pin -> fo/pout, after a schedule's E kernels; rows:
+// of those without a coefficient row only.
 cudaError_t launch_plate_e(const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fo, const PsiSet& pin,
-                           const PsiSet& pout, long long m, cudaStream_t st);
+                           const PsiSet& pout, bool rows, long long m, cudaStream_t st);
 
 // Fused schedule (yee_sweep.cu): one kernel per time step sweeps the whole grid, fields A -> B,
 // CPML memory pin -> pout.
@@ -56,14 +59,7 @@ struct FusedMaps {  // tensor maps of buffer A
     CUtensorMap e[3];
     CUtensorMap rec;  // coefficient rows (StepParams::rec)
 };
-// Coefficients of the CPML slabs by coefficient row, for the sweep's nodes whose row is not the
-// background's: entry (row, l) of axis a at e[a][row * (the axis's slab planes) + l], l counting the
-// low slab's planes and then the high slab's: the two E curl coefficients along the axis over kappa,
-// then the factors of the CPML memory; likewise h.
-struct SlabRows {
-    const float4* e[3];
-    const float4* h[3];
-};
+cudaError_t launch_count_general(const DeviceGrid& g, const uint16_t* rec, const int4* nodes, int n, int* count, cudaStream_t st);
 cudaError_t launch_slab_rows(const DeviceGrid& g, const MatCoef* coef, int n_rows, float* const prof_kappa[6], float4* out,
                              cudaStream_t st);
 
@@ -75,7 +71,6 @@ struct SweepStep {
     const long long* base;  // device step counter that m counts from (captured launches), or NULL: the
                             // sources' signals are then read on the device
     int mat;                // coefficient rows other than the background's in a CPML slab or on a low wall
-    SlabRows rows;          // with mat
     float sig[kSweepSources];
 };
 cudaError_t sweep_configure();

@@ -113,7 +113,6 @@ struct SweepArgs {
     const ProbeAt* probes;  // probes outside the CPML slabs (n of them), sampled one step late: see k_sweep
     int n_probes_at;
     int late;               // the step before this one belongs to the same call
-    SlabRows rows;          // kMat
     float sig[kSweepSources];  // this step's signal of each source
 };
 
@@ -201,15 +200,6 @@ __device__ __forceinline__ void slow_node(const SweepArgs* pa, SweepSmem<Idx>* p
             for (int a = 0; a < 3; ++a) sample(p, rr, 3 + a, i, j, kh, pre[a]);
     }
     fo.hx[n] = out[0]; fo.hy[n] = out[1]; fo.hz[n] = out[2];
-}
-
-__device__ __forceinline__ void sample_at(const ProbeAt& r, const FieldPtrs& f, const StepParams& p, long long m) {
-    const float* c[6] = {f.ex, f.ey, f.ez, f.hx, f.hy, f.hz};
-    const float* a = c[0];
-#pragma unroll
-    for (int q = 1; q < 6; ++q)
-        if (r.comp == q) a = c[q];
-    p.probe_ring[m % p.ring_cap * p.n_probes + r.id] = a[r.node];
 }
 
 struct Quad {
@@ -317,7 +307,7 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
     const int Lx = g.pxn + g.pxp, Ly = g.pyn + g.pyp, Lz = g.pzn + g.pzp;
     const int lx = i < g.pxn ? i : i - (g.nx - Lx), ly = j < g.pyn ? j : j - (g.ny - Ly);
     auto lz = [&](int k) { return k < g.pzn ? k : k - (g.nz - Lz); };
-    const SlabRows& SR = A.rows;
+    const SlabRows& SR = p.rows;
     const Idx nij = (Idx)j * (Idx)g.pitch + (Idx)i;
     Idx n = (Idx)k0 * (Idx)g.plane + nij;
     const int bgm = p.bg.mat;
@@ -948,10 +938,9 @@ __global__ void __launch_bounds__(NTH, kWide ? 2 : 3) k_sweep(const __grid_const
     // Probes outside the CPML slabs hold the step's final values, so they are read from the finished
     // fields: here the step before (its fields are this step's input), and after a call's last step by
     // k_sample_probes. Probes inside a slab are sampled by the slow path, before the CPML correction.
-    if (A.late && blockIdx.x * NTH < (unsigned)A.n_probes_at) {
-        const int q = blockIdx.x * NTH + tid;
-        if (q < A.n_probes_at) sample_at(A.probes[q], A.fi, p, S.m - 1);
-    }
+    if (A.late)
+        for (long long q = (long long)blockIdx.x * NTH + tid; q < A.n_probes_at; q += (long long)gridDim.x * NTH)
+            sample_at(A.probes[q], A.fi, p, S.m - 1);
     // own quads, then those of the halo row and the halo column (spare threads repeat the last one)
     const bool own = tid < NOWN;
     const int h = min(tid - NOWN, QX + TY - 1);
@@ -989,40 +978,22 @@ __global__ void k_sample_probes(const __grid_constant__ StepParams p, const __gr
 cudaError_t launch_sample_probes(const StepParams& p, const FieldPtrs& f, const ProbeAt* probes, int n, const long long* base,
                                  long long m, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(n + 127) / 128, 1, 1);
-    cfg.blockDim = dim3(128, 1, 1);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_sample_probes, p, f, probes, n, base, m);
+    return launch_dependent(k_sample_probes, dim3((unsigned)(n + 127) / 128), dim3(128), 0, st, p, f, probes, n, base, m);
 }
 
 cudaError_t launch_sweep(const FusedMaps& maps, const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fo,
                          const PsiSet& pin, const PsiSet& pout, const SweepPlan& sg, const SweepStep& ss, long long m,
                          cudaStream_t st) {
-    SweepArgs args{maps, p, fo, pin, pout, sg, m, ss.base, fi, ss.probes, ss.n_probes, ss.late, ss.rows, {}};
+    SweepArgs args{maps, p, fo, pin, pout, sg, m, ss.base, fi, ss.probes, ss.n_probes, ss.late, {}};
     std::copy(ss.sig, ss.sig + kSweepSources, args.sig);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(sg.nbx * sg.nby * sg.chunks()), 1, 1);
-    cfg.blockDim = dim3(NTH, 1, 1);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     const bool idx32 = p.g.plane * (long long)(p.g.nz + 1) < (1LL << 31) && p.psi_total < (1LL << 31);
-    cfg.dynamicSmemBytes = idx32 ? sweep_smem<uint32_t>() : sweep_smem<unsigned long long>();
-    const bool wide = !ss.base && cfg.gridDim.x <= kSweepWideCtas;
+    const unsigned ctas = (unsigned)(sg.nbx * sg.nby * sg.chunks());
+    const bool wide = !ss.base && ctas <= kSweepWideCtas;
     using K = void (*)(const SweepArgs);
     const K k = idx32 ? ss.mat ? wide ? K(k_sweep<uint32_t, true, true>) : K(k_sweep<uint32_t, true, false>)
                                : wide ? K(k_sweep<uint32_t, false, true>) : K(k_sweep<uint32_t, false, false>)
                       : ss.mat ? K(k_sweep<unsigned long long, true, false>) : K(k_sweep<unsigned long long, false, false>);
-    return cudaLaunchKernelEx(&cfg, k, args);
+    return launch_dependent(k, dim3(ctas), dim3(NTH), idx32 ? sweep_smem<uint32_t>() : sweep_smem<unsigned long long>(), st, args);
 }
 
 // Tensor maps of the sweep: H tiles with a one-node halo (x from 4 nodes before the tile: a TMA box

@@ -2,33 +2,70 @@
 //
 // This is the reference's own order of work (calc_e then calc_h, solver fdtdrav.h:3222-3333)
 // expressed over the compact data layout. It runs at any grid size and is the schedule the fused
-// sweep is checked against bit for bit; both call the same e_update / h_update.
-#include "node_global.cuh"
+// sweep is checked against bit for bit; both call the same update primitives (yee_common.cuh).
+//
+// Every pass may start while the one before it drains (launch_dependent): on small grids, a few
+// microseconds of work a pass, that and the shorter passes by row took a step of 24^3 from 13.5 to 7.5 us,
+// of 64^3 from 17.5 to 11.3.
+#include "node_rows.cuh"
+#include "tma.cuh"
 
 namespace fdtd {
 
-// CTAs of 256 per SM the one-node-per-thread kernels are compiled for: 6 caps them at 40 registers
-// (48 warps resident; the general path spills a few words), which measured 4-7 % faster at 512^3
-// than the compiler's own choice of 48 registers (5 CTAs).
-#ifndef FDTD_TWO_PASS_MIN_BLOCKS
-#define FDTD_TWO_PASS_MIN_BLOCKS 6
-#endif
-template <typename Idx>
-__global__ void __launch_bounds__(256, FDTD_TWO_PASS_MIN_BLOCKS) k_update_e(const __grid_constant__ StepParams p, FieldPtrs f,
-                                                  const __grid_constant__ PsiSet ps, long long m) {
-    const int i = blockIdx.x * 32 + threadIdx.x;
-    const int j = blockIdx.y * 8 + threadIdx.y;
-    if (i >= p.g.nx || j >= p.g.ny) return;
-    e_node_global<false, false, false, Idx>(p, f, f, ps, ps, i, j, blockIdx.z, m);
+// Grids of up to this many nodes take the kernels by coefficient row (node_rows.cuh), larger ones those
+// by node class (node_global.cuh), whose byte per node and sixth CTA an SM tell where HBM bounds the
+// pass. Per step, class / row: 128^3 45.2 / 39.8 us, 160^3 94 / 89, 200^3 174 / 175, 225^3 248 / 259, 400^3 1082 /
+// 1172.
+constexpr long long kRowsNodes = 7LL << 20;
+
+// CTAs of 256 per SM the kernels are compiled for. By class: 6 caps them at 40 registers (48 warps
+// resident; the general path spills a few words), which measured 4-7 % faster at 512^3 than the
+// compiler's own choice of 48 registers (5 CTAs). By row: 5, without spills in the common path
+// (128^3: 6 CTAs 42.0, 5 CTAs 39.9, 4 CTAs 43.6 us).
+template <bool kRows>
+constexpr int kCtas = kRows ? 5 : 6;
+
+// The nodes [b.x0, b.x1) x [b.y0, b.y1) x [b.z0, ..).
+// Probes outside the CPML slabs hold the step's final values, so the kernels by row read them from the
+// finished fields, a thread per probe: the H pass E's of its step, the next step's E pass H's (`late`,
+// a step of the same call), and k_sample_probes those of a call's last step. (Kernels by class look
+// each node up in its plane's list, which on a plane of 30 probes takes longer than the update.) Probes in
+// a slab hold the value before the CPML correction and are the general path's.
+struct ProbeList {
+    const ProbeAt* at;
+    int n, late;
+};
+__device__ __forceinline__ void sample_list(const StepParams& p, const FieldPtrs& f, const ProbeList& l, bool h, long long m) {
+    const long long block = ((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+    for (long long q = block * 256 + threadIdx.y * 32 + threadIdx.x; q < l.n; q += 256LL * gridDim.x * gridDim.y * gridDim.z) {
+        const ProbeAt r = l.at[q];
+        if ((r.comp >= 3) == h) sample_at(r, f, p, m);
+    }
 }
 
-template <typename Idx>
-__global__ void __launch_bounds__(256, FDTD_TWO_PASS_MIN_BLOCKS) k_update_h(const __grid_constant__ StepParams p, FieldPtrs f,
-                                                  const __grid_constant__ PsiSet ps, long long m) {
-    const int i = blockIdx.x * 32 + threadIdx.x;
-    const int j = blockIdx.y * 8 + threadIdx.y;
-    if (i >= p.g.nx || j >= p.g.ny) return;
-    h_node_global<false, Idx>(p, f, f, f, ps, ps, i, j, blockIdx.z, m);
+template <typename Idx, bool kRows>
+__global__ void __launch_bounds__(256, kCtas<kRows>)
+    k_update_e(const __grid_constant__ StepParams p, const __grid_constant__ FieldPtrs f, const __grid_constant__ PsiSet ps,
+               const __grid_constant__ NodeBox b, const __grid_constant__ ProbeList probes, const __grid_constant__ StepIndex step) {
+    grid_dependency_wait();
+    grid_launch_dependents();
+    if (kRows && probes.late) sample_list(p, f, probes, true, step.at() - 1);
+    const int i = b.x0 + blockIdx.x * 32 + threadIdx.x, j = b.y0 + blockIdx.y * 8 + threadIdx.y, k = b.z0 + blockIdx.z;
+    if (i >= b.x1 || j >= b.y1) return;
+    if constexpr (kRows) e_node_rows<Idx>(p, f, ps, i, j, k, step);
+    else e_node_global<false, false, false, Idx>(p, f, f, ps, ps, i, j, k, step.at());
+}
+template <typename Idx, bool kRows>
+__global__ void __launch_bounds__(256, kCtas<kRows>)
+    k_update_h(const __grid_constant__ StepParams p, const __grid_constant__ FieldPtrs f, const __grid_constant__ PsiSet ps,
+               const __grid_constant__ NodeBox b, const __grid_constant__ ProbeList probes, const __grid_constant__ StepIndex step) {
+    grid_dependency_wait();
+    grid_launch_dependents();
+    if (kRows && probes.n > 0) sample_list(p, f, probes, false, step.at());
+    const int i = b.x0 + blockIdx.x * 32 + threadIdx.x, j = b.y0 + blockIdx.y * 8 + threadIdx.y, k = b.z0 + blockIdx.z;
+    if (i >= b.x1 || j >= b.y1) return;
+    if constexpr (kRows) h_node_rows<Idx>(p, f, ps, i, j, k, step);
+    else h_node_global<false, Idx>(p, f, f, f, ps, ps, i, j, k, step.at());
 }
 
 // E of the nodes of the design region's edge box [d0, d3] x [d1, d4] x [d2, d5] (node class
@@ -50,20 +87,22 @@ __global__ void __launch_bounds__(256) k_design_e(const __grid_constant__ StepPa
 }
 
 // E of the nodes with a plate-covered edge (node class kPlateNode, which the other E kernels leave
-// alone): one thread per listed node, plate-aware coefficients.
+// alone): one thread per listed node, plate-aware coefficients. rows: k_update_e has done those that have
+// a coefficient row (all but probes and lumped edges in a slab and rows beyond the table).
 __global__ void __launch_bounds__(128) k_plate_e(const __grid_constant__ StepParams p, FieldPtrs fi, FieldPtrs fo,
                                                  const __grid_constant__ PsiSet pin,
-                                                 const __grid_constant__ PsiSet pout, long long m) {
+                                                 const __grid_constant__ PsiSet pout, bool rows, long long m) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= p.n_plate_nodes) return;
     const int4 v = p.plate_nodes[q];
+    if (rows && p.rec[(long long)v.z * p.g.plane + (long long)v.y * p.g.pitch + v.x] < kRecGeneral) return;
     e_node_global<false, false, true>(p, fi, fo, pin, pout, v.x, v.y, v.z, m);
 }
 
 cudaError_t launch_plate_e(const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fo, const PsiSet& pin,
-                           const PsiSet& pout, long long m, cudaStream_t st) {
-    if (p.n_plate_nodes <= 0) return cudaSuccess;
-    k_plate_e<<<(p.n_plate_nodes + 127) / 128, 128, 0, st>>>(p, fi, fo, pin, pout, m);
+                           const PsiSet& pout, bool rows, long long m, cudaStream_t st) {
+    if ((rows ? p.n_plate_general : p.n_plate_nodes) <= 0) return cudaSuccess;
+    k_plate_e<<<(p.n_plate_nodes + 127) / 128, 128, 0, st>>>(p, fi, fo, pin, pout, rows, m);
     return cudaGetLastError();
 }
 
@@ -76,98 +115,47 @@ cudaError_t launch_design_e(const StepParams& p, const FieldPtrs& fi, const Fiel
     return cudaGetLastError();
 }
 
-// Two-pass kernels whose step index is *base + s: a CUDA graph captured once replays them while
-// a counter on the device advances (the batched chain form).
-template <typename Idx>
-__global__ void __launch_bounds__(256, FDTD_TWO_PASS_MIN_BLOCKS) k_update_e_rel(const __grid_constant__ StepParams p,
-                                                                                 FieldPtrs f,
-                                                                                 const __grid_constant__ PsiSet ps,
-                                                                                 const long long* __restrict__ base, int s) {
-    const int i = blockIdx.x * 32 + threadIdx.x;
-    const int j = blockIdx.y * 8 + threadIdx.y;
-    if (i >= p.g.nx || j >= p.g.ny) return;
-    e_node_global<false, false, false, Idx>(p, f, f, ps, ps, i, j, blockIdx.z, *base + s);
-}
-template <typename Idx>
-__global__ void __launch_bounds__(256, FDTD_TWO_PASS_MIN_BLOCKS) k_update_h_rel(const __grid_constant__ StepParams p,
-                                                                                 FieldPtrs f,
-                                                                                 const __grid_constant__ PsiSet ps,
-                                                                                 const long long* __restrict__ base, int s) {
-    const int i = blockIdx.x * 32 + threadIdx.x;
-    const int j = blockIdx.y * 8 + threadIdx.y;
-    if (i >= p.g.nx || j >= p.g.ny) return;
-    h_node_global<false, Idx>(p, f, f, f, ps, ps, i, j, blockIdx.z, *base + s);
+template <typename Idx, bool kRows>
+static cudaError_t two_pass(const StepParams& p, const FieldPtrs& f, const PsiSet& ps, const NodeBox& b, const ProbeList& probes,
+                            const StepIndex& step, cudaStream_t st) {
+    const dim3 grid((b.x1 - b.x0 + 31) / 32, (b.y1 - b.y0 + 7) / 8, b.z1 - b.z0), block(32, 8, 1);
+    cudaError_t e = launch_dependent(k_update_e<Idx, kRows>, grid, block, 0, st, p, f, ps, b, probes, step);
+    if (e == cudaSuccess) e = launch_design_e(p, f, f, ps, ps, step.m, st);
+    if (e == cudaSuccess) e = launch_plate_e(p, f, f, ps, ps, kRows, step.m, st);
+    if (e == cudaSuccess) e = launch_dependent(k_update_h<Idx, kRows>, grid, block, 0, st, p, f, ps, b, probes, step);
+    return e;
 }
 
-cudaError_t launch_two_pass_rel(const StepParams& p, const FieldPtrs& f, const PsiSet& ps, const long long* base, int s,
-                                cudaStream_t st) {
+// One step over the nodes of b: E, the design region's and the plate nodes' E, H.
+static cudaError_t two_pass(const StepParams& p, const FieldPtrs& f, const PsiSet& ps, const NodeBox& b, const ProbeList& probes,
+                            const StepIndex& step, cudaStream_t st) {
+    const DeviceGrid& g = p.g;
+    // 32-bit node offsets when every offset (plus one plane of lookahead) fits
+    if (g.plane * (long long)(g.nz + 1) >= (1LL << 31)) return two_pass<long long, false>(p, f, ps, b, probes, step, st);
+    if ((long long)g.nx * g.ny * g.nz > kRowsNodes) return two_pass<uint32_t, false>(p, f, ps, b, probes, step, st);
+    return two_pass<uint32_t, true>(p, f, ps, b, probes, step, st);
+}
+
+cudaError_t launch_two_pass_rel(const StepParams& p, const FieldPtrs& f, const PsiSet& ps, const ProbeAt* probes, int n_probes,
+                                const long long* base, int s, cudaStream_t st) {
     if (p.deps || p.n_plate_nodes > 0) return cudaErrorInvalidValue;  // no design region, no plates
-    dim3 block(32, 8, 1);
-    dim3 grid((p.g.nx + 31) / 32, (p.g.ny + 7) / 8, p.g.nz);
-    const bool idx32 = p.g.plane * (long long)(p.g.nz + 1) < (1LL << 31);
-    if (idx32) k_update_e_rel<uint32_t><<<grid, block, 0, st>>>(p, f, ps, base, s);
-    else k_update_e_rel<long long><<<grid, block, 0, st>>>(p, f, ps, base, s);
-    if (idx32) k_update_h_rel<uint32_t><<<grid, block, 0, st>>>(p, f, ps, base, s);
-    else k_update_h_rel<long long><<<grid, block, 0, st>>>(p, f, ps, base, s);
-    return cudaGetLastError();
+    return two_pass(p, f, ps, NodeBox{0, 0, 0, p.g.nx, p.g.ny, p.g.nz}, ProbeList{probes, n_probes, s > 0}, StepIndex{base, s}, st);
 }
 
-// Two-pass kernels over the nodes [b.x0, b.x1) x [b.y0, b.y1) x [b.z0, b.z1) only (the adjoint's
-// segment recompute, whose nodes outside a shrinking box around the design region are never read
-// again). Same per-node code, so the nodes inside give the same bits as a whole-grid step.
-template <typename Idx>
-__global__ void __launch_bounds__(256, FDTD_TWO_PASS_MIN_BLOCKS) k_update_e_box(const __grid_constant__ StepParams p,
-                                                                                 FieldPtrs f,
-                                                                                 const __grid_constant__ PsiSet ps,
-                                                                                 NodeBox b, long long m) {
-    const int i = b.x0 + blockIdx.x * 32 + threadIdx.x;
-    const int j = b.y0 + blockIdx.y * 8 + threadIdx.y;
-    if (i >= b.x1 || j >= b.y1) return;
-    e_node_global<false, false, false, Idx>(p, f, f, ps, ps, i, j, b.z0 + blockIdx.z, m);
-}
-template <typename Idx>
-__global__ void __launch_bounds__(256, FDTD_TWO_PASS_MIN_BLOCKS) k_update_h_box(const __grid_constant__ StepParams p,
-                                                                                 FieldPtrs f,
-                                                                                 const __grid_constant__ PsiSet ps,
-                                                                                 NodeBox b, long long m) {
-    const int i = b.x0 + blockIdx.x * 32 + threadIdx.x;
-    const int j = b.y0 + blockIdx.y * 8 + threadIdx.y;
-    if (i >= b.x1 || j >= b.y1) return;
-    h_node_global<false, Idx>(p, f, f, f, ps, ps, i, j, b.z0 + blockIdx.z, m);
-}
-
+// The nodes [b.x0, b.x1) x [b.y0, b.y1) x [b.z0, b.z1) only (the adjoint's segment recompute, whose
+// nodes outside a shrinking box around the design region are never read again). Same per-node code, so
+// the nodes inside give the same bits as a whole-grid step; the steps' probes stand in the ring already.
 cudaError_t launch_two_pass_box(const StepParams& p, const FieldPtrs& f, const PsiSet& ps, const NodeBox& b, long long m,
                                 cudaStream_t st) {
     const DeviceGrid& g = p.g;
     if (b.x0 < 0 || b.y0 < 0 || b.z0 < 0 || b.x1 > g.nx || b.y1 > g.ny || b.z1 > g.nz) return cudaErrorInvalidValue;
     if (b.x1 <= b.x0 || b.y1 <= b.y0 || b.z1 <= b.z0) return cudaSuccess;
-    const dim3 block(32, 8, 1);
-    const dim3 grid((b.x1 - b.x0 + 31) / 32, (b.y1 - b.y0 + 7) / 8, b.z1 - b.z0);
-    const bool idx32 = g.plane * (long long)(g.nz + 1) < (1LL << 31);
-    if (idx32) k_update_e_box<uint32_t><<<grid, block, 0, st>>>(p, f, ps, b, m);
-    else k_update_e_box<long long><<<grid, block, 0, st>>>(p, f, ps, b, m);
-    cudaError_t e = launch_design_e(p, f, f, ps, ps, m, st);
-    if (e == cudaSuccess) e = launch_plate_e(p, f, f, ps, ps, m, st);
-    if (e != cudaSuccess) return e;
-    if (idx32) k_update_h_box<uint32_t><<<grid, block, 0, st>>>(p, f, ps, b, m);
-    else k_update_h_box<long long><<<grid, block, 0, st>>>(p, f, ps, b, m);
-    return cudaGetLastError();
+    return two_pass(p, f, ps, b, ProbeList{}, StepIndex{nullptr, m}, st);
 }
 
-cudaError_t launch_two_pass(const StepParams& p, const FieldPtrs& f, const PsiSet& ps, long long m,
-                            cudaStream_t st) {
-    dim3 block(32, 8, 1);
-    dim3 grid((p.g.nx + 31) / 32, (p.g.ny + 7) / 8, p.g.nz);
-    // 32-bit node offsets when every offset (plus one plane of lookahead) fits
-    const bool idx32 = p.g.plane * (long long)(p.g.nz + 1) < (1LL << 31);
-    if (idx32) k_update_e<uint32_t><<<grid, block, 0, st>>>(p, f, ps, m);
-    else k_update_e<long long><<<grid, block, 0, st>>>(p, f, ps, m);
-    cudaError_t e = launch_design_e(p, f, f, ps, ps, m, st);
-    if (e == cudaSuccess) e = launch_plate_e(p, f, f, ps, ps, m, st);
-    if (e != cudaSuccess) return e;
-    if (idx32) k_update_h<uint32_t><<<grid, block, 0, st>>>(p, f, ps, m);
-    else k_update_h<long long><<<grid, block, 0, st>>>(p, f, ps, m);
-    return cudaGetLastError();
+cudaError_t launch_two_pass(const StepParams& p, const FieldPtrs& f, const PsiSet& ps, const ProbeAt* probes, int n_probes, bool late,
+                            long long m, cudaStream_t st) {
+    return two_pass(p, f, ps, NodeBox{0, 0, 0, p.g.nx, p.g.ny, p.g.nz}, ProbeList{probes, n_probes, late}, StepIndex{nullptr, m}, st);
 }
 
 }  // namespace fdtd

@@ -36,9 +36,10 @@ enum { FDTD_EX = 0, FDTD_EY = 1, FDTD_EZ = 2, FDTD_HX = 3, FDTD_HY = 4, FDTD_HZ 
 
 /* Update-kernel schedules (fdtd_set_schedule). */
 enum {
-    FDTD_SCHEDULE_AUTO = 0,   /* FUSED or TWO_PASS by the grid's size (the measured faster one),
-                                 chosen by the first step or fdtd_tune_schedule; TWO_PASS where the
-                                 second buffers do not fit or the first step is captured */
+    FDTD_SCHEDULE_AUTO = 0,   /* FUSED or TWO_PASS by the grid's size (the measured faster one);
+                                 TWO_PASS until the steps asked for repay FUSED's second buffers
+                                 (5 to 200, fewer the larger the grid; or fdtd_tune_schedule) and
+                                 where those do not fit or the step is captured */
     FDTD_SCHEDULE_TWO_PASS = 1, /* E pass then H pass per step, in place (the reference's order) */
     FDTD_SCHEDULE_FUSED = 2,  /* one z-marching sweep of the whole grid per step over ping-pong
                                  field buffers (second buffers are allocated by the first step)  */

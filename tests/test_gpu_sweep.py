@@ -114,3 +114,26 @@ def test_sweep_plates_sources_and_background(gpu_lib, seed):
               background=S.Material(eps_r=2.0, sigma_e=0.01, mu_r=1.5, sigma_m=40.0))
     for schedule in (0, 2, 3):
         check(sc, schedule, (3, 1, 4))
+
+
+@pytest.mark.parametrize("schedule", [1, 2])
+def test_more_probes_than_threads(gpu_lib, schedule):
+    """Every component of every node a probe, twice over: more probes than the step's kernels have
+    threads. Outside the CPML each holds the field after its step."""
+    import torch
+    from fdtd_gb300 import solver
+    nx, ny, nz, p, steps = 20, 18, 16, 3, 3
+    sc = case((nx, ny, nz), (p,) * 6, 3, n_sources=1)
+    pts = [(i, j, k) for k in range(p, nz - p) for j in range(p, ny - p) for i in range(p, nx - p)]
+    sc.probes = [S.Probe(c, *q) for _ in range(2) for q in pts for c in range(6)]
+    with solver.Simulation.from_scenario(sc, schedule, probe_capacity=steps) as sim:
+        want = []
+        for _ in range(steps):
+            sim.step(1)
+            f = sim.fields()
+            want.append([f[c][k, j, i] for i, j, k in pts for c in range(6)] * 2)
+        assert bitwise_equal(sim.read_probes(0, steps), np.array(want, np.float32))
+    with solver.Simulation.from_scenario(sc, schedule, probe_capacity=steps) as sim:
+        sim.step(steps)
+        assert bitwise_equal(sim.read_probes(0, steps), np.array(want, np.float32))
+    assert np.abs(np.array(want)).max() > 0

@@ -241,6 +241,7 @@ __device__ __forceinline__ void st_mask2(float* a, float* b, const Quad& x, cons
 __device__ __forceinline__ int row_at(const uint2& c, int r) { return (int)((r < 2 ? c.x : c.y) >> (16 * (r & 1)) & 0xffffu); }
 __device__ __forceinline__ float pick(const Quad& q, int r) { return r == 0 ? q.v[0] : r == 1 ? q.v[1] : r == 2 ? q.v[2] : q.v[3]; }
 
+__device__ __forceinline__ void prefetch_l1(const void* a) { asm volatile("prefetch.global.L1 [%0];" ::"l"(a)); }
 __device__ __forceinline__ void cp_async16(float4* dst, const float* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(saddr(dst)), "l"(src) : "memory");
 }
@@ -431,9 +432,11 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                 // rows per node; in a slab background nodes take the tabulated curl coefficients, and
                 // without kMat the others the slow path
                 mixed = true;
-                if constexpr (kWide) {
+                if constexpr (kWide || !kEdge) {
                     // (component by component, so that the four nodes' loads are in flight together: the quads
-                    // of a material's surface decide how long the plane takes)
+                    // of a material's surface decide how long the plane takes. Tiles at the edge have no
+                    // registers left for it with three CTAs an SM, and spills cost more: 512^3 28.4 -> 28.1 ms for
+                    // 20 steps with it in the interior tiles)
                     int c[4];
 #pragma unroll
                     for (int r = 0; r < 4; ++r) {
@@ -489,6 +492,15 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                         }
                     }
                 } else {
+                    // (their rows on the way to L1 together, E's and H's, which the next plane step wants: the loads
+                    // below come one row after the other)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const char* a = reinterpret_cast<const char*>(p.coef + (row_at(cw, r) < kRecGeneral ? row_at(cw, r) : 0));
+                        prefetch_l1(a);
+                        prefetch_l1(a + 32);
+                        prefetch_l1(a + 64);
+                    }
                     int cur = -1;
                     float4 a{}, b{}, d{};
 #pragma unroll
@@ -673,7 +685,7 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                 }
             } else {
                 mixed = true;
-                if constexpr (kWide) {
+                if constexpr (kWide || !kEdge) {
                     int c[4];
 #pragma unroll
                     for (int r = 0; r < 4; ++r) {

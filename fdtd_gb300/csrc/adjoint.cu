@@ -22,6 +22,7 @@
 // step (edges of the design region carry no CPML term and no lumped element).
 #include "yee_common.cuh"
 #include "adjoint.h"
+#include "tma.cuh"
 
 namespace fdtd {
 
@@ -67,30 +68,31 @@ __device__ __forceinline__ long long node(const DeviceGrid& g, int i, int j, int
 // ---- transpose of calc_h (h_update) -------------------------------------------------------
 // G_E slots (written by k_adj_e): 0 Ex->Hz, 1 Ex->Hy, 2 Ey->Hx, 3 Ey->Hz, 4 Ez->Hy, 5 Ez->Hx.
 // G_H slots (written here):        0 Hx->Ey, 1 Hx->Ez, 2 Hy->Ez, 3 Hy->Ex, 4 Hz->Ex, 5 Hz->Ey.
-// 5 CTAs of 256 per SM (48 registers; k_adj_e spills a few words): measured 14 % faster for the
-// reverse sweep at 128^3 than the compiler's own 80 registers (3 CTAs).
+// CTAs of 256 per SM: at 128^3 the 192-step gradient took 30.1 ms with 4 (64 registers, no spills), 30.7 with
+// 5 and 31.1 with 6.
 #ifndef FDTD_ADJ_MIN_BLOCKS
-#define FDTD_ADJ_MIN_BLOCKS 5
+#define FDTD_ADJ_MIN_BLOCKS 4
 #endif
-// General path of k_adj_h. kBg: a node of class kUniformGeneral + background (CPML slabs and
-// boundary planes in the usual layouts): uniform cells and background tables decided at compile
-// time, as in the forward's specialisation.
-template <bool kBg>
-__device__ __forceinline__ void adj_h_general(const StepParams& p, const AdjState& a, const PsiSet& psa, int i, int j,
-                                              int k, long long n, int c, float lx, float ly, float lz) {
+// General path of k_adj_h, out of line.
+__device__ __noinline__ void adj_h_general(const StepParams* pp, const AdjState* pa, const PsiSet* pps, int i, int j, int k, float lx,
+                                           float ly, float lz) {
+    const StepParams& p = *pp;
+    const AdjState& a = *pa;
+    const PsiSet& psa = *pps;
     const DeviceGrid& g = p.g;
-    const long long P = g.plane, R = g.pitch;
+    const long long P = g.plane, R = g.pitch, n = node(g, i, j, k);
+    const int c = p.cls[n];
     const bool kp = k < g.nz - 1, jp = j < g.ny - 1, ip = i < g.nx - 1;
     const uint8_t* mat = p.mat;
-    const bool one = kBg || c < kInterfaceNode;  // seven cells of one material, given by the class
-    const int m0 = kBg ? p.bg.mat : one ? c - kUniformGeneral : mat[n];
+    const bool one = c >= kUniformGeneral && c < kInterfaceNode;  // seven cells of one material, given by the class
+    const int m0 = one ? c - kUniformGeneral : mat[n];
     const int mi = one ? m0 : i > 0 ? mat[n - 1] : 0, mj = one ? m0 : j > 0 ? mat[n - R] : 0;
     const int mk = one ? m0 : k > 0 ? mat[n - P] : 0;
     const bool hx_m = jp && kp, hy_m = ip && kp, hz_m = ip && jp;
     const bool xs = in_slab(i, g.nx, g.pxn, g.pxp), ys = in_slab(j, g.ny, g.pyn, g.pyp), zs = in_slab(k, g.nz, g.pzn, g.pzp);
     const int bg = p.bg.mat;
-    const bool ux = kBg || m0 == mi, uy = kBg || m0 == mj, uz = kBg || m0 == mk;
-    const bool on_bg = kBg || m0 == bg;
+    const bool ux = m0 == mi, uy = m0 == mj, uz = m0 == mk;
+    const bool on_bg = m0 == bg;
     const Coef3 cx = h_coef(p, 0, i == 0, ux, m0, mi);
     const Coef3 cy = h_coef(p, 1, j == 0, uy, m0, mj);
     const Coef3 cz = h_coef(p, 2, k == 0, uz, m0, mk);
@@ -126,46 +128,112 @@ __device__ __forceinline__ void adj_h_general(const StepParams& p, const AdjStat
     a.gh[0][n] = g0; a.gh[1][n] = g1; a.gh[2][n] = g2; a.gh[3][n] = g3; a.gh[4][n] = g4; a.gh[5][n] = g5;
 }
 
-__global__ void __launch_bounds__(256, FDTD_ADJ_MIN_BLOCKS) k_adj_h(const __grid_constant__ StepParams p, AdjState a,
+// The CPML terms of a node on one axis: its face and offset there, the two old values.
+struct AdjSlab {
+    int face, q, l;  // l: the slab plane (SlabRows)
+    float old0, old1;
+};
+template <bool kE>
+__device__ __forceinline__ AdjSlab adj_slab(const DeviceGrid& g, const PsiSet& psa, int axis, int i, int j, int k) {
+    AdjSlab s;
+    int side;
+    s.q = axis == 0 ? psi_off_x(g, i, j, k, side) : axis == 1 ? psi_off_y(g, i, j, k, side) : psi_off_z(g, i, j, k, side);
+    s.face = 2 * axis + side;
+    const int at = axis == 0 ? i : axis == 1 ? j : k, n = axis == 0 ? g.nx : axis == 1 ? g.ny : g.nz;
+    const int pn = axis == 0 ? g.pxn : axis == 1 ? g.pyn : g.pzn, pp = axis == 0 ? g.pxp : axis == 1 ? g.pyp : g.pzp;
+    s.l = side ? at - (n - pp) + pn : at;
+    const PsiFace& f = psa.f[s.face];
+    s.old0 = (kE ? f.e[0] : f.h[0])[s.q];
+    s.old1 = (kE ? f.e[1] : f.h[1])[s.q];
+    return s;
+}
+// One term of adj_comp: memory v' = b (v + f L), contribution g + a (v + f L). t: {b, a}; f: the factor.
+__device__ __forceinline__ float adj_psi(float* mem, const float2& t, float f, float old, float L, float g) {
+    const float mm = __fmaf_rn(f, L, old);
+    *mem = t.x * mm;
+    return __fmaf_rn(t.y, mm, g);
+}
+__device__ __forceinline__ float2 lo2(const float4* t) { return __ldg(reinterpret_cast<const float2*>(t)); }
+__device__ __forceinline__ float2 hi2(const float4* t) { return __ldg(reinterpret_cast<const float2*>(t) + 1); }
+
+// By coefficient row like the two-pass kernels (node_rows.cuh): the background's coefficients are constants,
+// a slab's come from its axis' table or the slab row table, other rows' from the row table; the rest
+// is called out of line. At 128^3 bound by L2: a pass moves 18 floats a node and the gathers' neighbours,
+// 300 MB in 33 us, of a 151 MB state that does not quite stay there.
+template <typename Idx>
+__global__ void __launch_bounds__(256, FDTD_ADJ_MIN_BLOCKS) k_adj_h(const __grid_constant__ StepParams p, const __grid_constant__ AdjState a,
                                                const __grid_constant__ PsiSet psa) {
+    grid_dependency_wait();
+    grid_launch_dependents();
     const DeviceGrid& g = p.g;
     const int i = blockIdx.x * 32 + threadIdx.x;
     const int j = blockIdx.y * 8 + threadIdx.y;
     const int k = blockIdx.z;
     if (i >= g.nx || j >= g.ny) return;
-    const long long n = node(g, i, j, k);
-    const long long P = g.plane, R = g.pitch;
+    const Idx P = (Idx)g.plane, R = (Idx)g.pitch, n = (Idx)k * P + (Idx)j * R + (Idx)i;
     const bool kp = k < g.nz - 1, jp = j < g.ny - 1, ip = i < g.nx - 1;
+    const int c = p.rec[n];
     // finish the transpose of the previous reverse step's calc_e: gather G_E
     float lx = a.l[3][n] + a.ge[2][n] - (kp ? a.ge[2][n + P] : 0.f) + a.ge[5][n] - (jp ? a.ge[5][n + R] : 0.f);
     float ly = a.l[4][n] + a.ge[1][n] - (kp ? a.ge[1][n + P] : 0.f) + a.ge[4][n] - (ip ? a.ge[4][n + 1] : 0.f);
     float lz = a.l[5][n] + a.ge[0][n] - (jp ? a.ge[0][n + R] : 0.f) + a.ge[3][n] - (ip ? a.ge[3][n + 1] : 0.f);
-
-    const int c = p.cls[n];
-    if (c < kUniformGeneral) {  // fast-path node: table coefficients, every component, no CPML
-        const MatCoef* mc = p.coef + c;
-        const float4 x = __ldg(&mc->h[0]), y = __ldg(&mc->h[1]), z = __ldg(&mc->h[2]);
-        a.l[3][n] = x.x * lx; a.l[4][n] = y.x * ly; a.l[5][n] = z.x * lz;
-        a.gh[0][n] = x.y * lx; a.gh[1][n] = x.z * lx; a.gh[2][n] = y.y * ly;
-        a.gh[3][n] = y.z * ly; a.gh[4][n] = z.y * lz; a.gh[5][n] = z.z * lz;
+    const bool xs = in_slab(i, g.nx, g.pxn, g.pxp), ys = in_slab(j, g.ny, g.pyn, g.pyp), zs = in_slab(k, g.nz, g.pzn, g.pzp);
+    AdjSlab X{}, Y{}, Z{};
+    if (xs) X = adj_slab<false>(g, psa, 0, i, j, k);
+    if (ys) Y = adj_slab<false>(g, psa, 1, i, j, k);
+    if (zs) Z = adj_slab<false>(g, psa, 2, i, j, k);
+    const BgNode& B = p.bgn;
+    const bool own = c != p.bg.mat, low = (own || !B.low_ok) && (i == 0 || j == 0 || k == 0);
+    if (c >= kRecGeneral || low || (own && (xs || ys || zs) && !p.rows.h[0])) {
+        adj_h_general(&p, &a, &psa, i, j, k, lx, ly, lz);
         return;
     }
-    if (c == kUniformGeneral + p.bg.mat) adj_h_general<true>(p, a, psa, i, j, k, n, c, lx, ly, lz);
-    else adj_h_general<false>(p, a, psa, i, j, k, n, c, lx, ly, lz);
+    float ax = B.ha[0], ay = B.ha[1], az = B.ha[2];
+    float cx0 = B.hc[0], cx1 = B.hc[1], cy0 = B.hc[2], cy1 = B.hc[3], cz0 = B.hc[4], cz1 = B.hc[5];
+    if (own) {
+        const float4 x = __ldg(&p.coef[c].h[0]), y = __ldg(&p.coef[c].h[1]), z = __ldg(&p.coef[c].h[2]);
+        ax = x.x; cx0 = x.y; cx1 = x.z; ay = y.x; cy0 = y.y; cy1 = y.z; az = z.x; cz0 = z.y; cz1 = z.z;
+    }
+    const int rx = c * (g.pxn + g.pxp) + X.l, ry = c * (g.pyn + g.pyp) + Y.l, rz = c * (g.pzn + g.pzp) + Z.l;
+    if (xs) { const float2 t = lo2(own ? p.rows.h[0] + rx : p.th[0] + i); cy0 = t.x; cz1 = t.y; }
+    if (ys) { const float2 t = lo2(own ? p.rows.h[1] + ry : p.th[1] + j); cx1 = t.x; cz0 = t.y; }
+    if (zs) { const float2 t = lo2(own ? p.rows.h[2] + rz : p.th[2] + k); cx0 = t.x; cy1 = t.y; }
+    const bool mx = jp && kp, my = ip && kp, mz = ip && jp;
+    float g0 = mx ? cx0 * lx : 0.f, g1 = mx ? cx1 * lx : 0.f, g2 = my ? cy0 * ly : 0.f, g3 = my ? cy1 * ly : 0.f;
+    float g4 = mz ? cz0 * lz : 0.f, g5 = mz ? cz1 * lz : 0.f;
+    if (xs) {
+        const float2 t = hi2(p.th[0] + i), f = own ? hi2(p.rows.h[0] + rx) : make_float2(B.ch[0], B.ch[1]);
+        if (my) g2 = adj_psi(psa.f[X.face].h[0] + X.q, t, f.x, X.old0, ly, g2);
+        if (mz) g5 = adj_psi(psa.f[X.face].h[1] + X.q, t, f.y, X.old1, lz, g5);
+    }
+    if (ys) {
+        const float2 t = hi2(p.th[1] + j), f = own ? hi2(p.rows.h[1] + ry) : make_float2(B.ch[2], B.ch[3]);
+        if (mx) g1 = adj_psi(psa.f[Y.face].h[0] + Y.q, t, f.x, Y.old0, lx, g1);
+        if (mz) g4 = adj_psi(psa.f[Y.face].h[1] + Y.q, t, f.y, Y.old1, lz, g4);
+    }
+    if (zs) {
+        const float2 t = hi2(p.th[2] + k), f = own ? hi2(p.rows.h[2] + rz) : make_float2(B.ch[4], B.ch[5]);
+        if (mx) g0 = adj_psi(psa.f[Z.face].h[0] + Z.q, t, f.x, Z.old0, lx, g0);
+        if (my) g3 = adj_psi(psa.f[Z.face].h[1] + Z.q, t, f.y, Z.old1, ly, g3);
+    }
+    a.l[3][n] = mx ? ax * lx : lx; a.l[4][n] = my ? ay * ly : ly; a.l[5][n] = mz ? az * lz : lz;
+    a.gh[0][n] = g0; a.gh[1][n] = g1; a.gh[2][n] = g2; a.gh[3][n] = g3; a.gh[4][n] = g4; a.gh[5][n] = g5;
 }
 
 // ---- transpose of calc_e (e_update), FoM source and design gradient ------------------------
-// General path of k_adj_e, specialised like adj_h_general (background nodes carry no lumped edge
-// and lie outside the design edge box).
-template <bool kBg>
-__device__ __forceinline__ void adj_e_general(const StepParams& p, const AdjState& a, const PsiSet& psa,
-                                              const AdjStep& st, int i, int j, int k, long long n, int c, float lx,
-                                              float ly, float lz) {
+// General path of k_adj_e, out of line.
+__device__ __noinline__ void adj_e_general(const StepParams* pp, const AdjState* pa, const PsiSet* pps, const AdjStep* pst, int i,
+                                           int j, int k, float lx, float ly, float lz) {
+    const StepParams& p = *pp;
+    const AdjState& a = *pa;
+    const PsiSet& psa = *pps;
+    const AdjStep& st = *pst;
     const DeviceGrid& g = p.g;
-    const long long P = g.plane, R = g.pitch;
+    const long long P = g.plane, R = g.pitch, n = node(g, i, j, k);
+    const int c = p.cls[n];
     const uint8_t* mat = p.mat;
-    const bool one = kBg || c < kInterfaceNode;  // seven cells of one material, given by the class
-    const int m0 = kBg ? p.bg.mat : one ? c - kUniformGeneral : mat[n];
+    const bool one = c >= kUniformGeneral && c < kInterfaceNode;  // seven cells of one material, given by the class
+    const int m0 = one ? c - kUniformGeneral : mat[n];
     const int mi = one ? m0 : i > 0 ? mat[n - 1] : 0, mj = one ? m0 : j > 0 ? mat[n - R] : 0;
     const int mk = one ? m0 : k > 0 ? mat[n - P] : 0;
     const int mij = one ? m0 : (i > 0 && j > 0) ? mat[n - 1 - R] : 0;
@@ -175,16 +243,16 @@ __device__ __forceinline__ void adj_e_general(const StepParams& p, const AdjStat
     const bool ex_m = i < g.nx - 1 && in_y && in_z, ey_m = in_x && j < g.ny - 1 && in_z, ez_m = in_x && in_y && k < g.nz - 1;
     const bool xs = in_slab(i, g.nx, g.pxn, g.pxp), ys = in_slab(j, g.ny, g.pyn, g.pyp), zs = in_slab(k, g.nz, g.pzn, g.pzp);
     const int bg = p.bg.mat;
-    const bool ux = kBg || (m0 == mj && m0 == mk && m0 == mjk);
-    const bool uy = kBg || (m0 == mi && m0 == mk && m0 == mik);
-    const bool uz = kBg || (m0 == mi && m0 == mj && m0 == mij);
-    const bool on_bg = kBg || m0 == bg;
-    const Coef3 cx = e_coef<!kBg>(p, 0, ux, m0, mj, mk, mjk, i, j, k);
-    const Coef3 cy = e_coef<!kBg>(p, 1, uy, m0, mi, mk, mik, i, j, k);
-    const Coef3 cz = e_coef<!kBg>(p, 2, uz, m0, mi, mj, mij, i, j, k);
+    const bool ux = m0 == mj && m0 == mk && m0 == mjk;
+    const bool uy = m0 == mi && m0 == mk && m0 == mik;
+    const bool uz = m0 == mi && m0 == mj && m0 == mij;
+    const bool on_bg = m0 == bg;
+    const Coef3 cx = e_coef<true>(p, 0, ux, m0, mj, mk, mjk, i, j, k);
+    const Coef3 cy = e_coef<true>(p, 1, uy, m0, mi, mk, mik, i, j, k);
+    const Coef3 cz = e_coef<true>(p, 2, uz, m0, mi, mj, mij, i, j, k);
 
     // design gradient: lambda here is dJ/dE^{m+1}; E^m and E^{m+1} come from the saved design E
-    if (!kBg && st.acc) {  // background nodes lie outside the design edge box
+    if (st.acc) {
         const int* d = p.dbox;
         const int ei = i - d[0], ej = j - d[1], ek = k - d[2];
         const int bx = d[3] - d[0] + 1, by = d[4] - d[1] + 1, bzz = d[5] - d[2] + 1;
@@ -197,13 +265,9 @@ __device__ __forceinline__ void adj_e_general(const StepParams& p, const AdjStat
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 if (!on[c] || !has_design(p, mm[c][0], mm[c][1], mm[c][2], mm[c][3])) continue;
-                float eps, sig;
-                edge_material(p, c, i, j, k, mm[c][0], mm[c][1], mm[c][2], mm[c][3], eps, sig);
-                const double e0 = g.eps0, dt = g.dt;
-                const double den = 2.0 * (double)eps * e0 + dt * (double)sig;
-                const double dca = 4.0 * e0 * dt * (double)sig / (den * den);
+                const double2 w = st.weight[c * ne + e];
                 const double em = st.e_old[c * ne + e], ep = st.e_new[c * ne + e];
-                const double v = (double)lam[c] * (dca * em - 2.0 * e0 / den * (ep - (double)cc[c].a * em));
+                const double v = (double)lam[c] * (w.x * em - w.y * (ep - (double)cc[c].a * em));
                 st.acc[c * ne + e] += v;
             }
         }
@@ -232,7 +296,7 @@ __device__ __forceinline__ void adj_e_general(const StepParams& p, const AdjStat
         PsiTerm t1{nullptr, 0, 0, 0, 0}, t2{nullptr, 0, 0, 0, 0};
         if (xs) { const int q = psi_off_x(g, i, j, k, side); t1 = psi_term(psa.f[side].e[1] + q, p.bex[i], p.aex[i], __fmul_rn(cz.bp, g.dx)); }
         if (ys) { const int q = psi_off_y(g, i, j, k, side); t2 = psi_term(psa.f[2 + side].e[1] + q, p.bey[j], p.aey[j], __fmul_rn(cz.bm, g.dy)); }
-        const bool plane_lumped = !kBg && p.lumped_k[k] < p.lumped_k[k + 1];  // background nodes carry none
+        const bool plane_lumped = p.lumped_k[k] < p.lumped_k[k + 1];
         const LumpedEdge* L = plane_lumped ? find_lumped(p, i, j, k, 2) : nullptr;  // design handles have no Ex edges
         float aa, c1, c2;
         if (L) { aa = L->ceze; c1 = L->cezhy; c2 = L->cezhx; }
@@ -247,33 +311,102 @@ __device__ __forceinline__ void adj_e_general(const StepParams& p, const AdjStat
     a.ge[0][n] = g0; a.ge[1][n] = g1; a.ge[2][n] = g2; a.ge[3][n] = g3; a.ge[4][n] = g4; a.ge[5][n] = g5;
 }
 
-__global__ void __launch_bounds__(256, FDTD_ADJ_MIN_BLOCKS) k_adj_e(const __grid_constant__ StepParams p, AdjState a,
-                                               const __grid_constant__ PsiSet psa, AdjStep st) {
+// By coefficient row, as k_adj_h.
+template <typename Idx>
+__global__ void __launch_bounds__(256, FDTD_ADJ_MIN_BLOCKS) k_adj_e(const __grid_constant__ StepParams p, const __grid_constant__ AdjState a,
+                                               const __grid_constant__ PsiSet psa, const __grid_constant__ AdjStep st) {
+    grid_dependency_wait();
+    grid_launch_dependents();
     const DeviceGrid& g = p.g;
     const int i = blockIdx.x * 32 + threadIdx.x;
     const int j = blockIdx.y * 8 + threadIdx.y;
     const int k = blockIdx.z;
     if (i >= g.nx || j >= g.ny) return;
-    const long long n = node(g, i, j, k);
-    const long long P = g.plane, R = g.pitch;
+    const Idx P = (Idx)g.plane, R = (Idx)g.pitch, n = (Idx)k * P + (Idx)j * R + (Idx)i;
+    const int c = p.rec[n];
     // finish the transpose of calc_h: gather G_H
     float lx = a.l[0][n] + (k > 0 ? a.gh[3][n - P] : 0.f) - a.gh[3][n] + (j > 0 ? a.gh[4][n - R] : 0.f) - a.gh[4][n];
     float ly = a.l[1][n] + (k > 0 ? a.gh[0][n - P] : 0.f) - a.gh[0][n] + (i > 0 ? a.gh[5][n - 1] : 0.f) - a.gh[5][n];
     float lz = a.l[2][n] + (j > 0 ? a.gh[1][n - R] : 0.f) - a.gh[1][n] + (i > 0 ? a.gh[2][n - 1] : 0.f) - a.gh[2][n];
-    if (n == st.probe) lz += st.source;  // dJ/dEz(p) of the sample taken in this step
-
-    const int c = p.cls[n];
-    if (c < kUniformGeneral) {  // fast-path node: table coefficients, every component, no CPML,
-                                // no lumped edge, outside the design edge box
-        const MatCoef* mc = p.coef + c;
-        const float4 x = __ldg(&mc->e[0]), y = __ldg(&mc->e[1]), z = __ldg(&mc->e[2]);
-        a.l[0][n] = x.x * lx; a.l[1][n] = y.x * ly; a.l[2][n] = z.x * lz;
-        a.ge[0][n] = x.y * lx; a.ge[1][n] = x.z * lx; a.ge[2][n] = y.y * ly;
-        a.ge[3][n] = y.z * ly; a.ge[4][n] = z.y * lz; a.ge[5][n] = z.z * lz;
+    if ((long long)n == st.probe) lz += st.source;  // dJ/dEz(p) of the sample taken in this step
+    const bool xs = in_slab(i, g.nx, g.pxn, g.pxp), ys = in_slab(j, g.ny, g.pyn, g.pyp), zs = in_slab(k, g.nz, g.pzn, g.pzp);
+    AdjSlab X{}, Y{}, Z{};
+    if (xs) X = adj_slab<true>(g, psa, 0, i, j, k);
+    if (ys) Y = adj_slab<true>(g, psa, 1, i, j, k);
+    if (zs) Z = adj_slab<true>(g, psa, 2, i, j, k);
+    const BgNode& B = p.bgn;
+    const bool own = c != p.bg.mat;
+    if (c >= kRecGeneral || (own && (xs || ys || zs) && !p.rows.e[0])) {  // the design edge box among them
+        adj_e_general(&p, &a, &psa, &st, i, j, k, lx, ly, lz);
         return;
     }
-    if (c == kUniformGeneral + p.bg.mat) adj_e_general<true>(p, a, psa, st, i, j, k, n, c, lx, ly, lz);
-    else adj_e_general<false>(p, a, psa, st, i, j, k, n, c, lx, ly, lz);
+    float ax = B.ea[0], ay = B.ea[1], az = B.ea[2];
+    float cx0 = B.ec[0], cx1 = B.ec[1], cy0 = B.ec[2], cy1 = B.ec[3], cz0 = B.ec[4], cz1 = B.ec[5];
+    if (own) {
+        const float4 x = __ldg(&p.coef[c].e[0]), y = __ldg(&p.coef[c].e[1]), z = __ldg(&p.coef[c].e[2]);
+        ax = x.x; cx0 = x.y; cx1 = x.z; ay = y.x; cy0 = y.y; cy1 = y.z; az = z.x; cz0 = z.y; cz1 = z.z;
+    }
+    const int rx = c * (g.pxn + g.pxp) + X.l, ry = c * (g.pyn + g.pyp) + Y.l, rz = c * (g.pzn + g.pzp) + Z.l;
+    if (xs) { const float2 t = lo2(own ? p.rows.e[0] + rx : p.te[0] + i); cy1 = t.x; cz0 = t.y; }
+    if (ys) { const float2 t = lo2(own ? p.rows.e[1] + ry : p.te[1] + j); cx0 = t.x; cz1 = t.y; }
+    if (zs) { const float2 t = lo2(own ? p.rows.e[2] + rz : p.te[2] + k); cx1 = t.x; cy0 = t.y; }
+    bool mx, my, mz;
+    e_masks(g, i, j, k, mx, my, mz);
+    float g0 = mx ? cx0 * lx : 0.f, g1 = mx ? cx1 * lx : 0.f, g2 = my ? cy0 * ly : 0.f, g3 = my ? cy1 * ly : 0.f;
+    float g4 = mz ? cz0 * lz : 0.f, g5 = mz ? cz1 * lz : 0.f;
+    if (xs) {
+        const float2 t = hi2(p.te[0] + i), f = own ? hi2(p.rows.e[0] + rx) : make_float2(B.ce[0], B.ce[1]);
+        if (my) g3 = adj_psi(psa.f[X.face].e[0] + X.q, t, f.x, X.old0, ly, g3);
+        if (mz) g4 = adj_psi(psa.f[X.face].e[1] + X.q, t, f.y, X.old1, lz, g4);
+    }
+    if (ys) {
+        const float2 t = hi2(p.te[1] + j), f = own ? hi2(p.rows.e[1] + ry) : make_float2(B.ce[2], B.ce[3]);
+        if (mx) g0 = adj_psi(psa.f[Y.face].e[0] + Y.q, t, f.x, Y.old0, lx, g0);
+        if (mz) g5 = adj_psi(psa.f[Y.face].e[1] + Y.q, t, f.y, Y.old1, lz, g5);
+    }
+    if (zs) {
+        const float2 t = hi2(p.te[2] + k), f = own ? hi2(p.rows.e[2] + rz) : make_float2(B.ce[4], B.ce[5]);
+        if (mx) g1 = adj_psi(psa.f[Z.face].e[0] + Z.q, t, f.x, Z.old0, lx, g1);
+        if (my) g2 = adj_psi(psa.f[Z.face].e[1] + Z.q, t, f.y, Z.old1, ly, g2);
+    }
+    a.l[0][n] = mx ? ax * lx : lx; a.l[1][n] = my ? ay * ly : ly; a.l[2][n] = mz ? az * lz : lz;
+    a.ge[0][n] = g0; a.ge[1][n] = g1; a.ge[2][n] = g2; a.ge[3][n] = g3; a.ge[4][n] = g4; a.ge[5][n] = g5;
+}
+
+// AdjStep::weight of the edges of the design edge box with a design cell: {da/deps, 2 eps0 / den} (the
+// head of this file), the same in every step. Their FP64 divisions in every reverse step held the
+// design region's CTAs back: k_adj_e 49 us against k_adj_h's 32 at 128^3 with a 32 x 32 x 16 region.
+__global__ void k_adj_weights(const __grid_constant__ StepParams p, double2* out) {
+    const DeviceGrid& g = p.g;
+    const int* d = p.dbox;
+    const int bx = d[3] - d[0] + 1, by = d[4] - d[1] + 1, bz = d[5] - d[2] + 1;
+    const long long ne = (long long)bx * by * bz, e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (e >= ne) return;
+    const int i = d[0] + (int)(e % bx), j = d[1] + (int)((e / bx) % by), k = d[2] + (int)(e / ((long long)bx * by));
+    const long long P = g.plane, R = g.pitch, n = node(g, i, j, k);  // an interior node (fdtd_set_design_region)
+    const uint8_t* mat = p.mat;
+    const int m0 = mat[n], mi = mat[n - 1], mj = mat[n - R], mk = mat[n - P];
+    const int mij = mat[n - 1 - R], mik = mat[n - 1 - P], mjk = mat[n - R - P];
+    const int mm[3][4] = {{m0, mj, mk, mjk}, {m0, mi, mk, mik}, {m0, mi, mj, mij}};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        double2 w = make_double2(0.0, 0.0);
+        if (has_design(p, mm[c][0], mm[c][1], mm[c][2], mm[c][3])) {
+            float eps, sig;
+            edge_material(p, c, i, j, k, mm[c][0], mm[c][1], mm[c][2], mm[c][3], eps, sig);
+            const double e0 = g.eps0, dt = g.dt;
+            const double den = 2.0 * (double)eps * e0 + dt * (double)sig;
+            w = make_double2(4.0 * e0 * dt * (double)sig / (den * den), 2.0 * e0 / den);
+        }
+        out[c * ne + e] = w;
+    }
+}
+
+cudaError_t launch_adj_weights(const StepParams& p, double2* out, cudaStream_t s) {
+    const int* d = p.dbox;
+    const long long ne = (long long)(d[3] - d[0] + 1) * (d[4] - d[1] + 1) * (d[5] - d[2] + 1);
+    k_adj_weights<<<(unsigned)((ne + 127) / 128), 128, 0, s>>>(p, out);
+    return cudaGetLastError();
 }
 
 // After a forward step: the FoM sample Ez(p) and, when `snap` is set, the E components over the
@@ -315,11 +448,11 @@ __global__ void k_grad_finalize(const double* acc, int dx, int dy, int dz, doubl
 
 cudaError_t launch_adj_step(const StepParams& p, const AdjState& a, const PsiSet& psa, const AdjStep& st,
                             cudaStream_t s) {
-    dim3 block(32, 8, 1);
-    dim3 grid((p.g.nx + 31) / 32, (p.g.ny + 7) / 8, p.g.nz);
-    k_adj_h<<<grid, block, 0, s>>>(p, a, psa);
-    k_adj_e<<<grid, block, 0, s>>>(p, a, psa, st);
-    return cudaGetLastError();
+    const dim3 block(32, 8, 1), grid((p.g.nx + 31) / 32, (p.g.ny + 7) / 8, p.g.nz);
+    const bool idx32 = p.g.plane * (long long)(p.g.nz + 1) < (1LL << 31);
+    const cudaError_t e = launch_dependent(idx32 ? k_adj_h<uint32_t> : k_adj_h<unsigned long long>, grid, block, 0, s, p, a, psa);
+    if (e != cudaSuccess) return e;
+    return launch_dependent(idx32 ? k_adj_e<uint32_t> : k_adj_e<unsigned long long>, grid, block, 0, s, p, a, psa, st);
 }
 
 cudaError_t launch_after_step(const float* ex, const float* ey, const float* ez, const DeviceGrid& g, long long probe,

@@ -23,8 +23,11 @@ struct AdjStep {
     double* acc;
     const float* e_old;
     const float* e_new;
+    const double2* weight;  // per edge like acc (launch_adj_weights)
 };
 
+// The design gradient's weight of each edge of the design edge box, for AdjStep::weight (3 x box volume).
+cudaError_t launch_adj_weights(const StepParams& p, double2* out, cudaStream_t s);
 // One reverse step (k_adj_h then k_adj_e).
 cudaError_t launch_adj_step(const StepParams& p, const AdjState& a, const PsiSet& psa, const AdjStep& st, cudaStream_t s);
 // FoM sample of a forward step (Ez at node `probe` into *sample) and, if snap != NULL, the E

@@ -196,6 +196,7 @@ struct fdtd_handle {
         char* ckpt = nullptr;          // checkpoints (K > 0) and the final state
         long long ckpt_slots = 0;
         double* acc = nullptr;         // per-edge gradient accumulators
+        double2* weight = nullptr;     // and weights (AdjStep::weight)
         double* grad = nullptr;        // per-cell gradient
         int* no_probe_k = nullptr;     // per-plane probe offsets, all zero: the recompute samples nothing
         int S = 0;                     // box checkpoints every S steps inside a segment (0: none)
@@ -1795,6 +1796,7 @@ int adj_prepare(fdtd_handle* h, long long n, int K) {
         (rc = adj_alloc(h, (void**)&A.hist, sizeof(float) * 3 * (size_t)ne * (size_t)A.hist_slots)) ||
         (rc = adj_alloc(h, (void**)&A.ckpt, (size_t)fdtd_state_bytes(h) * (size_t)A.ckpt_slots)) ||
         (rc = adj_alloc(h, (void**)&A.acc, sizeof(double) * 3 * (size_t)ne)) ||
+        (rc = adj_alloc(h, (void**)&A.weight, sizeof(double2) * 3 * (size_t)ne)) ||
         (rc = adj_alloc(h, (void**)&A.grad, sizeof(double) * nd)) ||
         (rc = adj_alloc(h, (void**)&A.no_probe_k, sizeof(int) * (size_t)(h->g.nz + 1))))
         return rc;
@@ -1971,11 +1973,12 @@ int adj_backward_enqueue(fdtd_handle* h) {
     const long long ne = edge_box_volume(h->dbox);
     CUDA_TRY(cudaMemsetAsync(A.acc, 0, sizeof(double) * 3 * (size_t)ne, h->stream));
     const StepParams p = make_params(h);
+    CUDA_TRY(launch_adj_weights(p, A.weight, h->stream));
     const float two_dt = 2.0f * h->g.dt;
     int rc;
     if (A.K == 0) {
         for (long long m = A.n - 1; m >= 0; --m) {
-            const AdjStep st{A.probe, two_dt * A.host_samples[(size_t)m], A.acc, adj_slot(h, m), adj_slot(h, m + 1)};
+            const AdjStep st{A.probe, two_dt * A.host_samples[(size_t)m], A.acc, adj_slot(h, m), adj_slot(h, m + 1), A.weight};
             CUDA_TRY(launch_adj_step(p, A.st, A.psa, st, h->stream));
         }
     } else {
@@ -2020,7 +2023,7 @@ int adj_backward_enqueue(fdtd_handle* h) {
             CUDA_TRY(cudaStreamWaitEvent(A.rev, ev_rec[sg & 1], 0));
             const long long len = std::min<long long>(A.K, A.n - sg * A.K);
             for (long long t = len - 1; t >= 0; --t) {
-                const AdjStep st{A.probe, two_dt * A.host_samples[(size_t)(sg * A.K + t)], A.acc, slot(sg, t), slot(sg, t + 1)};
+                const AdjStep st{A.probe, two_dt * A.host_samples[(size_t)(sg * A.K + t)], A.acc, slot(sg, t), slot(sg, t + 1), A.weight};
                 CUDA_TRY(launch_adj_step(p, A.st, A.psa, st, A.rev));
             }
             CUDA_TRY(cudaEventRecord(ev_rev[sg & 1], A.rev));

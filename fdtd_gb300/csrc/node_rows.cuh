@@ -23,10 +23,15 @@ struct StepIndex {
     __device__ __forceinline__ long long at() const { return base ? *base + m : m; }
 };
 
-template <typename Idx>
+// kDesign: the grid has a design region (the other grids' pass is kept free of its code: 128^3 39.9 against
+// 41.8 us a step).
+template <typename Idx, bool kDesign>
 static __device__ __noinline__ void e_node_general(const StepParams* p, const FieldPtrs* f, const PsiSet* ps, const StepIndex* step,
                                                    int i, int j, int k) {
-    e_node_global<false, false, false, Idx>(*p, *f, *f, *ps, *ps, i, j, k, step->at());
+    if (kDesign && p->rec[(Idx)k * (Idx)p->g.plane + (Idx)j * (Idx)p->g.pitch + (Idx)i] == (kRecGeneral | kDesignNode))
+        e_node_global<true>(*p, *f, *f, *ps, *ps, i, j, k, step->at());
+    else
+        e_node_global<false, false, false, Idx>(*p, *f, *f, *ps, *ps, i, j, k, step->at());
 }
 template <typename Idx>
 static __device__ __noinline__ void h_node_general(const StepParams* p, const FieldPtrs* f, const PsiSet* ps, const StepIndex* step,
@@ -70,7 +75,7 @@ __device__ __forceinline__ PsiSlot<Idx> psi_slot_z(const StepParams& p, int i, i
 __device__ __forceinline__ float2 curl_pair(const float4* t) { return __ldg(reinterpret_cast<const float2*>(t)); }
 __device__ __forceinline__ float2 psi_pair(const float4* t) { return __ldg(reinterpret_cast<const float2*>(t) + 1); }
 
-template <typename Idx>
+template <typename Idx, bool kDesign>
 __device__ __forceinline__ void e_node_rows(const StepParams& p, const FieldPtrs& f, const PsiSet& ps, int i, int j, int k,
                                             const StepIndex& step) {
     const DeviceGrid& g = p.g;
@@ -90,8 +95,7 @@ __device__ __forceinline__ void e_node_rows(const StepParams& p, const FieldPtrs
     const BgNode& B = p.bgn;
     const bool own = c != p.bg.mat;
     if (c >= kRecGeneral || (own && slab && !p.rows.e[0])) {
-        if (c == (kRecGeneral | kDesignNode)) return;  // k_design_e's
-        e_node_general<Idx>(&p, &f, &ps, &step, i, j, k);
+        e_node_general<Idx, kDesign>(&p, &f, &ps, &step, i, j, k);
         return;
     }
     float ax = B.ea[0], ay = B.ea[1], az = B.ea[2];

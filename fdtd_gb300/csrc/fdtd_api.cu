@@ -163,7 +163,8 @@ struct fdtd_handle {
     int* d_probe_ids = nullptr;
     float** d_waves = nullptr;
     long long* d_wave_len = nullptr;
-    std::vector<float*> d_wave_bufs;
+    char* lumped_tables = nullptr;  // the allocation of the lumped edges' and waveforms' tables
+    char* probe_tables = nullptr;   // and of the probes' and their ring
     int* d_lumped_box = nullptr;
     float* d_lumped_r = nullptr;
     int* d_lumped_owner = nullptr;
@@ -541,37 +542,40 @@ int fdtd_create(const fdtd_grid* grid, fdtd_handle** out) {
         if (launch_fill(h->field[0][c], V, kTiny, nullptr) != cudaSuccess) return cleanup(fail(FDTD_ERR_CUDA, "fill failed"));
     }
     if (h->alloc((void**)&h->mat, (size_t)V) != cudaSuccess) return cleanup(fail(FDTD_ERR_OOM, "material index allocation failed"));
-    if (h->alloc((void**)&h->props, sizeof(MatProps) * kMaxMaterials) != cudaSuccess ||
-        h->alloc((void**)&h->coef, sizeof(MatCoef) * (kMaxMaterials + 1)) != cudaSuccess ||
-        h->alloc((void**)&h->status, sizeof(int)) != cudaSuccess || h->alloc((void**)&h->small, 4 * sizeof(int)) != cudaSuccess)
-        return cleanup(fail(FDTD_ERR_OOM, "table allocation failed"));
+    // the tables every handle keeps, in one allocation
     const int ns[3] = {g.nx, g.ny, g.nz};
-    for (int a = 0; a < 3; ++a)
-        for (int q = 0; q < 6; ++q)
-            if (h->alloc((void**)&h->prof[6 * a + q], sizeof(float) * ns[a]) != cudaSuccess)
-                return cleanup(fail(FDTD_ERR_OOM, "profile allocation failed"));
-    for (int a = 0; a < 3; ++a)
-        for (int q = 0; q < 4; ++q)
-            if (h->alloc((void**)&h->bg_curl[4 * a + q], sizeof(float) * ns[a]) != cudaSuccess)
-                return cleanup(fail(FDTD_ERR_OOM, "profile allocation failed"));
-    {   // the packed tables, in one allocation
-        float4* t = nullptr;
-        if (h->alloc((void**)&t, sizeof(float4) * 2 * (size_t)(ns[0] + ns[1] + ns[2])) != cudaSuccess)
-            return cleanup(fail(FDTD_ERR_OOM, "profile allocation failed"));
-        for (int a = 0; a < 3; ++a) {
-            h->te[a] = t;
-            h->th[a] = t + ns[a];
-            t += 2 * ns[a];
-        }
-    }
-    if (h->alloc((void**)&h->d_kappa_ptrs, sizeof(float*) * 6) != cudaSuccess ||
-        h->alloc((void**)&h->d_bg_ptrs, sizeof(float*) * 12) != cudaSuccess)
-        return cleanup(fail(FDTD_ERR_OOM, "table allocation failed"));
     {
-        float* kp[6];
-        for (int a = 0; a < 3; ++a) { kp[2 * a] = h->prof[6 * a + 4]; kp[2 * a + 1] = h->prof[6 * a + 5]; }
-        if (cudaMemcpy(h->d_kappa_ptrs, kp, sizeof(kp), cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(h->d_bg_ptrs, h->bg_curl, sizeof(h->bg_curl), cudaMemcpyHostToDevice) != cudaSuccess)
+        std::vector<std::pair<void**, size_t>> parts;
+        size_t total = 0;
+        auto part = [&](auto** p, size_t n) {
+            parts.push_back({(void**)p, total});
+            total += (n * sizeof(**p) + 255) / 256 * 256;
+        };
+        part(&h->iface_table, kIfaceTableSize);
+        part(&h->iface_keys, kIfaceTableSize);
+        part(&h->iface_slot_row, kIfaceTableSize);
+        part(&h->iface_counters, 2);
+        part(&h->props, kMaxMaterials);
+        part(&h->coef, kMaxMaterials + 1);
+        part(&h->status, 1);
+        part(&h->small, 4);
+        for (int a = 0; a < 3; ++a) {
+            for (int q = 0; q < 6; ++q) part(&h->prof[6 * a + q], ns[a]);
+            for (int q = 0; q < 4; ++q) part(&h->bg_curl[4 * a + q], ns[a]);
+            part(&h->te[a], ns[a]);
+            part(&h->th[a], ns[a]);
+        }
+        part(&h->d_kappa_ptrs, 6 + 12);
+        char* base = nullptr;
+        if (h->alloc((void**)&base, total) != cudaSuccess) return cleanup(fail(FDTD_ERR_OOM, "table allocation failed"));
+        for (auto& q : parts) *q.first = base + q.second;
+        h->d_bg_ptrs = h->d_kappa_ptrs + 6;
+    }
+    {
+        float* ptrs[6 + 12];
+        for (int a = 0; a < 3; ++a) { ptrs[2 * a] = h->prof[6 * a + 4]; ptrs[2 * a + 1] = h->prof[6 * a + 5]; }
+        std::copy(h->bg_curl, h->bg_curl + 12, ptrs + 6);
+        if (cudaMemcpy(h->d_kappa_ptrs, ptrs, sizeof(ptrs), cudaMemcpyHostToDevice) != cudaSuccess)
             return cleanup(fail(FDTD_ERR_CUDA, "pointer table upload failed"));
     }
     // CPML memory: x faces (nz, ny, P), y faces (nz, P, pitch), z faces (P, ny, pitch)
@@ -585,14 +589,9 @@ int fdtd_create(const fdtd_grid* grid, fdtd_handle** out) {
     }
     rc = alloc_psi_set(h, 0);
     if (rc) return cleanup(rc);
-    // node classes, coefficient rows and the interface-key set, which every preparation builds:
-    // allocated here, while the fills run
-    if (h->alloc((void**)&h->cls, (size_t)V) != cudaSuccess ||
-        h->alloc((void**)&h->rec, (size_t)V * sizeof(uint16_t)) != cudaSuccess ||
-        h->alloc((void**)&h->iface_table, sizeof(unsigned long long) * kIfaceTableSize) != cudaSuccess ||
-        h->alloc((void**)&h->iface_keys, sizeof(unsigned long long) * kIfaceTableSize) != cudaSuccess ||
-        h->alloc((void**)&h->iface_slot_row, sizeof(int) * kIfaceTableSize) != cudaSuccess ||
-        h->alloc((void**)&h->iface_counters, sizeof(int) * 2) != cudaSuccess)
+    // node classes and coefficient rows, which every preparation builds: allocated here, while the
+    // fills run
+    if (h->alloc((void**)&h->cls, (size_t)V) != cudaSuccess || h->alloc((void**)&h->rec, (size_t)V * sizeof(uint16_t)) != cudaSuccess)
         return cleanup(fail(FDTD_ERR_OOM, "node class allocation failed"));
     if (cudaMemsetAsync(h->cls, kGeneral, (size_t)V, nullptr) != cudaSuccess)
         return cleanup(fail(FDTD_ERR_CUDA, "memset failed"));
@@ -1128,12 +1127,24 @@ int64_t fdtd_device_bytes(const fdtd_handle* h) { return h ? h->bytes : -1; }
 
 namespace {
 
+// Small tables made on the host and kept on the device in one allocation filled by one copy: each of
+// their own cost a handle some 5 us to allocate, 10 to fill and 5 to free.
+struct TablePack {
+    std::vector<char> bytes;
+    template <class T>
+    size_t add(const T* src, size_t n) {  // the table's offset
+        const size_t at = (bytes.size() + 255) / 256 * 256;
+        bytes.resize(at + sizeof(T) * std::max<size_t>(n, 1));
+        if (n) std::memcpy(bytes.data() + at, src, sizeof(T) * n);
+        return at;
+    }
+    size_t padded() const { return (bytes.size() + 255) / 256 * 256; }
+};
+
 int build_lumped(fdtd_handle* h) {
     // free the previous tables
-    h->release(h->d_lumped); h->release(h->d_lumped_k); h->release(h->d_waves); h->release(h->d_wave_len);
-    h->release(h->d_lumped_box); h->release(h->d_lumped_r); h->release(h->d_lumped_owner);
-    for (float* w : h->d_wave_bufs) h->release(w);
-    h->d_wave_bufs.clear();
+    h->release(h->lumped_tables);
+    h->lumped_tables = nullptr;
     h->d_lumped = nullptr; h->d_lumped_k = nullptr; h->d_waves = nullptr; h->d_wave_len = nullptr;
     h->d_lumped_box = nullptr; h->d_lumped_r = nullptr; h->d_lumped_owner = nullptr;
     const DeviceGrid& g = h->g;
@@ -1158,40 +1169,39 @@ int build_lumped(fdtd_handle* h) {
     for (int k = 0; k < g.nz; ++k) koff[k + 1] += koff[k];
     const size_t ne = se.size();
     h->n_lumped_edges = (int)ne;
-    CUDA_TRY(h->alloc((void**)&h->d_lumped_k, sizeof(int) * (g.nz + 1)));
-    CUDA_TRY(cudaMemcpy(h->d_lumped_k, koff.data(), sizeof(int) * (g.nz + 1), cudaMemcpyHostToDevice));
-    CUDA_TRY(h->alloc((void**)&h->d_lumped, sizeof(LumpedEdge) * std::max<size_t>(ne, 1)));
+    std::vector<int> boxes;
+    std::vector<float> rs;
+    for (const LumpedDef& L : h->lumped) { boxes.insert(boxes.end(), L.box, L.box + 6); rs.push_back(L.resistance); }
+    TablePack t;
+    const size_t at_k = t.add(koff.data(), koff.size()), at_e = t.add(se.data(), ne), at_b = t.add(boxes.data(), boxes.size());
+    const size_t at_r = t.add(rs.data(), rs.size()), at_o = t.add(so.data(), so.size());
+    // waveforms, then their addresses and lengths
+    const size_t nw = h->waves.size();
+    std::vector<size_t> at_w;
+    std::vector<long long> lens(std::max<size_t>(nw, 1), 0);
+    for (size_t w = 0; w < nw; ++w) {
+        at_w.push_back(t.add(h->waves[w].data(), h->waves[w].size()));
+        lens[w] = (long long)h->waves[w].size();
+    }
+    const size_t at_l = t.add(lens.data(), lens.size());
+    std::vector<float*> ptrs(std::max<size_t>(nw, 1), nullptr);
+    const size_t at_p = t.add(ptrs.data(), ptrs.size());
+    CUDA_TRY(h->alloc((void**)&h->lumped_tables, t.bytes.size()));
+    char* base = h->lumped_tables;
+    for (size_t w = 0; w < nw; ++w) ptrs[w] = (float*)(base + at_w[w]);
+    std::memcpy(t.bytes.data() + at_p, ptrs.data(), sizeof(float*) * ptrs.size());
+    CUDA_TRY(cudaMemcpy(base, t.bytes.data(), t.bytes.size(), cudaMemcpyHostToDevice));
+    h->d_lumped_k = (int*)(base + at_k);
+    h->d_lumped = (LumpedEdge*)(base + at_e);
+    h->d_waves = (float**)(base + at_p);
+    h->d_wave_len = (long long*)(base + at_l);
     if (ne) {
-        std::vector<int> boxes;
-        std::vector<float> rs;
-        for (const LumpedDef& L : h->lumped) { boxes.insert(boxes.end(), L.box, L.box + 6); rs.push_back(L.resistance); }
-        CUDA_TRY(h->alloc((void**)&h->d_lumped_box, sizeof(int) * boxes.size()));
-        CUDA_TRY(h->alloc((void**)&h->d_lumped_r, sizeof(float) * rs.size()));
-        CUDA_TRY(h->alloc((void**)&h->d_lumped_owner, sizeof(int) * ne));
-        CUDA_TRY(cudaMemcpy(h->d_lumped, se.data(), sizeof(LumpedEdge) * ne, cudaMemcpyHostToDevice));
-        CUDA_TRY(cudaMemcpy(h->d_lumped_box, boxes.data(), sizeof(int) * boxes.size(), cudaMemcpyHostToDevice));
-        CUDA_TRY(cudaMemcpy(h->d_lumped_r, rs.data(), sizeof(float) * rs.size(), cudaMemcpyHostToDevice));
-        CUDA_TRY(cudaMemcpy(h->d_lumped_owner, so.data(), sizeof(int) * ne, cudaMemcpyHostToDevice));
+        h->d_lumped_box = (int*)(base + at_b);
+        h->d_lumped_r = (float*)(base + at_r);
+        h->d_lumped_owner = (int*)(base + at_o);
         CUDA_TRY(launch_lumped_coefs(g, h->mat, h->props, h->d_lumped, h->d_lumped_box, h->d_lumped_r,
                                      h->d_lumped_owner, (int)ne, h->stream));
     }
-    // waveforms
-    const size_t nw = h->waves.size();
-    std::vector<float*> ptrs(std::max<size_t>(nw, 1), nullptr);
-    std::vector<long long> lens(std::max<size_t>(nw, 1), 0);
-    for (size_t w = 0; w < nw; ++w) {
-        float* d = nullptr;
-        CUDA_TRY(h->alloc((void**)&d, sizeof(float) * std::max<size_t>(h->waves[w].size(), 1)));
-        if (!h->waves[w].empty())
-            CUDA_TRY(cudaMemcpy(d, h->waves[w].data(), sizeof(float) * h->waves[w].size(), cudaMemcpyHostToDevice));
-        h->d_wave_bufs.push_back(d);
-        ptrs[w] = d;
-        lens[w] = (long long)h->waves[w].size();
-    }
-    CUDA_TRY(h->alloc((void**)&h->d_waves, sizeof(float*) * ptrs.size()));
-    CUDA_TRY(h->alloc((void**)&h->d_wave_len, sizeof(long long) * lens.size()));
-    CUDA_TRY(cudaMemcpy(h->d_waves, ptrs.data(), sizeof(float*) * ptrs.size(), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(h->d_wave_len, lens.data(), sizeof(long long) * lens.size(), cudaMemcpyHostToDevice));
     h->dirty_lumped = false;
     return FDTD_OK;
 }
@@ -1315,13 +1325,6 @@ size_t special_nodes(const fdtd_handle* h, std::vector<int4>& out) {
 // classes and plates are final.
 int build_interface_rows(fdtd_handle* h) {
     const DeviceGrid& g = h->g;
-    if (!h->rec) CUDA_TRY(h->alloc((void**)&h->rec, (size_t)vol(h) * sizeof(uint16_t)));
-    if (!h->iface_table) {
-        CUDA_TRY(h->alloc((void**)&h->iface_table, sizeof(unsigned long long) * kIfaceTableSize));
-        CUDA_TRY(h->alloc((void**)&h->iface_keys, sizeof(unsigned long long) * kIfaceTableSize));
-        CUDA_TRY(h->alloc((void**)&h->iface_slot_row, sizeof(int) * kIfaceTableSize));
-        CUDA_TRY(h->alloc((void**)&h->iface_counters, sizeof(int) * 2));
-    }
     // distinct keys on the device; only they come to the host (two small copies)
     CUDA_TRY(launch_iface_set(g, h->cls, h->mat, h->iface_table, h->iface_counters, h->iface_keys, h->stream));
     int counters[2] = {0, 0};
@@ -1430,9 +1433,9 @@ int build_slab_rows(fdtd_handle* h) {
 }
 
 int build_probes(fdtd_handle* h) {
-    h->release(h->d_probes); h->release(h->d_probe_k); h->release(h->d_probe_ids); h->release(h->ring);
+    h->release(h->probe_tables);
+    h->probe_tables = nullptr;
     h->d_probes = nullptr; h->d_probe_k = nullptr; h->d_probe_ids = nullptr; h->ring = nullptr;
-    h->release(h->d_probes_at);
     h->d_probes_at = nullptr;
     const DeviceGrid& g = h->g;
     const size_t np = h->probes.size();
@@ -1444,10 +1447,6 @@ int build_probes(fdtd_handle* h) {
         at.push_back(ProbeAt{r.comp, (int)q, (long long)r.k * g.plane + (long long)r.j * g.pitch + r.i});
     }
     h->n_probes_at = (int)at.size();
-    if (!at.empty()) {
-        CUDA_TRY(h->alloc((void**)&h->d_probes_at, sizeof(ProbeAt) * at.size()));
-        CUDA_TRY(cudaMemcpy(h->d_probes_at, at.data(), sizeof(ProbeAt) * at.size(), cudaMemcpyHostToDevice));
-    }
     std::vector<int> order(np);
     for (size_t q = 0; q < np; ++q) order[q] = (int)q;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return h->probes[a].k < h->probes[b].k; });
@@ -1456,15 +1455,17 @@ int build_probes(fdtd_handle* h) {
     std::vector<int> koff(g.nz + 1, 0);
     for (const Probe& p : sp) koff[p.k + 1]++;
     for (int k = 0; k < g.nz; ++k) koff[k + 1] += koff[k];
-    CUDA_TRY(h->alloc((void**)&h->d_probe_k, sizeof(int) * (g.nz + 1)));
-    CUDA_TRY(cudaMemcpy(h->d_probe_k, koff.data(), sizeof(int) * (g.nz + 1), cudaMemcpyHostToDevice));
-    CUDA_TRY(h->alloc((void**)&h->d_probes, sizeof(Probe) * std::max<size_t>(np, 1)));
-    CUDA_TRY(h->alloc((void**)&h->d_probe_ids, sizeof(int) * std::max<size_t>(np, 1)));
-    if (np) {
-        CUDA_TRY(cudaMemcpy(h->d_probes, sp.data(), sizeof(Probe) * np, cudaMemcpyHostToDevice));
-        CUDA_TRY(cudaMemcpy(h->d_probe_ids, order.data(), sizeof(int) * np, cudaMemcpyHostToDevice));
-    }
-    CUDA_TRY(h->alloc((void**)&h->ring, sizeof(float) * (size_t)h->ring_cap * std::max<size_t>(np, 1)));
+    TablePack t;
+    const size_t at_a = t.add(at.data(), at.size()), at_k = t.add(koff.data(), koff.size());
+    const size_t at_p = t.add(sp.data(), np), at_i = t.add(order.data(), np), at_r = t.padded();
+    CUDA_TRY(h->alloc((void**)&h->probe_tables, at_r + sizeof(float) * (size_t)h->ring_cap * std::max<size_t>(np, 1)));
+    char* base = h->probe_tables;
+    CUDA_TRY(cudaMemcpy(base, t.bytes.data(), t.bytes.size(), cudaMemcpyHostToDevice));
+    h->d_probes_at = (ProbeAt*)(base + at_a);
+    h->d_probe_k = (int*)(base + at_k);
+    h->d_probes = (Probe*)(base + at_p);
+    h->d_probe_ids = (int*)(base + at_i);
+    h->ring = (float*)(base + at_r);
     h->dirty_probes = false;
     return FDTD_OK;
 }
@@ -1495,10 +1496,6 @@ int ensure_prepared(fdtd_handle* h) {
         int rc = build_lumped(h);
         if (rc) return rc;
         // node classes depend on the material index and the lumped edges
-        if (!h->cls) {
-            CUDA_TRY(h->alloc((void**)&h->cls, (size_t)vol(h)));
-            CUDA_TRY(cudaMemsetAsync(h->cls, kGeneral, (size_t)vol(h), h->stream));
-        }
         CUDA_TRY(launch_node_class(h->g, h->mat, h->d_lumped, h->n_lumped_edges, h->has_design ? h->dbox : nullptr, h->cls,
                                    h->stream));
         rc = build_plates(h);

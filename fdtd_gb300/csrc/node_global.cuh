@@ -1,5 +1,6 @@
-// Per-node E and H updates reading the fields from global memory: the two-pass schedule, the
-// shell passes of the fused schedule, the design-region kernel and the batched launch share them.
+// Per-node E and H updates by node class, reading the fields from global memory: the two-pass kernels by
+// class, the general path of those by row, the design-region and plate kernels and the batched launch
+// share them.
 #pragma once
 
 #include "yee_common.cuh"
@@ -12,17 +13,12 @@ namespace fdtd {
 // and its class byte together (one round of memory latency); fast-path nodes (class below
 // kUniformGeneral) then update from the material table, interface nodes from their row of the
 // coefficient table, the rest also gather the seven cell materials and take
-// e_update / h_update. kDesign (k_design_e only): skip the class test and average the per-cell
+// e_update / h_update. kDesign (design nodes only): skip the class test and average the per-cell
 // eps_r of design cells. kPlate (k_plate_e only): plate-covered edges take the plate's sigma_e;
 // the other kernels leave plate nodes (class kPlateNode) alone, CPML memory included.
 // Idx: the integer type of node offsets; uint32_t when the field arrays hold fewer than 2^31
-// elements, which saves the 64-bit address arithmetic of every load and store. kSlabs: the CPML
-// slabs (bit 0 x, 1 y, 2 z) the caller's nodes may lie in; the other slab tests compile out.
-// kEarly: a CPML node's old psi is loaded together with its fields (the addresses depend only on
-// the node's position) instead of after its class has chosen the path; one round of memory latency
-// less, a few more registers live across the loads.
-template <bool kDesign = false, bool kCoherent = false, bool kPlate = false, typename Idx = long long, int kSlabs = 7,
-          bool kEarly = false>
+// elements, which saves the 64-bit address arithmetic of every load and store.
+template <bool kDesign = false, bool kCoherent = false, bool kPlate = false, typename Idx = long long>
 __device__ __forceinline__ void e_node_global(const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fo,
                                               const PsiSet& pin, const PsiSet& pout, int i, int j, int k, long long m) {
     const DeviceGrid& g = p.g;
@@ -37,9 +33,6 @@ __device__ __forceinline__ void e_node_global(const StepParams& p, const FieldPt
     nb.hy_km = k > 0 ? fi.hy[n - P] : 0.f;
     nb.hz_im = i > 0 ? fi.hz[n - 1] : 0.f;
     nb.hz_jm = j > 0 ? fi.hz[n - R] : 0.f;
-    PsiOld po;
-    if (kEarly && !kDesign) psi_preload<true, kCoherent, kSlabs>(g, pin.f, i, j, k, po);
-    const PsiOld* pop = (kEarly && !kDesign) ? &po : nullptr;
     const int c = kDesign ? kGeneral : p.cls[n];
     float out[3], pre[3];
     if (c < kUniformGeneral || c == kInterfaceNode) {
@@ -65,10 +58,10 @@ __device__ __forceinline__ void e_node_global(const StepParams& p, const FieldPt
         // plate nodes are k_plate_e's, CPML memory included: the other kernels store nothing of them
         const PsiIO io{pin.f, pout.f, kPlate || c != kPlateNode};
         if (!kDesign && !kPlate && c == kUniformGeneral + p.bg.mat) {  // CPML / boundary background node
-            e_update<false, kCoherent, false, true, kSlabs>(p, nb, i, j, k, m, false, io, out, pre, pop);
+            e_update<false, kCoherent, false, true>(p, nb, i, j, k, m, false, io, out, pre);
         } else {
             const bool plane_lumped = p.lumped_k[k] < p.lumped_k[k + 1];
-            e_update<kDesign, kCoherent, kPlate, false, kSlabs>(p, nb, i, j, k, m, plane_lumped, io, out, pre, pop);
+            e_update<kDesign, kCoherent, kPlate, false>(p, nb, i, j, k, m, plane_lumped, io, out, pre);
         }
     }
     // k_design_e writes the design region's E, k_plate_e the plate nodes' E
@@ -88,7 +81,7 @@ __device__ __forceinline__ void e_node_global(const StepParams& p, const FieldPt
 }
 
 // H reads the old H from `fi` and the new E from `fe`.
-template <bool kCoherent = false, typename Idx = long long, int kSlabs = 7, bool kEarly = false>
+template <bool kCoherent = false, typename Idx = long long>
 __device__ __forceinline__ void h_node_global(const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fe,
                                               const FieldPtrs& fo, const PsiSet& pin, const PsiSet& pout, int i, int j,
                                               int k, long long m) {
@@ -104,9 +97,6 @@ __device__ __forceinline__ void h_node_global(const StepParams& p, const FieldPt
     nb.ex_kp = k < g.nz - 1 ? fe.ex[n + P] : 0.f;
     nb.ex_jp = j < g.ny - 1 ? fe.ex[n + R] : 0.f;
     nb.ey_ip = i < g.nx - 1 ? fe.ey[n + 1] : 0.f;
-    PsiOld po;
-    if (kEarly) psi_preload<false, kCoherent, kSlabs>(g, pin.f, i, j, k, po);
-    const PsiOld* pop = kEarly ? &po : nullptr;
     const int c = p.cls[n];
     float out[3], pre[3];
     if (c < kUniformGeneral || c == kInterfaceNode) {
@@ -126,8 +116,8 @@ __device__ __forceinline__ void h_node_global(const StepParams& p, const FieldPt
             nb.mk = k > 0 ? mat[n - P] : 0;
         }
         const PsiIO io{pin.f, pout.f, true};
-        if (c == kUniformGeneral + p.bg.mat) h_update<kCoherent, true, kSlabs>(p, nb, i, j, k, io, out, pre, pop);  // background node
-        else h_update<kCoherent, false, kSlabs>(p, nb, i, j, k, io, out, pre, pop);
+        if (c == kUniformGeneral + p.bg.mat) h_update<kCoherent, true>(p, nb, i, j, k, io, out, pre);  // background node
+        else h_update<kCoherent, false>(p, nb, i, j, k, io, out, pre);
     }
     fo.hx[n] = out[0]; fo.hy[n] = out[1]; fo.hz[n] = out[2];
     if (p.probe_k[k] < p.probe_k[k + 1]) {

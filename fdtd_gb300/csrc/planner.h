@@ -1,7 +1,9 @@
-// Work planner of the fused schedule (host only, no CUDA types: also compiled on its own by the
-// CPU tests, which check that the items cover every node exactly once).
+// Work planners (host only, no CUDA types: also compiled on their own by the CPU tests, which check
+// that the items cover every node exactly once). plan_sweep plans the fused schedule's sweep;
+// plan_fused planned an earlier form of it, a sweep of the interior tiles and passes over the rest, and
+// is reached by its tests only.
 //
-// A fused step reads buffer A and writes buffer B. Its nodes are split into
+// plan_fused. A fused step reads buffer A and writes buffer B. Its nodes are split into
 //   * interior items {x0, y0, k0, k1}: a kTileX x kTileY column over planes [k0, k1) whose nodes
 //     and E halo are all interior (no CPML slab, no boundary plane), for the TMA sweep;
 //   * shell items {x0, y0, k, code} for the per-node shell passes: blocks of up to 256 nodes of

@@ -396,9 +396,9 @@ namespace fdtd {
 // cells agree, the reference's averages otherwise), so an interior node's update is the table
 // form with the same bits. Interior nodes whose key has no row take the general path, with the
 // same bits too. The rows of nodes in CPML slabs or on boundary planes (classes kGeneral and
-// kUniformGeneral + m) serve the CPML sweep, which divides the curl coefficients by the CPML
-// kappa and applies the boundary rules itself; the per-node kernels keep their general path for
-// those nodes. Lumped edges get no row (launch_rec_general).
+// kUniformGeneral + m) serve the kernels by row, which take the curl coefficients over kappa from
+// the axis tables or SlabRows and apply the boundary rules themselves; the kernels by class keep their
+// general path for those nodes. Lumped edges get rows of their own afterwards (special_row).
 namespace {
 __device__ __forceinline__ unsigned long long cell_key(const uint8_t* mat, const DeviceGrid& g, int i, int j, int k) {
     const long long R = g.pitch, P = g.plane, n = (long long)k * P + (long long)j * R + i;
@@ -569,7 +569,7 @@ __global__ void k_iface_coefs(const __grid_constant__ StepParams p, const unsign
     const int mk = (int)((key >> 24) & 0xff), mij = (int)((key >> 32) & 0xff), mik = (int)((key >> 40) & 0xff);
     const int mjk = (int)((key >> 48) & 0xff);
     // position-free coefficients: no design cells (those nodes are kDesignNode); CPML kappa and
-    // boundary faces are the CPML sweep's
+    // boundary faces are the kernels' own
     const Coef3 ex = e_coef(p, 0, m0 == mj && m0 == mk && m0 == mjk, m0, mj, mk, mjk, 1, 1, 1);
     const Coef3 ey = e_coef(p, 1, m0 == mi && m0 == mk && m0 == mik, m0, mi, mk, mik, 1, 1, 1);
     const Coef3 ez = e_coef(p, 2, m0 == mi && m0 == mj && m0 == mij, m0, mi, mj, mij, 1, 1, 1);

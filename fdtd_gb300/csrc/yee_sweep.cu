@@ -156,7 +156,7 @@ __device__ __forceinline__ void slow_node(const SweepArgs* pa, SweepSmem<Idx>* p
         nb.ex = TE[0]; nb.ey = TE[EF]; nb.ez = TE[2 * EF];
         const PsiIO io{pa->pin.f, pa->pout.f, own && store_e};
         if (c < kRecGeneral) {
-            e_update_diff<false, false, false, false, 7, true>(p, nb, d, i, j, k, m, false, io, out, pre, nullptr, c);
+            e_update_diff<false, false, false, false, true>(p, nb, d, i, j, k, m, false, io, out, pre, c);
         } else {
             const uint8_t* mat = p.mat;
             nb.m0 = mat[n];
@@ -167,7 +167,7 @@ __device__ __forceinline__ void slow_node(const SweepArgs* pa, SweepSmem<Idx>* p
             nb.mik = (i > 0 && k > 0) ? mat[n - 1 - PL] : 0;
             nb.mjk = (j > 0 && k > 0) ? mat[n - R - PL] : 0;
             const bool lumped = p.lumped_k[k] < p.lumped_k[k + 1];
-            e_update_diff<true, false, true, false, 7>(p, nb, d, i, j, k, m, lumped, io, out, pre);
+            e_update_diff<true, false, true, false>(p, nb, d, i, j, k, m, lumped, io, out, pre);
             if (own && store_e && p.probe_k[k] < p.probe_k[k + 1])
                 for (int a = 0; a < 3; ++a) sample(p, rr, a, i, j, k, pre[a]);
         }
@@ -188,14 +188,14 @@ __device__ __forceinline__ void slow_node(const SweepArgs* pa, SweepSmem<Idx>* p
     const long long n = (long long)kh * PL + (long long)j * R + i;
     const PsiIO io{pa->pin.f, pa->pout.f, true};
     if (cp < kRecGeneral) {
-        h_update_diff<false, false, 7, true>(p, nb, f, i, j, kh, io, out, pre, nullptr, cp);
+        h_update_diff<false, false, true>(p, nb, f, i, j, kh, io, out, pre, cp);
     } else {
         const uint8_t* mat = p.mat;
         nb.m0 = mat[n];
         nb.mi = i > 0 ? mat[n - 1] : 0;
         nb.mj = j > 0 ? mat[n - R] : 0;
         nb.mk = kh > 0 ? mat[n - PL] : 0;
-        h_update_diff<false, false, 7>(p, nb, f, i, j, kh, io, out, pre);
+        h_update_diff<false, false>(p, nb, f, i, j, kh, io, out, pre);
         if (p.probe_k[kh] < p.probe_k[kh + 1])
             for (int a = 0; a < 3; ++a) sample(p, rr, 3 + a, i, j, kh, pre[a]);
     }

@@ -41,7 +41,7 @@ def parse():
     ap.add_argument("--impl", choices=["ours", "reference"], default="ours")
     ap.add_argument("--config", choices=["512", "256", "64", "hbm"], default="512")
     ap.add_argument("--schedule", type=int, default=0,
-                    help="0 auto, 1 two-pass, 2 fused, 3 fused with the CPML sweep (not chosen by auto)")
+                    help="0 auto, 1 two-pass, 2 fused, 3 the same as 2")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--no-adjoint", action="store_true")
@@ -261,17 +261,14 @@ def fp64_error():
 TWO_PASS_DRAM_BYTES_PER_CELL = 78.15
 
 
-# DRAM bytes per cell update of one fused step (k_shell_e + k_sweep_interior + k_shell_h),
-# dram__bytes_read.sum + dram__bytes_write.sum from ncu captures of these kernels (the launch-list
-# commands in profiles/yee_step_boxes512_launch_list.md): 63.59 B on the 512^3 bench workload
-# itself, 72.77 B at 256^3, where the shell share is larger. Refreshed whenever the kernels change.
-FUSED_DRAM_BYTES_PER_CELL = {"512": 63.59, "256": 72.77}
+# DRAM bytes per cell update of one fused step (k_sweep), dram__bytes_read.sum + dram__bytes_write.sum
+# from ncu captures (profiles/update_kernels_counters.md): 59.07 B on the 512^3 random-box grid, 61.97 B at
+# 256^3, where the CPML share is larger. Refreshed whenever the kernel changes.
+FUSED_DRAM_BYTES_PER_CELL = {"512": 59.07, "256": 61.97}
 
 
 def measured_traffic(schedule, cells, config):
-    if schedule == 3:
-        return None  # not profiled
-    if schedule == 2:
+    if schedule in (2, 3):  # the same kernel
         per_cell = FUSED_DRAM_BYTES_PER_CELL.get(config)
         if per_cell is None:
             return None  # no capture of this workload's DRAM bytes
@@ -296,7 +293,7 @@ def bench_ours(args, rank, world):
     sim = solver.Simulation.from_scenario(sc, args.schedule, material_index=mat, probe_capacity=total_steps)
     sim.set_stream(stream.cuda_stream)
     sim.prepare()
-    sim.tune_schedule()  # AUTO: time both schedules on this grid (state kept) and keep the faster
+    sim.tune_schedule()  # AUTO: choose now, before the warm-up
     sim.step(args.warmup)
     sim.synchronize()
     active = sim.active_schedule

@@ -890,11 +890,13 @@ __global__ void __launch_bounds__(NTH, kWide ? 2 : 3) k_sweep(const __grid_const
     const StepParams& p = A.p;
     const DeviceGrid& g = p.g;
     const int tid = threadIdx.x;
-    // item: chunk outer, tiles inner (x fastest), so the CTAs in flight work on neighbouring planes
+    // item: chunk outer, tiles inner (x fastest), so the CTAs in flight work on neighbouring planes; every
+    // other step from the top down, beginning with what the step before wrote last and L2 still holds
+    // (225 x 190 x 163 3.27 -> 3.24 ms for 24 steps)
     int b = blockIdx.x;
     const int bx = b % A.sg.nbx;
     b /= A.sg.nbx;
-    const int by = b % A.sg.nby, ch = b / A.sg.nby;
+    const int by = b % A.sg.nby, ch = A.m & 1 ? A.sg.chunks() - 1 - b / A.sg.nby : b / A.sg.nby;
     const int x0 = bx * TX, y0 = by * TY;
     const int k0 = A.sg.chunk(ch), k1 = A.sg.chunk(ch + 1);
     const int kfirst = k0 - 1;  // the planes k0 - 1 .. k1, at most kMaxSweepPlanes (plan_sweep)

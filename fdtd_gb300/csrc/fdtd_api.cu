@@ -1339,7 +1339,6 @@ int build_interface_rows(fdtd_handle* h) {
         std::sort(hk.begin(), hk.end());
         hk.erase(std::unique(hk.begin(), hk.end()), hk.end());
         if (hk.size() > (size_t)kMaxInterfaceRows) hk.resize((size_t)kMaxInterfaceRows);  // the rest stay general
-        // pageable source: the copy has taken the data when the call returns
         CUDA_TRY(cudaMemcpyAsync(h->iface_keys, hk.data(), hk.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice,
                                  h->stream));
     }
@@ -1409,6 +1408,7 @@ int build_interface_rows(fdtd_handle* h) {
     h->n_iface_rows = n_rows;
     h->n_coef_rows = kFirstInterfaceRow + n_rows + n_special;
     CUDA_TRY(cudaMemcpyAsync(&h->edge_mat, h->small, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    CUDA_TRY(cudaStreamSynchronize(h->stream));  // edge_mat is here, and the copies from this function's vectors are done
     return FDTD_OK;
 }
 
@@ -1491,7 +1491,6 @@ int ensure_prepared(fdtd_handle* h) {
         h->dirty_materials = false;
         h->dirty_lumped = true;
     }
-    const bool rows = h->dirty_lumped;
     if (h->dirty_lumped) {
         int rc = build_lumped(h);
         if (rc) return rc;
@@ -1502,6 +1501,8 @@ int ensure_prepared(fdtd_handle* h) {
         if (rc) return rc;
         if (h->n_plate_nodes > 0) CUDA_TRY(launch_class_nodes(h->g, h->d_plate_nodes, h->n_plate_nodes, kPlateNode, h->cls, h->stream));
         rc = build_interface_rows(h);
+        if (rc) return rc;
+        rc = build_slab_rows(h);
         if (rc) return rc;
     }
     if (h->dirty_probes) {
@@ -1514,11 +1515,8 @@ int ensure_prepared(fdtd_handle* h) {
         CUDA_TRY(launch_count_general(h->g, h->rec, h->d_plate_nodes, h->n_plate_nodes, h->small + 1, h->stream));
         CUDA_TRY(cudaMemcpyAsync(&h->n_plate_general, h->small + 1, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     }
+    // every table is in place on return: the next step may run on another stream (fdtd_set_stream)
     CUDA_TRY(cudaStreamSynchronize(h->stream));
-    if (rows) {
-        int rc = build_slab_rows(h);
-        if (rc) return rc;
-    }
     h->prepared = true;
     return FDTD_OK;
 }

@@ -1504,6 +1504,7 @@ int ensure_prepared(fdtd_handle* h) {
         if (rc) return rc;
         rc = build_slab_rows(h);
         if (rc) return rc;
+        if (!h->slab_rows) CUDA_TRY(launch_rec_slab_plates(h->g, h->d_plate_nodes, h->n_plate_nodes, h->rec, h->stream));
     }
     if (h->dirty_probes) {
         int rc = build_probes(h);

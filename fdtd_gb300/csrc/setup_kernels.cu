@@ -540,6 +540,23 @@ cudaError_t launch_rec_probes(const DeviceGrid& g, const Probe* probes, int n, u
     return cudaGetLastError();
 }
 
+// The plate nodes inside a CPML slab, where the slab rows are missing: the kernels by row leave such a
+// node's row alone then, and k_plate_e goes by the general mark.
+__global__ void k_rec_slab_plates(uint16_t* rec, DeviceGrid g, const int4* nodes, int n) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    const int4 v = nodes[q];
+    if (!in_slab(v.x, g.nx, g.pxn, g.pxp) && !in_slab(v.y, g.ny, g.pyn, g.pyp) && !in_slab(v.z, g.nz, g.pzn, g.pzp)) return;
+    uint16_t& r = rec[(long long)v.z * g.plane + (long long)v.y * g.pitch + v.x];
+    if (r < kRecGeneral) r = (uint16_t)(kRecGeneral | kPlateNode);
+}
+
+cudaError_t launch_rec_slab_plates(const DeviceGrid& g, const int4* nodes, int n, uint16_t* rec, cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    k_rec_slab_plates<<<(n + 127) / 128, 128, 0, st>>>(rec, g, nodes, n);
+    return cudaGetLastError();
+}
+
 // How many of the listed nodes take the general path.
 __global__ void k_count_general(const uint16_t* rec, DeviceGrid g, const int4* nodes, int n, int* count) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;

@@ -131,6 +131,8 @@ cudaError_t launch_iface_coefs(const StepParams& p, const unsigned long long* ke
 // The nodes of the probes inside a CPML slab to the general path (after launch_iface_rows), which
 // samples them before the CPML correction.
 cudaError_t launch_rec_probes(const DeviceGrid& g, const Probe* probes, int n, uint16_t* rec, cudaStream_t st);
+// The listed plate nodes inside a CPML slab to the general path (grids without SlabRows).
+cudaError_t launch_rec_slab_plates(const DeviceGrid& g, const int4* nodes, int n, uint16_t* rec, cudaStream_t st);
 // Coefficient rows of listed nodes ({i, j, k, source or -1}: nodes with plate-covered or lumped
 // edges, which no seven-cell key describes). launch_special_set collects their distinct rows by a
 // 64-bit hash of the row and the source in the set of launch_iface_set (bit 63: a source), the list

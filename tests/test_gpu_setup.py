@@ -51,3 +51,33 @@ def test_prepare_waits_for_its_kernels(gpu_lib):
         assert stream.query()
         assert sim.device_bytes() > 2e8  # the table was built
         sim.synchronize()
+
+
+@pytest.mark.parametrize("schedule", [1, 2])
+def test_plates_in_slabs_without_the_slab_rows(gpu_lib, schedule):
+    """Some 30000 rows times 300 slab planes are more than the table of slab coefficients may hold (256 MiB): it is
+    not built, and plates in the slabs are updated all the same, as the oracle has them."""
+    import oracle
+    from conftest import bitwise_equal
+    from fdtd_gb300 import solver
+    n, pml, block = 110, 50, 30
+    sc, index = rows_case(n, pml, block)
+    assert key_count(index) < 32000 and key_count(index) * 6 * pml * SLAB_ROW_BYTES > 257 * 2**20
+    sc.plates = [S.Plate(2, (35, 30, 55, 100, 80, 55), 1e10, 1e7),  # from slab to slab through the middle
+                 S.Plate(0, (70, 35, 40, 70, 90, 70), 3e3, 1e10),   # inside an x slab
+                 S.Plate(1, (40, 0, 35, 60, 0, 60), 1e5, 1e6)]      # on a low wall
+    c = n // 2
+    sc.sources = [S.LumpedSource((c, c, c + 2, c, c, c + 3), 50.0, sc.sources[0].waveform)]
+    sc.probes = [S.Probe(S.EX, 75, 55, 55), S.Probe(S.EY, 70, 60, 55), S.Probe(S.EZ, 70, 60, 50)]
+    rng = np.random.default_rng(4)
+    start = np.zeros((6, n, n, n), np.float32)
+    start[:, 1:-1, 1:-1, 1:-1] = rng.standard_normal((6, n - 2, n - 2, n - 2)).astype(np.float32)
+    with solver.Simulation.from_scenario(sc, schedule, material_index=index, probe_capacity=sc.steps) as sim:
+        for q in range(6):
+            sim.set_field(q, start[q])
+        sim.step(sc.steps)
+        sim.synchronize()
+        got, fields, prof = sim.read_probes(0, sc.steps), sim.fields(), sim.cpml_profiles()
+        assert sim.device_bytes() < 250e6  # without the table
+    want, want_fields = oracle.run(sc, init_fields=start, profile_override=prof)
+    assert bitwise_equal(got, want) and bitwise_equal(fields, want_fields)

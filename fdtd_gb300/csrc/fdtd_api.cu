@@ -350,7 +350,8 @@ int alloc_psi_set(fdtd_handle* h, int s) {
     if (h->alloc((void**)&base, total) != cudaSuccess) return fail(FDTD_ERR_OOM, "CPML memory allocation failed");
     h->psi_base[s] = base;
     h->psi[s].base = (float*)base;
-    if (launch_fill((float*)base, (long long)(total / sizeof(float)), kTiny, nullptr) != cudaSuccess)
+    // on the handle's stream, whose steps write the set next (at creation still the legacy stream)
+    if (launch_fill((float*)base, (long long)(total / sizeof(float)), kTiny, h->stream) != cudaSuccess)
         return fail(FDTD_ERR_CUDA, "fill failed");
     for (int f = 0; f < 6; ++f) {
         if (h->psi_elems[f] <= 0) continue;

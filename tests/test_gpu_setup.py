@@ -81,3 +81,31 @@ def test_plates_in_slabs_without_the_slab_rows(gpu_lib, schedule):
         assert sim.device_bytes() < 250e6  # without the table
     want, want_fields = oracle.run(sc, init_fields=start, profile_override=prof)
     assert bitwise_equal(got, want) and bitwise_equal(fields, want_fields)
+
+
+def test_second_buffers_filled_on_the_handles_stream(gpu_lib):
+    """The fused schedule's second CPML set is filled on the stream that the steps run on: with the legacy stream busy,
+    a handle on a non-blocking stream gets the same state."""
+    import torch
+    from fdtd_gb300 import solver
+    sc = S.vacuum_cube(40, 8, pml=8, name="fill")
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    start = [torch.rand((40, 40, 40), generator=gen, device="cuda") - 0.5 for _ in range(6)]
+    stream = torch.cuda.Stream()
+    states = []
+    for busy in (False, True):
+        with solver.Simulation.from_scenario(sc, 2) as sim:
+            sim.set_stream(stream.cuda_stream)
+            for c, f in enumerate(start):
+                sim.set_field_device(c, f.data_ptr())
+            sim.prepare()
+            state = torch.zeros(sim.state_bytes(), dtype=torch.uint8, device="cuda")
+            torch.cuda.synchronize()
+            if busy:
+                torch.cuda._sleep(200_000_000)  # some 0.1 s on the legacy stream
+            sim.step(5)
+            torch.cuda.synchronize()
+            sim.save_state(state.data_ptr())
+            torch.cuda.synchronize()
+            states.append(state)
+    assert torch.equal(*states)

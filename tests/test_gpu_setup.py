@@ -89,6 +89,7 @@ def test_second_buffers_filled_on_the_handles_stream(gpu_lib):
     import torch
     from fdtd_gb300 import solver
     sc = S.vacuum_cube(40, 8, pml=8, name="fill")
+    sc.sources, sc.probes = [], []
     gen = torch.Generator(device="cuda").manual_seed(5)
     start = [torch.rand((40, 40, 40), generator=gen, device="cuda") - 0.5 for _ in range(6)]
     stream = torch.cuda.Stream()

@@ -74,6 +74,17 @@ struct SweepPlan {
         return c == chunks() ? nz : zhi + (int)((long long)(c - n_lo - n_mid) * (nz - zhi) / n_hi);
     }
 };
+// The sweep's ring of n stages. Plane q of a chunk (0: the plane below its first) lies in stage(q), its copy
+// completes the phase with parity(q) of that stage's barrier. At the top of plane step k, before its copy is
+// issued, the planes up to k - 2 have arrived and those below drain_end(k) have been asked for: a chunk that
+// gives up there waits for the planes from drain_begin(k) on, the one whose wait failed among them.
+struct SweepRing {
+    FDTD_HD static constexpr int stage(int q, int n) { return q % n; }
+    FDTD_HD static constexpr unsigned parity(int q, int n) { return (unsigned)(q / n) & 1u; }
+    FDTD_HD static constexpr int drain_begin(int k) { return k - 1; }
+    FDTD_HD static constexpr int drain_end(int k, int k1, int n) { return (k + n - 2 < k1 ? k + n - 2 : k1) + 1; }
+};
+
 // share: the part of the device the grid has to itself (1 / n for one of n grids swept at once).
 SweepPlan plan_sweep(const PlanGrid& g, double share = 1.0);
 

@@ -33,7 +33,7 @@
 // background's have their slab coefficients in a table (SlabRows), since divisions in line made grids
 // with materials in the slabs 10-20 % slower (128^3 73 -> 60 us).
 // All arithmetic is that of yee_common.cuh, so the results equal the two-pass schedule's bits.
-// Every wait on a TMA barrier is bounded: on timeout the kernel records an error in the status
+// Every wait on a TMA barrier is bounded: on timeout the kernel uses nothing of that plane, records an error in the status
 // word, drains its own copies (again bounded) and exits.
 #define FDTD_RARE __forceinline__  // calls in the slow path would spill the march's state (512^3: 31.0 -> 28.6 ms for 20 steps)
 #include <cuda.h>
@@ -354,16 +354,12 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
 #pragma unroll 1
     for (int k = k0;; ++k) {
         if (__syncthreads_or(!ok)) {
-            // a plane never arrived: record it, wait (bounded) for the copies still in flight, exit
+            // a plane never arrived: record it, wait (bounded) for the copies that may still be in flight, exit
             if (kEdge) cp_async_wait_all();
             if (threadIdx.x == 0) {
                 atomic_flag(p.status, 1);
-                int r = s;
-                uint32_t par = parity;
-                for (int q = k; q <= min(k1, k + NST - 2); ++q) {
-                    mbar_wait(&S.bar[r], par);
-                    if (++r == NST) { r = 0; par ^= 1u; }
-                }
+                for (int q = SweepRing::drain_begin(k); q < SweepRing::drain_end(k, k1, NST); ++q)
+                    mbar_wait(&S.bar[SweepRing::stage(q - kfirst, NST)], SweepRing::parity(q - kfirst, NST));
             }
             __syncthreads();
             return;
@@ -397,6 +393,7 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                 }
         }
         ok = mbar_wait(&S.bar[s], parity);
+        if (!ok) continue;  // the stage holds anything: no row of it may index a table, nothing is stored
         const Quad hx = lds4(T + H_OFF), hy = lds4(T + H_OFF + HF), hz = lds4(T + H_OFF + 2 * HF);
         const uint2 cw = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(S.stage[s] + 3 * H_BYTES + 3 * E_BYTES) + t);
         Quad vx, vy, vz;

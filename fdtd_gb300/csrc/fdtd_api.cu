@@ -702,6 +702,11 @@ int fdtd_add_brick(fdtd_handle* h, const int32_t box[6], int32_t material) {
     return FDTD_OK;
 }
 
+// Whether a lumped Ez element's edges (cells i-1..i, j-1..j each) touch cells of the design box d.
+static bool touches_design(const int32_t* b, const int32_t* d) {
+    return b[0] - 1 < d[3] && d[0] <= b[3] && b[1] - 1 < d[4] && d[1] <= b[4] && b[2] < d[5] && d[2] < b[5];
+}
+
 static int check_lumped_box(fdtd_handle* h, int32_t axis, const int32_t box[6], float r) {
     if (!box) return fail(FDTD_ERR_INVALID, "box is NULL");
     if (axis != 0 && axis != 2) return fail(FDTD_ERR_INVALID, "lumped elements are x- (axis 0) or z-directed (axis 2)");
@@ -712,6 +717,8 @@ static int check_lumped_box(fdtd_handle* h, int32_t axis, const int32_t box[6], 
         if (is < 1 || ie > g.nx - 2 || is > ie || js < 1 || je > g.ny - 2 || js > je || ks < 0 || ke > g.nz - 1 ||
             ks >= ke)
             return fail(FDTD_ERR_INVALID, "lumped box outside the updated Ez edges or empty (k range is half-open)");
+        if (h->has_design && touches_design(box, h->dbox))
+            return fail(FDTD_ERR_INVALID, "a lumped element touches the design region");
     } else {
         // defineSourceX's Ex edges i in [is,ie), j in [js,ie], k in [ks,ke]; Ex is updated for
         // i < nx-1, 0 < j < ny-1, 0 < k < nz-1 (fdtdrav.h:665); je enters only its resistance
@@ -1297,19 +1304,21 @@ int build_plates(fdtd_handle* h) {
 
 // The nodes whose coefficients no seven-cell key describes but a row can: those with a plate-covered
 // edge (none of them a lumped edge), and those with a lumped edge outside the CPML slabs, with the
-// source that drives their Ez edge (-1: none; sources past kSweepSources stay on the general path).
-// {i, j, k, source}.
+// source that drives their Ez edge (-1: none; sources past kSweepSources stay on the general path). Nodes of
+// the design edge box have no row: the design cells' eps_r changes without new rows. {i, j, k, source}.
 constexpr size_t kSpecialEach = 256;
 size_t special_nodes(const fdtd_handle* h, std::vector<int4>& out) {
     const DeviceGrid& g = h->g;
-    constexpr int kInSlab = kSweepSources;  // never a row
-    std::map<long long, int> lumped;        // node -> source
+    constexpr int kNoRow = kSweepSources;
+    std::map<long long, int> lumped;  // node -> source
+    const int* d = h->dbox;
     for (const LumpedDef& L : h->lumped)
         lumped_edges(L, [&](int i, int j, int k) {
+            const bool design = h->has_design && i >= d[0] && i <= d[3] && j >= d[1] && j <= d[4] && k >= d[2] && k <= d[5];
             const bool slab = in_slab_host(i, g.nx, g.pxn, g.pxp) || in_slab_host(j, g.ny, g.pyn, g.pyp) ||
                               in_slab_host(k, g.nz, g.pzn, g.pzp);
             int& s = lumped.emplace(((long long)k * g.ny + j) * g.nx + i, -1).first->second;
-            s = std::max(s, slab ? kInSlab : L.source);
+            s = std::max(s, slab || design ? kNoRow : L.source);
         });
     auto node = [&](long long v, int s) {
         return make_int4((int)(v % g.nx), (int)((v / g.nx) % g.ny), (int)(v / ((long long)g.nx * g.ny)), s);
@@ -1692,11 +1701,8 @@ extern "C" int fdtd_set_design_region(fdtd_handle* h, const int32_t box[6], cons
     for (const LumpedDef& L : h->lumped)
         if (L.axis != 2)
             return fail(FDTD_ERR_STATE, "a design region cannot be combined with x-directed lumped elements");
-    for (const LumpedDef& L : h->lumped) {  // the cells of a lumped Ez edge (i,j): i-1..i, j-1..j
-        const int* b = L.box;
-        if (b[0] - 1 < box[3] && box[0] <= b[3] && b[1] - 1 < box[4] && box[1] <= b[4] && b[2] < box[5] && box[2] < b[5])
-            return fail(FDTD_ERR_INVALID, "a lumped element touches the design region");
-    }
+    for (const LumpedDef& L : h->lumped)
+        if (touches_design(L.box, box)) return fail(FDTD_ERR_INVALID, "a lumped element touches the design region");
     const size_t nd = (size_t)(box[3] - box[0]) * (box[4] - box[1]) * (box[5] - box[2]);
     for (size_t q = 0; q < nd; ++q)
         if (!(eps_r[q] > 0.f) || !std::isfinite(eps_r[q])) return fail(FDTD_ERR_INVALID, "design eps_r must be positive");

@@ -356,9 +356,14 @@ __global__ void k_node_class(const uint8_t* __restrict__ mat, uint8_t* __restric
         node_class(mat, cls, g, dlo, dhi, i, j, k);
 }
 
+// A node of the design edge box stays kDesignNode (an Ez lumped element may stand on the region's top
+// face): its Ex and Ey take the design cells' eps_r, its Ez the lumped override, which the design kernels
+// look for.
 __global__ void k_class_lumped(uint8_t* cls, DeviceGrid g, const LumpedEdge* edges, int n_edges) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < n_edges) cls[(long long)edges[q].k * g.plane + (long long)edges[q].j * g.pitch + edges[q].i] = kGeneral;
+    if (q >= n_edges) return;
+    uint8_t& c = cls[(long long)edges[q].k * g.plane + (long long)edges[q].j * g.pitch + edges[q].i];
+    if (c != kDesignNode) c = kGeneral;
 }
 
 __global__ void k_class_nodes(uint8_t* cls, DeviceGrid g, const int4* nodes, int n, uint8_t value) {
@@ -516,11 +521,13 @@ __device__ __forceinline__ void iface_row(uint8_t* __restrict__ cls, const uint8
     rec[n] = (uint16_t)r;
 }
 
-// Lumped edges keep the general path in every schedule (their E update is the lumped override).
+// Lumped edges keep the general path in every schedule (their E update is the lumped override); those of
+// the design edge box are marked as its nodes already.
 __global__ void k_rec_general(uint16_t* rec, DeviceGrid g, const LumpedEdge* edges, int n_edges) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < n_edges)
-        rec[(long long)edges[q].k * g.plane + (long long)edges[q].j * g.pitch + edges[q].i] = (uint16_t)(kRecGeneral | kGeneral);
+    if (q >= n_edges) return;
+    uint16_t& r = rec[(long long)edges[q].k * g.plane + (long long)edges[q].j * g.pitch + edges[q].i];
+    if (r != (kRecGeneral | kDesignNode)) r = (uint16_t)(kRecGeneral | kGeneral);
 }
 
 // The nodes of probes inside a CPML slab too: the general path samples them before the CPML

@@ -119,6 +119,7 @@ struct fdtd_handle {
     SrcRow* src_rows = nullptr;
     ProbeAt* d_probes_at = nullptr;   // probes outside the CPML slabs
     int n_probes_at = 0;
+    int h_bg = 0;                     // StepParams::h_bg
     int edge_mat = 0;                 // rows other than the background's in a slab or on a low wall (read back by ensure_prepared)
     float4* slab_rows = nullptr;      // SlabRows, with edge_mat (NULL: too many rows, their nodes take the general path)
     int n_coef_rows = 0;
@@ -290,6 +291,7 @@ StepParams make_params(fdtd_handle* h) {
     p.bgn = h->bg_node;
     p.src_row0 = h->src_row0;
     p.src_rows = h->src_rows;
+    p.h_bg = h->h_bg;
     std::copy(h->te, h->te + 3, p.te);
     std::copy(h->th, h->th + 3, p.th);
     std::copy(h->psi_off, h->psi_off + 6, p.psi_off);
@@ -384,14 +386,15 @@ void* tensor_map_encoder() {
 // two-pass against sweep per step, boxes outside the CPML: 40^3 8.5 / 7.4 us, 64^3 11.3 / 10.4, 72^3 14.5 /
 // 15.9, 96^3 20.9 / 20.7, 112^3 31.7 / 34.3, 128^3 39.8 / 45.3, 136^3 60.0 / 59.0, 144^3 70 / 65, 160^3 89 / 78,
 // 200^3 175 / 129, 225^3 247 / 182. In between, where the fields sit in L2 and the sweep's CTAs do not
-// fill the device evenly, two-pass is ahead. Boxes that touch the CPML make the sweep's tiles there
-// slower than the others: 40^3 8.5 / 8.7 us, 64^3 11.3 / 12.5, 128^3 40 / 62, 160^3 90 / 113, 192^3 145 / 188,
-// 200^3 176 / 157, 225^3 253 / 217. Grids below kAutoSweepCells, a few CTAs' work, gain little. Grids with
+// fill the device evenly, two-pass is ahead. Materials that lie in the CPML make the sweep's tiles there
+// slower than the others. Boxes and a half space through every slab: 64^3 16.3 / 17.3 us, 128^3 51 / 62, 144^3
+// 81.7 / 81.5, 160^3 100 / 97, 192^3 162 / 137, 225^3 283 / 237, 256^3 349 / 247; of magnetic materials, whose H
+// coefficients differ from the background's: 160^3 101 / 120, 192^3 162 / 165, 200^3 213 / 202. Grids below kAutoSweepCells, a few CTAs' work, gain little. Grids with
 // a design region take the sweep from kAutoDesignCells on (smaller ones record in their two-pass
 // kernels). Two-pass also serves where the second buffers cannot be allocated.
 constexpr long long kAutoSweepCells = 32LL << 10;
 constexpr long long kAutoTwoPassLo = 300LL << 10, kAutoTwoPassHi = 2450LL << 10;
-constexpr long long kAutoEdgeHi = 7400LL << 10;  // with slab_rows, two-pass below this
+constexpr long long kAutoEdgeHi = 3LL << 20, kAutoEdgeMagneticHi = 7LL << 20;  // with slab_rows, two-pass below this
 constexpr long long kAutoDesignCells = 64LL << 20;
 
 // The background material's coefficients (StepParams::bgn), evaluated on the host with the rounding steps of
@@ -482,7 +485,7 @@ void auto_choose(fdtd_handle* h, int64_t n) {
     const long long cells = (long long)h->g.nx * h->g.ny * h->g.nz;
     const bool small = cells < kAutoTwoPassLo;
     if (h->has_design ? cells < kAutoDesignCells
-        : h->slab_rows ? cells < kAutoEdgeHi
+        : h->slab_rows ? cells < (h->h_bg ? kAutoEdgeHi : kAutoEdgeMagneticHi)
                        : cells < kAutoSweepCells || (!small && cells < kAutoTwoPassHi)) {
         h->auto_choice = FDTD_SCHEDULE_TWO_PASS;
         return;
@@ -600,7 +603,6 @@ int fdtd_create(const fdtd_grid* grid, fdtd_handle** out) {
     if (cudaMemset(h->mat, 0, (size_t)V) != cudaSuccess || cudaMemset(h->status, 0, sizeof(int)) != cudaSuccess)
         return cleanup(fail(FDTD_ERR_CUDA, "memset failed"));
     h->materials.push_back(axes_of(fdtd_material{1.0f, kTiny, 1.0f, kTiny}));
-    h->sweep = plan_sweep(PlanGrid{g.nx, g.ny, g.nz, g.pxn, g.pxp, g.pyn, g.pyp, g.pzn, g.pzp});
     cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return cleanup(fail(FDTD_ERR_CUDA, std::string("init: ") + cudaGetErrorString(e)));
     *out = h;
@@ -1417,8 +1419,12 @@ int build_interface_rows(fdtd_handle* h) {
     CUDA_TRY(launch_iface_coefs(pi, h->iface_keys, n_rows, h->coef_rows, h->stream));
     h->n_iface_rows = n_rows;
     h->n_coef_rows = kFirstInterfaceRow + n_rows + n_special;
-    CUDA_TRY(cudaMemcpyAsync(&h->edge_mat, h->small, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(cudaStreamSynchronize(h->stream));  // edge_mat is here, and the copies from this function's vectors are done
+    CUDA_TRY(launch_rows_h(h->coef_rows, h->n_coef_rows, 0, h->small + 1, h->stream));
+    int marks[2] = {0, 0};
+    CUDA_TRY(cudaMemcpyAsync(marks, h->small, sizeof(marks), cudaMemcpyDeviceToHost, h->stream));
+    CUDA_TRY(cudaStreamSynchronize(h->stream));  // (the copies from this function's vectors are done, too)
+    h->edge_mat = marks[0];
+    h->h_bg = !marks[1];
     return FDTD_OK;
 }
 
@@ -1514,6 +1520,8 @@ int ensure_prepared(fdtd_handle* h) {
         if (rc) return rc;
         rc = build_slab_rows(h);
         if (rc) return rc;
+        const DeviceGrid& g = h->g;
+        h->sweep = plan_sweep(PlanGrid{g.nx, g.ny, g.nz, g.pxn, g.pxp, g.pyn, g.pyp, g.pzn, g.pzp}, 1.0, h->slab_rows != nullptr);
         if (!h->slab_rows) CUDA_TRY(launch_rec_slab_plates(h->g, h->d_plate_nodes, h->n_plate_nodes, h->rec, h->stream));
     }
     if (h->dirty_probes) {
@@ -1523,8 +1531,8 @@ int ensure_prepared(fdtd_handle* h) {
     CUDA_TRY(launch_rec_probes(h->g, h->d_probes, (int)h->probes.size(), h->rec, h->stream));
     h->n_plate_general = 0;
     if (!h->plates.empty() && h->n_plate_nodes > 0) {
-        CUDA_TRY(launch_count_general(h->g, h->rec, h->d_plate_nodes, h->n_plate_nodes, h->small + 1, h->stream));
-        CUDA_TRY(cudaMemcpyAsync(&h->n_plate_general, h->small + 1, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+        CUDA_TRY(launch_count_general(h->g, h->rec, h->d_plate_nodes, h->n_plate_nodes, h->small + 2, h->stream));
+        CUDA_TRY(cudaMemcpyAsync(&h->n_plate_general, h->small + 2, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     }
     // every table is in place on return: the next step may run on another stream (fdtd_set_stream)
     CUDA_TRY(cudaStreamSynchronize(h->stream));

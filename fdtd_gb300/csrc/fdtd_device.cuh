@@ -187,6 +187,7 @@ struct StepParams {
     long long psi_off[6], psi_stride[6];
     long long psi_total;
     SlabRows rows;  // e[0] NULL: not built (no such nodes, or too many rows)
+    int h_bg;       // every row has the background's H coefficients (no magnetic material)
     // design region: cells of material kDesign inside dbox = [d0,d3) x [d1,d4) x [d2,d5) take eps_r
     // from deps ((d5-d2), (d4-d1), (d3-d0), x fastest); NULL when the handle has none
     const float* deps;

@@ -2,6 +2,7 @@
 #include "planner.h"
 
 #include <algorithm>
+#include <cmath>
 
 namespace fdtd {
 
@@ -56,7 +57,12 @@ std::vector<int> starts(int lo, int hi, int size, int align, bool overlap) {
 // run in several waves, cuts at the z slabs keep the slabs' rules out of the middle chunks (512^3 1.36 ->
 // 1.33 ms); in a single wave they would only start a second one (281 x 123 x 162: 131 us with the cuts,
 // 121 without).
-SweepPlan plan_sweep(const PlanGrid& g, double share) {
+//
+// rows: materials lie in the CPML slabs. Their chunks take up to twice as long as the others, so a single wave of
+// long ones ends with most of the device idle (192^3 with a half space: 284 us a step, 137 with chunks of 8
+// planes cut at the z slabs). Chunks of 8 to 32 planes then, for some eight waves, and always the cuts: 144^3 106 ->
+// 82 us, 225^3 243 -> 236, 256^3 268 -> 252, 400^3 750 either way; grids whose plan has shorter chunks anyway keep it.
+SweepPlan plan_sweep(const PlanGrid& g, double share, bool rows) {
 #ifndef FDTD_SWEEP_SLOTS
 #define FDTD_SWEEP_SLOTS 3
 #endif
@@ -74,9 +80,16 @@ SweepPlan plan_sweep(const PlanGrid& g, double share) {
             p.n_mid = nch;
         }
     }
-    const int kc = (g.nz + p.n_mid - 1) / p.n_mid;
+    int kc = (g.nz + p.n_mid - 1) / p.n_mid;
+    constexpr int kRowsChunk = 8, kRowsWaves = 8;
+    const bool cut = rows && kc >= kRowsChunk;
+    if (cut) {
+        kc = (int)std::ceil((double)tiles * g.nz / (kRowsWaves * slots));
+        kc = std::min(std::max(kc, kRowsChunk), kMaxSweepChunk);
+        p.n_mid = (g.nz + kc - 1) / kc;
+    }
     const int lo = g.pzn > 1 ? g.pzn : 1, hi = (g.pzp > 1 ? g.nz - g.pzp : g.nz - 1) - 1;
-    if (kc >= 24 && hi - lo >= kc && tiles * p.n_mid > slots) {
+    if (hi - lo >= kc && (cut || (kc >= 24 && tiles * p.n_mid > slots))) {
         auto chunks = [&](int n) { return (n + kc - 1) / kc; };
         p.zlo = lo;
         p.zhi = hi;

@@ -85,8 +85,9 @@ struct SweepRing {
     FDTD_HD static constexpr int drain_end(int k, int k1, int n) { return (k + n - 2 < k1 ? k + n - 2 : k1) + 1; }
 };
 
-// share: the part of the device the grid has to itself (1 / n for one of n grids swept at once).
-SweepPlan plan_sweep(const PlanGrid& g, double share = 1.0);
+// share: the part of the device the grid has to itself (1 / n for one of n grids swept at once). rows: materials
+// lie in the CPML slabs (SlabRows).
+SweepPlan plan_sweep(const PlanGrid& g, double share = 1.0, bool rows = false);
 
 // Planes per interior item (see plan_chunk in planner.cpp).
 int plan_chunk(const PlanGrid& g);

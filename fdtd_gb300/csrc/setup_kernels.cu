@@ -223,6 +223,21 @@ __global__ void k_slab_rows(const MatCoef* __restrict__ coef, DeviceGrid g, int 
     out[n_rows * L + q] = make_float4(__fdiv_rn(h0, km[a][at]), __fdiv_rn(h1, km[a][at]), __fmul_rn(h0, size), __fmul_rn(h1, size));
 }
 
+__global__ void k_rows_h(const MatCoef* __restrict__ coef, int n_rows, int bg, int* differ) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n_rows) return;
+    const uint32_t *a = reinterpret_cast<const uint32_t*>(coef[q].h), *b = reinterpret_cast<const uint32_t*>(coef[bg].h);
+    for (int w = 0; w < (int)(sizeof(MatCoef::h) / 4); ++w)
+        if (a[w] != b[w]) *differ = 1;
+}
+
+cudaError_t launch_rows_h(const MatCoef* coef, int n_rows, int bg, int* differ, cudaStream_t st) {
+    const cudaError_t e = cudaMemsetAsync(differ, 0, sizeof(int), st);
+    if (e != cudaSuccess || n_rows <= 0) return e;
+    k_rows_h<<<(n_rows + 127) / 128, 128, 0, st>>>(coef, n_rows, bg, differ);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_slab_rows(const DeviceGrid& g, const MatCoef* coef, int n_rows, float* const kappa[6], float4* out,
                              cudaStream_t st) {
     const int L = max(g.pxn + g.pxp, max(g.pyn + g.pyp, g.pzn + g.pzp));

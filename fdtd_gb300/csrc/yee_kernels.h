@@ -60,6 +60,8 @@ struct FusedMaps {  // tensor maps of buffer A
     CUtensorMap rec;  // coefficient rows (StepParams::rec)
 };
 cudaError_t launch_count_general(const DeviceGrid& g, const uint16_t* rec, const int4* nodes, int n, int* count, cudaStream_t st);
+// *differ (device int) becomes 1 if a row's H coefficients are not those of row bg.
+cudaError_t launch_rows_h(const MatCoef* coef, int n_rows, int bg, int* differ, cudaStream_t st);
 cudaError_t launch_slab_rows(const DeviceGrid& g, const MatCoef* coef, int n_rows, float* const prof_kappa[6], float4* out,
                              cudaStream_t st);
 

@@ -15,7 +15,8 @@
 // Coefficients. A quad whose four nodes share a coefficient row loads it once (the background's comes
 // with the kernel parameters); in a CPML slab the curl coefficients along the slab's axis come from
 // the axis' table for background nodes (StepParams::te, th: divided by kappa) and from SlabRows for
-// other rows. Quads of several rows take them node by node. What is left (lumped edges in a slab,
+// other rows. Quads of several rows load them component by component, or node by node where the registers
+// do not allow that. Where no material is magnetic (StepParams::h_bg), H looks at no rows at all. What is left (lumped edges in a slab,
 // design nodes, probes in a slab, keys beyond the table) runs e_update_diff / h_update_diff (slow_node).
 // Old CPML memory of the y and z faces is fetched a plane ahead with cp.async into slots of the
 // thread's own.
@@ -237,6 +238,18 @@ __device__ __forceinline__ void st_mask2(float* a, float* b, const Quad& x, cons
         }
     }
 }
+// The halves of an entry of SlabRows: curl coefficients, factors of the CPML memory.
+__device__ __forceinline__ float2 curl2(const float4* t) { return __ldg(reinterpret_cast<const float2*>(t)); }
+__device__ __forceinline__ float2 psi2(const float4* t) { return __ldg(reinterpret_cast<const float2*>(t) + 1); }
+// The curl coefficients along x of the nodes of a mask, entry r for node r.
+__device__ __forceinline__ void curl_x(Quad& c0, Quad& c1, const float4* t, int mask) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+        if (mask >> r & 1) {
+            const float2 f = curl2(t + r);
+            c0.v[r] = f.x; c1.v[r] = f.y;
+        }
+}
 // The row of node r of a quad.
 __device__ __forceinline__ int row_at(const uint2& c, int r) { return (int)((r < 2 ? c.x : c.y) >> (16 * (r & 1)) & 0xffffu); }
 __device__ __forceinline__ float pick(const Quad& q, int r) { return r == 0 ? q.v[0] : r == 1 ? q.v[1] : r == 2 ? q.v[2] : q.v[3]; }
@@ -252,7 +265,10 @@ __device__ __forceinline__ Quad quad_of(const float4& f) { return Quad{f.x, f.y,
 // The march of one thread's quad at tile row `row`, first column `col`. kEdge: the tile (halo
 // included) meets a CPML slab or a wall in x (wx) or y (wy), or the chunk one in z; without it no
 // node does. kMat: rows other than the background's lie in a slab or on a low wall (without it the
-// few that may, beside general nodes, take the slow path).
+// few that may, beside general nodes, take the slow path). Their quads of one row take the background's
+// way through the step, with coefficients from the tables: node by node, a load waiting for the one
+// before it, they held their tiles up (a half space and boxes through the slabs, us a step: 225^3 300 -> 244,
+// 320^3 567 -> 444; with the chunks of plan_sweep 237 and 419).
 template <typename Idx, bool kEdge, bool kMat, bool kWide>
 __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int x0, int y0, int k0, int k1, int row,
                                       int col, bool own, bool wx, bool wy) {
@@ -405,19 +421,24 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
             vx = lds4(TE); vy = lds4(TE + EF); vz = lds4(TE + 2 * EF);
             const int c0 = (int)(cw.x & 0xffffu);
             bool mixed = false;
-            if (cw.x == cw.y && cw.x == (uint32_t)c0 * 0x10001u && (kEdge ? c0 == bgm && !xslow : c0 < p.src_row0)) {
-                // one row for the quad (in tiles at the edge, the background's)
+            const bool bg = kEdge && !kMat ? true : c0 == bgm;
+            if (cw.x == cw.y && cw.x == (uint32_t)c0 * 0x10001u && (kEdge && !kMat ? c0 == bgm : c0 < p.src_row0) && !(kEdge && xslow)) {
+                // one row for the quad (in tiles at the edge without kMat, the background's)
                 float4 a = make_float4(B.ea[0], B.ec[0], B.ec[1], 0.f), b = make_float4(B.ea[1], B.ec[2], B.ec[3], 0.f);
                 float4 d = make_float4(B.ea[2], B.ec[4], B.ec[5], 0.f);
-                if (!kEdge && c0 != bgm) {
+                if (!bg) {
                     const MatCoef* mc = p.coef + c0;
                     a = __ldg(&mc->e[0]); b = __ldg(&mc->e[1]); d = __ldg(&mc->e[2]);
                 }
                 Quad x0c = {b.z, b.z, b.z, b.z}, x1c = {d.y, d.y, d.y, d.y};
-                if (kEdge) {  // curl coefficients along a slab's axis, over kappa
+                if (kEdge && bg) {  // curl coefficients along a slab's axis, over kappa
                     if (ys) { a.y = S.ye[row].x; d.z = S.ye[row].y; }
                     if (zs) { a.z = S.ze[q].x; b.y = S.ze[q].y; }
                     if (xs) { x0c = lds4(&S.xe[0][col]); x1c = lds4(&S.xe[1][col]); }
+                } else if (kEdge) {
+                    if (ys) { const float2 f = curl2(SR.e[1] + c0 * Ly + ly); a.y = f.x; d.z = f.y; }
+                    if (zs) { const float2 f = curl2(SR.e[2] + c0 * Lz + lz(k)); a.z = f.x; b.y = f.y; }
+                    if (xs) curl_x(x0c, x1c, SR.e[0] + c0 * Lx + lx, xs);
                 }
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
@@ -552,10 +573,13 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                 }
                 const int st = store_e ? in4 & ~slow : 0;
                 // v0 and v1 plus the quad's CPML memory u0, u1 along an axis (factors b0, b1, or its rows')
-                const bool own_rows = kMat && (mixed || c0 != bgm);
                 auto add = [&](Quad& v0, Quad& v1, const Quad& u0, const Quad& u1, float b0, float b1, const float4* T, int L, int l,
                                int dl, int nodes) {
-                    if (own_rows) {
+                    if (kMat && !mixed && !bg) {  // the quad's row's (the same on every plane of the slabs)
+                        const float2 f = psi2(T + c0 * L);
+                        b0 = f.x; b1 = f.y;
+                    }
+                    if (kMat && mixed) {
 #pragma unroll
                         for (int r = 0; r < 4; ++r) {
                             const int c = row_at(cw, r);
@@ -647,8 +671,9 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
             const float ezi = ep[2 * NF + 4], eyi = ep[NF + 4];
             const bool low_jk = kEdge && (j == 0 || kh == 0);  // faces on a low wall take the default entry
             Quad ux = hxp, uy = hyp, uz = hzp;
-            const int c0 = (int)(cp.x & 0xffffu);
-            bool mixed = false;
+            bool one = cp.x == cp.y && cp.x == (cp.x & 0xffffu) * 0x10001u, mixed = false;  // one row for the quad
+            int c0 = (int)(cp.x & 0xffffu);
+            if (kMat && p.h_bg && !((cp.x | cp.y) & kRecGeneral * 0x10001u)) { c0 = bgm; one = true; }
             // the row that component `comp` of node r (row c) takes: the default entry's on a low wall
             auto hrow = [&](int c, int r, int comp) {
                 if (!kEdge || !kMat) return c;
@@ -660,19 +685,25 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                 if (rq != rp) { const float4 o = __ldg(T + rq * L + l); f.y = o.y; f.w = o.w; }
                 return f;
             };
-            const bool table = c0 == bgm && (!low_jk || B.low_ok);  // the tabulated coefficients apply
-            if (cp.x == cp.y && cp.x == (uint32_t)c0 * 0x10001u &&
-                (kEdge ? table && !xslow && (i > 0 || B.low_ok) : c0 < kRecGeneral)) {
+            const bool bg = kEdge && !kMat ? true : c0 == bgm;
+            // one row for the quad: the background's where its tabulated coefficients apply, with kMat another
+            // one off the low walls
+            if (one && (kEdge ? (kMat && !bg ? c0 < kRecGeneral && !low_jk && i > 0 : c0 == bgm && ((!low_jk && i > 0) || B.low_ok)) && !xslow
+                              : c0 < kRecGeneral)) {
                 float4 a = make_float4(B.ha[0], B.hc[0], B.hc[1], 0.f), b = make_float4(B.ha[1], B.hc[2], B.hc[3], 0.f);
                 float4 d = make_float4(B.ha[2], B.hc[4], B.hc[5], 0.f);
-                if (!kEdge && c0 != bgm) {
+                if (!bg) {
                     a = __ldg(&p.coef[c0].h[0]); b = __ldg(&p.coef[c0].h[1]); d = __ldg(&p.coef[c0].h[2]);
                 }
                 Quad x0c = {b.y, b.y, b.y, b.y}, x1c = {d.z, d.z, d.z, d.z};
-                if (kEdge) {
+                if (kEdge && bg) {
                     if (ys) { a.z = S.yh[row].x; d.y = S.yh[row].y; }
                     if (zsh) { a.y = S.zh[q - 1].x; b.z = S.zh[q - 1].y; }
                     if (xs) { x0c = lds4(&S.xh[0][col]); x1c = lds4(&S.xh[1][col]); }
+                } else if (kEdge) {
+                    if (ys) { const float2 f = curl2(SR.h[1] + c0 * Ly + ly); a.z = f.x; d.y = f.y; }
+                    if (zsh) { const float2 f = curl2(SR.h[2] + c0 * Lz + lz(kh)); a.y = f.x; b.z = f.y; }
+                    if (xs) curl_x(x0c, x1c, SR.h[0] + c0 * Lx + lx, xs);
                 }
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
@@ -784,10 +815,13 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                     my = klh ? lt4 : 0;
                     mz = ylt ? lt4 : 0;
                 }
-                const bool own_rows = kMat && (mixed || !table);
                 auto add = [&](Quad& v0, Quad& v1, const Quad& u0, const Quad& u1, float b0, float b1, const float4* T, int L, int l,
                                int dl, int nodes, int p0, int p1) {
-                    if (own_rows) {
+                    if (kMat && !mixed && !bg) {
+                        const float2 f = psi2(T + c0 * L);
+                        b0 = f.x; b1 = f.y;
+                    }
+                    if (kMat && mixed) {
 #pragma unroll
                         for (int r = 0; r < 4; ++r) {
                             const int c = row_at(cp, r);

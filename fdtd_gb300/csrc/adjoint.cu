@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(256, FDTD_ADJ_MIN_BLOCKS) k_adj_e(const __grid
     if (zs) Z = adj_slab<true>(g, psa, 2, i, j, k);
     const BgNode& B = p.bgn;
     const bool own = c != p.bg.mat;
-    if (c >= kRecGeneral || (own && (xs || ys || zs) && !p.rows.e[0])) {  // the design edge box among them
+    if (c >= kRecGeneral || (c >= p.des_row0 && c < p.des_row1) || (own && (xs || ys || zs) && !p.rows.e[0])) {  // the design edge box among them
         adj_e_general(&p, &a, &psa, &st, i, j, k, lx, ly, lz);
         return;
     }

@@ -117,11 +117,15 @@ struct fdtd_handle {
     int n_iface_rows = 0;
     int src_row0 = kRecGeneral;       // rows of lumped source edges (StepParams::src_row0)
     SrcRow* src_rows = nullptr;
+    int des_row0 = kRecGeneral, des_row1 = 0;  // rows of design nodes, and their E coefficients (StepParams::dcoef)
+    float4* dcoef = nullptr;          // (in d_deps' allocation; NULL: no room for them)
     ProbeAt* d_probes_at = nullptr;   // probes outside the CPML slabs
     int n_probes_at = 0;
     int h_bg = 0;                     // StepParams::h_bg
+    bool edge_rows = false;           // materials or plates may lie in the slabs (build_slab_rows)
     int edge_mat = 0;                 // rows other than the background's in a slab or on a low wall (read back by ensure_prepared)
     float4* slab_rows = nullptr;      // SlabRows, with edge_mat (NULL: too many rows, their nodes take the general path)
+    size_t slab_bytes = 0;
     int n_coef_rows = 0;
     int4* d_special = nullptr;        // special_nodes, while and after their rows are built
     // interface-key hash set and its lists (launch_iface_set / launch_iface_rows)
@@ -291,6 +295,9 @@ StepParams make_params(fdtd_handle* h) {
     p.bgn = h->bg_node;
     p.src_row0 = h->src_row0;
     p.src_rows = h->src_rows;
+    p.des_row0 = h->des_row0;
+    p.des_row1 = h->des_row1;
+    p.dcoef = h->dcoef;
     p.h_bg = h->h_bg;
     std::copy(h->te, h->te + 3, p.te);
     std::copy(h->th, h->th + 3, p.th);
@@ -389,13 +396,14 @@ void* tensor_map_encoder() {
 // fill the device evenly, two-pass is ahead. Materials that lie in the CPML make the sweep's tiles there
 // slower than the others. Boxes and a half space through every slab: 64^3 16.3 / 17.3 us, 128^3 51 / 62, 144^3
 // 81.7 / 81.5, 160^3 100 / 97, 192^3 162 / 137, 225^3 283 / 237, 256^3 349 / 247; of magnetic materials, whose H
-// coefficients differ from the background's: 160^3 101 / 120, 192^3 162 / 165, 200^3 213 / 202. Grids below kAutoSweepCells, a few CTAs' work, gain little. Grids with
-// a design region take the sweep from kAutoDesignCells on (smaller ones record in their two-pass
-// kernels). Two-pass also serves where the second buffers cannot be allocated.
+// coefficients differ from the background's: 160^3 101 / 120, 192^3 162 / 165, 200^3 213 / 202. Grids below kAutoSweepCells, a few CTAs' work, gain little. A
+// design region changes little (d^3 cells of n^3, 256 / 32 322 / 222 us, 256 / 128 449 / 241, 512 / 256 3118 / 1443), but an
+// adjoint's forward takes its records in the two-pass kernels below kAutoAdjointCells. Two-pass also serves
+// where the second buffers cannot be allocated.
 constexpr long long kAutoSweepCells = 32LL << 10;
 constexpr long long kAutoTwoPassLo = 300LL << 10, kAutoTwoPassHi = 2450LL << 10;
 constexpr long long kAutoEdgeHi = 3LL << 20, kAutoEdgeMagneticHi = 7LL << 20;  // with slab_rows, two-pass below this
-constexpr long long kAutoDesignCells = 64LL << 20;
+constexpr long long kAutoAdjointCells = 64LL << 20;
 
 // The background material's coefficients (StepParams::bgn), evaluated on the host with the rounding steps of
 // k_material_tables (coef3, harm2; IEEE float operations and fma on both sides).
@@ -484,9 +492,8 @@ void auto_choose(fdtd_handle* h, int64_t n) {
     if (h->schedule != FDTD_SCHEDULE_AUTO || h->auto_choice != FDTD_SCHEDULE_AUTO) return;
     const long long cells = (long long)h->g.nx * h->g.ny * h->g.nz;
     const bool small = cells < kAutoTwoPassLo;
-    if (h->has_design ? cells < kAutoDesignCells
-        : h->slab_rows ? cells < (h->h_bg ? kAutoEdgeHi : kAutoEdgeMagneticHi)
-                       : cells < kAutoSweepCells || (!small && cells < kAutoTwoPassHi)) {
+    if (h->edge_rows ? cells < (h->h_bg ? kAutoEdgeHi : kAutoEdgeMagneticHi)
+                     : cells < kAutoSweepCells || (!small && cells < kAutoTwoPassHi)) {
         h->auto_choice = FDTD_SCHEDULE_TWO_PASS;
         return;
     }
@@ -1332,6 +1339,47 @@ size_t special_nodes(const fdtd_handle* h, std::vector<int4>& out) {
     return out.size();
 }
 
+// The list of distinct keys that a set's launch left on the device (unsorted).
+int read_keys(fdtd_handle* h, std::vector<unsigned long long>& keys) {
+    constexpr size_t kFew = 512;  // most sets are small: copied with the count, one wait
+    int counters[2] = {0, 0};
+    keys.resize(kFew);
+    auto copy = [&](size_t n) {
+        return cudaMemcpyAsync(keys.data(), h->iface_keys, n * sizeof(unsigned long long), cudaMemcpyDeviceToHost, h->stream);
+    };
+    CUDA_TRY(cudaMemcpyAsync(counters, h->iface_counters, sizeof(counters), cudaMemcpyDeviceToHost, h->stream));
+    CUDA_TRY(copy(kFew));
+    CUDA_TRY(cudaStreamSynchronize(h->stream));
+    keys.resize((size_t)std::min(counters[1], kIfaceTableSize));
+    if (keys.size() > kFew) {
+        CUDA_TRY(copy(keys.size()));
+        CUDA_TRY(cudaStreamSynchronize(h->stream));
+    }
+    return FDTD_OK;
+}
+
+// Rows of the design edge box's nodes (launch_design_set), at most `room` of them from row `first` on, and
+// their E coefficients. keys: of the rows. Without room for the coefficients there are no rows, and the
+// nodes take the general path.
+int build_design_rows(fdtd_handle* h, int room, int first, std::vector<unsigned long long>& keys) {
+    h->des_row0 = kRecGeneral;
+    h->des_row1 = 0;
+    const int* d = h->dbox;
+    if (!h->dcoef || room <= 0) return FDTD_OK;
+    StepParams p = make_params(h);
+    p.coef = h->coef;
+    CUDA_TRY(launch_design_coefs(p, h->dcoef, h->stream));
+    CUDA_TRY(launch_design_set(h->g, d, h->cls, h->mat, h->iface_table, h->iface_counters, h->iface_keys, h->stream));
+    int rc = read_keys(h, keys);
+    if (rc) return rc;
+    std::sort(keys.begin(), keys.end());
+    if (keys.size() > (size_t)room) keys.resize((size_t)room);
+    CUDA_TRY(cudaMemcpyAsync(h->iface_keys, keys.data(), keys.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice, h->stream));
+    CUDA_TRY(launch_design_rows(h->g, d, h->cls, h->mat, h->iface_table, h->iface_keys, (int)keys.size(), first, h->iface_slot_row, h->rec,
+                                h->stream));
+    return FDTD_OK;
+}
+
 // Interface rows (kInterfaceNode and kGeneral nodes): gather the seven-cell keys, sort and unique
 // them here, then write each node's coefficient row and the rows themselves. Runs after the node
 // classes and plates are final.
@@ -1339,15 +1387,10 @@ int build_interface_rows(fdtd_handle* h) {
     const DeviceGrid& g = h->g;
     // distinct keys on the device; only they come to the host (two small copies)
     CUDA_TRY(launch_iface_set(g, h->cls, h->mat, h->iface_table, h->iface_counters, h->iface_keys, h->stream));
-    int counters[2] = {0, 0};
-    CUDA_TRY(cudaMemcpyAsync(counters, h->iface_counters, sizeof(counters), cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(cudaStreamSynchronize(h->stream));
-    const int n = std::min(counters[1], kIfaceTableSize);
-    std::vector<unsigned long long> hk((size_t)n);
-    if (n > 0) {
-        CUDA_TRY(cudaMemcpyAsync(hk.data(), h->iface_keys, (size_t)n * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                                 h->stream));
-        CUDA_TRY(cudaStreamSynchronize(h->stream));
+    std::vector<unsigned long long> hk;
+    int rc = read_keys(h, hk);
+    if (rc) return rc;
+    if (!hk.empty()) {
         std::sort(hk.begin(), hk.end());
         hk.erase(std::unique(hk.begin(), hk.end()), hk.end());
         if (hk.size() > (size_t)kMaxInterfaceRows) hk.resize((size_t)kMaxInterfaceRows);  // the rest stay general
@@ -1357,7 +1400,11 @@ int build_interface_rows(fdtd_handle* h) {
     const int n_rows = (int)hk.size();
     CUDA_TRY(launch_iface_rows(g, h->cls, h->mat, h->iface_table, h->iface_keys, n_rows, h->iface_slot_row, h->rec,
                                h->small, h->stream));
-    CUDA_TRY(launch_rec_general(g, h->d_lumped, h->n_lumped_edges, h->rec, h->stream));
+    std::vector<unsigned long long> dk;
+    rc = build_design_rows(h, kMaxInterfaceRows - n_rows, kFirstInterfaceRow + n_rows, dk);
+    if (rc) return rc;
+    const int n_design = (int)dk.size();
+    CUDA_TRY(launch_rec_general(g, h->d_lumped, h->n_lumped_edges, h->cls, h->rec, h->stream));
     StepParams p = make_params(h);  // the rows come from the material rows and properties, plates and lumped edges
     p.coef = h->coef;
     // nodes with plate-covered edges, and lumped edges outside the CPML slabs: rows of their own
@@ -1365,7 +1412,7 @@ int build_interface_rows(fdtd_handle* h) {
     std::vector<unsigned long long> sk;
     h->release(h->d_special);
     h->d_special = nullptr;
-    const int room = kMaxInterfaceRows - n_rows;
+    const int room = kMaxInterfaceRows - n_rows - n_design;
     // a few such nodes (lumped edges): a row each; more (plates): their distinct rows
     const bool each = special_nodes(h, special) <= kSpecialEach && (int)special.size() <= room;
     std::stable_sort(special.begin(), special.end(), [](const int4& a, const int4& b) { return (a.w >= 0) < (b.w >= 0); });
@@ -1377,11 +1424,7 @@ int build_interface_rows(fdtd_handle* h) {
         for (size_t q = 0; q < special.size(); ++q) sk.push_back(special[q].w >= 0 ? 1ull << 63 : 0ull);
     } else if (room > 0) {
         CUDA_TRY(launch_special_set(p, h->d_special, (int)special.size(), h->iface_table, h->iface_counters, h->iface_keys, h->stream));
-        CUDA_TRY(cudaMemcpyAsync(counters, h->iface_counters, sizeof(counters), cudaMemcpyDeviceToHost, h->stream));
-        CUDA_TRY(cudaStreamSynchronize(h->stream));
-        sk.resize((size_t)std::min(counters[1], kIfaceTableSize));
-        CUDA_TRY(cudaMemcpyAsync(sk.data(), h->iface_keys, sk.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, h->stream));
-        CUDA_TRY(cudaStreamSynchronize(h->stream));
+        if ((rc = read_keys(h, sk))) return rc;
         std::sort(sk.begin(), sk.end());  // source rows (bit 63) last
         if (sk.size() > (size_t)room) sk.resize((size_t)room);
     }
@@ -1394,11 +1437,11 @@ int build_interface_rows(fdtd_handle* h) {
     h->src_rows = nullptr;
     h->src_row0 = kRecGeneral;
     h->n_iface_rows = 0;
-    CUDA_TRY(h->alloc((void**)&h->coef_rows, sizeof(MatCoef) * (size_t)(kFirstInterfaceRow + n_rows + n_special)));
+    const int first = kFirstInterfaceRow + n_rows + n_design;
+    CUDA_TRY(h->alloc((void**)&h->coef_rows, sizeof(MatCoef) * (size_t)(first + n_special)));
     CUDA_TRY(cudaMemcpyAsync(h->coef_rows, h->coef, sizeof(MatCoef) * (size_t)kFirstInterfaceRow, cudaMemcpyDeviceToDevice,
                              h->stream));
     if (n_special > 0) {
-        const int first = kFirstInterfaceRow + n_rows;
         if (n_special > n_plain) {
             CUDA_TRY(h->alloc((void**)&h->src_rows, sizeof(SrcRow) * (size_t)(n_special - n_plain)));
             h->src_row0 = first + n_plain;
@@ -1409,16 +1452,21 @@ int build_interface_rows(fdtd_handle* h) {
             CUDA_TRY(cudaMemcpyAsync(h->iface_keys, sk.data(), sk.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice, h->stream));
             CUDA_TRY(launch_special_rows(p, h->d_special, (int)special.size(), h->iface_table, h->iface_keys, n_special, n_plain,
                                          first, h->iface_slot_row, h->coef_rows, h->src_rows, h->rec, h->stream));
-            CUDA_TRY(cudaMemcpyAsync(h->iface_keys, hk.data(), hk.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice, h->stream));
         }
     }
+    // the sets above used the list: the keys of the interface rows, then of the design rows, once more
+    hk.insert(hk.end(), dk.begin(), dk.end());
+    if (!each || n_design > 0)
+        CUDA_TRY(cudaMemcpyAsync(h->iface_keys, hk.data(), hk.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice, h->stream));
     StepParams pi{};
     pi.g = g;
     pi.props = h->props;
     pi.coef = h->coef;
-    CUDA_TRY(launch_iface_coefs(pi, h->iface_keys, n_rows, h->coef_rows, h->stream));
+    CUDA_TRY(launch_iface_coefs(pi, h->iface_keys, n_rows + n_design, h->coef_rows, h->stream));
     h->n_iface_rows = n_rows;
-    h->n_coef_rows = kFirstInterfaceRow + n_rows + n_special;
+    h->n_coef_rows = first + n_special;
+    h->des_row0 = n_design > 0 ? first - n_design : h->src_row0;
+    h->des_row1 = n_design > 0 ? first : 0;
     CUDA_TRY(launch_rows_h(h->coef_rows, h->n_coef_rows, 0, h->small + 1, h->stream));
     int marks[2] = {0, 0};
     CUDA_TRY(cudaMemcpyAsync(marks, h->small, sizeof(marks), cudaMemcpyDeviceToHost, h->stream));
@@ -1429,20 +1477,27 @@ int build_interface_rows(fdtd_handle* h) {
 }
 
 // The slab coefficients by row, where rows other than the background's lie in a slab or on a low wall
-// (4 MB for 1000 rows and 60 slab planes; up to kSlabRowsLimit).
+// (4 MB for 1000 rows and 60 slab planes; up to kSlabRowsLimit), and for design rows, which the sweep's
+// kernels with that table take.
 constexpr size_t kSlabRowsLimit = 256u << 20;
 int build_slab_rows(fdtd_handle* h) {
     const DeviceGrid& g = h->g;
-    h->release(h->slab_rows);
-    h->slab_rows = nullptr;
-    if (!h->edge_mat && h->plates.empty() && h->bg_node.low_ok) return FDTD_OK;
+    h->edge_rows = h->edge_mat || !h->plates.empty() || !h->bg_node.low_ok;
     const long long L = (long long)g.pxn + g.pxp + g.pyn + g.pyp + g.pzn + g.pzp;
-    const size_t bytes = std::max<size_t>(1, (size_t)(2 * h->n_coef_rows * L) * sizeof(float4));
-    if (bytes > kSlabRowsLimit || h->alloc((void**)&h->slab_rows, bytes) != cudaSuccess) {
-        cudaGetLastError();
+    size_t bytes = std::max<size_t>(1, (size_t)(2 * h->n_coef_rows * L) * sizeof(float4));
+    if ((!h->edge_rows && h->des_row1 == 0) || bytes > kSlabRowsLimit) bytes = 0;
+    if (bytes != h->slab_bytes) {
+        h->release(h->slab_rows);
         h->slab_rows = nullptr;
-        return FDTD_OK;
+        h->slab_bytes = 0;
+        if (bytes > 0 && h->alloc((void**)&h->slab_rows, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            h->slab_rows = nullptr;
+            return FDTD_OK;
+        }
+        h->slab_bytes = bytes;
     }
+    if (!h->slab_rows) return FDTD_OK;
     float* const kappa[6] = {h->prof[4], h->prof[10], h->prof[16], h->prof[5], h->prof[11], h->prof[17]};
     CUDA_TRY(launch_slab_rows(g, h->coef_rows, h->n_coef_rows, kappa, h->slab_rows, h->stream));
     return FDTD_OK;
@@ -1522,7 +1577,12 @@ int ensure_prepared(fdtd_handle* h) {
         if (rc) return rc;
         const DeviceGrid& g = h->g;
         h->sweep = plan_sweep(PlanGrid{g.nx, g.ny, g.nz, g.pxn, g.pxp, g.pyn, g.pyp, g.pzn, g.pzp}, 1.0, h->slab_rows != nullptr);
-        if (!h->slab_rows) CUDA_TRY(launch_rec_slab_plates(h->g, h->d_plate_nodes, h->n_plate_nodes, h->rec, h->stream));
+        if (!h->slab_rows) {  // what it would have served takes the general path
+            CUDA_TRY(launch_rec_slab_plates(h->g, h->d_plate_nodes, h->n_plate_nodes, h->rec, h->stream));
+            if (h->des_row1 > 0) CUDA_TRY(launch_rec_design_general(h->g, h->dbox, h->cls, h->rec, h->stream));
+            h->des_row0 = h->src_row0;
+            h->des_row1 = 0;
+        }
     }
     if (h->dirty_probes) {
         int rc = build_probes(h);
@@ -1718,7 +1778,15 @@ extern "C" int fdtd_set_design_region(fdtd_handle* h, const int32_t box[6], cons
     if (!same) {
         h->release(h->d_deps);
         h->d_deps = nullptr;
-        CUDA_TRY(h->alloc((void**)&h->d_deps, nd * sizeof(float)));
+        h->dcoef = nullptr;
+        const size_t at = (nd * sizeof(float) + 255) / 256 * 256;
+        const size_t ne = (size_t)(box[3] - box[0] + 1) * (box[4] - box[1] + 1) * (box[5] - box[2] + 1);
+        if (h->alloc((void**)&h->d_deps, at + 3 * ne * sizeof(float4)) == cudaSuccess) {
+            h->dcoef = (float4*)((char*)h->d_deps + at);
+        } else {  // the cells alone: their nodes take the general path
+            cudaGetLastError();
+            CUDA_TRY(h->alloc((void**)&h->d_deps, nd * sizeof(float)));
+        }
         int b[6];
         for (int q = 0; q < 6; ++q) b[q] = box[q];
         CUDA_TRY(launch_paint(h->mat, g, b, (uint8_t)kDesign, h->stream));
@@ -1916,10 +1984,11 @@ int adj_forward_enqueue(fdtd_handle* h, int64_t n, int32_t checkpoint_every, int
         CUDA_TRY(launch_after_step(h->field[c][0], h->field[c][1], h->field[c][2], g, A.probe, nullptr, h->dbox, adj_slot(h, 0),
                                    h->stream));
     }
-    auto_choose(h, n);
-    // two-pass steps take their records in k_design_e (no launch of their own): the E of the
-    // design edge box is final there, and so is every other E
-    const bool two_pass = !use_fused(h);
+    // AUTO's choice holds for large grids: two-pass steps take their records in the E pass (by class in
+    // k_design_e), without a launch of their own
+    const bool small = h->schedule == FDTD_SCHEDULE_AUTO && (long long)g.nx * g.ny * g.nz < kAutoAdjointCells;
+    if (!small) auto_choose(h, n);
+    const bool two_pass = small || !use_fused(h);
     StepParams pa = make_params(h);
     if (two_pass) {
         const int* d = h->dbox;

@@ -179,6 +179,11 @@ struct StepParams {
     // coefficient rows from src_row0 on belong to lumped source edges (kRecGeneral: none do)
     int src_row0;
     const SrcRow* src_rows;
+    // rows des_row0 .. des_row1 - 1 belong to nodes of the design edge box: such a row holds the node's H
+    // coefficients, its E coefficients lie in dcoef (three arrays of the box volume, x fastest: Ex, Ey, Ez).
+    // Without a design region des_row0 = src_row0, des_row1 = 0
+    int des_row0, des_row1;
+    const float4* dcoef;
     // the same curl coefficients packed with the CPML profiles, per axis and node: {slot 0, slot 1,
     // b, a} of E and of H (BgCurl's slots)
     const float4 *te[3], *th[3];

@@ -28,7 +28,8 @@ struct StepIndex {
 template <typename Idx, bool kDesign>
 static __device__ __noinline__ void e_node_general(const StepParams* p, const FieldPtrs* f, const PsiSet* ps, const StepIndex* step,
                                                    int i, int j, int k) {
-    if (kDesign && p->rec[(Idx)k * (Idx)p->g.plane + (Idx)j * (Idx)p->g.pitch + (Idx)i] == (kRecGeneral | kDesignNode))
+    const int c = kDesign ? p->rec[(Idx)k * (Idx)p->g.plane + (Idx)j * (Idx)p->g.pitch + (Idx)i] : 0;
+    if (kDesign && (c == (kRecGeneral | kDesignNode) || (c >= p->des_row0 && c < p->des_row1)))
         e_node_global<true>(*p, *f, *f, *ps, *ps, i, j, k, step->at());
     else
         e_node_global<false, false, false, Idx>(*p, *f, *f, *ps, *ps, i, j, k, step->at());
@@ -94,7 +95,7 @@ __device__ __forceinline__ void e_node_rows(const StepParams& p, const FieldPtrs
     if (zs) { Z = psi_slot_z<Idx>(p, i, j, k); }
     const BgNode& B = p.bgn;
     const bool own = c != p.bg.mat;
-    if (c >= kRecGeneral || (own && slab && !p.rows.e[0])) {
+    if (c >= kRecGeneral || (kDesign && c >= p.des_row0 && c < p.des_row1) || (own && slab && !p.rows.e[0])) {
         e_node_general<Idx, kDesign>(&p, &f, &ps, &step, i, j, k);
         return;
     }

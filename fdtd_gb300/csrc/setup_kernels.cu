@@ -536,13 +536,13 @@ __device__ __forceinline__ void iface_row(uint8_t* __restrict__ cls, const uint8
     rec[n] = (uint16_t)r;
 }
 
-// Lumped edges keep the general path in every schedule (their E update is the lumped override); those of
-// the design edge box are marked as its nodes already.
-__global__ void k_rec_general(uint16_t* rec, DeviceGrid g, const LumpedEdge* edges, int n_edges) {
+// Lumped edges keep the general path in every schedule (their E update is the lumped override), in the
+// design edge box as its nodes.
+__global__ void k_rec_general(uint16_t* rec, DeviceGrid g, const LumpedEdge* edges, int n_edges, const uint8_t* cls) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n_edges) return;
-    uint16_t& r = rec[(long long)edges[q].k * g.plane + (long long)edges[q].j * g.pitch + edges[q].i];
-    if (r != (kRecGeneral | kDesignNode)) r = (uint16_t)(kRecGeneral | kGeneral);
+    const long long n = (long long)edges[q].k * g.plane + (long long)edges[q].j * g.pitch + edges[q].i;
+    rec[n] = (uint16_t)(kRecGeneral | (cls[n] == kDesignNode ? kDesignNode : kGeneral));
 }
 
 // The nodes of probes inside a CPML slab too: the general path samples them before the CPML
@@ -592,9 +592,98 @@ cudaError_t launch_count_general(const DeviceGrid& g, const uint16_t* rec, const
     return cudaGetLastError();
 }
 
-cudaError_t launch_rec_general(const DeviceGrid& g, const LumpedEdge* edges, int n_edges, uint16_t* rec, cudaStream_t st) {
+cudaError_t launch_rec_general(const DeviceGrid& g, const LumpedEdge* edges, int n_edges, const uint8_t* cls, uint16_t* rec,
+                               cudaStream_t st) {
     if (n_edges <= 0) return cudaSuccess;
-    k_rec_general<<<(n_edges + 127) / 128, 128, 0, st>>>(rec, g, edges, n_edges);
+    k_rec_general<<<(n_edges + 127) / 128, 128, 0, st>>>(rec, g, edges, n_edges, cls);
+    return cudaGetLastError();
+}
+
+namespace {
+struct DesignBox {
+    int d[6];
+    __host__ __device__ long long volume() const { return (long long)(d[3] - d[0] + 1) * (d[4] - d[1] + 1) * (d[5] - d[2] + 1); }
+};
+// Node e of the box, x fastest.
+__device__ __forceinline__ int3 design_node(const DesignBox& b, long long e) {
+    const int bx = b.d[3] - b.d[0] + 1, by = b.d[4] - b.d[1] + 1;
+    return make_int3(b.d[0] + (int)(e % bx), b.d[1] + (int)((e / bx) % by), b.d[2] + (int)(e / ((long long)bx * by)));
+}
+DesignBox design_box(const int* d) { return DesignBox{{d[0], d[1], d[2], d[3], d[4], d[5]}}; }
+}  // namespace
+
+__global__ void k_design_insert(const uint8_t* __restrict__ cls, const uint8_t* __restrict__ mat, DeviceGrid g, DesignBox b,
+                                unsigned long long* table, int* filled) {
+    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (e >= b.volume()) return;
+    const int3 v = design_node(b, e);
+    if (cls[(long long)v.z * g.plane + (long long)v.y * g.pitch + v.x] == kDesignNode)
+        iface_insert(table, filled, cell_key(mat, g, v.x, v.y, v.z));
+}
+__global__ void k_design_rows(const uint8_t* __restrict__ cls, const uint8_t* __restrict__ mat, DeviceGrid g, DesignBox b,
+                              const unsigned long long* __restrict__ table, const int* __restrict__ slot_row, int first, uint16_t* rec) {
+    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (e >= b.volume()) return;
+    const int3 v = design_node(b, e);
+    const long long n = (long long)v.z * g.plane + (long long)v.y * g.pitch + v.x;
+    if (cls[n] != kDesignNode) return;
+    const int s = find_slot(table, cell_key(mat, g, v.x, v.y, v.z)), row = s >= 0 ? slot_row[s] : -1;
+    if (row >= 0) rec[n] = (uint16_t)(first + row);
+}
+// The general path's coefficients (e_coef with design cells), once instead of in every step.
+__global__ void k_design_coefs(const __grid_constant__ StepParams p, DesignBox b, float4* out) {
+    const long long ne = b.volume(), e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (e >= ne) return;
+    const int3 v = design_node(b, e);
+    const unsigned long long key = cell_key(p.mat, p.g, v.x, v.y, v.z);
+    const int m0 = (int)(key & 0xff), mi = (int)((key >> 8) & 0xff), mj = (int)((key >> 16) & 0xff);
+    const int mk = (int)((key >> 24) & 0xff), mij = (int)((key >> 32) & 0xff), mik = (int)((key >> 40) & 0xff);
+    const int mjk = (int)((key >> 48) & 0xff);
+    const Coef3 c[3] = {e_coef<true>(p, 0, m0 == mj && m0 == mk && m0 == mjk, m0, mj, mk, mjk, v.x, v.y, v.z),
+                        e_coef<true>(p, 1, m0 == mi && m0 == mk && m0 == mik, m0, mi, mk, mik, v.x, v.y, v.z),
+                        e_coef<true>(p, 2, m0 == mi && m0 == mj && m0 == mij, m0, mi, mj, mij, v.x, v.y, v.z)};
+    for (int q = 0; q < 3; ++q) out[q * ne + e] = make_float4(c[q].a, c[q].bp, c[q].bm, 0.f);
+}
+
+cudaError_t launch_design_set(const DeviceGrid& g, const int* dbox, const uint8_t* cls, const uint8_t* mat, unsigned long long* table,
+                              int* counters, unsigned long long* keys, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(table, 0xff, sizeof(unsigned long long) * kIfaceTableSize, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(counters, 0, 2 * sizeof(int), st);
+    if (e != cudaSuccess) return e;
+    const DesignBox b = design_box(dbox);
+    k_design_insert<<<(unsigned)((b.volume() + 255) / 256), 256, 0, st>>>(cls, mat, g, b, table, counters);
+    k_iface_compact<<<kIfaceTableSize / 256, 256, 0, st>>>(table, keys, counters + 1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_design_rows(const DeviceGrid& g, const int* dbox, const uint8_t* cls, const uint8_t* mat,
+                               const unsigned long long* table, const unsigned long long* keys, int n_keys, int first, int* slot_row,
+                               uint16_t* rec, cudaStream_t st) {
+    const cudaError_t e = cudaMemsetAsync(slot_row, 0xff, sizeof(int) * kIfaceTableSize, st);
+    if (e != cudaSuccess || n_keys <= 0) return e;
+    const DesignBox b = design_box(dbox);
+    k_iface_slot_rows<<<(n_keys + 127) / 128, 128, 0, st>>>(table, keys, n_keys, slot_row);
+    k_design_rows<<<(unsigned)((b.volume() + 255) / 256), 256, 0, st>>>(cls, mat, g, b, table, slot_row, first, rec);
+    return cudaGetLastError();
+}
+
+__global__ void k_rec_design_general(const uint8_t* __restrict__ cls, DeviceGrid g, DesignBox b, uint16_t* rec) {
+    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (e >= b.volume()) return;
+    const int3 v = design_node(b, e);
+    const long long n = (long long)v.z * g.plane + (long long)v.y * g.pitch + v.x;
+    if (cls[n] == kDesignNode) rec[n] = (uint16_t)(kRecGeneral | kDesignNode);
+}
+
+cudaError_t launch_rec_design_general(const DeviceGrid& g, const int* dbox, const uint8_t* cls, uint16_t* rec, cudaStream_t st) {
+    const DesignBox b = design_box(dbox);
+    k_rec_design_general<<<(unsigned)((b.volume() + 255) / 256), 256, 0, st>>>(cls, g, b, rec);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_design_coefs(const StepParams& p, float4* dcoef, cudaStream_t st) {
+    const DesignBox b = design_box(p.dbox);
+    k_design_coefs<<<(unsigned)((b.volume() + 127) / 128), 128, 0, st>>>(p, b, dcoef);
     return cudaGetLastError();
 }
 

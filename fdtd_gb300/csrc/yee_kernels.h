@@ -149,7 +149,20 @@ cudaError_t launch_special_set(const StepParams& p, const int4* nodes, int n, un
 cudaError_t launch_special_rows(const StepParams& p, const int4* nodes, int n, const unsigned long long* table,
                                 const unsigned long long* keys, int n_keys, int n_plain, int first, int* slot_row,
                                 MatCoef* coef, SrcRow* src, uint16_t* rec, cudaStream_t st);
-// The lumped edges' nodes back to kRecGeneral | kGeneral in rec (after launch_iface_rows).
-cudaError_t launch_rec_general(const DeviceGrid& g, const LumpedEdge* edges, int n_edges, uint16_t* rec, cudaStream_t st);
+// The lumped edges' nodes back to kRecGeneral | class in rec (after launch_iface_rows and launch_design_rows).
+cudaError_t launch_rec_general(const DeviceGrid& g, const LumpedEdge* edges, int n_edges, const uint8_t* cls, uint16_t* rec,
+                               cudaStream_t st);
+// Rows of the nodes of the design edge box (class kDesignNode), like those of the interface nodes: their
+// distinct keys, then the nodes' entries of rec (row first + q for the sorted key q; nodes without one stay
+// general). launch_iface_coefs computes the rows, whose H coefficients apply.
+cudaError_t launch_design_set(const DeviceGrid& g, const int* dbox, const uint8_t* cls, const uint8_t* mat, unsigned long long* table,
+                              int* counters, unsigned long long* keys, cudaStream_t st);
+cudaError_t launch_design_rows(const DeviceGrid& g, const int* dbox, const uint8_t* cls, const uint8_t* mat,
+                               const unsigned long long* table, const unsigned long long* keys, int n_keys, int first, int* slot_row,
+                               uint16_t* rec, cudaStream_t st);
+// The nodes of the design edge box back to the general path.
+cudaError_t launch_rec_design_general(const DeviceGrid& g, const int* dbox, const uint8_t* cls, uint16_t* rec, cudaStream_t st);
+// StepParams::dcoef from the material index, the table and the design cells' eps_r.
+cudaError_t launch_design_coefs(const StepParams& p, float4* dcoef, cudaStream_t st);
 
 }  // namespace fdtd

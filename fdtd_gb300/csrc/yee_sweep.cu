@@ -265,7 +265,10 @@ __device__ __forceinline__ Quad quad_of(const float4& f) { return Quad{f.x, f.y,
 // The march of one thread's quad at tile row `row`, first column `col`. kEdge: the tile (halo
 // included) meets a CPML slab or a wall in x (wx) or y (wy), or the chunk one in z; without it no
 // node does. kMat: rows other than the background's lie in a slab or on a low wall (without it the
-// few that may, beside general nodes, take the slow path). Their quads of one row take the background's
+// few that may, beside general nodes, take the slow path), or the grid has a design region, whose rows' E
+// coefficients are each node's own (StepParams::dcoef; node by node on the slow path a region of 256^3 cells
+// in 512^3 cost 2.4 ms of a step's 3.7, now 0.14 of 1.44; in the other kernels the test for such rows cost
+// boxes 2 %). Their quads of one row take the background's
 // way through the step, with coefficients from the tables: node by node, a load waiting for the one
 // before it, they held their tiles up (a half space and boxes through the slabs, us a step: 225^3 300 -> 244,
 // 320^3 567 -> 444; with the chunks of plan_sweep 237 and 419).
@@ -422,7 +425,8 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
             const int c0 = (int)(cw.x & 0xffffu);
             bool mixed = false;
             const bool bg = kEdge && !kMat ? true : c0 == bgm;
-            if (cw.x == cw.y && cw.x == (uint32_t)c0 * 0x10001u && (kEdge && !kMat ? c0 == bgm : c0 < p.src_row0) && !(kEdge && xslow)) {
+            if (cw.x == cw.y && cw.x == (uint32_t)c0 * 0x10001u &&
+                (kEdge ? (kMat ? c0 < p.des_row0 : c0 == bgm) && !xslow : c0 < (kMat ? p.des_row0 : p.src_row0))) {
                 // one row for the quad (in tiles at the edge without kMat, the background's)
                 float4 a = make_float4(B.ea[0], B.ec[0], B.ec[1], 0.f), b = make_float4(B.ea[1], B.ec[2], B.ec[3], 0.f);
                 float4 d = make_float4(B.ea[2], B.ec[4], B.ec[5], 0.f);
@@ -450,6 +454,17 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                 // rows per node; in a slab background nodes take the tabulated curl coefficients, and
                 // without kMat the others the slow path
                 mixed = true;
+                // where a component's E coefficients of node r (row c) lie (without kMat the grid has no design rows)
+                long long dq = 0, dn = 0;
+                if (kMat && p.des_row1 > 0) {
+                    const int* d = p.dbox;
+                    const long long bx = d[3] - d[0] + 1, by = d[4] - d[1] + 1;
+                    dn = bx * by * (d[5] - d[2] + 1);
+                    dq = ((k - d[2]) * by + (j - d[1])) * bx + (i - d[0]);
+                }
+                auto e_row = [&](int c, int r, int comp) {
+                    return kMat && c >= p.des_row0 && c < p.des_row1 ? p.dcoef + (comp * dn + dq + r) : &p.coef[c].e[comp];
+                };
                 if constexpr (kWide || !kEdge) {
                     // (component by component, so that the four nodes' loads are in flight together: the quads
                     // of a material's surface decide how long the plane takes. Tiles at the edge have no
@@ -480,7 +495,7 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                     auto rows = [&](int comp) {
 #pragma unroll
                         for (int r = 0; r < 4; ++r) {
-                            const float4 f = __ldg(&p.coef[c[r]].e[comp]);
+                            const float4 f = __ldg(e_row(c[r], r, comp));
                             f0.v[r] = f.x; f1.v[r] = f.y; f2.v[r] = f.z;
                         }
                     };
@@ -530,9 +545,8 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                             continue;
                         }
                         if (c != cur) {
-                            const MatCoef* mc = p.coef + c;
-                            a = __ldg(&mc->e[0]); b = __ldg(&mc->e[1]); d = __ldg(&mc->e[2]);
-                            cur = c;
+                            a = __ldg(e_row(c, r, 0)); b = __ldg(e_row(c, r, 1)); d = __ldg(e_row(c, r, 2));
+                            cur = kMat && c >= p.des_row0 && c < p.des_row1 ? -1 : c;  // (a design row's are the node's own)
                             if (!kMat || c == bgm) {
                                 if (kEdge && ys) { a.y = S.ye[row].x; d.z = S.ye[row].y; }
                                 if (kEdge && zs) { a.z = S.ze[q].x; b.y = S.ze[q].y; }
@@ -685,11 +699,11 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                 if (rq != rp) { const float4 o = __ldg(T + rq * L + l); f.y = o.y; f.w = o.w; }
                 return f;
             };
+            const bool table = c0 == bgm && (!low_jk || B.low_ok);  // the tabulated coefficients apply
             const bool bg = kEdge && !kMat ? true : c0 == bgm;
             // one row for the quad: the background's where its tabulated coefficients apply, with kMat another
             // one off the low walls
-            if (one && (kEdge ? (kMat && !bg ? c0 < kRecGeneral && !low_jk && i > 0 : c0 == bgm && ((!low_jk && i > 0) || B.low_ok)) && !xslow
-                              : c0 < kRecGeneral)) {
+            if (one && (kEdge ? (kMat && !bg ? c0 < kRecGeneral && !low_jk && i > 0 : table && (i > 0 || B.low_ok)) && !xslow : c0 < kRecGeneral)) {
                 float4 a = make_float4(B.ha[0], B.hc[0], B.hc[1], 0.f), b = make_float4(B.ha[1], B.hc[2], B.hc[3], 0.f);
                 float4 d = make_float4(B.ha[2], B.hc[4], B.hc[5], 0.f);
                 if (!bg) {

@@ -63,12 +63,11 @@ static __device__ FDTD_RARE Coef3 h_coef_mixed(const MatProps* props, int axis, 
 static __device__ FDTD_RARE float kappa_div(float c, float kappa) { return __fdiv_rn(c, kappa); }
 
 // eps_r of axis `axis` of cell (ci, cj, ck) holding material m: the design array for design
-// cells (isotropic).
+// cells (isotropic). Cells of an earlier design box outside the present one hold the base material.
 __device__ __forceinline__ float cell_eps(const StepParams& p, int m, int axis, int ci, int cj, int ck) {
-    if (m == kDesign && p.deps) {
-        const int* d = p.dbox;
+    const int* d = p.dbox;
+    if (m == kDesign && p.deps && ci >= d[0] && ci < d[3] && cj >= d[1] && cj < d[4] && ck >= d[2] && ck < d[5])
         return p.deps[((long long)(ck - d[2]) * (d[4] - d[1]) + (cj - d[1])) * (d[3] - d[0]) + (ci - d[0])];
-    }
     return p.props[m].a[axis].eps;
 }
 // The averaged eps_r and sigma_e of E edge `comp` at node (i, j, k) over its four cells in the

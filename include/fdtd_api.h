@@ -284,7 +284,8 @@ int fdtd_marching_loop(
  * index 255 (so the table may hold at most 255 materials), painted over what they held. The E edges
  * of the region must be interior nodes (outside the CPML slabs and the boundary planes) and no
  * lumped element may touch it, whether added before or after (FDTD_ERR_INVALID; its lowest edges may
- * stand on the region's top face). Calling again with the same box only replaces eps_r. */
+ * stand on the region's top face). Calling again with the same box only replaces eps_r; with another box,
+ * cells of the old one outside it keep the base material (with `base`'s eps_r). */
 int fdtd_set_design_region(fdtd_handle* h, const int32_t box[6], const fdtd_material* base, const float* eps_r);
 
 /* Figure of merit J = sum over the next n steps of dt * Ez(i,j,k)^2, Ez sampled after each step's E

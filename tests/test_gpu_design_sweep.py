@@ -97,3 +97,30 @@ def test_auto_takes_the_sweep(gpu_lib):
             out.append((J, g, sim.fields()))
     assert out[0][0] == out[1][0] and np.array_equal(out[0][1], out[1][1]) and np.abs(out[0][1]).max() > 0
     assert bitwise_equal(out[0][2], out[1][2])
+
+
+@pytest.mark.parametrize("schedule", [1, 2])
+@pytest.mark.parametrize("box", [(10, 8, 7, 16, 14, 11), (14, 11, 9, 19, 16, 14), (16, 8, 11, 19, 14, 14)])
+def test_region_moved(gpu_lib, schedule, box):
+    """A second region that overlaps the first, or touches it: the first one's other cells hold the base material."""
+    import oracle
+    from fdtd_gb300 import solver
+    sc, _ = grid((26, 24, 22), 4)
+    sc.steps, sc.design_mu = 30, 1.0
+    sc.sources = [S.LumpedSource((7, 11, 9, 7, 11, 10), 50.0, np.random.default_rng(1).standard_normal(30).astype(np.float32))]
+    first = (12, 9, 8, 16, 14, 11)
+    rng = np.random.default_rng(6)
+    size = lambda b: (b[5] - b[2], b[4] - b[1], b[3] - b[0])  # noqa: E731
+    eps = rng.uniform(1, 12, size(box)).astype(np.float32)
+    with solver.Simulation.from_scenario(sc, schedule, probe_capacity=64) as sim:
+        sim.set_design_region(first, rng.uniform(1, 12, size(first)).astype(np.float32), sigma_e=0.02)
+        sim.prepare()
+        sim.set_design_region(box, eps, sigma_e=0.02)
+        sim.step(sc.steps)
+        sim.synchronize()
+        p, f, prof = sim.read_probes(0, sc.steps), sim.fields(), sim.cpml_profiles()
+    sc.materials.append(S.Material(eps_r=1.0, sigma_e=0.02))
+    sc.bricks += [S.Brick(first, 1), S.Brick(box, 1)]  # both boxes hold the base material; the oracle adds eps_r
+    po, fo = oracle.run(sc, profile_override=prof, design=(box, eps.astype(np.float64)))
+    assert np.abs(po).max() > 0
+    assert bitwise_equal(p, po) and bitwise_equal(f, fo)

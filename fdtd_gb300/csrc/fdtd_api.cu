@@ -904,7 +904,8 @@ namespace {
 // What the sweep of the handle's next step takes besides its fields; late: the step before it is
 // one of the same call, whose probes are still to be sampled.
 SweepStep sweep_step(const fdtd_handle* h, bool late) {
-    SweepStep s{h->d_probes_at, h->n_probes_at, late, nullptr, h->slab_rows != nullptr, {}};
+    const int kind = !h->slab_rows ? kSweepPlain : h->des_row1 > 0 ? kSweepDesign : kSweepMat;
+    SweepStep s{h->d_probes_at, h->n_probes_at, late, nullptr, kind, {}};
     for (size_t w = 0; w < h->waves.size() && w < (size_t)kSweepSources; ++w)
         s.sig[w] = h->step < (long long)h->waves[w].size() ? h->waves[w][(size_t)h->step] : 0.f;
     return s;

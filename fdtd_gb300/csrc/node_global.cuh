@@ -80,6 +80,29 @@ __device__ __forceinline__ void e_node_global(const StepParams& p, const FieldPt
     }
 }
 
+// E of a design node with a row (StepParams::des_row0): its coefficients come from StepParams::dcoef. An
+// interior node without a lumped edge: every component, no CPML memory. kSample: probes too.
+__device__ __forceinline__ bool design_row(const StepParams& p, int row) { return row >= p.des_row0 && row < p.des_row1; }
+template <bool kSample, typename Idx = long long>
+__device__ __forceinline__ void e_node_design(const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fo, int i, int j, int k,
+                                              long long m) {
+    const DeviceGrid& g = p.g;
+    const Idx P = (Idx)g.plane, R = (Idx)g.pitch, n = (Idx)k * P + (Idx)j * R + (Idx)i;
+    const int* d = p.dbox;
+    const long long bx = d[3] - d[0] + 1, by = d[4] - d[1] + 1, ne = bx * by * (d[5] - d[2] + 1);
+    const long long q = ((k - d[2]) * by + (j - d[1])) * bx + (i - d[0]);
+    const float4 a = __ldg(p.dcoef + q), b = __ldg(p.dcoef + ne + q), c = __ldg(p.dcoef + 2 * ne + q);
+    const float hx = fi.hx[n], hy = fi.hy[n], hz = fi.hz[n];
+    float v[3] = {upd3(a.x, fi.ex[n], a.y, __fsub_rn(hz, fi.hz[n - R]), a.z, __fsub_rn(hy, fi.hy[n - P])),
+                  upd3(b.x, fi.ey[n], b.y, __fsub_rn(hx, fi.hx[n - P]), b.z, __fsub_rn(hz, fi.hz[n - 1])),
+                  upd3(c.x, fi.ez[n], c.y, __fsub_rn(hy, fi.hy[n - 1]), c.z, __fsub_rn(hx, fi.hx[n - R]))};
+    fo.ex[n] = v[0]; fo.ey[n] = v[1]; fo.ez[n] = v[2];
+    if (p.design_snap) { p.design_snap[q] = v[0]; p.design_snap[ne + q] = v[1]; p.design_snap[2 * ne + q] = v[2]; }
+    if (p.fom_sample && (long long)n == p.fom_node) *p.fom_sample = v[2];
+    if (kSample && p.probe_k[k] < p.probe_k[k + 1])
+        for (int s = 0; s < 3; ++s) sample(p, m % p.ring_cap, s, i, j, k, v[s]);
+}
+
 // H reads the old H from `fi` and the new E from `fe`.
 template <bool kCoherent = false, typename Idx = long long>
 __device__ __forceinline__ void h_node_global(const StepParams& p, const FieldPtrs& fi, const FieldPtrs& fe,

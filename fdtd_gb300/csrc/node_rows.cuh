@@ -29,7 +29,9 @@ template <typename Idx, bool kDesign>
 static __device__ __noinline__ void e_node_general(const StepParams* p, const FieldPtrs* f, const PsiSet* ps, const StepIndex* step,
                                                    int i, int j, int k) {
     const int c = kDesign ? p->rec[(Idx)k * (Idx)p->g.plane + (Idx)j * (Idx)p->g.pitch + (Idx)i] : 0;
-    if (kDesign && (c == (kRecGeneral | kDesignNode) || (c >= p->des_row0 && c < p->des_row1)))
+    if (kDesign && design_row(*p, c))
+        e_node_design<false, Idx>(*p, *f, *f, i, j, k, 0);
+    else if (kDesign && c == (kRecGeneral | kDesignNode))
         e_node_global<true>(*p, *f, *f, *ps, *ps, i, j, k, step->at());
     else
         e_node_global<false, false, false, Idx>(*p, *f, *f, *ps, *ps, i, j, k, step->at());
@@ -95,7 +97,7 @@ __device__ __forceinline__ void e_node_rows(const StepParams& p, const FieldPtrs
     if (zs) { Z = psi_slot_z<Idx>(p, i, j, k); }
     const BgNode& B = p.bgn;
     const bool own = c != p.bg.mat;
-    if (c >= kRecGeneral || (kDesign && c >= p.des_row0 && c < p.des_row1) || (own && slab && !p.rows.e[0])) {
+    if (c >= kRecGeneral || (kDesign && design_row(p, c)) || (own && slab && !p.rows.e[0])) {
         e_node_general<Idx, kDesign>(&p, &f, &ps, &step, i, j, k);
         return;
     }

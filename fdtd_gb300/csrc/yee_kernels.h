@@ -65,6 +65,9 @@ cudaError_t launch_rows_h(const MatCoef* coef, int n_rows, int bg, int* differ, 
 cudaError_t launch_slab_rows(const DeviceGrid& g, const MatCoef* coef, int n_rows, float* const prof_kappa[6], float4* out,
                              cudaStream_t st);
 
+// What a grid asks of the sweep: nothing but its rows; coefficient rows other than the background's in a
+// CPML slab or on a low wall (SlabRows); a design region's rows besides.
+enum { kSweepPlain = 0, kSweepMat = 1, kSweepDesign = 2 };
 constexpr int kSweepSources = 8;  // lumped sources whose signal comes with the launch
 struct SweepStep {
     const ProbeAt* probes;  // probes outside the CPML slabs
@@ -72,7 +75,7 @@ struct SweepStep {
     int late;               // sample them for step m - 1 from fi
     const long long* base;  // device step counter that m counts from (captured launches), or NULL: the
                             // sources' signals are then read on the device
-    int mat;                // coefficient rows other than the background's in a CPML slab or on a low wall
+    int kind;
     float sig[kSweepSources];
 };
 cudaError_t sweep_configure();

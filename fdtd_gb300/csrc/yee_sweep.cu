@@ -265,16 +265,17 @@ __device__ __forceinline__ Quad quad_of(const float4& f) { return Quad{f.x, f.y,
 // The march of one thread's quad at tile row `row`, first column `col`. kEdge: the tile (halo
 // included) meets a CPML slab or a wall in x (wx) or y (wy), or the chunk one in z; without it no
 // node does. kMat: rows other than the background's lie in a slab or on a low wall (without it the
-// few that may, beside general nodes, take the slow path), or the grid has a design region, whose rows' E
-// coefficients are each node's own (StepParams::dcoef; node by node on the slow path a region of 256^3 cells
-// in 512^3 cost 2.4 ms of a step's 3.7, now 0.14 of 1.44; in the other kernels the test for such rows cost
-// boxes 2 %). Their quads of one row take the background's
+// few that may, beside general nodes, take the slow path). Their quads of one row take the background's
 // way through the step, with coefficients from the tables: node by node, a load waiting for the one
 // before it, they held their tiles up (a half space and boxes through the slabs, us a step: 225^3 300 -> 244,
-// 320^3 567 -> 444; with the chunks of plan_sweep 237 and 419).
-template <typename Idx, bool kEdge, bool kMat, bool kWide>
+// 320^3 567 -> 444; with the chunks of plan_sweep 237 and 419). kDesign (with kMat): the grid has a design
+// region, whose rows' E coefficients are each node's own (StepParams::dcoef): on the slow path a region of
+// 256^3 cells in 512^3 cost 2.4 ms of a step's 3.7, now 0.14 of 1.49. A kernel of their own, as the test for
+// such rows cost the others 1 to 8 %.
+template <typename Idx, bool kEdge, int kKind, bool kWide>
 __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int x0, int y0, int k0, int k1, int row,
                                       int col, bool own, bool wx, bool wy) {
+    constexpr bool kMat = kKind != kSweepPlain, kDesign = kKind == kSweepDesign;
     const StepParams& p = A.p;
     const DeviceGrid& g = p.g;
     const FieldPtrs& fo = A.fo;
@@ -426,7 +427,7 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
             bool mixed = false;
             const bool bg = kEdge && !kMat ? true : c0 == bgm;
             if (cw.x == cw.y && cw.x == (uint32_t)c0 * 0x10001u &&
-                (kEdge ? (kMat ? c0 < p.des_row0 : c0 == bgm) && !xslow : c0 < (kMat ? p.des_row0 : p.src_row0))) {
+                (kEdge ? (kMat ? c0 < (kDesign ? p.des_row0 : p.src_row0) : c0 == bgm) && !xslow : c0 < (kDesign ? p.des_row0 : p.src_row0))) {
                 // one row for the quad (in tiles at the edge without kMat, the background's)
                 float4 a = make_float4(B.ea[0], B.ec[0], B.ec[1], 0.f), b = make_float4(B.ea[1], B.ec[2], B.ec[3], 0.f);
                 float4 d = make_float4(B.ea[2], B.ec[4], B.ec[5], 0.f);
@@ -454,16 +455,16 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                 // rows per node; in a slab background nodes take the tabulated curl coefficients, and
                 // without kMat the others the slow path
                 mixed = true;
-                // where a component's E coefficients of node r (row c) lie (without kMat the grid has no design rows)
+                // where a component's E coefficients of node r (row c) lie
                 long long dq = 0, dn = 0;
-                if (kMat && p.des_row1 > 0) {
+                if (kDesign) {
                     const int* d = p.dbox;
                     const long long bx = d[3] - d[0] + 1, by = d[4] - d[1] + 1;
                     dn = bx * by * (d[5] - d[2] + 1);
                     dq = ((k - d[2]) * by + (j - d[1])) * bx + (i - d[0]);
                 }
                 auto e_row = [&](int c, int r, int comp) {
-                    return kMat && c >= p.des_row0 && c < p.des_row1 ? p.dcoef + (comp * dn + dq + r) : &p.coef[c].e[comp];
+                    return kDesign && c >= p.des_row0 && c < p.des_row1 ? p.dcoef + (comp * dn + dq + r) : &p.coef[c].e[comp];
                 };
                 if constexpr (kWide || !kEdge) {
                     // (component by component, so that the four nodes' loads are in flight together: the quads
@@ -546,7 +547,7 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
                         }
                         if (c != cur) {
                             a = __ldg(e_row(c, r, 0)); b = __ldg(e_row(c, r, 1)); d = __ldg(e_row(c, r, 2));
-                            cur = kMat && c >= p.des_row0 && c < p.des_row1 ? -1 : c;  // (a design row's are the node's own)
+                            cur = kDesign && c >= p.des_row0 && c < p.des_row1 ? -1 : c;  // (a design row's are the node's own)
                             if (!kMat || c == bgm) {
                                 if (kEdge && ys) { a.y = S.ye[row].x; d.z = S.ye[row].y; }
                                 if (kEdge && zs) { a.z = S.ze[q].x; b.y = S.ze[q].y; }
@@ -928,7 +929,7 @@ __device__ __forceinline__ void march(const SweepArgs& A, SweepSmem<Idx>& S, int
 
 }  // namespace
 
-template <typename Idx, bool kMat, bool kWide>
+template <typename Idx, int kKind, bool kWide>
 __global__ void __launch_bounds__(NTH, kWide ? 2 : 3) k_sweep(const __grid_constant__ SweepArgs A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     SweepSmem<Idx>& S = *reinterpret_cast<SweepSmem<Idx>*>(smem_raw);
@@ -1007,23 +1008,31 @@ __global__ void __launch_bounds__(NTH, kWide ? 2 : 3) k_sweep(const __grid_const
     const bool wx = x0 < max(g.pxn, 1) || x0 + TX >= min(g.nx - g.pxp, g.nx - 1);
     const bool wy = y0 < max(g.pyn, 1) || y0 + TY >= min(g.ny - g.pyp, g.ny - 1);
     const bool wz = k0 < max(g.pzn, 1) || k1 >= min(g.nz - g.pzp, g.nz - 1);  // E(k0) .. E(k1), H(k0) .. H(k1 - 1)
-    if (wx || wy || wz) march<Idx, true, kMat, kWide>(A, S, x0, y0, k0, k1, row, col, own, wx, wy);
-    else march<Idx, false, kMat, kWide>(A, S, x0, y0, k0, k1, row, col, own, false, false);
+    if (wx || wy || wz) march<Idx, true, kKind, kWide>(A, S, x0, y0, k0, k1, row, col, own, wx, wy);
+    else march<Idx, false, kKind, kWide>(A, S, x0, y0, k0, k1, row, col, own, false, false);
 }
 
 template <typename Idx>
 constexpr int sweep_smem() { return (int)sizeof(SweepSmem<Idx>); }
 
-template <typename Idx, bool kMat, bool kWide>
-cudaError_t configure() {
-    return cudaFuncSetAttribute(k_sweep<Idx, kMat, kWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, sweep_smem<Idx>());
+// The kernel for a grid's kind; 64-bit offsets have no two-CTA form (such grids fill the device).
+using SweepKernel = void (*)(const SweepArgs);
+template <typename Idx, bool kWide>
+SweepKernel sweep_kernel(int kind) {
+    return kind == kSweepPlain ? SweepKernel(k_sweep<Idx, kSweepPlain, kWide>)
+           : kind == kSweepMat ? SweepKernel(k_sweep<Idx, kSweepMat, kWide>)
+                               : SweepKernel(k_sweep<Idx, kSweepDesign, kWide>);
 }
 cudaError_t sweep_configure() {
     cudaError_t e = cudaSuccess;
-    for (cudaError_t (*f)() : {configure<uint32_t, false, false>, configure<uint32_t, false, true>, configure<uint32_t, true, false>,
-                               configure<uint32_t, true, true>, configure<unsigned long long, false, false>,
-                               configure<unsigned long long, true, false>})
-        if (e == cudaSuccess) e = f();
+    auto configure = [&](SweepKernel k, int smem) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    };
+    for (int kind : {kSweepPlain, kSweepMat, kSweepDesign}) {
+        configure(sweep_kernel<uint32_t, false>(kind), sweep_smem<uint32_t>());
+        configure(sweep_kernel<uint32_t, true>(kind), sweep_smem<uint32_t>());
+        configure(sweep_kernel<unsigned long long, false>(kind), sweep_smem<unsigned long long>());
+    }
     return e;
 }
 
@@ -1048,10 +1057,9 @@ cudaError_t launch_sweep(const FusedMaps& maps, const StepParams& p, const Field
     const bool idx32 = p.g.plane * (long long)(p.g.nz + 1) < (1LL << 31) && p.psi_total < (1LL << 31);
     const unsigned ctas = (unsigned)(sg.nbx * sg.nby * sg.chunks());
     const bool wide = !ss.base && ctas <= kSweepWideCtas;
-    using K = void (*)(const SweepArgs);
-    const K k = idx32 ? ss.mat ? wide ? K(k_sweep<uint32_t, true, true>) : K(k_sweep<uint32_t, true, false>)
-                               : wide ? K(k_sweep<uint32_t, false, true>) : K(k_sweep<uint32_t, false, false>)
-                      : ss.mat ? K(k_sweep<unsigned long long, true, false>) : K(k_sweep<unsigned long long, false, false>);
+    const SweepKernel k = !idx32 ? sweep_kernel<unsigned long long, false>(ss.kind)
+                          : wide ? sweep_kernel<uint32_t, true>(ss.kind)
+                                 : sweep_kernel<uint32_t, false>(ss.kind);
     return launch_dependent(k, dim3(ctas), dim3(NTH), idx32 ? sweep_smem<uint32_t>() : sweep_smem<unsigned long long>(), st, args);
 }
 

@@ -89,7 +89,8 @@ __global__ void __launch_bounds__(256) k_design_e(const __grid_constant__ StepPa
     const int j = d[1] + blockIdx.y * 8 + threadIdx.y;
     const int k = d[2] + blockIdx.z;
     if (i > d[3] || j > d[4]) return;
-    e_node_global<true>(p, fi, fo, pin, pout, i, j, k, m);
+    if (design_row(p, p.rec[(long long)k * p.g.plane + (long long)j * p.g.pitch + i])) e_node_design<true>(p, fi, fo, i, j, k, m);
+    else e_node_global<true>(p, fi, fo, pin, pout, i, j, k, m);
 }
 
 // E of the nodes with a plate-covered edge (node class kPlateNode, which the other E kernels leave

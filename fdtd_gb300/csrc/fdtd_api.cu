@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -105,7 +106,7 @@ struct fdtd_handle {
     int cur = 0;
     bool have_second = false;
     FusedMaps maps[2];  // the sweep's tensor maps per input buffer
-    char* psi_base[2] = {nullptr, nullptr};  // the allocation holding each CPML memory set
+    std::shared_ptr<void> second;  // device memory of the second buffers, perhaps shared with other handles of a batch
     long long psi_off[6] = {}, psi_stride[6] = {}, psi_total = 0;  // its arrays by face (StepParams::psi_off)
     float4 *te[3] = {}, *th[3] = {};   // StepParams::te, th
     BgNode bg_node{};
@@ -338,34 +339,28 @@ int validate_grid(const fdtd_grid* g) {
 
 int ensure_prepared(fdtd_handle* h);
 
-// One set of CPML memory slabs (4 arrays per face), initialised to 1.2e-38.
-// CPML memory set s: the 24 arrays (4 per face) in one allocation, each array on a 256-byte
-// boundary, filled with the initial value by one launch (separate allocations of this size cost
-// tens of microseconds each).
-int alloc_psi_set(fdtd_handle* h, int s) {
-    size_t off[6], bytes[6], total = 0;
+// The layout of a CPML memory set: the 24 arrays (4 per face), each on a 256-byte boundary.
+void psi_layout(fdtd_handle* h) {
+    long long total = 0;
     for (int f = 0; f < 6; ++f) {
-        bytes[f] = ((size_t)h->psi_elems[f] * sizeof(float) + 255) / 256 * 256;
-        off[f] = total;
-        total += 4 * bytes[f];
-        h->psi_off[f] = (long long)(off[f] / sizeof(float));
-        h->psi_stride[f] = (long long)(bytes[f] / sizeof(float));
+        h->psi_stride[f] = (h->psi_elems[f] + 63) / 64 * 64;
+        h->psi_off[f] = total;
+        total += 4 * h->psi_stride[f];
     }
-    h->psi_total = (long long)(total / sizeof(float));
+    h->psi_total = total;
+}
+
+// CPML memory set s at `base` (psi_total floats), filled with the initial value by one launch on the
+// handle's stream, whose steps write the set next (at creation still the legacy stream).
+int place_psi_set(fdtd_handle* h, int s, float* base) {
     h->psi[s] = PsiSet{};
-    h->psi_base[s] = nullptr;
-    if (total == 0) return FDTD_OK;
-    char* base = nullptr;
-    if (h->alloc((void**)&base, total) != cudaSuccess) return fail(FDTD_ERR_OOM, "CPML memory allocation failed");
-    h->psi_base[s] = base;
-    h->psi[s].base = (float*)base;
-    // on the handle's stream, whose steps write the set next (at creation still the legacy stream)
-    if (launch_fill((float*)base, (long long)(total / sizeof(float)), kTiny, h->stream) != cudaSuccess)
-        return fail(FDTD_ERR_CUDA, "fill failed");
+    if (h->psi_total == 0) return FDTD_OK;
+    h->psi[s].base = base;
+    if (launch_fill(base, h->psi_total, kTiny, h->stream) != cudaSuccess) return fail(FDTD_ERR_CUDA, "fill failed");
     for (int f = 0; f < 6; ++f) {
         if (h->psi_elems[f] <= 0) continue;
         float* a[4];
-        for (int q = 0; q < 4; ++q) a[q] = (float*)(base + off[f] + (size_t)q * bytes[f]);
+        for (int q = 0; q < 4; ++q) a[q] = base + h->psi_off[f] + q * h->psi_stride[f];
         h->psi[s].f[f].e[0] = a[0]; h->psi[s].f[f].e[1] = a[1];
         h->psi[s].f[f].h[0] = a[2]; h->psi[s].f[f].h[1] = a[3];
     }
@@ -438,20 +433,25 @@ BgNode make_bg_node(const DeviceGrid& g, const fdtd_material_axes& m) {
     return b;
 }
 
-// Second field buffer, second CPML set and the TMA tensor maps of both buffers for the sweep.
-int ensure_fused(fdtd_handle* h) {
-    if (h->have_second) return FDTD_OK;
+// Bytes of a handle's second buffers for the sweep: six fields, then a CPML set.
+size_t second_bytes(const fdtd_handle* h) {
+    return ((6 * (size_t)vol(h) * sizeof(float) + 255) / 256 + ((size_t)h->psi_total * sizeof(float) + 255) / 256) * 256;
+}
+
+// The second buffers at `base`, in device memory that `owner` keeps, and the TMA tensor maps of both
+// buffers; the caller waits for the handle's stream before it sets have_second.
+int place_second(fdtd_handle* h, const std::shared_ptr<void>& owner, char* base) {
+    const long long V = vol(h);
+    h->second = owner;
+    h->bytes += (long long)second_bytes(h);
+    for (int c = 0; c < 6; ++c) h->field[1][c] = (float*)base + c * V;
     // no copy of the state and no fill: a fused step writes every node of its target buffer; only
     // the row padding, which no kernel writes, gets buffer 0's initial value so that saved states
     // agree
-    const long long V = vol(h);
-    float* base = nullptr;  // the six fields in one allocation (separate ones cost tens of microseconds each)
-    CUDA_TRY(h->alloc((void**)&base, 6 * (size_t)V * sizeof(float)));
-    for (int c = 0; c < 6; ++c) h->field[1][c] = base + c * V;
     DeviceGrid all = h->g;
     all.nz *= 6;
-    CUDA_TRY(launch_fill_padding(base, all, kTiny, h->stream));
-    int rc = alloc_psi_set(h, 1);
+    CUDA_TRY(launch_fill_padding((float*)base, all, kTiny, h->stream));
+    int rc = place_psi_set(h, 1, (float*)(base + (6 * (size_t)V * sizeof(float) + 255) / 256 * 256));
     if (rc) return rc;
     void* enc = tensor_map_encoder();
     if (!enc) return fail(FDTD_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
@@ -461,26 +461,51 @@ int ensure_fused(fdtd_handle* h) {
         if (encode_sweep_maps(&h->maps[b], h->g, hh, ee, h->rec, enc) != 0)
             return fail(FDTD_ERR_CUDA, "tensor map encoding failed");
     }
-    CUDA_TRY(sweep_configure());
-    CUDA_TRY(cudaStreamSynchronize(h->stream));
-    h->have_second = true;
     return FDTD_OK;
 }
+
+// Gives the second buffers back; the state must be in buffer 0.
+void release_second(fdtd_handle* h) {
+    if (h->second) h->bytes -= (long long)second_bytes(h);
+    h->second.reset();
+    for (int c = 0; c < 6; ++c) h->field[1][c] = nullptr;
+    h->psi[1] = PsiSet{};
+    h->have_second = false;
+}
+
+// Second buffers for the n handles of hs (none of which has any) in one allocation, which the last of
+// them gives back: an allocation each costs 45 us, which a batch's first call felt. All or none.
+int alloc_second(fdtd_handle* const* hs, size_t n) {
+    size_t total = 0;
+    for (size_t q = 0; q < n; ++q) total += second_bytes(hs[q]);
+    char* base = nullptr;
+    CUDA_TRY(cudaMalloc((void**)&base, total));
+    const std::shared_ptr<void> owner(base, [](void* p) { cudaFree(p); });
+    auto place = [&]() -> int {
+        CUDA_TRY(sweep_configure());
+        char* at = base;
+        for (size_t q = 0; q < n; at += second_bytes(hs[q]), ++q) {
+            const int rc = place_second(hs[q], owner, at);
+            if (rc) return rc;
+        }
+        for (size_t q = 0; q < n; ++q)
+            if (q == 0 || hs[q]->stream != hs[q - 1]->stream) CUDA_TRY(cudaStreamSynchronize(hs[q]->stream));
+        return FDTD_OK;
+    };
+    const int rc = place();
+    for (size_t q = 0; q < n; ++q) {
+        if (rc) release_second(hs[q]);
+        else hs[q]->have_second = true;
+    }
+    return rc;
+}
+
+int ensure_fused(fdtd_handle* h) { return h->have_second ? FDTD_OK : alloc_second(&h, 1); }
 
 // AUTO runs two-pass until auto_choose has taken the fused schedule.
 bool use_fused(const fdtd_handle* h) {
     return h->schedule == FDTD_SCHEDULE_FUSED || h->schedule == FDTD_SCHEDULE_FUSED_CPML ||
            (h->schedule == FDTD_SCHEDULE_AUTO && h->auto_choice == FDTD_SCHEDULE_FUSED);
-}
-
-// Frees what ensure_fused allocated; the state must be in buffer 0.
-void release_fused(fdtd_handle* h) {
-    h->release(h->field[1][0]);  // the allocation holds all six
-    for (int c = 0; c < 6; ++c) h->field[1][c] = nullptr;
-    h->release(h->psi_base[1]);
-    h->psi_base[1] = nullptr;
-    h->psi[1] = PsiSet{};
-    h->have_second = false;
 }
 
 // AUTO's choice, made by fdtd_tune_schedule (n < 0) or by the call whose n steps bring the handle to
@@ -511,7 +536,6 @@ void auto_choose(fdtd_handle* h, int64_t n) {
         h->auto_choice = FDTD_SCHEDULE_FUSED;
     } else {  // no room for the second buffers
         cudaGetLastError();
-        if (h->cur == 0) release_fused(h);
         h->auto_choice = FDTD_SCHEDULE_TWO_PASS;
     }
 }
@@ -598,7 +622,11 @@ int fdtd_create(const fdtd_grid* grid, fdtd_handle** out) {
         else n = (long long)P[f] * g.ny * g.pitch;
         h->psi_elems[f] = n;
     }
-    rc = alloc_psi_set(h, 0);
+    psi_layout(h);
+    float* psi = nullptr;
+    if (h->psi_total > 0 && h->alloc((void**)&psi, (size_t)h->psi_total * sizeof(float)) != cudaSuccess)
+        return cleanup(fail(FDTD_ERR_OOM, "CPML memory allocation failed"));
+    rc = place_psi_set(h, 0, psi);
     if (rc) return cleanup(rc);
     // node classes and coefficient rows, which every preparation builds: allocated here, while the
     // fills run
@@ -1628,7 +1656,7 @@ bool g_scratch_configured[kMaxScratchDevices] = {};
 size_t align_up(size_t v) { return (v + kScratchAlign - 1) / kScratchAlign * kScratchAlign; }
 
 // Offsets of the pieces of the scratch for handle h: 6 fields, then the 24 CPML arrays, laid out
-// like a CPML memory set (alloc_psi_set).
+// like a CPML memory set (psi_layout).
 struct ScratchLayout {
     size_t field[6];
     size_t psi;
@@ -2205,6 +2233,8 @@ struct fdtd_batch {
     std::vector<cudaEvent_t> chain_events;  // [0]: fork, [1 + q]: join of instance q
     unsigned long long chain_sig = 0;       // of the current descriptors
     std::vector<char> sweep;                // instances whose chain runs the sweep (two-pass otherwise)
+    long long steps_asked = 0;              // of the chain form
+    bool no_room = false;                   // for the second buffers of instances under AUTO
 };
 
 namespace {
@@ -2213,6 +2243,11 @@ namespace {
 // fewer halo planes, short ones give the device more CTAs. 64 instances of 32^3 to 96^3, 32 steps:
 // 14.5 ms with a share of 1, 14.6 with 2, 14.8 with 4; 16 of them 5.1, 3.9 and 3.5; 8 of 64^3 2.3, 1.8 and 2.0.
 constexpr double kBatchShare = 2.0;
+
+// What the second buffers of a batch's instances cost, us: the allocation, each instance's fills and
+// tensor maps, each byte; and what the sweep saves per cell and step: 64 instances of 32^3 to 96^3 0.73 ->
+// 0.48 ms a step, 24 of 48^3 to 96^3 0.33 -> 0.24, 256 of 32^3 to 96^3 2.94 -> 1.89.
+constexpr double kBatchAllocUs = 200.0, kBatchEachUs = 20.0, kBatchByteUs = 0.3e-6, kBatchSavedUs = 12e-6 / 1.048576;
 
 void batch_drop_graph(fdtd_batch* b) {
     for (auto& G : b->graphs) {
@@ -2268,26 +2303,44 @@ int batch_set_config(fdtd_batch* b, int cluster, int threads) {
 }
 
 // Which instances' chains run the sweep: in a batch of at least kBatchSweepCells altogether, those from
-// kAutoSweepCells on whose schedule allows it and that have room for second buffers. Smaller batches
-// leave the device partly idle, and two passes have the shorter chain of dependent loads. Measured,
+// kAutoSweepCells on whose schedule allows it and that have second buffers. Smaller batches leave the
+// device partly idle, and two passes have the shorter chain of dependent loads. Measured,
 // two-pass against sweep, ms for 32 steps of n cubes: 4 x 64^3 0.77 / 1.05, 2 x 96^3 1.02 / 1.38,
 // 16 x 40^3 1.40 / 1.83, 8 x 64^3 1.61 / 1.78, 16 x 48^3 2.11 / 2.18, 16 x 56^3 3.6 / 2.8, 4 x 96^3 2.67 / 2.36,
 // 16 x (32 to 96) 4.24 / 3.96, 64 x 40^3 8.5 / 6.2, 64 x 64^3 18.7 / 12.0, 16 x 128^3 23.2 / 15.7.
+// Instances under AUTO get their second buffers together, once the steps asked of the batch (n < 0: a
+// tuning run) repay them, and where they leave as much memory free as they take.
 constexpr long long kBatchSweepCells = 2560LL << 10;
-void batch_choose(fdtd_batch* b) {
+void batch_choose(fdtd_batch* b, long long n) {
     auto cells = [](const fdtd_handle* h) { return (long long)h->g.nx * h->g.ny * h->g.nz; };
     long long total = 0;
     for (const fdtd_handle* h : b->hs) total += cells(h);
+    if (n > 0) b->steps_asked += n;
+    std::vector<fdtd_handle*> want, fused;  // without second buffers: under AUTO, under FUSED
+    double saved = 0.0, cost = kBatchAllocUs;
+    size_t bytes = 0;
     for (size_t q = 0; q < b->hs.size(); ++q) {
         fdtd_handle* h = b->hs[q];
-        bool s = total >= kBatchSweepCells && cells(h) >= kAutoSweepCells && h->schedule != FDTD_SCHEDULE_TWO_PASS;
-        if (s && ensure_fused(h) != FDTD_OK) {
-            cudaGetLastError();
-            if (h->cur == 0) release_fused(h);
-            s = false;
-        }
-        b->sweep[q] = s;
+        b->sweep[q] = total >= kBatchSweepCells && cells(h) >= kAutoSweepCells && h->schedule != FDTD_SCHEDULE_TWO_PASS;
+        if (!b->sweep[q] || h->have_second) continue;
+        (h->schedule == FDTD_SCHEDULE_AUTO ? want : fused).push_back(h);
+        if (h->schedule != FDTD_SCHEDULE_AUTO) continue;
+        saved += kBatchSavedUs * (double)cells(h);
+        cost += kBatchEachUs + kBatchByteUs * (double)second_bytes(h);
+        bytes += second_bytes(h);
     }
+    if (n >= 0 && saved * (double)b->steps_asked < cost) want.clear();
+    size_t free_b = 0, all_b = 0;
+    if (!want.empty() && (b->no_room || cudaMemGetInfo(&free_b, &all_b) != cudaSuccess || 2 * bytes > free_b)) {
+        b->no_room = true;
+        want.clear();
+    }
+    want.insert(want.end(), fused.begin(), fused.end());
+    if (!want.empty() && alloc_second(want.data(), want.size()) != FDTD_OK) {
+        cudaGetLastError();
+        b->no_room = true;
+    }
+    for (size_t q = 0; q < b->hs.size(); ++q) b->sweep[q] = b->sweep[q] && b->hs[q]->have_second;
 }
 
 // `steps` sweep steps of instance q on stream cs, counted from its device step counter.
@@ -2386,17 +2439,17 @@ unsigned long long descriptor_signature(const fdtd_batch* b) {
         word(b->sweep[q]);
         word((unsigned long long)x->cur);
         word((unsigned long long)(uintptr_t)x->field[1][0]);
-        word((unsigned long long)(uintptr_t)x->psi_base[1]);
+        word((unsigned long long)(uintptr_t)x->psi[1].base);
         word((unsigned long long)(uintptr_t)x->d_probes_at);
         word((unsigned long long)x->n_probes_at);
     }
     return h;
 }
-int batch_run(fdtd_batch* b, long long steps) {
+int batch_run(fdtd_batch* b, long long steps, bool tuning = false) {
     int rc = batch_refresh(b);
     if (rc) return rc;
     if (b->cluster == -1) {
-        batch_choose(b);
+        batch_choose(b, tuning ? -1 : steps);
         b->chain_sig = descriptor_signature(b);
     }
     cudaGraphExec_t ex = nullptr;
@@ -2569,7 +2622,7 @@ extern "C" int fdtd_batch_tune(fdtd_batch* b, int64_t steps, double* best_ms) {
             float ms = 0.f;
             for (int rep = 0; rep < 2 && !rc; ++rep) {
                 cudaEventRecord(e0, b->stream);
-                if ((rc = batch_run(b, steps))) break;
+                if ((rc = batch_run(b, steps, true))) break;
                 cudaEventRecord(e1, b->stream);
                 if (cudaEventSynchronize(e1) != cudaSuccess) { rc = fail(FDTD_ERR_CUDA, "tuning run failed"); break; }
                 cudaEventElapsedTime(&ms, e0, e1);

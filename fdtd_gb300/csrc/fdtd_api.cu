@@ -2244,10 +2244,12 @@ namespace {
 // 14.5 ms with a share of 1, 14.6 with 2, 14.8 with 4; 16 of them 5.1, 3.9 and 3.5; 8 of 64^3 2.3, 1.8 and 2.0.
 constexpr double kBatchShare = 2.0;
 
-// What the second buffers of a batch's instances cost, us: the allocation, each instance's fills and
-// tensor maps, each byte; and what the sweep saves per cell and step: 64 instances of 32^3 to 96^3 0.73 ->
-// 0.48 ms a step, 24 of 48^3 to 96^3 0.33 -> 0.24, 256 of 32^3 to 96^3 2.94 -> 1.89.
-constexpr double kBatchAllocUs = 200.0, kBatchEachUs = 20.0, kBatchByteUs = 0.3e-6, kBatchSavedUs = 12e-6 / 1.048576;
+// What the second buffers of a batch's instances cost, us, less what a first call saves by capturing one
+// kernel a step in place of two: the allocation, each instance's fills and tensor maps, each byte; and what
+// the sweep saves per cell and step: 64 instances of 32^3 to 96^3 0.73 -> 0.48 ms a step, 24 of 48^3 to 96^3
+// 0.33 -> 0.24, 256 of 32^3 to 96^3 2.94 -> 1.89. A first call of 5 steps, two-pass / with the buffers: 64
+// instances 6.2 / 5.5 ms, 256 28.9 / 23.3, 16 of 96^3 to 128^3 3.6 / 3.0; of one step, 64 instances 2.5 / 2.9.
+constexpr double kBatchAllocUs = 100.0, kBatchEachUs = 8.0, kBatchByteUs = 0.2e-6, kBatchSavedUs = 12e-6 / 1.048576;
 
 void batch_drop_graph(fdtd_batch* b) {
     for (auto& G : b->graphs) {

@@ -473,11 +473,28 @@ void release_second(fdtd_handle* h) {
     h->have_second = false;
 }
 
+// Whether the handle's stream is under capture (an error, on the legacy stream next to another's capture,
+// counts as not).
+bool capturing(const fdtd_handle* h) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess) cudaGetLastError();
+    return cs != cudaStreamCaptureStatusNone;
+}
+
 // Second buffers for the n handles of hs (none of which has any) in one allocation, which the last of
 // them gives back: an allocation each costs 45 us, which a batch's first call felt. All or none.
 int alloc_second(fdtd_handle* const* hs, size_t n) {
     size_t total = 0;
-    for (size_t q = 0; q < n; ++q) total += second_bytes(hs[q]);
+    for (size_t q = 0; q < n; ++q) {
+        if (capturing(hs[q])) return fail(FDTD_ERR_STATE, "second buffers cannot be allocated while the handle's stream is captured");
+        total += second_bytes(hs[q]);
+    }
+    // (a capture that goes on elsewhere in the program takes no harm from the allocation)
+    struct Relaxed {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+        ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    } relaxed;
     char* base = nullptr;
     CUDA_TRY(cudaMalloc((void**)&base, total));
     const std::shared_ptr<void> owner(base, [](void* p) { cudaFree(p); });
@@ -512,10 +529,19 @@ bool use_fused(const fdtd_handle* h) {
 // where the second buffers repay what it costs to allocate and free them: measured 0.2 ms at 64^3,
 // 0.55 at 256^3, 0.84 at 28 M cells, against the 1, 92 and 190 us that the sweep saves a step; some
 // 200 steps at 64^3, 20 at 160^3, 5 from 256^3 on. The buffers are allocated here, not under stream
-// capture: a handle stepped there takes two-pass until later.
+// capture: a handle stepped there takes two-pass until later. Below kAutoCaptureCells it keeps to two-pass
+// from then on: the captured step is replayed on the buffer that it was captured with, where the state
+// must stay (an odd number of sweeps leaves it in the other one). Larger grids may be captured under the
+// sweep, in even counts.
+constexpr long long kAutoCaptureCells = 8LL << 20;
 void auto_choose(fdtd_handle* h, int64_t n) {
-    if (h->schedule != FDTD_SCHEDULE_AUTO || h->auto_choice != FDTD_SCHEDULE_AUTO) return;
+    if (h->schedule != FDTD_SCHEDULE_AUTO || h->auto_choice == FDTD_SCHEDULE_TWO_PASS) return;
     const long long cells = (long long)h->g.nx * h->g.ny * h->g.nz;
+    if (n >= 0 && cells < kAutoCaptureCells && capturing(h)) {
+        h->auto_choice = FDTD_SCHEDULE_TWO_PASS;
+        return;
+    }
+    if (h->auto_choice != FDTD_SCHEDULE_AUTO) return;
     const bool small = cells < kAutoTwoPassLo;
     if (h->edge_rows ? cells < (h->h_bg ? kAutoEdgeHi : kAutoEdgeMagneticHi)
                      : cells < kAutoSweepCells || (!small && cells < kAutoTwoPassHi)) {
@@ -526,11 +552,7 @@ void auto_choose(fdtd_handle* h, int64_t n) {
         if (n > 0) h->auto_steps += n;
         const double saved = small ? 1.0 : std::max(1.0, 7e-6 * (cells - 2.2e6)), cost = 200.0 + 23e-6 * cells;
         if (n >= 0 && h->auto_steps * saved < cost) return;
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-            cudaGetLastError();
-            return;
-        }
+        if (capturing(h)) return;
     }
     if (ensure_fused(h) == FDTD_OK) {
         h->auto_choice = FDTD_SCHEDULE_FUSED;

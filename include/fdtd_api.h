@@ -38,11 +38,13 @@ enum { FDTD_EX = 0, FDTD_EY = 1, FDTD_EZ = 2, FDTD_HX = 3, FDTD_HY = 4, FDTD_HZ 
 enum {
     FDTD_SCHEDULE_AUTO = 0,   /* FUSED or TWO_PASS by the grid's size (the measured faster one);
                                  TWO_PASS until the steps asked for repay FUSED's second buffers
-                                 (5 to 200, fewer the larger the grid; or fdtd_tune_schedule) and
-                                 where those do not fit or the step is captured */
+                                 (5 to 200, fewer the larger the grid; or fdtd_tune_schedule),
+                                 where those do not fit, and from a captured step on below 8 Mi
+                                 cells. The call that allocates them waits for the handle's stream */
     FDTD_SCHEDULE_TWO_PASS = 1, /* E pass then H pass per step, in place (the reference's order) */
     FDTD_SCHEDULE_FUSED = 2,  /* one z-marching sweep of the whole grid per step over ping-pong
-                                 field buffers (second buffers are allocated by the first step)  */
+                                 field buffers (second buffers are allocated by the first step, not
+                                 under capture; captured for replay, a call takes an even count) */
     FDTD_SCHEDULE_FUSED_CPML = 3 /* the same sweep as FUSED, which covers the CPML */
 };
 

@@ -1051,9 +1051,8 @@ int fdtd_set_field(fdtd_handle* h, int32_t comp, const float* in) {
     if (!h || !in) return fail(FDTD_ERR_INVALID, "NULL argument");
     if (comp < 0 || comp > 5) return fail(FDTD_ERR_INVALID, "component must be 0..5");
     const DeviceGrid& g = h->g;
-    for (int b = 0; b < (h->have_second ? 2 : 1); ++b)
-        CUDA_TRY(cudaMemcpy2DAsync(h->field[b][comp], (size_t)g.pitch * 4, in, (size_t)g.nx * 4, (size_t)g.nx * 4,
-                                   (size_t)g.ny * g.nz, cudaMemcpyHostToDevice, h->stream));
+    CUDA_TRY(cudaMemcpy2DAsync(h->field[h->cur][comp], (size_t)g.pitch * 4, in, (size_t)g.nx * 4, (size_t)g.nx * 4,
+                               (size_t)g.ny * g.nz, cudaMemcpyHostToDevice, h->stream));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     return FDTD_OK;
 }
@@ -1071,9 +1070,8 @@ int fdtd_set_field_device(fdtd_handle* h, int32_t comp, const float* in) {
     if (!h || !in) return fail(FDTD_ERR_INVALID, "NULL argument");
     if (comp < 0 || comp > 5) return fail(FDTD_ERR_INVALID, "component must be 0..5");
     const DeviceGrid& g = h->g;
-    for (int b = 0; b < (h->have_second ? 2 : 1); ++b)
-        CUDA_TRY(cudaMemcpy2DAsync(h->field[b][comp], (size_t)g.pitch * 4, in, (size_t)g.nx * 4, (size_t)g.nx * 4,
-                                   (size_t)g.ny * g.nz, cudaMemcpyDeviceToDevice, h->stream));
+    CUDA_TRY(cudaMemcpy2DAsync(h->field[h->cur][comp], (size_t)g.pitch * 4, in, (size_t)g.nx * 4, (size_t)g.nx * 4,
+                               (size_t)g.ny * g.nz, cudaMemcpyDeviceToDevice, h->stream));
     return FDTD_OK;
 }
 
@@ -1082,15 +1080,15 @@ int fdtd_set_field_device(fdtd_handle* h, int32_t comp, const float* in) {
 namespace {
 
 // Copy the dynamic state (6 fields, then the 24 CPML arrays) to or from a device buffer on the
-// handle's stream, without synchronising. Loading writes both field buffers of the fused schedule.
+// handle's stream, without synchronising. Loading writes the current buffer only: a sweep writes every
+// node of the other one.
 int state_copy(fdtd_handle* h, void* buf, bool save) {
     char* p = (char*)buf;
     const size_t V = (size_t)vol(h) * sizeof(float);
-    const int a = h->cur, nb = h->have_second ? 2 : 1;
+    const int a = h->cur;
     for (int c = 0; c < 6; ++c, p += V) {
         if (save) CUDA_TRY(cudaMemcpyAsync(p, h->field[a][c], V, cudaMemcpyDeviceToDevice, h->stream));
-        else
-            for (int b = 0; b < nb; ++b) CUDA_TRY(cudaMemcpyAsync(h->field[b][c], p, V, cudaMemcpyDeviceToDevice, h->stream));
+        else CUDA_TRY(cudaMemcpyAsync(h->field[a][c], p, V, cudaMemcpyDeviceToDevice, h->stream));
     }
     for (int f = 0; f < 6; ++f) {
         const size_t n = (size_t)h->psi_elems[f] * sizeof(float);
@@ -1147,9 +1145,8 @@ int fdtd_load_state(fdtd_handle* h, const void* buf) {
         if (hdr[1] != h->g.nx || hdr[2] != h->g.ny || hdr[3] != h->g.nz) return fail(FDTD_ERR_INVALID, "state belongs to another grid");
         h->step = hdr[0];
     }
-    const int nb = h->have_second ? 2 : 1;
     for (int c = 0; c < 6; ++c, p += V)
-        for (int b = 0; b < nb; ++b) CUDA_TRY(cudaMemcpyAsync(h->field[b][c], p, V, cudaMemcpyDeviceToDevice, h->stream));
+        CUDA_TRY(cudaMemcpyAsync(h->field[h->cur][c], p, V, cudaMemcpyDeviceToDevice, h->stream));
     for (int f = 0; f < 6; ++f) {
         const size_t n = (size_t)h->psi_elems[f] * sizeof(float);
         float* arr[4];

@@ -384,20 +384,23 @@ void* tensor_map_encoder() {
     return fn;
 }
 
-// AUTO: the fused schedule (one sweep per step) or two passes, by the grid's cells. Measured on GB300,
-// two-pass against sweep per step, boxes outside the CPML: 40^3 8.5 / 7.4 us, 64^3 11.3 / 10.4, 72^3 14.5 /
-// 15.9, 96^3 20.9 / 20.7, 112^3 31.7 / 34.3, 128^3 39.8 / 45.3, 136^3 60.0 / 59.0, 144^3 70 / 65, 160^3 89 / 78,
-// 200^3 175 / 129, 225^3 247 / 182. In between, where the fields sit in L2 and the sweep's CTAs do not
-// fill the device evenly, two-pass is ahead. Materials that lie in the CPML make the sweep's tiles there
-// slower than the others. Boxes and a half space through every slab: 64^3 16.3 / 17.3 us, 128^3 51 / 62, 144^3
-// 81.7 / 81.5, 160^3 100 / 97, 192^3 162 / 137, 225^3 283 / 237, 256^3 349 / 247; of magnetic materials, whose H
-// coefficients differ from the background's: 160^3 101 / 120, 192^3 162 / 165, 200^3 213 / 202. Grids below kAutoSweepCells, a few CTAs' work, gain little. A
-// design region changes little (d^3 cells of n^3, 256 / 32 322 / 222 us, 256 / 128 449 / 241, 512 / 256 3118 / 1443), but an
+// AUTO: the fused schedule (one sweep per step) or two passes, by the grid's cells. Measured on GB300, 10-cell
+// CPML, two-pass against sweep, us a step. 32 boxes clear of the CPML: 36^3 7.8 / 8.1, 40^3 8.7 / 8.1, 48^3 8.6 / 8.1,
+// 56^3 10.3 / 11.9, 64^3 11.5 / 11.5, 65^3 14.6 / 18.2, 80^3 17.3 / 18.0, 96^3 21.9 / 22.6, 112^3 33.5 / 35.8, 128^3 42.2 /
+// 49.1, 132^3 61.8 / 63.0, 136^3 65.4 / 63.9, 144^3 70.3 / 70.6, 160^3 87.9 / 85.8, 192^3 146 / 143, 200^3 189 / 140, 256^3
+// 318 / 226; vacuum gains more (64^3 11.5 / 10.3, 96^3 21.7 / 18.8, 128^3 41.7 / 49.1, 160^3 86.9 / 81.0). In between,
+// where the fields sit in L2 and the sweep's CTAs do not fill the device evenly, two-pass is ahead. Materials
+// that lie in the CPML make the sweep's tiles there slower than the others. Boxes and a half space through every
+// slab: 64^3 16.1 / 17.2, 96^3 26.8 / 34.2, 128^3 50.1 / 60.5, 144^3 80.6 / 80.1, 152^3 89.6 / 92.0, 160^3 99.4 / 94.6,
+// 192^3 160 / 134, 225^3 279 / 236, 256^3 345 / 245; a half space alone 128^3 49.1 / 53.8, 136^3 73.6 / 69.8, 152^3 88.1 /
+// 79.6; of magnetic materials, whose H coefficients differ from the background's: 160^3 99 / 118, 192^3 160 / 163,
+// 200^3 210 / 200, 225^3 280 / 283, 256^3 345 / 283. Grids below kAutoSweepCells, a few CTAs' work, gain little. A
+// design region changes little (d^3 cells of n^3, 256 / 32 318 / 219, 256 / 128 387 / 241, 512 / 256 3118 / 1459), but an
 // adjoint's forward takes its records in the two-pass kernels below kAutoAdjointCells. Two-pass also serves
 // where the second buffers cannot be allocated.
 constexpr long long kAutoSweepCells = 32LL << 10;
-constexpr long long kAutoTwoPassLo = 300LL << 10, kAutoTwoPassHi = 2450LL << 10;
-constexpr long long kAutoEdgeHi = 3LL << 20, kAutoEdgeMagneticHi = 7LL << 20;  // with slab_rows, two-pass below this
+constexpr long long kAutoTwoPassLo = 264LL << 10, kAutoTwoPassHi = 2450LL << 10;
+constexpr long long kAutoEdgeHi = 3LL << 20, kAutoEdgeMagneticHi = 7LL << 20;  // materials in the slabs: two-pass below
 constexpr long long kAutoAdjointCells = 64LL << 20;
 
 // The background material's coefficients (StepParams::bgn), evaluated on the host with the rounding steps of

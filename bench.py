@@ -262,7 +262,7 @@ TWO_PASS_DRAM_BYTES_PER_CELL = 78.15
 
 
 # DRAM bytes per cell update of one fused step (k_sweep), dram__bytes_read.sum + dram__bytes_write.sum
-# from ncu captures (profiles/update_kernels_counters.md): 59.07 B on the 512^3 random-box grid, 61.97 B at
+# from ncu captures: 59.07 B on the 512^3 random-box grid, 61.97 B at
 # 256^3, where the CPML share is larger. Refreshed whenever the kernel changes.
 FUSED_DRAM_BYTES_PER_CELL = {"512": 59.07, "256": 61.97}
 

@@ -70,9 +70,7 @@ __device__ __forceinline__ long long node(const DeviceGrid& g, int i, int j, int
 // G_H slots (written here):        0 Hx->Ey, 1 Hx->Ez, 2 Hy->Ez, 3 Hy->Ex, 4 Hz->Ex, 5 Hz->Ey.
 // CTAs of 256 per SM: at 128^3 the 192-step gradient took 30.1 ms with 4 (64 registers, no spills), 30.7 with
 // 5 and 31.1 with 6.
-#ifndef FDTD_ADJ_MIN_BLOCKS
-#define FDTD_ADJ_MIN_BLOCKS 4
-#endif
+constexpr int kAdjCtas = 4;
 // General path of k_adj_h, out of line.
 __device__ __noinline__ void adj_h_general(const StepParams* pp, const AdjState* pa, const PsiSet* pps, int i, int j, int k, float lx,
                                            float ly, float lz) {
@@ -161,7 +159,7 @@ __device__ __forceinline__ float2 hi2(const float4* t) { return __ldg(reinterpre
 // is called out of line. At 128^3 bound by L2: a pass moves 18 floats a node and the gathers' neighbours,
 // 300 MB in 33 us, of a 151 MB state that does not quite stay there.
 template <typename Idx>
-__global__ void __launch_bounds__(256, FDTD_ADJ_MIN_BLOCKS) k_adj_h(const __grid_constant__ StepParams p, const __grid_constant__ AdjState a,
+__global__ void __launch_bounds__(256, kAdjCtas) k_adj_h(const __grid_constant__ StepParams p, const __grid_constant__ AdjState a,
                                                const __grid_constant__ PsiSet psa) {
     grid_dependency_wait();
     grid_launch_dependents();
@@ -314,7 +312,7 @@ __device__ __noinline__ void adj_e_general(const StepParams* pp, const AdjState*
 // By coefficient row, as k_adj_h. The planes from the top down: it begins with what k_adj_h wrote last, which
 // is still in L2 (the 192-step gradient 26.8 -> 25.9 ms).
 template <typename Idx>
-__global__ void __launch_bounds__(256, FDTD_ADJ_MIN_BLOCKS) k_adj_e(const __grid_constant__ StepParams p, const __grid_constant__ AdjState a,
+__global__ void __launch_bounds__(256, kAdjCtas) k_adj_e(const __grid_constant__ StepParams p, const __grid_constant__ AdjState a,
                                                const __grid_constant__ PsiSet psa, const __grid_constant__ AdjStep st) {
     grid_dependency_wait();
     grid_launch_dependents();

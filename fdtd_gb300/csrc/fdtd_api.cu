@@ -1656,8 +1656,8 @@ int ensure_prepared(fdtd_handle* h) {
 // ---------------------------------------------------------------------------------------------
 // fdtd_step_static_scratch: the fused sweep with its ping-pong target in a static device array.
 //
-// fdtd_step under FDTD_SCHEDULE_FUSED allocates a second field set, a second CPML set and the work
-// list on its first call. Callers that cannot allocate while stepping (device memory reserved in
+// fdtd_step under FDTD_SCHEDULE_FUSED allocates a second field set and a second CPML set on its first
+// call. Callers that cannot allocate while stepping (device memory reserved in
 // full by their own pool; loops that must not let cudaMalloc / cudaFree synchronise the device)
 // use this entry point instead: the same kernels alternate between the handle's buffers and a
 // fixed array of FDTD_STEP_STATIC_SCRATCH_BYTES, and no device memory is allocated.

@@ -8,7 +8,7 @@
 // recurrence factors come from its axis' table in one 16-byte load, and other rows' from the row
 // tables. Nodes on the general path call out of line, so that their code costs the others neither
 // registers nor instruction cache. Probes are not looked for here: see ProbeList. At
-// 128^3 a step takes 39.8 us against 45.2 by class, at 64^3 11.3 against 13.9.
+// 128^3 a step takes 41.4 us against 45.7 by class, at 64^3 11.5 against 15.0.
 #pragma once
 
 #include "node_global.cuh"
@@ -23,8 +23,7 @@ struct StepIndex {
     __device__ __forceinline__ long long at() const { return base ? *base + m : m; }
 };
 
-// kDesign: the grid has a design region (the other grids' pass is kept free of its code: 128^3 39.9 against
-// 41.8 us a step).
+// kDesign: the grid has a design region (the other grids' pass is kept free of its code, which cost 5 % at 128^3).
 template <typename Idx, bool kDesign>
 static __device__ __noinline__ void e_node_general(const StepParams* p, const FieldPtrs* f, const PsiSet* ps, const StepIndex* step,
                                                    int i, int j, int k) {

@@ -51,7 +51,7 @@ std::vector<int> starts(int lo, int hi, int size, int align, bool overlap) {
 }  // namespace
 
 // Chunks per tile column. A chunk of n planes costs about n + 1.2 plane steps (the plane below is
-// streamed, the E of the plane above recomputed), and FDTD_SWEEP_SLOTS CTAs run at once on each of the
+// streamed, the E of the plane above recomputed), and kSweepSlots CTAs run at once on each of the
 // 152 SMs, so short grids want enough chunks to fill the device and tall ones few. The cheapest count
 // wins (320 x 240 x 300: with n + 2 281 us a step, with n + 1.2 274). Where the chunks come out long and
 // run in several waves, cuts at the z slabs keep the slabs' rules out of the middle chunks (512^3 1.36 ->
@@ -63,10 +63,8 @@ std::vector<int> starts(int lo, int hi, int size, int align, bool overlap) {
 // planes cut at the z slabs). Chunks of 8 to 32 planes then, for some eight waves, and always the cuts: 144^3 106 ->
 // 82 us, 225^3 243 -> 236, 256^3 268 -> 252, 400^3 750 either way; grids whose plan has shorter chunks anyway keep it.
 SweepPlan plan_sweep(const PlanGrid& g, double share, bool rows) {
-#ifndef FDTD_SWEEP_SLOTS
-#define FDTD_SWEEP_SLOTS 3
-#endif
-    const double slots = std::max(1.0, FDTD_SWEEP_SLOTS * 152 * share);
+    constexpr int kSweepSlots = 3;
+    const double slots = std::max(1.0, kSweepSlots * 152 * share);
     SweepPlan p{(g.nx + kTileX - 1) / kTileX, (g.ny + kSweepRows - 1) / kSweepRows, g.nz, 0, g.nz, 0, 1, 0};
     const long long tiles = (long long)p.nbx * p.nby;
     double best = -1.0;

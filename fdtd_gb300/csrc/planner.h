@@ -53,10 +53,7 @@ struct PlanGrid {
 // cut into chunks of planes of nearly equal length: n_lo chunks of the planes below zlo, n_mid of
 // [zlo, zhi) and n_hi of the rest. The middle chunks, and the E above their top plane, meet neither a
 // z slab nor a z wall; grids where cutting there does not pay have n_mid chunks only (zlo 0, zhi nz).
-#ifndef FDTD_SWEEP_ROWS
-#define FDTD_SWEEP_ROWS 16
-#endif
-constexpr int kSweepRows = FDTD_SWEEP_ROWS;
+constexpr int kSweepRows = 16;
 constexpr int kMaxSweepChunk = 32;                   // planes of a chunk
 constexpr int kMaxSweepPlanes = kMaxSweepChunk + 2;  // planes a chunk streams
 #ifdef __CUDACC__

@@ -137,8 +137,9 @@ __device__ __forceinline__ bool plane_has_plate(const StepParams& p, int k) {
 // E-edge coefficients (setCoefficients, fdtdrav.h:1280-1303). `uni`: the four cells around the
 // edge hold material m0, so the table entry applies. comp: 0 = Ex, 1 = Ey, 2 = Ez; the Cb cell
 // sizes are Ex (dy, dz), Ey (dz, dx), Ez (dx, dy). kDesignAware: edges touching the design region
-// average the per-cell eps_r. The update kernels compile without it (their registers, and with
-// them their occupancy, would grow); the design region's E is then redone by k_design_e.
+// average the per-cell eps_r. The kernels by class compile without it (their registers, and with them their
+// occupancy, would grow): there the design region's E is k_design_e's. The sweep and the kernels by row
+// take it on their general path and take the region's other nodes' from a table (StepParams::dcoef).
 template <bool kDesignAware = false>
 __device__ __forceinline__ Coef3 e_coef(const StepParams& p, int comp, bool uni, int m0, int m1, int m2, int m3, int i,
                                         int j, int k) {

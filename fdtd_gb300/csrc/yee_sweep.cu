@@ -16,26 +16,28 @@
 // with the kernel parameters); in a CPML slab the curl coefficients along the slab's axis come from
 // the axis' table for background nodes (StepParams::te, th: divided by kappa) and from SlabRows for
 // other rows. Quads of several rows load them component by component, or node by node where the registers
-// do not allow that. Where no material is magnetic (StepParams::h_bg), H looks at no rows at all. What is left (lumped edges in a slab,
-// design nodes, probes in a slab, keys beyond the table) runs e_update_diff / h_update_diff (slow_node).
+// do not allow that. With materials in the slabs of which none is magnetic (StepParams::h_bg), H looks at no
+// rows. What is left (lumped edges and probes in a slab, design nodes with a lumped edge, keys beyond the table)
+// runs e_update_diff / h_update_diff (slow_node).
 // Old CPML memory of the y and z faces is fetched a plane ahead with cp.async into slots of the
 // thread's own.
 //
 // What bounds it: on grids beyond L2, HBM and the latency of a plane step; on smaller ones the latency
 // of a plane step alone (15 warps an SM, about 650 instructions per quad and step, a third of the
-// issue slots) and, with materials in the slabs, the tiles that hold them. Measured per step, against
-// the schedule it replaced (a sweep of the interior tiles, then one-node-per-thread passes over the
-// CPML shell): 512^3 random boxes 1.650 -> 1.38 ms, 256^3 0.302 -> 0.240 ms, 1024 x 1024 x 896 10.4 ->
-// 8.8 ms; against two-pass, 64^3 18.4 -> 10.5 us. One node per thread in the same march ran 2.0 ms at 512^3
+// issue slots) and, with materials in the slabs, the tiles that hold them. Measured per step with boxes clear of
+// the CPML, against the schedule it replaced (a sweep of the interior tiles, then one-node-per-thread passes over
+// the CPML shell): 512^3 1.59 -> 1.30 ms, 256^3 0.279 -> 0.226, 1024 x 1024 x 896 10.4 -> 8.3; against the two passes
+// of that time, 64^3 18.3 -> 11.5 us. One node per thread in the same march ran 2.0 ms at 512^3
 // (352 instructions per node against about 165). 3 CTAs an SM (128 registers) against 2: 512^3 1.39 /
 // 1.55 ms, 128^3 52 / 61 us. Registers decide much: spills of 100 bytes in the march cost 5 % at 512^3 and
 // 20 % at 64^3, so old H of a plane is read again from its stage at the end of the step rather than
-// kept through it; and code, as the march should fit the instruction cache: rows other than the
-// background's have their slab coefficients in a table (SlabRows), since divisions in line made grids
-// with materials in the slabs 10-20 % slower (128^3 73 -> 60 us).
+// kept through it (of the kernels here, those of materials in the slabs spill 32 to 72 bytes in the two-CTA
+// and the 64-bit form, the others none); and code, as the march should fit the instruction cache: rows other than
+// the background's have their slab coefficients in a table (SlabRows), since divisions in line made grids
+// with materials in the slabs 10-20 % slower.
 // All arithmetic is that of yee_common.cuh, so the results equal the two-pass schedule's bits.
-// Every wait on a TMA barrier is bounded: on timeout the kernel uses nothing of that plane, records an error in the status
-// word, drains its own copies (again bounded) and exits.
+// Every wait on a TMA barrier is bounded: on timeout the kernel uses nothing of that plane, records an
+// error in the status word, drains its own copies (again bounded) and exits.
 #define FDTD_RARE __forceinline__  // calls in the slow path would spill the march's state (512^3: 31.0 -> 28.6 ms for 20 steps)
 #include <cuda.h>
 
@@ -51,15 +53,12 @@ namespace fdtd {
 namespace {
 
 // Stages of the ring: a third one left less of the SM's memory to L1 and was 12-20 % slower.
-#ifndef FDTD_SWEEP_STAGES
-#define FDTD_SWEEP_STAGES 2
-#endif
 constexpr int TX = kTileX, TY = kSweepRows;
 constexpr int QX = TX / 4;                // quads per row
 constexpr int NOWN = QX * TY;             // threads with a quad of the tile; then the halo row and column
 constexpr int NTH = NOWN + (QX + TY + 31) / 32 * 32;
 static_assert(NOWN % 32 == 0, "own quads fill whole warps");
-constexpr int NST = FDTD_SWEEP_STAGES;    // planes in the ring
+constexpr int NST = 2;                    // planes in the ring
 // A grid swept alone of up to this many CTAs: two of 168 registers an SM run the grid at once (kWide) instead of three of 128:
 // a plane step is shorter with the registers to have the loads of a quad of several rows in flight
 // together (64^3: vacuum 11.0 -> 10.4 us a step, boxes 12.5 -> 10.5, boxes that touch a CPML slab 16.7 -> 12.6).
@@ -124,9 +123,10 @@ __device__ __forceinline__ float sweep_sig(const SweepArgs& A, int source) {
     return m < A.p.wave_len[source] ? A.p.waves[source][m] : 0.f;
 }
 
-// Slow path, out of line: nodes on the general path (lumped edges, plates, design nodes, probes,
-// keys beyond the table), nodes of another material than the background in a CPML slab, and H faces
-// of such nodes on the low walls. bits: 1 E(k), 2 H(k-1), 4 a node of the tile (stored, probes
+// Slow path, one node at a time (in line: a call would spill the march's state): nodes on the general path
+// (lumped edges and probes in a slab, design nodes with a lumped edge, keys beyond the table), nodes of another
+// material than the background in a CPML slab where there is no SlabRows table, and H faces of such nodes on
+// the low walls. bits: 1 E(k), 2 H(k-1), 4 a node of the tile (stored, probes
 // sampled), 8 E(k) is this chunk's. Old H of plane k - 1 and the node's row there come with the
 // call, the rest from the shared-memory tiles.
 template <typename Idx>

@@ -4,12 +4,12 @@
 // expressed over the compact data layout. It runs at any grid size and is the schedule the fused
 // sweep is checked against bit for bit; both call the same update primitives (yee_common.cuh).
 //
-// Every pass may start while the one before it drains (launch_dependent): on small grids, a few
-// microseconds of work a pass, that and the shorter passes by row took a step of 24^3 from 13.5 to 7.5 us,
-// of 64^3 from 17.5 to 11.3.
+// Every pass may start while the one before it drains (launch_dependent). A step with boxes clear of the CPML, us,
+// without that / now: 24^3 12.4 / 7.0, 64^3 16.5 / 11.5, 128^3 45.2 / 41.4, 160^3 92.5 / 88.0.
 //
 // The H pass goes through the planes from the top down: it begins with what the E pass wrote last, which L2
-// still holds when the grid as a whole does not fit (160^3 93.9 -> 85.2 us, 225^3 247 -> 243).
+// still holds when the grid as a whole does not fit. From the bottom up / now: 160^3 94.3 / 88.0, 192^3 152 / 146,
+// 225^3 257 / 252.
 #include "node_rows.cuh"
 #include "tma.cuh"
 
@@ -17,14 +17,14 @@ namespace fdtd {
 
 // Grids of up to this many nodes take the kernels by coefficient row (node_rows.cuh), larger ones those
 // by node class (node_global.cuh), whose byte per node and sixth CTA an SM tell where HBM bounds the
-// pass. Per step, class / row: 128^3 45.2 / 39.8 us, 160^3 94 / 89, 200^3 174 / 175, 225^3 248 / 259, 400^3 1082 /
-// 1172.
+// pass. Per step, class / row, us: 24^3 9.0 / 7.0, 64^3 15.0 / 11.5, 128^3 45.7 / 41.4, 160^3 91.9 / 88.0, 192^3 147 /
+// 146, 200^3 189 / 189, 225^3 252 / 270, 256^3 318 / 332.
 constexpr long long kRowsNodes = 7LL << 20;
 
 // CTAs of 256 per SM the kernels are compiled for. By class: 6 caps them at 40 registers (48 warps
 // resident; the general path spills a few words), which measured 4-7 % faster at 512^3 than the
 // compiler's own choice of 48 registers (5 CTAs). By row: 5, without spills in the common path
-// (128^3: 6 CTAs 42.0, 5 CTAs 39.9, 4 CTAs 43.6 us).
+// (at 128^3 6 CTAs were 5 % slower, 4 CTAs 9 %).
 template <bool kRows>
 constexpr int kCtas = kRows ? 5 : 6;
 
@@ -39,7 +39,7 @@ struct ProbeList {
     int n, late;
 };
 __device__ __forceinline__ void sample_list(const StepParams& p, const FieldPtrs& f, const ProbeList& l, bool h, long long m) {
-    if (blockIdx.z != 0) return;  // one plane's blocks: the others do not even look (128^3 43.3 -> 40.5 us a step)
+    if (blockIdx.z != 0) return;  // one plane's blocks: the others do not even look (128^3 44.0 -> 41.4 us a step)
     const int block = blockIdx.y * gridDim.x + blockIdx.x, step = 256 * gridDim.x * gridDim.y;
     for (long long q = block * 256 + threadIdx.y * 32 + threadIdx.x; q < l.n; q += step) {
         const ProbeAt r = l.at[q];

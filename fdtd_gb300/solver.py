@@ -294,7 +294,7 @@ class Simulation:
         return _lib.fdtd_current_step(self._h)
 
     def tune_schedule(self) -> None:
-        """Under SCHEDULE_AUTO, choose the schedule now by timing both (the handle's state is kept)."""
+        """Under SCHEDULE_AUTO, choose the schedule now (by the grid; the state is kept)."""
         _check(_lib.fdtd_tune_schedule(self._h))
 
     @property

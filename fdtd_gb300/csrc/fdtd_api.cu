@@ -442,7 +442,7 @@ size_t second_bytes(const fdtd_handle* h) {
 }
 
 // The second buffers at `base`, in device memory that `owner` keeps, and the TMA tensor maps of both
-// buffers; the caller waits for the handle's stream before it sets have_second.
+// buffers. The fills run on the handle's stream.
 int place_second(fdtd_handle* h, const std::shared_ptr<void>& owner, char* base) {
     const long long V = vol(h);
     h->second = owner;
@@ -485,8 +485,9 @@ bool capturing(const fdtd_handle* h) {
 }
 
 // Second buffers for the n handles of hs (none of which has any) in one allocation, which the last of
-// them gives back: an allocation each costs 45 us, which a batch's first call felt. All or none.
-int alloc_second(fdtd_handle* const* hs, size_t n) {
+// them gives back: an allocation each costs 45 us, which a batch's first call felt. All or none. wait: for the
+// fills, where the next steps run on another stream.
+int alloc_second(fdtd_handle* const* hs, size_t n, bool wait) {
     size_t total = 0;
     for (size_t q = 0; q < n; ++q) {
         if (capturing(hs[q])) return fail(FDTD_ERR_STATE, "second buffers cannot be allocated while the handle's stream is captured");
@@ -508,7 +509,7 @@ int alloc_second(fdtd_handle* const* hs, size_t n) {
             const int rc = place_second(hs[q], owner, at);
             if (rc) return rc;
         }
-        for (size_t q = 0; q < n; ++q)
+        for (size_t q = 0; q < n && wait; ++q)
             if (q == 0 || hs[q]->stream != hs[q - 1]->stream) CUDA_TRY(cudaStreamSynchronize(hs[q]->stream));
         return FDTD_OK;
     };
@@ -520,7 +521,7 @@ int alloc_second(fdtd_handle* const* hs, size_t n) {
     return rc;
 }
 
-int ensure_fused(fdtd_handle* h) { return h->have_second ? FDTD_OK : alloc_second(&h, 1); }
+int ensure_fused(fdtd_handle* h) { return h->have_second ? FDTD_OK : alloc_second(&h, 1, false); }
 
 // AUTO runs two-pass until auto_choose has taken the fused schedule.
 bool use_fused(const fdtd_handle* h) {
@@ -2360,7 +2361,7 @@ void batch_choose(fdtd_batch* b, long long n) {
         want.clear();
     }
     want.insert(want.end(), fused.begin(), fused.end());
-    if (!want.empty() && alloc_second(want.data(), want.size()) != FDTD_OK) {
+    if (!want.empty() && alloc_second(want.data(), want.size(), true) != FDTD_OK) {
         cudaGetLastError();
         b->no_room = true;
     }

@@ -31,7 +31,7 @@
 // (352 instructions per node against about 165). 3 CTAs an SM (128 registers) against 2: 512^3 1.39 /
 // 1.55 ms, 128^3 52 / 61 us. Registers decide much: spills of 100 bytes in the march cost 5 % at 512^3 and
 // 20 % at 64^3, so old H of a plane is read again from its stage at the end of the step rather than
-// kept through it (of the kernels here, those of materials in the slabs spill 32 to 72 bytes in the two-CTA
+// kept through it (of the kernels here, those of materials in the slabs spill 40 to 72 bytes in the two-CTA
 // and the 64-bit form, the others none); and code, as the march should fit the instruction cache: rows other than
 // the background's have their slab coefficients in a table (SlabRows), since divisions in line made grids
 // with materials in the slabs 10-20 % slower.

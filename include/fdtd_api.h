@@ -40,7 +40,7 @@ enum {
                                  TWO_PASS until the steps asked for repay FUSED's second buffers
                                  (5 to 200, fewer the larger the grid; or fdtd_tune_schedule),
                                  where those do not fit, and from a captured step on below 8 Mi
-                                 cells. The call that allocates them waits for the handle's stream */
+                                 cells */
     FDTD_SCHEDULE_TWO_PASS = 1, /* E pass then H pass per step, in place (the reference's order) */
     FDTD_SCHEDULE_FUSED = 2,  /* one z-marching sweep of the whole grid per step over ping-pong
                                  field buffers (second buffers are allocated by the first step, not

@@ -110,3 +110,32 @@ def test_second_buffers_filled_on_the_handles_stream(gpu_lib):
             torch.cuda.synchronize()
             states.append(state)
     assert torch.equal(*states)
+
+
+def test_auto_takes_the_sweep_without_waiting(gpu_lib):
+    """The call in which AUTO gets its second buffers enqueues its steps behind whatever the stream still does."""
+    import torch
+    from conftest import bitwise_equal
+    from fdtd_gb300 import solver
+    sc = S.vacuum_cube(48, 8, pml=8, name="no_wait")
+    sc.probes = []
+    stream = torch.cuda.Stream()
+    with solver.Simulation.from_scenario(sc, 0) as sim, solver.Simulation.from_scenario(sc, 1) as ref:
+        with solver.Simulation.from_scenario(sc, 2) as warm:  # the kernels are loaded
+            warm.step(2)
+            warm.synchronize()
+        sim.set_stream(stream.cuda_stream)
+        sim.step(10)
+        torch.cuda.synchronize()
+        assert sim.active_schedule == 1
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(1_000_000_000)  # some 0.5 s
+            slept = torch.cuda.Event()
+            slept.record(stream)
+        sim.step(390)
+        assert not slept.query()
+        assert sim.active_schedule == 2
+        sim.synchronize()
+        ref.step(400)
+        ref.synchronize()
+        assert bitwise_equal(sim.fields(), ref.fields())
